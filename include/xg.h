@@ -258,6 +258,11 @@ int xg_load(xg_circuit *c, const xg_load_flags *flags);
  *                   left-looking threshold-partial-pivot factorisation of the
  *                   given values (KLU's tol 0.001, diagonal preferred) that
  *                   fixes the pivot order and the L\U pattern; uploads them.
+ *                   Large matrices (8,192 rows and up) with long dependency
+ *                   chains are refactored by dense fronts over a nested-
+ *                   dissection tree instead, when their multipliers on the
+ *                   given values stay within the same tolerance; xg_lu_info
+ *                   and xg_lu_get_symbolic describe the analysis either way.
  * xg_lu_refactor  : GPU numeric refactorisation of new values (device CSR
  *                   values in the analysed pattern) with that pivot order.
  *                   Asynchronous; a zero or non-finite pivot is reported by

@@ -16,7 +16,7 @@ BUILD = os.path.join(PKG, "_build")
 LIBDIR = os.path.join(PKG, "_lib")
 LIB = os.path.join(LIBDIR, "libxg.so")
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
-FMA_SOURCES = {"lu_kernels.cu"}
+FMA_SOURCES = {"lu_kernels.cu", "lu_front.cu"}
 
 
 def _nvcc():

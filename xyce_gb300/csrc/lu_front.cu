@@ -1,0 +1,1006 @@
+// lu_front.cu — multifrontal refactorisation and solves of large Newton
+// matrices on the GPU (plan: lu_front.h).
+//
+// A tree level is one launch.  front_factor keeps a whole front in shared
+// memory, its columns dealt in blocks of 4 to the CTAs it takes: 1 to 16 of a
+// cluster, which several fronts share when they are small.  The owner of the
+// next pivot columns updates and eliminates them first, a row per thread in
+// registers, and signals the front's other CTAs through mbarriers in their
+// shared memory; those fetch the columns through distributed shared memory
+// while it goes on with its other columns.  An FP64 instruction takes a
+// sub-partition 66 cycles, dependent or not and however few lanes it has
+// (77 with all four busy), so what counts is the number of warp instructions:
+// the updates are dealt entry by entry over all lanes, and the pivots' serial
+// chain (reciprocal, multiplier, update, barrier) is kept to the fewest.  The
+// forward and backward solves are one launch that walks the tree by flags.
+//
+// Every sum has a fixed order: results repeat bit for bit.
+
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cmath>
+#include <memory>
+#include <vector>
+
+#include "lu_front.h"
+#include "xg_internal.h"
+#include "xg_smem.cuh"
+
+namespace xg {
+namespace {
+
+// Pivot columns eliminated at a time, and the unit of dealing columns: an
+// elimination costs a warp kNb (kNb + 1) / 2 FP64 instructions however many
+// of its lanes have rows, and the next columns' update kNb^2, all on the
+// pivots' serial chain; the hand-over between CTAs costs about 1,300 cycles.
+constexpr int kNb = 4;
+constexpr int kMaxCtas = 16;       // of one front
+constexpr size_t kSmemLimit = 225 * 1024, kSmemTarget = 56 * 1024;
+constexpr int kFlowThreads = 128;
+
+struct ChildDev {
+  int64_t inv, co, bv, map;
+  int b, front;
+};
+
+struct FrontDev {
+  const Front *front;
+  const ChildDev *child;
+  const int *idx, *map, *inv_map, *apos, *aidx;
+  const int *P, *Q;
+  void *l, *u, *c;                // factors and Schur complements (T)
+  void *rd, *y, *bv;              // reciprocal pivots, forward values, border sums (T)
+  double *xk;                     // unknowns by B column
+  unsigned *status;
+};
+
+__device__ __forceinline__ unsigned cluster_rank() {
+  unsigned r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ unsigned cluster_size() {
+  unsigned r;
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ unsigned smem_u32(const void *p) { return unsigned(__cvta_generic_to_shared(p)); }
+// One arrival at an mbarrier of another CTA of the cluster (its address from
+// remote()); what the caller saw or wrote before is visible to whoever sees it.
+__device__ __forceinline__ void signal(unsigned remote_bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(remote_bar) : "memory");
+}
+// Waits for the barrier's phase of this parity, at most `limit` polls.
+__device__ __forceinline__ bool await(unsigned bar, unsigned parity, int limit) {
+  for (int it = 0; it < limit; ++it) {
+    unsigned ok;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+        " selp.u32 %0, 1, 0, p;\n}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    if (ok) return true;
+  }
+  return false;
+}
+// This CTA's shared address p, in CTA `rank` of the cluster.
+__device__ __forceinline__ unsigned remote(const void *p, unsigned rank) {
+  unsigned a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(unsigned(__cvta_generic_to_shared(p))), "r"(rank));
+  return a;
+}
+// Four loads in flight at once from other CTAs' shared memory.
+__device__ __forceinline__ void remote_load4(const unsigned (&a)[4], double (&v)[4]) {
+  asm volatile(
+      "ld.shared::cluster.f64 %0, [%4];\n ld.shared::cluster.f64 %1, [%5];\n"
+      "ld.shared::cluster.f64 %2, [%6];\n ld.shared::cluster.f64 %3, [%7];"
+      : "=&d"(v[0]), "=&d"(v[1]), "=&d"(v[2]), "=&d"(v[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3])
+      : "memory");
+}
+__device__ __forceinline__ void remote_load4(const unsigned (&a)[4], float (&v)[4]) {
+  asm volatile(
+      "ld.shared::cluster.f32 %0, [%4];\n ld.shared::cluster.f32 %1, [%5];\n"
+      "ld.shared::cluster.f32 %2, [%6];\n ld.shared::cluster.f32 %3, [%7];"
+      : "=&f"(v[0]), "=&f"(v[1]), "=&f"(v[2]), "=&f"(v[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3])
+      : "memory");
+}
+
+// Columns of an m-column front that CTA r of C holds.
+__host__ __device__ inline int local_columns(int m, int r, int C) {
+  const int blocks = (m + kNb - 1) / kNb, mine = blocks > r ? (blocks - r + C - 1) / C : 0;
+  const bool last = mine > 0 && (blocks - 1) % C == r;
+  return mine * kNb - (last ? blocks * kNb - m : 0);
+}
+// An odd column stride: lanes on consecutive columns touch different banks.
+__host__ __device__ inline int column_stride(int m) { return m | 1; }
+
+size_t factor_smem(int m, int C, size_t tsz) {
+  const size_t ld = size_t(column_stride(m));
+  return ((C > 1 ? kNb : 0) + size_t(local_columns(m, 0, C))) * ld * tsz + (kNb * kNb + kNb) * tsz;
+}
+
+__device__ __forceinline__ bool bad_value(double u) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(u);
+  return (b << 1) == 0 || ((b >> 52) & 0x7ff) == 0x7ff;
+}
+__device__ __forceinline__ bool bad_value(float u) {
+  const unsigned b = __float_as_uint(u);
+  return (b << 1) == 0 || ((b >> 23) & 0xff) == 0xff;
+}
+
+__device__ __forceinline__ void report_pivot(unsigned *status, int row) {
+  atomicOr(status, 1u);
+  atomicMin(status + 1, unsigned(row));
+}
+
+// This CTA's place of column j, -1 if another CTA holds it.
+__device__ __forceinline__ int local_column(int j, int r, int C) {
+  const int b = j / kNb;
+  if (C == 1) return j;
+  return b % C == r ? (b / C) * kNb + j % kNb : -1;
+}
+
+// The columns this CTA holds, summed from A and the children's Schur
+// complements.  All threads take a child at a time, its entries in the order
+// they lie in memory: the loads of a child are all in flight at once, and a
+// child costs about one L2 round trip.  (A warp per column instead, children
+// in turn, cost a chain of three round trips per column and child: 50 us for
+// a single front of 32 rows.)
+template <class T>
+__device__ void assemble(const FrontDev &d, const Front &f, const double *__restrict__ a, T *F, int ld, int ncl,
+                         int r, int C) {
+  const int tid = threadIdx.x, bd = blockDim.x;
+  for (int e = tid; e < ncl * ld; e += bd) F[e] = T(0);
+  __syncthreads();
+  const int64_t e0 = f.acol, e1 = f.acol + f.na;
+  for (int64_t e = e0 + tid; e < e1; e += bd) {
+    const int at = __ldg(d.apos + e), lc = local_column(at / kFrontMax, r, C);
+    if (lc >= 0) F[size_t(lc) * ld + at % kFrontMax] = T(a[__ldg(d.aidx + e)]);
+  }
+  __syncthreads();
+  for (int c = f.child0; c < f.child1; ++c) {
+    const ChildDev g = d.child[c];
+    const int b = g.b, n = b * b;
+    const T *s = (const T *)d.c + g.co;
+    const int *map = d.map + g.map;
+    constexpr int kE = 4;
+    for (int e = tid; e < n; e += kE * bd) {
+      int at[kE];
+      T v[kE];
+#pragma unroll
+      for (int q = 0; q < kE; ++q) {
+        const int k = e + q * bd;
+        at[q] = -1;
+        v[q] = T(0);
+        if (k < n) {
+          const int j = k / b, lc = local_column(__ldg(map + j), r, C);
+          if (lc >= 0) {
+            at[q] = lc * ld + __ldg(map + k - j * b);
+            v[q] = __ldcg(s + k);
+          }
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < kE; ++q)
+        if (at[q] >= 0) F[at[q]] += v[q];
+    }
+    __syncthreads();
+  }
+}
+
+// 1 / u: a Halley step (the cubic member of Householder's family: with
+// e = 1 - u x, x (1 + e + e^2) leaves a relative error of e^3) from the
+// hardware's 20-bit approximation, three dependent multiply-adds where the
+// IEEE division has a longer chain; the pivots of a front follow one another
+// at its latency.  The division itself near the ends of the exponent range.
+__device__ __forceinline__ double pivot_reciprocal(double u) {
+  double x;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(u));
+  const double e = fma(-u, x, 1.0);
+  x = fma(x, fma(e, e, e), x);
+  const int ex = (__double2hiint(u) >> 20) & 0x7ff;
+  if (unsigned(ex - 64) > 1918u) x = 1.0 / u;
+  return x;
+}
+__device__ __forceinline__ float pivot_reciprocal(float u) { return 1.0f / u; }
+
+// Eliminates the pivot columns [k0, k0 + nb) that start at base, a row per
+// thread with its entries in registers, after applying the kNb pivots before
+// them (whose eliminated columns are prev; nullptr for the first block).
+// Step q sends pivot row q and its reciprocal through shared memory.
+template <class T>
+__device__ __forceinline__ void eliminate(const FrontDev &d, const Front &f, T *base, int ld, int k0, int nb,
+                                          const T *prev, T *su, T *sr) {
+  const int tid = threadIdx.x, i = k0 + tid;
+  const bool mine = i < f.m;
+  T v[kNb];
+#pragma unroll
+  for (int q = 0; q < kNb; ++q) v[q] = q < nb && mine ? base[size_t(q) * ld + i] : T(0);
+  if (prev && mine) {
+#pragma unroll
+    for (int q = 0; q < kNb; ++q) {
+      const T l = prev[q * ld + i];
+#pragma unroll
+      for (int s = 0; s < kNb; ++s)
+        if (s < nb) v[s] -= l * base[size_t(s) * ld + k0 - kNb + q];
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < kNb; ++q) {
+    if (q < nb) {
+      if (tid == q) {
+        const T rc = pivot_reciprocal(v[q]);
+        sr[q] = rc;
+#pragma unroll
+        for (int s = q + 1; s < kNb; ++s) su[q * kNb + s] = v[s];
+        ((T *)d.rd)[f.pv + k0 + q] = rc;
+        if (bad_value(v[q])) report_pivot(d.status, __ldg(d.idx + f.idx + k0 + q));
+      }
+      __syncthreads();
+      if (tid > q && mine) {
+        v[q] *= sr[q];
+#pragma unroll
+        for (int s = q + 1; s < kNb; ++s)
+          if (s < nb) v[s] -= v[q] * su[q * kNb + s];
+      }
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < kNb; ++q)
+    if (q < nb && mine) base[size_t(q) * ld + i] = v[q];
+}
+
+// Columns [l0, l1) of this CTA after the pivots [k0, k0 + nb), whose
+// eliminated columns are pan: their U rows, a column per thread, ...
+template <class T>
+__device__ __forceinline__ void update_u(T *F, int ld, int l0, int l1, const T *pan, int k0, int nb) {
+  for (int c = l0 + int(threadIdx.x); c < l1; c += blockDim.x) {
+    T *col = F + size_t(c) * ld + k0;
+    T u[kNb];
+#pragma unroll
+    for (int q = 0; q < kNb; ++q) u[q] = q < nb ? col[q] : T(0);
+#pragma unroll
+    for (int q = 1; q < kNb; ++q) {
+      if (q < nb) {
+#pragma unroll
+        for (int s = 0; s < q; ++s) u[q] -= pan[s * ld + k0 + q] * u[s];
+        col[q] = u[q];
+      }
+    }
+  }
+}
+// ... and the rows below, two entries per thread at a time (their chains of
+// kNb multiply-adds are independent).
+template <class T>
+__device__ __forceinline__ void update_rest(T *F, int ld, int l0, int l1, const T *pan, int k0, int nb, int m) {
+  const int tid = threadIdx.x, bd = blockDim.x, i0 = k0 + nb, rem = m - i0, n = rem * (l1 - l0);
+  for (int e = tid; e < n; e += 2 * bd) {
+    const int e2 = e + bd < n ? e + bd : e;
+    const int c = e / rem, i = i0 + (e - c * rem), c2 = e2 / rem, i2 = i0 + (e2 - c2 * rem);
+    T *col = F + size_t(l0 + c) * ld, *col2 = F + size_t(l0 + c2) * ld;
+    T acc = col[i], acc2 = col2[i2];
+    if (nb == kNb) {
+#pragma unroll
+      for (int q = 0; q < kNb; ++q) {
+        acc -= pan[q * ld + i] * col[k0 + q];
+        acc2 -= pan[q * ld + i2] * col2[k0 + q];
+      }
+    } else {
+      for (int q = 0; q < nb; ++q) {
+        acc -= pan[q * ld + i] * col[k0 + q];
+        acc2 -= pan[q * ld + i2] * col2[k0 + q];
+      }
+    }
+    col[i] = acc;
+    if (e2 != e) col2[i2] = acc2;
+  }
+}
+
+// One CTA's part of a front.
+template <class T>
+__device__ void factor_front(const FrontDev &d, const Front f, const double *__restrict__ a, unsigned char *raw,
+                             unsigned long long *bar, int limit) {
+  const int C = f.ctas, r = C > 1 ? int(cluster_rank()) & (C - 1) : 0, rank0 = int(cluster_rank()) - r;
+  const int m = f.m, p = f.p, ld = column_stride(m), tid = threadIdx.x, bd = blockDim.x;
+  const int ncl = local_columns(m, r, C);
+  T *su = reinterpret_cast<T *>(raw);       // pivot rows of the block being eliminated
+  T *sr = su + kNb * kNb;                   // and their reciprocal pivots
+  T *pb = sr + kNb;                         // another CTA's pivot columns
+  T *F = pb + (C > 1 ? size_t(kNb) * ld : 0);
+  assemble<T>(d, f, a, F, ld, ncl, r, C);
+  __syncthreads();
+  const int blocks = (p + kNb - 1) / kNb;
+  // Block jb's columns are final in its owner's shared memory: a thread tells
+  // each CTA of the front.  Barrier jb % C serves one block of each round of
+  // C; a CTA owns one block of a round itself, so no barrier completes twice
+  // before it is waited for.
+  auto hand_over = [&](int jb) {
+    __syncthreads();
+    if (tid < C) signal(remote(bar + jb % C, unsigned(rank0 + tid)));
+  };
+  if (r == 0) {
+    eliminate<T>(d, f, F, ld, 0, min(kNb, p), nullptr, su, sr);
+    if (C > 1) hand_over(0);
+  }
+  for (int jb = 0; jb < blocks; ++jb) {
+    const int k0 = jb * kNb, nb = min(kNb, p - k0), own = jb % C, lc0 = (jb / C) * kNb;
+    if (C > 1) {
+      if (!await(smem_u32(bar + own), unsigned(jb / C) & 1u, limit)) atomicOr(d.status, 2u);
+    } else {
+      __syncthreads();
+    }
+    const T *pan = F + size_t(lc0) * ld;
+    // this CTA's first column after the block
+    const int passed = jb >= r ? (jb - r) / C + 1 : 0;
+    int l0 = r == own ? lc0 + nb : min(passed * kNb, ncl);
+    if (r != own && l0 < ncl) {
+      const int rows = m - k0, cnt = nb * rows;
+      for (int e = tid; e < cnt; e += 4 * bd) {
+        unsigned src[4];
+        T *dst[4];
+        T v[4];
+#pragma unroll
+        for (int z = 0; z < 4; ++z) {
+          const int ez = min(e + z * bd, cnt - 1), q = ez / rows, i = k0 + ez - q * rows;
+          src[z] = remote(F + size_t(lc0 + q) * ld + i, unsigned(rank0 + own));
+          dst[z] = pb + q * ld + i;
+        }
+        remote_load4(src, v);
+#pragma unroll
+        for (int z = 0; z < 4; ++z) *dst[z] = v[z];  // past the end: the last entry again
+      }
+      pan = pb;
+    }
+    if (C > 1) __syncthreads();
+    const bool more = jb + 1 < blocks;
+    if (more && r == (jb + 1) % C) {
+      const int nbn = min(kNb, p - k0 - kNb);
+      update_u<T>(F, ld, l0, l0 + nbn, pan, k0, nb);
+      __syncthreads();
+      eliminate<T>(d, f, F + size_t(l0) * ld, ld, k0 + kNb, nbn, pan, su, sr);
+      if (C > 1) hand_over(jb + 1);
+      l0 += nbn;
+    }
+    if (l0 < ncl) {
+      update_u<T>(F, ld, l0, ncl, pan, k0, nb);
+      __syncthreads();
+      update_rest<T>(F, ld, l0, ncl, pan, k0, nb, m);
+    }
+    __syncthreads();
+  }
+  // factor and Schur complement, a warp per column
+  const int lane = tid & 31, b = m - p;
+  for (int lc = tid >> 5; lc < ncl; lc += bd >> 5) {
+    const int j = ((lc / kNb) * C + r) * kNb + lc % kNb;
+    const T *col = F + size_t(lc) * ld;
+    if (j < p) {
+      T *dst = (T *)d.l + f.lo + int64_t(j) * m;
+      for (int i = lane; i < m; i += 32) dst[i] = col[i];
+    } else {
+      T *dst = (T *)d.u + f.uo + int64_t(j - p) * p;
+      for (int i = lane; i < p; i += 32) dst[i] = col[i];
+      dst = (T *)d.c + f.co + int64_t(j - p) * b;
+      for (int i = lane; i < b; i += 32) dst[i] = col[p + i];
+    }
+  }
+}
+
+// slot: per CTA of the launch the front it works for (-1: none); a front's
+// Front::ctas CTAs are neighbours in one cluster.
+template <class T>
+__global__ void __launch_bounds__(kFrontMax) front_factor(FrontDev d, const double *__restrict__ a,
+                                                          const int *__restrict__ slot, const unsigned *limit_at) {
+  extern __shared__ __align__(16) unsigned char raw[];
+  __shared__ __align__(8) unsigned long long bar[kMaxCtas];
+  const int number = __ldg(slot + blockIdx.x), tid = threadIdx.x;
+  const bool shared_cluster = cluster_size() > 1;
+  if (tid == 0) {
+    for (int k = 0; k < kMaxCtas; ++k)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(bar + k)) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (shared_cluster) cluster_sync();  // every barrier of the cluster is ready
+  if (number >= 0) factor_front<T>(d, d.front[number], a, raw, bar, int(__ldg(limit_at)));
+  if (shared_cluster) cluster_sync();  // no CTA leaves while another may read its columns
+}
+
+// Opens a refactor: keeps A for the rows outside the tree and refinement,
+// resets the status.
+__global__ void front_open(const double *__restrict__ a, double *__restrict__ a_copy, int64_t nnz, unsigned *status) {
+  const int64_t t0 = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (t0 == 0) {
+    status[0] = 0;
+    status[1] = 0xffffffffu;
+  }
+  if (a_copy != a)
+    for (int64_t p = t0; p < nnz; p += int64_t(gridDim.x) * blockDim.x) a_copy[p] = a[p];
+}
+
+struct RowsDev {
+  const int *row, *diag, *col, *a;
+  const int64_t *ptr;
+};
+
+__global__ void front_check_rows(RowsDev R, int n, const double *__restrict__ a, unsigned *status) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    if (bad_value(a[R.diag[i]])) report_pivot(status, R.row[i]);
+}
+
+// One round of rows outside the tree (and the tree's right-hand sides, which
+// have no pivot here): a block per long row first, then a thread per row.
+// clear: flags the solve that follows starts from (nullptr: none).
+__global__ void __launch_bounds__(1024) front_rows(RowsDev R, int i0, int n_long, int n, const double *__restrict__ a,
+                                                   const double *__restrict__ b, const int *__restrict__ P,
+                                                   const int *__restrict__ Q, double *xk, double *x,
+                                                   unsigned *__restrict__ clear, int n_clear) {
+  __shared__ double part[32];
+  const int bd = blockDim.x;
+  if (clear)
+    for (int k = blockIdx.x * bd + threadIdx.x; k < n_clear; k += gridDim.x * bd) clear[k] = 0;
+  const bool is_long = int(blockIdx.x) < n_long;
+  const int i = is_long ? i0 + int(blockIdx.x) : i0 + n_long + (int(blockIdx.x) - n_long) * bd + int(threadIdx.x);
+  if (i >= i0 + n) return;
+  const int64_t e0 = R.ptr[i], e1 = R.ptr[i + 1];
+  const int k = R.row[i], dg = R.diag[i];
+  double s = 0.0;
+  if (is_long) {
+#pragma unroll 8
+    for (int64_t e = e0 + threadIdx.x; e < e1; e += bd) s += a[R.a[e]] * xk[R.col[e]];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x) return;
+    s = part[0];
+    for (int w = 1; w < bd >> 5; ++w) s += part[w];
+  } else {
+    for (int64_t e = e0; e < e1; ++e) s += a[R.a[e]] * xk[R.col[e]];
+  }
+  double v = b[P[k]] - s;
+  if (dg >= 0) {
+    v /= a[dg];
+    x[Q[k]] = v;
+  }
+  xk[k] = v;
+}
+
+// Children whose border sums (forward) a row gathers: loads of four children
+// in flight at once, added in their order.
+template <class T>
+__device__ __forceinline__ T gather_children(const FrontDev &d, const Front &f, int i) {
+  const T *bv = (const T *)d.bv;
+  T s = T(0);
+  int c = f.child0;
+  for (; c + 4 <= f.child1; c += 4) {
+    int at[4];
+    T v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) at[q] = __ldg(d.inv_map + d.child[c + q].inv + i);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) v[q] = at[q] >= 0 ? __ldcg(bv + d.child[c + q].bv + at[q]) : T(0);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) s += v[q];
+  }
+  for (; c < f.child1; ++c) {
+    const int at = __ldg(d.inv_map + d.child[c].inv + i);
+    if (at >= 0) s += __ldcg(bv + d.child[c].bv + at);
+  }
+  return s;
+}
+
+// y = L \ (right-hand side and the children's sums) for the front's pivots;
+// its border sums go to its parent.  Warp 0 resolves 32 pivots lane to lane
+// while the other warps fetch the entries they apply next (a block of one
+// warp does both in turn).
+template <class T>
+__device__ __forceinline__ void forward(const FrontDev &d, const Front &f, T *v) {
+  const int m = f.m, p = f.p, tid = threadIdx.x, bd = blockDim.x, lane = tid & 31;
+  const T *L = (const T *)d.l + f.lo;
+  for (int i = tid; i < m; i += bd) {
+    T s = gather_children<T>(d, f, i);
+    if (i < p) s += T(__ldcg(d.xk + __ldg(d.idx + f.idx + i)));
+    v[i] = s;
+  }
+  __syncthreads();
+  const int first = bd > 32 ? 32 : 0, step = bd - first;  // threads that apply
+  for (int kb = 0; kb < p; kb += 32) {
+    const int nb = min(32, p - kb);
+    T w[32];
+    const int i0 = kb + nb + tid - first;
+    if (tid < 32) {
+      T s = lane < nb ? v[kb + lane] : T(0);
+#pragma unroll
+      for (int t = 0; t < 32; ++t) w[t] = t < nb && lane > t && lane < nb ? L[int64_t(kb + t) * m + kb + lane] : T(0);
+#pragma unroll
+      for (int t = 0; t < 32; ++t) {
+        if (t < nb) {
+          const T vt = __shfl_sync(0xffffffffu, s, t);
+          if (lane > t) s -= w[t] * vt;
+        }
+      }
+      if (lane < nb) {
+        v[kb + lane] = s;
+        ((T *)d.y)[f.pv + kb + lane] = s;
+      }
+    } else if (i0 < m) {
+#pragma unroll
+      for (int t = 0; t < 32; ++t) w[t] = t < nb ? L[int64_t(kb + t) * m + i0] : T(0);
+    }
+    __syncthreads();
+    if (tid >= first) {
+      for (int i = i0; i < m; i += step) {
+        if (first == 0 || i != i0) {
+#pragma unroll
+          for (int t = 0; t < 32; ++t) w[t] = t < nb ? L[int64_t(kb + t) * m + i] : T(0);
+        }
+        T s = v[i];
+#pragma unroll
+        for (int t = 0; t < 32; ++t)
+          if (t < nb) s -= w[t] * v[kb + t];
+        v[i] = s;
+      }
+    }
+    __syncthreads();
+  }
+  for (int i = p + tid; i < m; i += bd) ((T *)d.bv)[f.bv + i - p] = v[i];
+}
+
+// x = U \ (y - the border's part) for the front's pivots, border first; v
+// holds p + b values and one per thread.
+template <class T>
+__device__ __forceinline__ void backward(const FrontDev &d, const Front &f, T *v, double *x) {
+  const int m = f.m, p = f.p, b = m - p, tid = threadIdx.x, bd = blockDim.x, lane = tid & 31;
+  T *xb = v + p;                      // the border's unknowns
+  T *red = xb + b;                    // partial sums, one per thread
+  const T *L = (const T *)d.l + f.lo, *U = (const T *)d.u + f.uo;
+  for (int j = tid; j < b; j += bd) xb[j] = T(__ldcg(d.xk + __ldg(d.idx + f.idx + p + j)));
+  __syncthreads();
+  // v = y - U x: threads in groups of one row each, a group per slice of the
+  // border, the slices added in order
+  const int rows = min(bd, (p + 31) & ~31), parts = bd / rows, part = tid / rows, ri = tid - part * rows;
+  for (int r0 = 0; r0 < p; r0 += rows) {
+    const int i = r0 + ri;
+    T s = T(0);
+    if (part < parts && i < p) {
+#pragma unroll 8
+      for (int j = part; j < b; j += parts) s += U[int64_t(j) * p + i] * xb[j];
+    }
+    red[tid] = s;
+    __syncthreads();
+    if (part == 0 && i < p) {
+      T t = __ldcg((const T *)d.y + f.pv + i);
+      for (int q = 0; q < parts; ++q) t -= red[q * rows + ri];
+      v[i] = t;
+    }
+    __syncthreads();
+  }
+  const int first = bd > 32 ? 32 : 0, step = bd - first;
+  for (int kb = ((p - 1) / 32) * 32; kb >= 0; kb -= 32) {
+    const int nb = min(32, p - kb);
+    T w[32];
+    const int i0 = tid - first;
+    if (tid < 32) {
+      T s = lane < nb ? v[kb + lane] : T(0);
+      const T rd = lane < nb ? ((const T *)d.rd)[f.pv + kb + lane] : T(0);
+#pragma unroll
+      for (int t = 0; t < 32; ++t) w[t] = t < nb && lane < t ? L[int64_t(kb + t) * m + kb + lane] : T(0);
+#pragma unroll
+      for (int t = 31; t >= 0; --t) {
+        if (t < nb) {
+          if (lane == t) s *= rd;
+          const T vt = __shfl_sync(0xffffffffu, s, t);
+          if (lane < t) s -= w[t] * vt;
+        }
+      }
+      if (lane < nb) {
+        v[kb + lane] = s;
+        const int k = __ldg(d.idx + f.idx + kb + lane);
+        d.xk[k] = double(s);
+        x[__ldg(d.Q + k)] = double(s);
+      }
+    } else if (i0 < kb) {
+#pragma unroll
+      for (int t = 0; t < 32; ++t) w[t] = t < nb ? L[int64_t(kb + t) * m + i0] : T(0);
+    }
+    __syncthreads();
+    if (tid >= first) {
+      for (int i = i0; i < kb; i += step) {
+        if (first == 0 || i != i0) {
+#pragma unroll
+          for (int t = 0; t < 32; ++t) w[t] = t < nb ? L[int64_t(kb + t) * m + i] : T(0);
+        }
+        T s = v[i];
+#pragma unroll
+        for (int t = 0; t < 32; ++t)
+          if (t < nb) s -= w[t] * v[kb + t];
+        v[i] = s;
+      }
+    }
+    __syncthreads();
+  }
+}
+
+template <class T>
+__global__ void __launch_bounds__(256) front_forward(FrontDev d, int f0) {
+  extern __shared__ __align__(16) unsigned char raw[];
+  const Front f = d.front[f0 + blockIdx.x];
+  forward<T>(d, f, reinterpret_cast<T *>(raw));
+}
+template <class T>
+__global__ void __launch_bounds__(256) front_backward(FrontDev d, int f0, double *x) {
+  extern __shared__ __align__(16) unsigned char raw[];
+  const Front f = d.front[f0 + blockIdx.x];
+  backward<T>(d, f, reinterpret_cast<T *>(raw), x);
+}
+
+// Polls a flag (acquire) until it is set, at most `limit` times.
+__device__ __forceinline__ bool wait_flag(const unsigned *p, int limit) {
+  unsigned v = 0;
+  for (int it = 0; it < limit; ++it) {
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    if (v) return true;
+    if (it > 32) __nanosleep(32);
+  }
+  return false;
+}
+
+// Both solves over the fronts above level 0 in one launch.  Blocks claim
+// fronts in order, children before parents, then in reverse; a front waits
+// (bounded) for its children's border sums, backward for its parent, so a
+// step up or down the tree costs a flag and the front's own work instead of
+// a launch that waits for the whole level.  Every front waited for was
+// claimed earlier by a running block, so the claims always advance.  flow:
+// the claim counter, then a forward and a backward flag per front, cleared
+// before the launch.
+template <class T>
+__global__ void __launch_bounds__(kFlowThreads) front_flow(FrontDev d, int first, int nf, unsigned *flow,
+                                                           const unsigned *limit_at, double *x) {
+  extern __shared__ __align__(16) unsigned char raw[];
+  __shared__ int claim;
+  const int count = nf - first, limit = int(__ldg(limit_at)), tid = threadIdx.x;
+  unsigned *fwd = flow + 1, *bwd = fwd + nf;
+  for (;;) {
+    if (tid == 0) claim = int(atomicAdd(flow, 1u));
+    __syncthreads();
+    const int t = claim;
+    if (t >= 2 * count) break;
+    const bool up = t < count;
+    const int k = up ? first + t : nf - 1 - (t - count);
+    const Front f = d.front[k];
+    bool ok = true;
+    if (up) {
+      for (int c = f.child0 + tid; c < f.child1; c += kFlowThreads) {
+        const int g = d.child[c].front;
+        if (g >= first) ok = wait_flag(fwd + g, limit) && ok;
+      }
+    } else if (tid == 0) {
+      ok = wait_flag(f.parent >= 0 ? bwd + f.parent : fwd + k, limit);
+    }
+    if (!ok) atomicOr(d.status, 2u);
+    __syncthreads();
+    if (up) forward<T>(d, f, reinterpret_cast<T *>(raw));
+    else backward<T>(d, f, reinterpret_cast<T *>(raw), x);
+    __syncthreads();
+    if (tid == 0) {
+      __threadfence();
+      asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"((up ? fwd : bwd) + k), "r"(1u) : "memory");
+    }
+  }
+}
+
+// The largest |multiplier| per front.
+template <class T>
+__global__ void __launch_bounds__(256) front_multipliers(FrontDev d, double *out) {
+  __shared__ double part[8];
+  const Front f = d.front[blockIdx.x];
+  const T *L = (const T *)d.l + f.lo;
+  double mx = 0.0;
+  for (int64_t e = threadIdx.x; e < int64_t(f.m) * f.p; e += 256) {
+    const int64_t j = e / f.m;
+    if (e - j * f.m > j) {
+      const double v = fabs(double(L[e]));
+      mx = v > mx || v != v ? v : mx;  // a NaN stays
+    }
+  }
+  // NaN-keeping maximum over the block
+  for (int o = 16; o > 0; o >>= 1) {
+    const double v = __shfl_xor_sync(0xffffffffu, mx, o);
+    mx = v > mx || v != v ? v : mx;
+  }
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = mx;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; ++w) mx = part[w] > mx || part[w] != part[w] ? part[w] : mx;
+    out[blockIdx.x] = mx;
+  }
+}
+
+struct Group {  // fronts of one level launched together
+  int f0, n;                      // solves of level 0
+  int slot0, grid, cluster, threads;
+  size_t smem, smem_fwd, smem_bwd;
+  int solve_threads;
+};
+
+}  // namespace
+
+struct FrontLu {
+  int n = 0, n_front = 0;
+  int precision = 0;
+  std::vector<Group> group;
+  std::vector<void *> owned;
+  FrontDev d{};
+  RowsDev before{}, core{}, after{};
+  std::vector<int> before_round, core_round, after_round;
+  int flow_first = 0, flow_grid = 0;  // fronts from here on (levels above 0) are solved in one launch
+  size_t n_low = 0;                   // groups of level 0
+  size_t flow_smem = 0;
+  unsigned *flow = nullptr;           // claim counter and flags
+  const int *slot = nullptr;          // the factor launches' CTAs: their fronts
+  ~FrontLu() {
+    for (void *p : owned) cudaFree(p);
+  }
+};
+
+namespace {
+
+// One allocation that the LU owns.
+template <class V>
+bool take(FrontLu *f, V **p, size_t count) {
+  *p = nullptr;
+  if (cudaMalloc((void **)p, sizeof(V) * std::max<size_t>(count, 1)) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  f->owned.push_back(*p);
+  return true;
+}
+template <class V>
+bool give(FrontLu *f, const V **p, const std::vector<V> &src) {
+  V *q = nullptr;
+  if (!take(f, &q, src.size())) return false;
+  *p = q;
+  return src.empty() ||
+         cudaMemcpy(q, src.data(), sizeof(V) * src.size(), cudaMemcpyHostToDevice) == cudaSuccess;
+}
+bool give_rows(FrontLu *f, RowsDev *R, const FrontRows &H) {
+  return give(f, &R->row, H.row) && give(f, &R->diag, H.diag) && give(f, &R->col, H.col) && give(f, &R->a, H.a) &&
+         give(f, &R->ptr, H.ptr);
+}
+
+template <class T>
+const void *factor_fn() {
+  return (const void *)front_factor<T>;
+}
+
+cudaError_t launch_factor(const FrontLu *f, const Group &g, const double *a, const unsigned *limit, cudaStream_t s) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(unsigned(g.grid));
+  cfg.blockDim = dim3(unsigned(g.threads));
+  cfg.dynamicSmemBytes = g.smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = unsigned(g.cluster);
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return f->precision == XG_LU_FP32 ? cudaLaunchKernelEx(&cfg, front_factor<float>, f->d, a, f->slot + g.slot0, limit)
+                                    : cudaLaunchKernelEx(&cfg, front_factor<double>, f->d, a, f->slot + g.slot0, limit);
+}
+
+constexpr double kWideWork = 6e4;  // multiply-adds one SM is left with
+
+}  // namespace
+
+FrontLu *front_create(const FrontPlan &plan, const LuSymbolic &S, int device, int precision, int *rc) {
+  *rc = XG_OK;
+  std::unique_ptr<FrontLu> f(new FrontLu);
+  f->n = plan.n;
+  f->n_front = int(plan.front.size());
+  f->precision = precision;
+  const size_t tsz = precision == XG_LU_FP32 ? sizeof(float) : sizeof(double);
+  const void *fn = precision == XG_LU_FP32 ? factor_fn<float>() : factor_fn<double>();
+  int sms = 0;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+  cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  std::vector<Front> front = plan.front;
+  std::vector<int> slot;
+  size_t most = 0;
+  for (size_t l = 0; l + 1 < plan.level.size(); ++l) {
+    const int at = plan.level[l], end = plan.level[l + 1];
+    // the small fronts of a level with many apart: their blocks are smaller
+    int first_small = at, first_low = at;
+    while (first_small < end && plan.front[first_small].m > kFrontMiddle) ++first_small;
+    while (first_low < end && plan.front[first_low].m > kFrontLow) ++first_low;
+    std::vector<int> cut = {at};
+    if (first_small > at && end - first_small > sms) cut.push_back(first_small);
+    if (first_low > cut.back() && end - first_low > 4 * sms) cut.push_back(first_low);
+    cut.push_back(end);
+    for (size_t q = 0; q + 1 < cut.size(); ++q) {
+      Group g{};
+      g.f0 = cut[q];
+      g.n = cut[q + 1] - cut[q];
+      int m = 0;
+      double total = 0.0;
+      for (int k = g.f0; k < g.f0 + g.n; ++k) {
+        m = std::max(m, front[k].m);
+        total += front_work(front[k].p, front[k].m);
+      }
+      g.threads = std::max(m <= kFrontLow ? 32 : 128, (m + 31) / 32 * 32);
+      g.solve_threads = m <= kFrontLow ? 32 : m <= kFrontMiddle ? 64 : 256;
+      // CTAs of a front: what brings its work down to an SM's share of the
+      // level (below kWideWork another halving gains less than its
+      // hand-overs cost) and its shared memory to a quarter of an SM's, so
+      // that fronts hide each other's waits; at least two column blocks each
+      const double share = std::max(kWideWork, total / sms);
+      std::vector<int> by_ctas[5];
+      for (int k = g.f0; k < g.f0 + g.n; ++k) {
+        Front &h = front[k];
+        int lg = 0;
+        const double w = front_work(h.p, h.m);
+        while (lg < 4 && (w > share * (1 << lg) || factor_smem(h.m, 1 << lg, tsz) > kSmemTarget) &&
+               (4 * kNb << lg) <= h.m)
+          ++lg;
+        while (lg < 4 && factor_smem(h.m, 1 << lg, tsz) > kSmemLimit) ++lg;
+        if (factor_smem(h.m, 1 << lg, tsz) > kSmemLimit) return nullptr;
+        h.ctas = 1 << lg;
+        by_ctas[lg].push_back(k);
+        g.smem = std::max(g.smem, factor_smem(h.m, h.ctas, tsz));
+      }
+      // widest first: powers of two pack the clusters without gaps
+      g.slot0 = int(slot.size());
+      g.cluster = 1;
+      for (int lg = 4; lg >= 0; --lg)
+        for (int k : by_ctas[lg]) {
+          g.cluster = std::max(g.cluster, 1 << lg);
+          slot.insert(slot.end(), size_t(1) << lg, k);
+        }
+      while ((slot.size() - size_t(g.slot0)) % size_t(g.cluster)) slot.push_back(-1);
+      g.grid = int(slot.size()) - g.slot0;
+      g.smem_fwd = size_t(m) * tsz;
+      g.smem_bwd = size_t(m + g.solve_threads) * tsz;
+      most = std::max(most, g.smem);
+      f->group.push_back(g);
+    }
+    if (l == 0) f->n_low = f->group.size();
+  }
+  f->flow_first = plan.level.size() > 1 ? plan.level[1] : f->n_front;
+  {
+    int mx = 0;
+    for (int k = f->flow_first; k < f->n_front; ++k) mx = std::max(mx, plan.front[k].m);
+    f->flow_smem = size_t(mx + kFlowThreads) * tsz;
+    const void *flow_fn = precision == XG_LU_FP32 ? (const void *)front_flow<float> : (const void *)front_flow<double>;
+    int occ = 0;
+    if (allow_dynamic_smem(flow_fn, f->flow_smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, flow_fn, kFlowThreads, f->flow_smem) != cudaSuccess)
+      return nullptr;
+    f->flow_grid = std::max(1, std::min(sms * std::max(occ, 1), f->n_front - f->flow_first));
+  }
+  if (allow_dynamic_smem(fn, most) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  std::vector<ChildDev> child(plan.child.size());
+  for (size_t k = 0; k < child.size(); ++k) {
+    const Front &g = plan.front[plan.child[k]];
+    child[k] = ChildDev{plan.inv[k], g.co, g.bv, g.map, g.m - g.p, plan.child[k]};
+  }
+  FrontDev &d = f->d;
+  unsigned char *l = nullptr, *u = nullptr, *c = nullptr, *rd = nullptr, *y = nullptr, *bv = nullptr;
+  const bool ok = give(f.get(), &d.front, front) && give(f.get(), &f->slot, slot) && give(f.get(), (const ChildDev **)&d.child, child) &&
+                  give(f.get(), &d.idx, plan.idx) && give(f.get(), &d.map, plan.map) &&
+                  give(f.get(), &d.inv_map, plan.inv_map) && give(f.get(), &d.apos, plan.apos) &&
+                  give(f.get(), &d.aidx, plan.aidx) &&
+                  give(f.get(), &d.P, S.P) && give(f.get(), &d.Q, plan.Q) && take(f.get(), &l, tsz * plan.n_l) &&
+                  take(f.get(), &u, tsz * plan.n_u) && take(f.get(), &c, tsz * plan.n_c) &&
+                  take(f.get(), &rd, tsz * plan.n_pv) && take(f.get(), &y, tsz * plan.n_pv) &&
+                  take(f.get(), &bv, tsz * plan.n_bv) &&
+                  take(f.get(), &f->flow, size_t(2 * f->n_front + 1)) && take(f.get(), &d.xk, size_t(plan.n)) &&
+                  give_rows(f.get(), &f->before, plan.before) && give_rows(f.get(), &f->core, plan.core) &&
+                  give_rows(f.get(), &f->after, plan.after);
+  if (!ok) {
+    *rc = XG_ERR_OOM;
+    return nullptr;
+  }
+  d.l = l;
+  d.u = u;
+  d.c = c;
+  d.rd = rd;
+  d.y = y;
+  d.bv = bv;
+  f->before_round = plan.before.round;
+  f->core_round = plan.core.round;
+  f->after_round = plan.after.round;
+  return f.release();
+}
+
+void front_destroy(FrontLu *f) { delete f; }
+
+int front_refactor(FrontLu *f, const double *dev_values, double *a_copy, int64_t nnz_a, unsigned *status,
+                   const unsigned *limit, void *stream) {
+  cudaStream_t s = (cudaStream_t)stream;
+  f->d.status = status;
+  front_open<<<int(std::min<int64_t>(1024, (nnz_a + 255) / 256)), 256, 0, s>>>(dev_values, a_copy, nnz_a, status);
+  count_launches(1);
+  for (const Group &g : f->group) {
+    if (launch_factor(f, g, dev_values, limit, s) != cudaSuccess) return XG_ERR_CUDA;
+    count_launches(1);
+  }
+  const RowsDev *rows[] = {&f->before, &f->after};
+  const std::vector<int> *round[] = {&f->before_round, &f->after_round};
+  for (int k = 0; k < 2; ++k) {
+    if (round[k]->empty() || !round[k]->back()) continue;
+    const int n = round[k]->back();
+    front_check_rows<<<std::min(1024, (n + 255) / 256), 256, 0, s>>>(*rows[k], n, a_copy, status);
+    count_launches(1);
+  }
+  return cudaGetLastError() == cudaSuccess ? XG_OK : XG_ERR_CUDA;
+}
+
+template <class T>
+static void solve_tree(FrontLu *f, double *x, unsigned *status, const unsigned *limit, cudaStream_t s) {
+  for (size_t k = 0; k < f->n_low; ++k) {
+    const Group &g = f->group[k];
+    front_forward<T><<<g.n, g.solve_threads, g.smem_fwd, s>>>(f->d, g.f0);
+    count_launches(1);
+  }
+  if (f->flow_first < f->n_front) {
+    f->d.status = status;
+    front_flow<T><<<f->flow_grid, kFlowThreads, f->flow_smem, s>>>(f->d, f->flow_first, f->n_front, f->flow, limit, x);
+    count_launches(1);
+  }
+  for (size_t k = f->n_low; k-- > 0;) {
+    const Group &g = f->group[k];
+    front_backward<T><<<g.n, g.solve_threads, g.smem_bwd, s>>>(f->d, g.f0, x);
+    count_launches(1);
+  }
+}
+
+int front_solve(FrontLu *f, const double *a_copy, const double *b, double *x, unsigned *status, const unsigned *limit,
+                void *stream) {
+  cudaStream_t s = (cudaStream_t)stream;
+  auto rows = [&](const RowsDev &R, const std::vector<int> &round, unsigned *clear) {
+    for (size_t k = 0; k + 2 < round.size(); k += 2) {
+      const int i0 = round[k], n_long = round[k + 1] - i0, n = round[k + 2] - i0;
+      if (!n) continue;
+      const int bd = n_long ? 1024 : 256;
+      front_rows<<<n_long + (n - n_long + bd - 1) / bd, bd, 0, s>>>(R, i0, n_long, n, a_copy, b, f->d.P, f->d.Q,
+                                                                    f->d.xk, x, clear, 2 * f->n_front + 1);
+      count_launches(1);
+    }
+  };
+  rows(f->before, f->before_round, nullptr);
+  rows(f->core, f->core_round, f->flow);
+  if (f->precision == XG_LU_FP32) solve_tree<float>(f, x, status, limit, s);
+  else solve_tree<double>(f, x, status, limit, s);
+  rows(f->after, f->after_round, nullptr);
+  return cudaGetLastError() == cudaSuccess ? XG_OK : XG_ERR_CUDA;
+}
+
+int front_max_multiplier(FrontLu *f, double *out, void *stream) {
+  cudaStream_t s = (cudaStream_t)stream;
+  double *dev = nullptr;
+  std::vector<double> h(size_t(f->n_front), 0.0);
+  if (cudaMalloc((void **)&dev, sizeof(double) * h.size()) != cudaSuccess) return XG_ERR_OOM;
+  if (f->precision == XG_LU_FP32) front_multipliers<float><<<f->n_front, 256, 0, s>>>(f->d, dev);
+  else front_multipliers<double><<<f->n_front, 256, 0, s>>>(f->d, dev);
+  count_launches(1);
+  cudaError_t e = cudaMemcpyAsync(h.data(), dev, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, s);
+  const cudaError_t e2 = cudaStreamSynchronize(s);
+  cudaFree(dev);
+  if (e != cudaSuccess || e2 != cudaSuccess) return XG_ERR_CUDA;
+  double mx = 0.0;
+  for (double v : h) mx = v > mx || v != v ? v : mx;
+  *out = mx;
+  return XG_OK;
+}
+
+}  // namespace xg

@@ -25,6 +25,9 @@
 //    trailing rows of one or two per level go to the chain kernel, 32
 //    columns at a time (lu_solve_chain, planned in lu_chain.h), and a long
 //    row no other row waits for to a block of its own (lu_solve_long).
+//  * large matrices (8,192 rows and up) whose dependency chains would cost
+//    more than a tree of dense fronts go to the multifrontal path
+//    (lu_front.h, lu_front.cu) instead; try_front below chooses.
 //  * precision: factors in FP64, or in FP32 with FP64 iterative refinement
 //    (r = b - A x with the FP64 matrix, solve, x += d).
 //
@@ -46,6 +49,7 @@
 #include "xg.h"
 #include "xg_internal.h"
 #include "lu_chain.h"
+#include "lu_front.h"
 #include "xg_lu.h"
 #include "xg_smem.cuh"
 
@@ -922,11 +926,35 @@ __global__ void __launch_bounds__(kChainLanes) lu_solve_chain(LuDev d, ChainDev 
   }
 }
 
-// r = b - A x   (FP64, one thread per row, entries in CSR order)
-__global__ void lu_residual(LuDev d, const double *__restrict__ a, const double *__restrict__ x,
-                            const double *__restrict__ b, double *__restrict__ r) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < d.n; i += gridDim.x * blockDim.x) {
+// r = b - A x   (FP64, one thread per row, entries in CSR order).  Rows of
+// more than kResidualLong entries (a supply node's row names every device on
+// it; one thread took 1 ms for 20,000) get a block each, the first n_long
+// blocks of the grid: a strided sum per thread, then a fixed tree.
+constexpr int kResidualLong = 128;
+constexpr int kResidualThreads = 256;
+__global__ void __launch_bounds__(kResidualThreads) lu_residual(LuDev d, const double *__restrict__ a,
+                                                                const double *__restrict__ x,
+                                                                const double *__restrict__ b, double *__restrict__ r,
+                                                                const int *__restrict__ long_rows, int n_long) {
+  if (int(blockIdx.x) < n_long) {
+    __shared__ double part[kResidualThreads / 32];
+    const int i = long_rows[blockIdx.x], p0 = __ldg(d.arp + i), p1 = __ldg(d.arp + i + 1);
+    double acc = 0.0;
+#pragma unroll 8
+    for (int p = p0 + threadIdx.x; p < p1; p += kResidualThreads) acc += a[p] * x[__ldg(d.aci + p)];
+    acc = warp_sum(acc);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = acc;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      for (int w = 1; w < kResidualThreads / 32; ++w) acc += part[w];
+      r[i] = b[i] - acc;
+    }
+    return;
+  }
+  const int blocks = gridDim.x - n_long;
+  for (int i = (blockIdx.x - n_long) * blockDim.x + threadIdx.x; i < d.n; i += blocks * blockDim.x) {
     const int p0 = __ldg(d.arp + i), p1 = __ldg(d.arp + i + 1);
+    if (p1 - p0 > kResidualLong) continue;
     double acc = b[i];
     for (int p = p0; p < p1; ++p) acc -= a[p] * x[__ldg(d.aci + p)];
     r[i] = acc;
@@ -1693,6 +1721,8 @@ struct xg_lu {
   void *d_rdiag = nullptr;                        // n of T: 1 / U(k,k)
   double *d_a = nullptr;                          // FP64 copy of A
   double *d_r = nullptr, *d_dx = nullptr;         // refinement work
+  int *d_res_long = nullptr;                      // rows of A the residual gives a block each
+  int n_res_long = 0;
   double *d_hv = nullptr, *d_hb = nullptr, *d_hx = nullptr;  // xg_lu_solve_host staging
   int grid_factor = 0, grid_solve = 0;
   int stage_cap = 0;                       // grid refactor: staged row entries per warp
@@ -1722,6 +1752,7 @@ struct xg_lu {
   int lvl_threads = 0;
   int *d_lvl = nullptr;                    // level lists, row starts and tail, one buffer
   xg::LvlDev lvl_dev{};
+  xg::FrontLu *front = nullptr;            // the multifrontal path (lu_front.h); nothing above then
   bool factored = false;
   xg::LuDev dev() const {
     return xg::LuDev{S.n, d_rp, d_ci, d_diag, d_lu2a, d_P, d_Q, d_arp, d_aci, d_urp, d_upos,
@@ -1754,14 +1785,20 @@ void free_lu(xg_lu *lu) {
                   lu->d_urp, lu->d_upos, lu->d_lvl,
                   lu->d_aci, lu->d_ctrl, lu->d_tdesc, lu->d_hpart, lu->d_solo, lu->d_long, lu->d_pending, lu->d_chain_blk, lu->d_chain_tiles, lu->d_chain_tsrc,
                   lu->d_chain_rowj, lu->d_chain_esrc, lu->d_chain_val, lu->d_val, lu->d_y, lu->d_z, lu->d_rdiag, lu->d_a,
-                  lu->d_r, lu->d_dx, lu->d_hv, lu->d_hb, lu->d_hx};
+                  lu->d_r, lu->d_dx, lu->d_res_long, lu->d_hv, lu->d_hb, lu->d_hx};
   for (void *p : ptrs)
     if (p) cudaFree(p);
+  if (lu->front) xg::front_destroy(lu->front);
 }
 
 template <class T>
 int refactor_t(xg_lu *lu, const double *dev_values) {
   xg::LuDev d = lu->dev();
+  if (lu->front) {
+    const int rc = xg::front_refactor(lu->front, dev_values, lu->d_a, lu->S.nnz_a, lu->d_ctrl + xg::C_STATUS,
+                                      lu->d_ctrl + xg::C_SPIN, lu->stream);
+    return rc ? cuda_fail(cudaGetLastError(), "multifrontal refactor") : XG_OK;
+  }
   if (lu->lvl) {
     xg::lu_factor_lvl<T><<<1, lu->lvl_threads, lu->smem_lvl_factor, lu->stream>>>(
         d, lu->lvl_dev, dev_values, lu->d_a, lu->S.nnz_a, (T *)lu->d_val, lu->nnz_lu);
@@ -1799,6 +1836,10 @@ int refactor_t(xg_lu *lu, const double *dev_values) {
 template <class T>
 int solve_once(xg_lu *lu, const double *b, double *x) {
   xg::LuDev d = lu->dev();
+  if (lu->front) {
+    const int rc = xg::front_solve(lu->front, lu->d_a, b, x, lu->d_ctrl + xg::C_STATUS, lu->d_ctrl + xg::C_SPIN, lu->stream);
+    return rc ? cuda_fail(cudaGetLastError(), "multifrontal solve") : XG_OK;
+  }
   if (lu->lvl) {
     xg::lu_solve_lvl<T><<<1, lu->lvl_threads, lu->smem_lvl_solve, lu->stream>>>(
         d, lu->lvl_dev, (const T *)lu->d_val, lu->nnz_lu, b, x);
@@ -1857,7 +1898,8 @@ int solve_t(xg_lu *lu, const double *b, double *x, int n_refine) {
   xg::LuDev d = lu->dev();
   const int nb = std::min(1024, (lu->S.n + 255) / 256);
   for (int it = 0; it < n_refine; ++it) {
-    xg::lu_residual<<<nb, 256, 0, lu->stream>>>(d, lu->d_a, x, b, lu->d_r); xg::count_launches(1);
+    xg::lu_residual<<<nb + lu->n_res_long, xg::kResidualThreads, 0, lu->stream>>>(d, lu->d_a, x, b, lu->d_r, lu->d_res_long,
+                                                                             lu->n_res_long); xg::count_launches(1);
     rc = solve_once<T>(lu, lu->d_r, lu->d_dx);
     if (rc) return rc;
     xg::lu_axpy<<<nb, 256, 0, lu->stream>>>(lu->S.n, lu->d_dx, x); xg::count_launches(1);
@@ -1880,12 +1922,71 @@ int refactor_solve_t(xg_lu *lu, const double *dev_values, const double *b, doubl
   XG_CU(cudaGetLastError());
   for (int it = 0; it < n_refine; ++it) {
     const int nb = std::min(1024, (lu->S.n + 255) / 256);
-    xg::lu_residual<<<nb, 256, 0, lu->stream>>>(d, lu->d_a, x, b, lu->d_r); xg::count_launches(1);
+    xg::lu_residual<<<nb + lu->n_res_long, xg::kResidualThreads, 0, lu->stream>>>(d, lu->d_a, x, b, lu->d_r, lu->d_res_long,
+                                                                             lu->n_res_long); xg::count_launches(1);
     int rc = solve_once<T>(lu, lu->d_r, lu->d_dx);
     if (rc) return rc;
     xg::lu_axpy<<<nb, 256, 0, lu->stream>>>(lu->S.n, lu->d_dx, x); xg::count_launches(1);
   }
   XG_CU(cudaGetLastError());
+  return XG_OK;
+}
+
+// Where the multifrontal path is tried.  Factors below kFrontMinRows rows
+// keep the bounded waits and the reported chain of the grid path, which their
+// callers observe.
+constexpr int kFrontMinRows = 8192;
+// The largest multiplier the chosen pivots may give in the tree's order: the
+// analysis accepts a pivot at 0.001 of its column (KLU's tolerance), which is
+// this bound on |L|; the order within the tree is another one, so it is
+// checked on the analysed values.
+constexpr double kFrontMaxMultiplier = 1e3;
+
+// The grid path's refactor and solve, modelled: 2.8 us a level of its
+// longest dependency chain and 25 ps a multiply-add (power grids of 8,634 to
+// 120,002 rows and logic blocks of 17,000 to 200,000 devices took 0.75 to 1.2
+// times that), and 0.6 us an entry of the longest L row, which one warp walks (a
+// 9,000-stage chain's supply row: 5.5 ms).
+double grid_seconds(const xg::LuSymbolic &S) {
+  int longest = 0;
+  for (int i = 0; i < S.n; ++i) longest = std::max(longest, S.diag[i] - S.rp[i]);
+  return std::max(2.8e-6 * S.levels + 25e-12 * S.refactor_flops, 0.6e-6 * longest);
+}
+
+// Tries the multifrontal path for an analysed matrix: lu->front when it is
+// modelled faster than the grid path and its multipliers stay within the
+// pivoting bound.  Measured, refactor and solve, grid / multifrontal: 74x70
+// power grid (8,634 rows) 1.10 / 0.76 ms, 200x200 7.2 / 2.6 ms, logic of
+// 17,000 devices 1.87 / 1.34 ms, of 200,000 21.4 / 2.9 ms.
+int try_front(xg_lu *lu, const int *rp, const int *ci, const double *values) {
+  const xg::LuSymbolic &S = lu->S;
+  xg::FrontPlan plan;
+  if (!xg::build_front_plan(S, rp, ci, &plan) || plan.seconds > grid_seconds(S)) return XG_OK;
+  int rc = XG_OK;
+  xg::FrontLu *f = xg::front_create(plan, S, lu->device, lu->precision, &rc);
+  if (!f) return XG_OK;  // no room: the grid path
+  double *dev_values = nullptr, most = 0.0;
+  unsigned status[2] = {1u, 0u};
+  cudaError_t e = cudaMalloc((void **)&dev_values, sizeof(double) * size_t(S.nnz_a));
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(dev_values, values, sizeof(double) * size_t(S.nnz_a), cudaMemcpyHostToDevice, lu->stream);
+  if (e == cudaSuccess) {
+    rc = xg::front_refactor(f, dev_values, dev_values, S.nnz_a, lu->d_ctrl + xg::C_STATUS, lu->d_ctrl + xg::C_SPIN,
+                            lu->stream);
+    if (!rc) rc = xg::front_max_multiplier(f, &most, lu->stream);
+    e = cudaMemcpyAsync(status, lu->d_ctrl + xg::C_STATUS, sizeof(status), cudaMemcpyDeviceToHost, lu->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(lu->stream);
+  }
+  if (dev_values) cudaFree(dev_values);
+  if (rc || e != cudaSuccess || status[0] || !(most <= kFrontMaxMultiplier)) {
+    xg::front_destroy(f);
+    if (e == cudaErrorMemoryAllocation) {
+      cudaGetLastError();
+      return XG_OK;
+    }
+    return rc ? rc : e != cudaSuccess ? cuda_fail(e, "xg_lu_analyze") : XG_OK;
+  }
+  lu->front = f;
   return XG_OK;
 }
 
@@ -1909,10 +2010,6 @@ extern "C" int xg_lu_analyze(xg_ctx *ctx, int n, const int *host_rowptr, const i
     xg::set_error(err);
     return XG_ERR_SINGULAR;
   }
-  if (!xg::lu_build_updates(lu->S)) {
-    xg::set_error("xg_lu_analyze: internal error, an update falls outside the L\\U pattern");
-    return XG_ERR_ARG;
-  }
   XG_CU(cudaSetDevice(lu->device));
   const xg::LuSymbolic &S = lu->S;
   lu->nnz_lu = S.rp[n];
@@ -1924,10 +2021,46 @@ extern "C" int xg_lu_analyze(xg_ctx *ctx, int n, const int *host_rowptr, const i
     free_lu(lu.get());
     return r;
   };
+  cudaError_t e = cudaSuccess;
+  auto fail_alloc = [&]() {
+    free_lu(lu.get());
+    return e == cudaErrorMemoryAllocation ? (xg::set_error("xg_lu_analyze: out of device memory"),
+                                             XG_ERR_OOM)
+                                          : cuda_fail(e, "xg_lu_analyze");
+  };
+  std::vector<int> res_long;
+  for (int i = 0; i < n; ++i)
+    if (arp[i + 1] - arp[i] > xg::kResidualLong) res_long.push_back(i);
+  lu->n_res_long = int(res_long.size());
+  if ((rc = upload(&lu->d_arp, arp)) || (rc = upload(&lu->d_aci, aci)) || (rc = upload(&lu->d_res_long, res_long)))
+    return fail(rc);
+  if ((e = cudaMalloc((void **)&lu->d_ctrl, sizeof(unsigned) * xg::C_N)) ||
+      (e = cudaMalloc((void **)&lu->d_a, sizeof(double) * size_t(S.nnz_a))) ||
+      (e = cudaMalloc((void **)&lu->d_r, sizeof(double) * size_t(n))) ||
+      (e = cudaMalloc((void **)&lu->d_dx, sizeof(double) * size_t(n))))
+    return fail_alloc();
+  {
+    unsigned init[xg::C_N] = {};
+    init[xg::C_SPIN] = unsigned(xg::kSpinLimit);
+    if ((e = cudaMemcpy(lu->d_ctrl, init, sizeof(init), cudaMemcpyHostToDevice))) {
+      free_lu(lu.get());
+      return cuda_fail(e, "xg_lu_analyze: cudaMemcpy");
+    }
+  }
+  if (n >= kFrontMinRows && !std::getenv("XG_LU_NO_FRONT")) {
+    if ((rc = try_front(lu.get(), host_rowptr, host_colidx, host_values))) return fail(rc);
+    if (lu->front) {
+      *out = lu.release();
+      return XG_OK;
+    }
+  }
+  if (!xg::lu_build_updates(lu->S)) {
+    xg::set_error("xg_lu_analyze: internal error, an update falls outside the L\\U pattern");
+    return fail(XG_ERR_ARG);
+  }
   if ((rc = upload(&lu->d_rp, S.rp)) || (rc = upload(&lu->d_ci, S.ci)) ||
       (rc = upload(&lu->d_diag, S.diag)) || (rc = upload(&lu->d_lu2a, S.lu2a)) ||
       (rc = upload(&lu->d_P, S.P)) || (rc = upload(&lu->d_Q, S.Q)) ||
-      (rc = upload(&lu->d_arp, arp)) || (rc = upload(&lu->d_aci, aci)) ||
       (rc = upload(&lu->d_urp, S.urp)) || (rc = upload(&lu->d_upos, S.upos)))
     return fail(rc);
   const int64_t nup = S.urp[n];
@@ -1937,27 +2070,10 @@ extern "C" int xg_lu_analyze(xg_ctx *ctx, int n, const int *host_rowptr, const i
   std::vector<int64_t>().swap(lu->S.urp);
   std::vector<int>().swap(lu->S.upos);
   const size_t tsz = precision == XG_LU_FP32 ? sizeof(float) : sizeof(double);
-  cudaError_t e = cudaSuccess;
-  if ((e = cudaMalloc((void **)&lu->d_ctrl, sizeof(unsigned) * xg::C_N)) ||
-      (e = cudaMalloc(&lu->d_val, tsz * size_t(lu->nnz_lu))) ||
+  if ((e = cudaMalloc(&lu->d_val, tsz * size_t(lu->nnz_lu))) ||
       (e = cudaMalloc(&lu->d_y, tsz * size_t(n))) || (e = cudaMalloc(&lu->d_z, tsz * size_t(n))) ||
-      (e = cudaMalloc(&lu->d_rdiag, tsz * size_t(n))) ||
-      (e = cudaMalloc((void **)&lu->d_a, sizeof(double) * size_t(S.nnz_a))) ||
-      (e = cudaMalloc((void **)&lu->d_r, sizeof(double) * size_t(n))) ||
-      (e = cudaMalloc((void **)&lu->d_dx, sizeof(double) * size_t(n)))) {
-    free_lu(lu.get());
-    return e == cudaErrorMemoryAllocation ? (xg::set_error("xg_lu_analyze: out of device memory"),
-                                             XG_ERR_OOM)
-                                          : cuda_fail(e, "xg_lu_analyze");
-  }
-  {
-    unsigned init[xg::C_N] = {};
-    init[xg::C_SPIN] = unsigned(xg::kSpinLimit);
-    if ((e = cudaMemcpy(lu->d_ctrl, init, sizeof(init), cudaMemcpyHostToDevice))) {
-      free_lu(lu.get());
-      return cuda_fail(e, "xg_lu_analyze: cudaMemcpy");
-    }
-  }
+      (e = cudaMalloc(&lu->d_rdiag, tsz * size_t(n))))
+    return fail_alloc();
   int sms = 0, occ = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, lu->device);
   {
