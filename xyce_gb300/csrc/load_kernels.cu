@@ -24,6 +24,7 @@
 
 #include <cstdint>
 
+#include "xg_dcmp.cuh"
 #include "xg_fast_rcp.cuh"
 #include "xg_internal.h"
 
@@ -108,34 +109,6 @@ __device__ __forceinline__ double fetlim(double vnew, double vold, double vto) {
     }
   }
   return vnew;
-}
-
-// DeviceSupport::qmeyer (N_DEV_DeviceSupport.C:545-631)
-__device__ __forceinline__ void qmeyer(double vgs, double vgd, double von, double vdsat,
-                                       double &capgs, double &capgd, double &capgb, double phi,
-                                       double cox) {
-  double vgst = vgs - von;
-  if (vgst <= -phi) {
-    capgb = cox / 2; capgs = 0; capgd = 0;
-  } else if (vgst <= -phi / 2) {
-    capgb = -vgst * cox / (2 * phi); capgs = 0; capgd = 0;
-  } else if (vgst <= 0) {
-    capgb = -vgst * cox / (2 * phi);
-    capgs = vgst * cox / (1.5 * phi) + cox / 3;
-    capgd = 0;
-  } else {
-    double vds = vgs - vgd;
-    if (vdsat <= vds) {
-      capgs = cox / 3; capgd = 0; capgb = 0;
-    } else {
-      double vddif = 2.0 * vdsat - vds;
-      double vddif1 = vdsat - vds;
-      double vddif2 = vddif * vddif;
-      capgd = cox * (1.0 - vdsat * vdsat / vddif2) / 3;
-      capgs = cox * (1.0 - vddif1 * vddif1 / vddif2) / 3;
-      capgb = 0;
-    }
-  }
 }
 
 // Term writer: term q of instance i at [q][i], so a warp's store of one term
@@ -376,6 +349,97 @@ __global__ void __launch_bounds__(256) diode_kernel(DevType t, DevOptions o, Fla
 }
 
 // ---- MOSFET level 1 (N_DEV_MOSFET1.C:2618-3427, 4103-4722), newMeyer off ----
+// Bound by FP64 issue, and a warp pays for every instruction any of its lanes
+// takes: with the model's branches as branches, a warp of the random netlist
+// issued 806 FP64 instructions where one thread needs 287.  So each
+// alternative is a choice of operands for one evaluation (the direction of
+// the channel, the junction that is limited, saturation or not) with the
+// arithmetic of the branch it stands for; comparisons are made on the bits
+// and polarity and mode are sign flips (xg_dcmp.cuh); quotients by vt share
+// one reciprocal; and a warp whose instances all have M = 1 skips the
+// products by M.  Nothing is formed that a card without body effect
+// (GAMMA = 0) or oxide capacitance would multiply by that zero.  On 300,000
+// devices: 806 -> 213 FP64 instructions a warp, 0.47 -> 0.133 ms (FMA build),
+// 0.49 -> 0.138 ms (exact build), FP64 pipe 82% busy.
+
+// fetlim: the limit is a bound on the step (s) or on the value (t).
+__device__ __forceinline__ double fetlim_select(double vnew, double vold, double vto) {
+  const double hi = fma(2.0, magnitude(vold - vto), 2.0);  // (exact products)
+  const double lo = fma(0.5, hi, 2.0);
+  const double vtox = vto + 3.5, delv = vnew - vold;
+  const bool down = le0(delv), on = ge(vold, vto), strong = ge(vold, vtox);
+  const double s = vold + (on ? (down ? -lo : hi) : (down ? -hi : lo));
+  const double t = vto + (on ? (strong ? 2.0 : down ? -0.5 : 4.0) : 0.5);
+  if (on ? strong && (!down || ge(vnew, vtox)) : down || le(vnew, t)) {
+    const double step = down ? -delv : delv, bound = on ? (down ? lo : hi) : (down ? hi : lo);
+    return (on && !down ? ge(step, bound) : gt(step, bound)) ? s : vnew;
+  }
+  if (!on) return t;
+  return down ? (gt(vnew, t) ? vnew : t) : (lt(vnew, t) ? vnew : t);
+}
+
+__device__ __forceinline__ double limvds_select(double vnew, double vold) {
+  const bool strong = ge(vold, 3.5), up = gt(vnew, vold);
+  double lim = up ? 4.0 : -0.5;
+  if (strong) lim = up ? (3.0 * vold) + 2.0 : 2.0;
+  if (up) return lt(vnew, lim) ? vnew : lim;
+  if (strong && !lt(vnew, 3.5)) return vnew;
+  return gt(vnew, lim) ? vnew : lim;
+}
+
+// pnjlim with y the reciprocal of vt; one logarithm for both of its forms.
+__device__ __forceinline__ double pnjlim_select(double vnew, double vold, double vt, double y, double vcrit) {
+  const double delv = vnew - vold;
+  if (!(gt(vnew, vcrit) && gt(magnitude(delv), vt + vt))) return vnew;
+  const bool pos = gt0(vold);
+  const double q = xg::quotient(pos ? delv : vnew, vt, y);
+  const double arg = pos ? 1 + q : q;
+  if (pos && !gt0(arg)) return vcrit;
+  return (pos ? vold : 0.0) + vt * log(arg);
+}
+
+// DeviceSupport::qmeyer (N_DEV_DeviceSupport.C:545-631); the caller exchanges
+// the gate-source and gate-drain sides in reverse mode.
+__device__ __forceinline__ void qmeyer_select(double vgs, double vgd, double von, double vdsat, double &capgs,
+                                              double &capgd, double &capgb, double phi, double cox) {
+  const double vgst = vgs - von;
+  capgs = capgd = 0.0;
+  if (le0(vgst)) {
+    if (le(vgst, -phi)) {
+      capgb = 0.5 * cox;
+    } else {
+      const double c = vgst * cox;
+      capgb = -c / (2 * phi);
+      if (!le(vgst, -0.5 * phi)) capgs = c / (1.5 * phi) + cox / 3;
+    }
+  } else {
+    const double vds = vgs - vgd;
+    capgb = 0;
+    if (le(vdsat, vds)) {
+      capgs = cox / 3;
+    } else {
+      const double vddif = 2.0 * vdsat - vds, vddif1 = vdsat - vds, vddif2 = vddif * vddif;
+      capgd = cox * (1.0 - vdsat * vdsat / vddif2) / 3;
+      capgs = cox * (1.0 - vddif1 * vddif1 / vddif2) / 3;
+    }
+  }
+}
+
+// One junction: conductance and current from its voltage v (sat the
+// saturation current, y the reciprocal of vt).  Without forward bias the
+// exponential is 1, which leaves sat / vt and the current gbv v.
+__device__ __forceinline__ void junction(double v, double sat, double vt, double y, double gmin, double &g, double &c) {
+  const bool fwd = !le0(v);
+  double ev = 1.0;
+  if (fwd) {
+    const double q = xg::quotient(v, vt, y);
+    ev = exp(lt(kMaxExpArg, q) ? kMaxExpArg : q);
+  }
+  g = xg::quotient(sat * ev, vt, y) + gmin;
+  const double cv = (fwd ? gmin : g) * v;
+  c = fwd ? sat * (ev - 1) + gmin * v : cv;
+}
+
 __global__ void __launch_bounds__(128) mos1_kernel(DevType t, DevOptions o, Flags f, LoadIO io) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= t.n || !instance_flags(t, i, f)) return;
@@ -384,7 +448,8 @@ __global__ void __launch_bounds__(128) mos1_kernel(DevType t, DevOptions o, Flag
 #define PRM(k) ld(p + (k) * n + i)
   const int li_d = ld(t.lid + i), li_g = ld(t.lid + n + i), li_s = ld(t.lid + 2 * n + i);
   const int li_b = ld(t.lid + 3 * n + i), li_dp = ld(t.lid + 4 * n + i), li_sp = ld(t.lid + 5 * n + i);
-  const int dtype = (int)PRM(XG_M1_DTYPE);
+  // the polarity (+-1) as a sign to flip
+  const int pol = __double2hiint(PRM(XG_M1_DTYPE)) & int(0x80000000);
   const double gamma = PRM(XG_M1_GAMMA);
   const double vt = PRM(XG_M1_VT), tPhi = PRM(XG_M1_TPHI);
   const double gmin = o.gmin;
@@ -399,8 +464,7 @@ __global__ void __launch_bounds__(128) mos1_kernel(DevType t, DevOptions o, Flag
 
   const double Vd = ld(io.sol + li_d), Vg = ld(io.sol + li_g), Vs = ld(io.sol + li_s);
   const double Vb = ld(io.sol + li_b), Vsp = ld(io.sol + li_sp), Vdp = ld(io.sol + li_dp);
-  const double Vddp = Vd - Vdp, Vssp = Vs - Vsp;
-  double vbs = dtype * (Vb - Vsp), vgs = dtype * (Vg - Vsp), vds = dtype * (Vdp - Vsp);
+  double vbs = flip(Vb - Vsp, pol), vgs = flip(Vg - Vsp, pol), vds = flip(Vdp - Vsp, pol);
   double vbd = vbs - vds, vgd = vgs - vds;
   const double vgs_orig = vgs, vds_orig = vds, vbs_orig = vbs, vbd_orig = vbd, vgd_orig = vgd;
 
@@ -408,12 +472,12 @@ __global__ void __launch_bounds__(128) mos1_kernel(DevType t, DevOptions o, Flag
   if (f.init_jct && !OFF && o.voltlim) {
     if (IC_GIVEN) {
       forced = true;
-      vds = dtype * PRM(XG_M1_ICVDS);
-      vgs = dtype * PRM(XG_M1_ICVGS);
-      vbs = dtype * PRM(XG_M1_ICVBS);
+      vds = flip(PRM(XG_M1_ICVDS), pol);
+      vgs = flip(PRM(XG_M1_ICVGS), pol);
+      vbs = flip(PRM(XG_M1_ICVBS), pol);
     } else {
       vbs = -1;
-      vgs = dtype * PRM(XG_M1_TVTO);
+      vgs = flip(PRM(XG_M1_TVTO), pol);
       vds = 0;
     }
     vbd = vbs - vds;
@@ -428,7 +492,7 @@ __global__ void __launch_bounds__(128) mos1_kernel(DevType t, DevOptions o, Flag
     if (!f.dcop) {
       vbs_old = ld(csto + O_VBS); vbd_old = ld(csto + O_VBD);
       vgs_old = ld(csto + O_VGS); vds_old = ld(csto + O_VDS);
-      Von = dtype * ld(csto + O_VON);
+      Von = flip(ld(csto + O_VON), pol);
     } else {
       vbs_old = vbs; vbd_old = vbd; vgs_old = vgs; vds_old = vds;
       Von = 0.0;
@@ -436,105 +500,90 @@ __global__ void __launch_bounds__(128) mos1_kernel(DevType t, DevOptions o, Flag
   } else {
     vbs_old = sto[O_VBS]; vbd_old = sto[O_VBD];
     vgs_old = sto[O_VGS]; vds_old = sto[O_VDS];
-    Von = dtype * sto[O_VON];
+    Von = flip(sto[O_VON], pol);
   }
-  const double vgd_old = vgs_old - vds_old;
+  const double y = 1.0 / vt;
 
   if (o.voltlim && !(f.init_fix && OFF)) {
-    int Check = 1;
-    if (vds_old >= 0) {
-      vgs = fetlim(vgs, vgs_old, Von);
-      vds = vgs - vgd;
-      vds = limvds(vds, vds_old);
-      vgd = vgs - vds;
-    } else {
-      vgd = fetlim(vgd, vgd_old, Von);
-      vds = vgs - vgd;
-      vds = -limvds(-vds, -vds_old);
-      vgs = vgd + vds;
-    }
-    if (vds >= 0.0) {
-      vbs = pnjlim(vbs, vbs_old, vt, PRM(XG_M1_SOURCEVCRIT), &Check);
-      vbd = vbs - vds;
-    } else {
-      vbd = pnjlim(vbd, vbd_old, vt, PRM(XG_M1_DRAINVCRIT), &Check);
-      vbs = vbd + vds;
-    }
+    // forward: vgs is limited, then vds, and vgd follows; reverse: vgd, -vds, vgs
+    const bool fwd = ge0(vds_old);
+    const int rev = fwd ? 0 : int(0x80000000);
+    const double vgd_old = vgs_old - vds_old;
+    const double vg = fetlim_select(fwd ? vgs : vgd, fwd ? vgs_old : vgd_old, Von);
+    vds = (fwd ? vg : vgs) - (fwd ? vgd : vg);
+    vds = flip(limvds_select(flip(vds, rev), flip(vds_old, rev)), rev);
+    const double other = vg + flip(vds, fwd ? int(0x80000000) : 0);
+    vgs = fwd ? vg : other;
+    vgd = fwd ? other : vg;
+    const bool pos = ge0(vds);
+    const double vb = pnjlim_select(pos ? vbs : vbd, pos ? vbs_old : vbd_old, vt, y,
+                                    pos ? PRM(XG_M1_SOURCEVCRIT) : PRM(XG_M1_DRAINVCRIT));
+    vbs = pos ? vb : vb + vds;
   }
   vbd = vbs - vds;
   vgd = vgs - vds;
   const double Vgb = vgs - vbs;
-  const bool origFlag = !(forced || vgs_orig != vgs || vds_orig != vds || vbs_orig != vbs ||
-                          vbd_orig != vbd || vgd_orig != vgd);
+  const bool origFlag = !(forced || ne(vgs_orig, vgs) || ne(vds_orig, vds) || ne(vbs_orig, vbs) ||
+                          ne(vbd_orig, vbd) || ne(vgd_orig, vgd));
 
   double gbs, cbs, gbd, cbd;
-  {
-    const double SourceSatCur = PRM(XG_M1_SOURCESATCUR), DrainSatCur = PRM(XG_M1_DRAINSATCUR);
-    if (vbs <= 0) {
-      gbs = SourceSatCur / vt;
-      gbs += gmin;
-      cbs = gbs * vbs;
-    } else {
-      double evbs = exp(dmin(kMaxExpArg, vbs / vt));
-      gbs = (SourceSatCur * evbs / vt + gmin);
-      cbs = (SourceSatCur * (evbs - 1) + gmin * vbs);
-    }
-    if (vbd <= 0) {
-      gbd = DrainSatCur / vt;
-      gbd += gmin;
-      cbd = gbd * vbd;
-    } else {
-      double evbd = exp(dmin(kMaxExpArg, vbd / vt));
-      gbd = (DrainSatCur * evbd / vt + gmin);
-      cbd = (DrainSatCur * (evbd - 1) + gmin * vbd);
-    }
-  }
-  const int mode = (vds >= 0) ? 1 : -1;
+  junction(vbs, PRM(XG_M1_SOURCESATCUR), vt, y, gmin, gbs, cbs);
+  junction(vbd, PRM(XG_M1_DRAINSATCUR), vt, y, gmin, gbd, cbd);
+  // an infinite or NaN voltage takes every operation, zeros times it included
+  const bool wild = !finite_bits(vbs) || !finite_bits(vgs) || !finite_bits(vds) || !finite_bits(vbs_orig) ||
+                    !finite_bits(vgs_orig) || !finite_bits(vds_orig);
+  const bool fwd = ge0(vds);  // mode
+  const int rev = fwd ? 0 : int(0x80000000);
+  const double vds_m = flip(vds, rev);
   double Vdsat, cdrain, gm, gds, gmbs;
   {
-    const double vbx = mode == 1 ? vbs : vbd;
-    double sarg;
-    if (vbx <= 0) {
-      sarg = sqrt(tPhi - vbx);
-    } else {
-      sarg = sqrt(tPhi);
-      sarg = sarg - vbx / (sarg + sarg);
-      sarg = dmax(0.0, sarg);
-    }
-    Von = (PRM(XG_M1_TVBI) * dtype) + gamma * sarg;
-    double vgst = (mode == 1 ? vgs : vgd) - Von;
-    Vdsat = dmax(vgst, 0.0);
-    double arg = sarg <= 0 ? 0 : gamma / (sarg + sarg);
-    if (vgst <= 0) {
-      cdrain = 0; gm = 0; gds = 0; gmbs = 0;
-    } else {
-      const double lambda = PRM(XG_M1_LAMBDA), Beta = PRM(XG_M1_BETA);
-      double betap = Beta * (1 + lambda * (vds * mode));
-      if (vgst <= (vds * mode)) {
-        cdrain = betap * vgst * vgst * .5;
-        gm = betap * vgst;
-        gds = lambda * Beta * vgst * vgst * .5;
-        gmbs = gm * arg;
-      } else {
-        cdrain = betap * (vds * mode) * (vgst - .5 * (vds * mode));
-        gm = betap * (vds * mode);
-        gds = betap * (vgst - (vds * mode)) + lambda * Beta * (vds * mode) * (vgst - .5 * (vds * mode));
-        gmbs = gm * arg;
+    const double vbx = fwd ? vbs : vbd;
+    const double tVbi = flip(PRM(XG_M1_TVBI), pol);
+    double arg = 0.0;
+    Von = tVbi;
+    if (wild || ne0(gamma)) {
+      const bool neg = le0(vbx);
+      double sarg = sqrt(neg ? tPhi - vbx : tPhi);
+      if (!neg) {
+        sarg = sarg - vbx / (sarg + sarg);
+        sarg = lt0(sarg) ? 0.0 : sarg;
       }
+      Von = tVbi + gamma * sarg;
+      arg = le0(sarg) ? 0 : gamma / (sarg + sarg);
+    }
+    const double vgst = (fwd ? vgs : vgd) - Von;
+    Vdsat = gt0(vgst) ? vgst : 0.0;
+    const bool off = le0(vgst), sat = le(vgst, vds_m);
+    const double lambda = PRM(XG_M1_LAMBDA), Beta = PRM(XG_M1_BETA);
+    // with w = vgst in saturation, vds below it: gm = betap w, the current
+    // gm (vgst - w/2), gds = betap (vgst - w) + lambda Beta w (vgst - w/2)
+    const double w = sat ? vgst : vds_m;
+    const double z = fma(-0.5, w, vgst);  // (exact product)
+    double betap = Beta, lb = 0.0;
+    if (wild || ne0(lambda)) {
+      betap = Beta * (1 + lambda * vds_m);
+      lb = lambda * Beta;
+    }
+    gm = betap * w;
+    cdrain = gm * z;
+    gds = sat ? 0.0 : betap * (vgst - w);
+    if (wild || ne0(lambda)) gds += lb * w * z;
+    gmbs = wild || ne0(arg) ? gm * arg : 0.0;
+    if (off) {
+      cdrain = 0; gm = 0; gds = 0; gmbs = 0;
     }
   }
-  const double von = dtype * Von;
 
   double qbs = 0, capbs = 0, qbd = 0, capbd = 0;
   {
     const double Cbs = PRM(XG_M1_CBS), Cbssw = PRM(XG_M1_CBSSW);
     const double Cbd = PRM(XG_M1_CBD), Cbdsw = PRM(XG_M1_CBDSW);
-    if (Cbs != 0 || Cbssw != 0 || Cbd != 0 || Cbdsw != 0) {
+    if (ne0(Cbs) || ne0(Cbssw) || ne0(Cbd) || ne0(Cbdsw)) {
       const double MJ = PRM(XG_M1_MJ), MJSW = PRM(XG_M1_MJSW);
       const double tDepCap = PRM(XG_M1_TDEPCAP), tBulkPot = PRM(XG_M1_TBULKPOT);
       double sarg, sargsw, arg;
-      if (Cbs != 0 || Cbssw != 0) {
-        if (vbs < tDepCap) {
+      if (ne0(Cbs) || ne0(Cbssw)) {
+        if (lt(vbs, tDepCap)) {
           arg = 1 - vbs / tBulkPot;
           if (MJ == MJSW) {
             sarg = sargsw = (MJ == .5) ? 1 / sqrt(arg) : exp(-MJ * log(arg));
@@ -550,8 +599,8 @@ __global__ void __launch_bounds__(128) mos1_kernel(DevType t, DevOptions o, Flag
           capbs = f2s + f3s * vbs;
         }
       }
-      if (Cbd != 0 || Cbdsw != 0) {
-        if (vbd < tDepCap) {
+      if (ne0(Cbd) || ne0(Cbdsw)) {
+        if (lt(vbd, tDepCap)) {
           arg = 1 - vbd / tBulkPot;
           if (MJ == .5 && MJSW == .5) {
             sarg = sargsw = 1 / sqrt(arg);
@@ -570,10 +619,14 @@ __global__ void __launch_bounds__(128) mos1_kernel(DevType t, DevOptions o, Flag
     }
   }
 
-  double capgs, capgd, capgb;
+  double capgs = 0.0, capgd = 0.0, capgb = 0.0;
   const double OxideCap = PRM(XG_M1_OXIDECAP);
-  if (mode > 0) qmeyer(vgs, vgd, Von, Vdsat, capgs, capgd, capgb, tPhi, OxideCap);
-  else qmeyer(vgd, vgs, Von, Vdsat, capgd, capgs, capgb, tPhi, OxideCap);
+  if (wild || ne0(OxideCap)) {
+    double c1, c2;
+    qmeyer_select(fwd ? vgs : vgd, fwd ? vgd : vgs, Von, Vdsat, c1, c2, capgb, tPhi, OxideCap);
+    capgs = fwd ? c1 : c2;
+    capgd = fwd ? c2 : c1;
+  }
 
   double Capgs, Capgd, Capgb;
   {
@@ -587,22 +640,20 @@ __global__ void __launch_bounds__(128) mos1_kernel(DevType t, DevOptions o, Flag
       Capgd = (capgd + ld(csta + S_CAPGD) + cgdo);
       Capgb = (capgb + ld(csta + S_CAPGB) + cgbo);
     }
-    Capgs *= (Capgs < 0.0) ? -1.0 : 1.0;
-    Capgd *= (Capgd < 0.0) ? -1.0 : 1.0;
-    Capgb *= (Capgb < 0.0) ? -1.0 : 1.0;
+    Capgs = magnitude(Capgs);
+    Capgd = magnitude(Capgd);
+    Capgb = magnitude(Capgb);
   }
   const double drainConductance = PRM(XG_M1_GD), sourceConductance = PRM(XG_M1_GS);
-  const double Idrain = drainConductance * Vddp;
-  const double Isource = sourceConductance * Vssp;
-  double Gm, Gmbs, nrmsum, revsum, cdreq;
-  if (mode >= 0) {
-    Gm = gm; Gmbs = gmbs; nrmsum = Gm + Gmbs; revsum = 0; cdreq = dtype * cdrain;
-  } else {
-    Gm = -gm; Gmbs = -gmbs; nrmsum = 0; revsum = -(Gm + Gmbs); cdreq = -(dtype)*cdrain;
-  }
+  const double Idrain = wild || ne0(drainConductance) ? drainConductance * (Vd - Vdp) : 0.0;
+  const double Isource = wild || ne0(sourceConductance) ? sourceConductance * (Vs - Vsp) : 0.0;
+  const double Gm = flip(gm, rev), Gmbs = flip(gmbs, rev);
+  const double gsum = ne0(gmbs) ? Gm + Gmbs : Gm;
+  const double nrmsum = fwd ? gsum : 0.0, revsum = fwd ? 0.0 : -gsum;
+  const double cdreq = flip(cdrain, pol ^ rev);
 
   // Master::updateState store / state writes
-  sto[O_VBD] = vbd; sto[O_VBS] = vbs; sto[O_VGS] = vgs; sto[O_VDS] = vds; sto[O_VON] = von;
+  sto[O_VBD] = vbd; sto[O_VBS] = vbs; sto[O_VGS] = vgs; sto[O_VDS] = vds; sto[O_VON] = flip(Von, pol);
   sta[S_CAPGS] = capgs; sta[S_CAPGD] = capgd; sta[S_CAPGB] = capgb;
   double qgs, qgd, qgb;
   if (f.dcop) {
@@ -610,83 +661,101 @@ __global__ void __launch_bounds__(128) mos1_kernel(DevType t, DevOptions o, Flag
   } else {
     qgs = ld(csta + S_QGS); qgd = ld(csta + S_QGD); qgb = ld(csta + S_QGB);
     double vgs1 = ld(csto + O_VGS), vbs1 = ld(csto + O_VBS), vds1 = ld(csto + O_VDS);
-    double vgb1 = vgs1 - vbs1, vgd1 = vgs1 - vds1;
-    qgs += Capgs * (vgs - vgs1);
-    qgd += Capgd * (vgd - vgd1);
-    qgb += Capgb * ((vgs - vbs) - vgb1);
+    if (wild || ne0(Capgs) || ne0(Capgd) || ne0(Capgb) || !finite_bits(vgs1) || !finite_bits(vbs1) ||
+        !finite_bits(vds1)) {
+      double vgb1 = vgs1 - vbs1, vgd1 = vgs1 - vds1;
+      qgs += Capgs * (vgs - vgs1);
+      qgd += Capgd * (vgd - vgd1);
+      qgb += Capgb * (Vgb - vgb1);
+    }
   }
   sta[S_QGS] = qgs; sta[S_QGD] = qgd; sta[S_QGB] = qgb; sta[S_QBD] = qbd; sta[S_QBS] = qbs;
 
-  // Master::loadDAEVectors
+  // Master::loadDAEVectors and loadDAEMatrices (pointer path; `-=` stored as
+  // the negated term), each value times M
   const double numberParallel = PRM(XG_M1_M);
 #undef PRM
   Terms T{io.terms + t.term0, n};
-  const double ceqbs = dtype * (cbs), ceqbd = dtype * (cbd);
-  const double ceqgb = 0.0, ceqgs = 0.0, ceqgd = 0.0;
-  T.put(0, i, drainConductance != 0.0 ? Idrain * numberParallel : 0.0);
-  T.put(1, i, (ceqgs + ceqgd + ceqgb) * numberParallel);
-  T.put(2, i, sourceConductance != 0.0 ? Isource * numberParallel : 0.0);
-  T.put(3, i, (ceqbs + ceqbd - ceqgb) * numberParallel);
-  T.put(4, i, (-Idrain - (ceqbd - cdreq + ceqgd)) * numberParallel);
-  T.put(5, i, (-Isource - (ceqbs + cdreq + ceqgs)) * numberParallel);
-  const double Qeqbs = dtype * (qbs), Qeqbd = dtype * (qbd), Qeqgb = dtype * (qgb);
-  const double Qeqgs = dtype * (qgs), Qeqgd = dtype * (qgd);
-  T.put(6, i, (Qeqgs + Qeqgd + Qeqgb) * numberParallel);
-  T.put(7, i, (Qeqbs + Qeqbd - Qeqgb) * numberParallel);
-  T.put(8, i, (-(Qeqbd + Qeqgd)) * numberParallel);
-  T.put(9, i, (-(Qeqbs + Qeqgs)) * numberParallel);
   const bool cap_on = f.tranop || f.acop || f.transient;
   const double gcgd = cap_on ? Capgd : 0.0, gcgs = cap_on ? Capgs : 0.0, gcgb = cap_on ? Capgb : 0.0;
   const double gcbs = cap_on ? capbs : 0.0, gcbd = cap_on ? capbd : 0.0;
-  if (!origFlag) {
-    const double dvgs = vgs - vgs_orig, dvgd = vgd - vgd_orig, dvbs = vbs - vbs_orig;
-    const double dvbd = vbd - vbd_orig, dvds = vds - vds_orig;
-    const double dvg = (mode > 0) ? dvgs : dvgd, dvb = (mode > 0) ? dvbs : dvbd;
-    T.put(10, i, (dtype * (+((gbd - gmin)) * (dvbd) + ((gbs - gmin)) * (dvbs))) * numberParallel);
-    T.put(11, i, (dtype * (-((gbd - gmin)) * (dvbd) + gds * (dvds) + Gm * dvg + Gmbs * dvb)) * numberParallel);
-    T.put(12, i, (dtype * (-((gbs - gmin)) * (dvbs) - gds * (dvds) - Gm * dvg - Gmbs * dvb)) * numberParallel);
-    const double dvgsb = vgs - vgs_orig - vbs + vbs_orig;
-    T.put(13, i, (dtype * (gcgd * (dvgd) + gcgs * (dvgs) + gcgb * dvgsb)) * numberParallel);
-    T.put(14, i, (dtype * (-(gcgb)*dvgsb + (gcgb) * (dvbd) + (gcbs) * (dvbs))) * numberParallel);
-    T.put(15, i, (dtype * (-(gcgd) * (dvgd) - (gcbd) * (dvbd))) * numberParallel);
-    T.put(16, i, (dtype * (-gcgs * (dvgs) - (gcbs) * (dvbs))) * numberParallel);
-  } else {
+  const bool caps = wild || ne0(gcgd) || ne0(gcgs) || ne0(gcgb) || ne0(gcbs) || ne0(gcbd);
+  auto stamp = [&](auto times) {
+    auto put = [&](int q, double v) { T.put(q, i, times(v)); };
+    auto both = [&](int q, int r, double v) {  // v and -v
+      const double a = times(v);
+      T.put(q, i, a);
+      T.put(r, i, -a);
+    };
+    const double ceqbs = flip(cbs, pol), ceqbd = flip(cbd, pol);
+    put(0, ne0(drainConductance) ? Idrain : 0.0);
+    put(1, 0.0);
+    put(2, ne0(sourceConductance) ? Isource : 0.0);
+    put(3, ceqbs + ceqbd);
+    put(4, -Idrain - (ceqbd - cdreq));
+    put(5, -Isource - (ceqbs + cdreq));
+    put(6, flip(qgs + qgd + qgb, pol));
+    put(7, flip(qbs + qbd - qgb, pol));
+    put(8, -flip(qbd + qgd, pol));
+    put(9, -flip(qbs + qgs, pol));
+    if (!origFlag) {
+      const double dvgs = vgs - vgs_orig, dvgd = vgd - vgd_orig, dvbs = vbs - vbs_orig;
+      const double dvbd = vbd - vbd_orig, dvds = vds - vds_orig;
+      const double dvg = fwd ? dvgs : dvgd, dvb = fwd ? dvbs : dvbd;
+      const double jd = (gbd - gmin) * dvbd, js = (gbs - gmin) * dvbs;
+      put(10, flip(jd + js, pol));
+      put(11, flip(-jd + gds * dvds + Gm * dvg + Gmbs * dvb, pol));
+      put(12, flip(-js - gds * dvds - Gm * dvg - Gmbs * dvb, pol));
+      if (!caps) {
 #pragma unroll
-    for (int q = 10; q <= 16; ++q) T.put(q, i, 0.0);
-  }
-  // Master::loadDAEMatrices (pointer path); `-=` stored as the negated term.
-  const double M = numberParallel;
-  T.put(17, i, drainConductance * M);
-  T.put(18, i, -(drainConductance * M));
-  T.put(19, i, sourceConductance * M);
-  T.put(20, i, -(sourceConductance * M));
-  T.put(21, i, (gbs + gbd) * M);
-  T.put(22, i, -(gbd * M));
-  T.put(23, i, -(gbs * M));
-  T.put(24, i, -(drainConductance * M));
-  T.put(25, i, (Gm)*M);
-  T.put(26, i, (-gbd + Gmbs) * M);
-  T.put(27, i, (drainConductance + gds + gbd + revsum) * M);
-  T.put(28, i, (-gds - nrmsum) * M);
-  T.put(29, i, -((Gm)*M));
-  T.put(30, i, -(sourceConductance * M));
-  T.put(31, i, -((gbs + Gmbs) * M));
-  T.put(32, i, -((gds + revsum) * M));
-  T.put(33, i, (sourceConductance + gds + gbs + nrmsum) * M);
-  T.put(34, i, (gcgd + gcgs + gcgb) * M);
-  T.put(35, i, -(gcgb * M));
-  T.put(36, i, -(gcgd * M));
-  T.put(37, i, -(gcgs * M));
-  T.put(38, i, -(gcgb * M));
-  T.put(39, i, (+gcbs + gcbd + gcgb) * M);
-  T.put(40, i, -(+gcbd * M));
-  T.put(41, i, -(+gcbs * M));
-  T.put(42, i, -gcgd * M);
-  T.put(43, i, -gcbd * M);
-  T.put(44, i, (+gcbd + gcgd) * M);
-  T.put(45, i, -(gcgs * M));
-  T.put(46, i, -(+gcbs * M));
-  T.put(47, i, (+gcbs + gcgs) * M);
+        for (int q = 13; q <= 16; ++q) T.put(q, i, 0.0);
+      } else {
+        const double dvgsb = vgs - vgs_orig - vbs + vbs_orig;
+        put(13, flip(gcgd * dvgd + gcgs * dvgs + gcgb * dvgsb, pol));
+        put(14, flip(-gcgb * dvgsb + gcgb * dvbd + gcbs * dvbs, pol));
+        put(15, flip(-gcgd * dvgd - gcbd * dvbd, pol));
+        put(16, flip(-gcgs * dvgs - gcbs * dvbs, pol));
+      }
+    } else {
+#pragma unroll
+      for (int q = 10; q <= 16; ++q) T.put(q, i, 0.0);
+    }
+    both(17, 18, drainConductance);
+    both(19, 20, sourceConductance);
+    put(21, gbs + gbd);
+    put(22, -gbd);
+    put(23, -gbs);
+    put(24, -drainConductance);
+    both(25, 29, Gm);
+    put(26, -gbd + Gmbs);
+    put(27, drainConductance + gds + gbd + revsum);
+    put(28, -gds - nrmsum);
+    put(30, -sourceConductance);
+    put(31, -(gbs + Gmbs));
+    put(32, -(gds + revsum));
+    put(33, sourceConductance + gds + gbs + nrmsum);
+    if (!caps) {
+#pragma unroll
+      for (int q = 34; q <= 47; ++q) T.put(q, i, 0.0);
+      return;
+    }
+    put(34, gcgd + gcgs + gcgb);
+    put(35, -gcgb);
+    put(36, -gcgd);
+    put(37, -gcgs);
+    put(38, -gcgb);
+    put(39, gcbs + gcbd + gcgb);
+    put(40, -gcbd);
+    put(41, -gcbs);
+    put(42, -gcgd);
+    put(43, -gcbd);
+    put(44, gcbd + gcgd);
+    put(45, -gcgs);
+    put(46, -gcbs);
+    put(47, gcbs + gcgs);
+  };
+  if (numberParallel == 1.0) stamp([](double v) { return v; });
+  else stamp([&](double v) { return v * numberParallel; });
 }
 
 #include "bsim3_eval.cuh"

@@ -1,0 +1,69 @@
+// xg_dcmp.cuh — FP64 tests, signs and shared-divisor quotients that spare the
+// FP64 pipe.
+//
+// GB300 issues an FP64 instruction to a sub-partition in 66 cycles however
+// few lanes need it, a comparison (DSETP) included; the integer pipe takes
+// one or two.  The comparisons of device models are therefore made on the
+// bits, with IEEE's results for every operand (signed zeros equal, NaN
+// unordered), and multiplication by a polarity of +-1 is a sign flip.
+#pragma once
+
+namespace xg {
+
+__device__ __forceinline__ unsigned long long dbits(double x) { return (unsigned long long)__double_as_longlong(x); }
+constexpr unsigned long long kInfBits = 0x7ff0000000000000ull;
+constexpr unsigned long long kSignBit = 0x8000000000000000ull;
+
+// x > 0, x >= 0, x < 0, x <= 0, x == 0, x != 0 (true for NaN), finite
+__device__ __forceinline__ bool gt0(double x) { return dbits(x) - 1ull < kInfBits; }
+__device__ __forceinline__ bool lt0(double x) { return (dbits(x) ^ kSignBit) - 1ull < kInfBits; }
+__device__ __forceinline__ bool ge0(double x) { return dbits(x) <= kInfBits || dbits(x) == kSignBit; }
+__device__ __forceinline__ bool le0(double x) { return (dbits(x) ^ kSignBit) <= kInfBits || dbits(x) == 0ull; }
+__device__ __forceinline__ bool ne0(double x) { return (dbits(x) << 1) != 0ull; }
+__device__ __forceinline__ bool finite_bits(double x) { return ((unsigned(__double2hiint(x)) >> 20) & 0x7ffu) != 0x7ffu; }
+
+// The magnitude with its sign as a two's-complement number: ordered as the
+// doubles are, both zeros 0, NaN outside +-kInfBits.
+__device__ __forceinline__ long long dkey(double x) {
+  const long long v = __double_as_longlong(x), m = v >> 63;
+  return (v ^ (m & 0x7fffffffffffffffll)) - m;
+}
+__device__ __forceinline__ bool lt(double a, double b) {
+  const long long x = dkey(a), y = dkey(b);
+  return x < y && x >= -(long long)kInfBits && y <= (long long)kInfBits;
+}
+__device__ __forceinline__ bool le(double a, double b) {
+  const long long x = dkey(a), y = dkey(b);
+  return x <= y && x >= -(long long)kInfBits && y <= (long long)kInfBits;
+}
+__device__ __forceinline__ bool gt(double a, double b) { return lt(b, a); }
+__device__ __forceinline__ bool ge(double a, double b) { return le(b, a); }
+// a != b (true for NaN)
+__device__ __forceinline__ bool ne(double a, double b) {
+  const long long x = dkey(a);
+  return x != dkey(b) || x > (long long)kInfBits || x < -(long long)kInfBits;
+}
+
+// x or -x by a mask of 0 or kSignBit's high word
+__device__ __forceinline__ double flip(double x, int sign) {
+  return __hiloint2double(__double2hiint(x) ^ sign, __double2loint(x));
+}
+__device__ __forceinline__ double magnitude(double x) {
+  return __hiloint2double(__double2hiint(x) & 0x7fffffff, __double2loint(x));
+}
+
+// a / b from y, the correctly rounded reciprocal of b: the quotient a y and
+// one correction by its remainder, which gives IEEE's rounding (P. Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000
+// processor", IBM J. Res. Dev. 34(1), 1990): three FP64 instructions where
+// the division takes at least six.  Quotients near the ends of the exponent
+// range (zero, subnormal, infinite and NaN among them) are divided.
+__device__ __forceinline__ double quotient(double a, double b, double y) {
+  double q = a * y;
+  const unsigned e = (unsigned(__double2hiint(q)) >> 20) & 0x7ffu;
+  if (e - 128u > 1791u) return a / b;
+  const double r = fma(-b, q, a);
+  return fma(r, y, q);
+}
+
+}  // namespace xg
