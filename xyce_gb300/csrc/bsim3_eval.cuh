@@ -14,6 +14,14 @@
 // charge-partition derivatives, all zero for nqsMod = 0) are left out: adding
 // +-0 never changes a sum's value.
 //
+// Bound by FP64 issue (81-85% of the pipe's cycles): comparisons are made on
+// the bits, polarity is a sign flip and the limiting evaluates one alternative
+// (xg_dcmp.cuh and the level-1 kernel's helpers), quotients share reciprocals
+// and square roots come with theirs.  On 300,000 devices a warp issues 1,724
+// FP64 instructions in the FMA build (2,002 with the model's branches and
+// comparisons as they stand) and 2,523 in the exact build (3,339): 1.185 ->
+// 1.043 ms and 1.92 -> 1.47 ms.
+//
 // Members the reference refreshes only when charges are computed (CAP*
 // capacitances, Qeqq*_Jdxp limiter charges, qg/qb/qd/qbs/qbd) live in a
 // device array carried from one load to the next, laid out [k*n + i].
@@ -28,34 +36,41 @@ constexpr double KQ = 1.6021918e-19;            // CONSTQ
 constexpr double KBOLTZ = 1.3806226e-23;        // CONSTboltz
 constexpr double CTOK = 273.15;                 // CONSTCtoK
 
-// Quotients.  The bit-exact build divides wherever the reference divides.
-// The FMA build (XG_FAST_DIV) multiplies by reciprocals instead: formed once
-// where several quotients share a denominator, read from the parameter block
-// where it is an instance constant, and otherwise taken by Newton-Raphson
-// from the hardware's approximation (xg::fast_rcp, four fused multiply-adds
-// against IEEE division's longer sequence); each quotient lands within ~1-2
-// ulp, inside the tolerance that build is held to.  A literal divisor
-// becomes a multiply by its reciprocal, folded at compile time.
-//   B3_RCOL(name, k)   declares a reciprocal read from parameter column k
-//   B3_RCP(name, x)    declares the reciprocal of x (FMA build only)
-//   B3_DIV(a, b, rb)   a / b, or a * rb
-//   B3_Q(a, b)         a / b, or a * fast_rcp(b)
-//   B3_DIVK(a, k)      a / k for a literal k, or a * (1 / k)
-//   B3_RSQRT(x)        1 / sqrt(x), or CUDA's rsqrt (within 1 ulp)
-#if XG_FAST_DIV
+// Quotients.  Where several share a denominator its reciprocal is formed once
+// (or read from the parameter block where it is an instance constant).  The
+// bit-exact build corrects a product with it to IEEE's quotient
+// (xg::quotient: three FP64 instructions for the 8.6 a division takes); the
+// FMA build takes the product, and reciprocals by xg::fast_rcp: each quotient
+// lands within ~1-2 ulp, inside the tolerance that build is held to.  A
+// literal divisor becomes a multiply by its reciprocal there, folded at
+// compile time.
+//   B3_RCOL(name, k)     declares a reciprocal read from parameter column k
+//   B3_RCP(name, x)      declares the reciprocal of x; B3_RCPX(x) is it
+//   B3_SQRTX(x, &r)      sqrt(x), its reciprocal in r
+//   B3_DIV(a, b, rb)     a / b
+//   B3_DIVP(a, b, rb)    a / b, rb a product of reciprocals (FMA build only)
+//   B3_Q(a, b)           a / b, or a * fast_rcp(b)
+//   B3_DIVK(a, k)        a / k for a literal k, or a * (1 / k)
+//   B3_RSQRT(x)          1 / sqrt(x), or CUDA's rsqrt (within 1 ulp)
 #define B3_RCOL(name, k) const double name = PRM(k)
+#if XG_FAST_DIV
 #define B3_RCP(name, x) const double name = xg::fast_rcp(x)
 #define B3_DIV(a, b, rb) ((a) * (rb))
+#define B3_DIVP(a, b, rb) ((a) * (rb))
 #define B3_Q(a, b) ((a) * xg::fast_rcp(b))
 #define B3_DIVK(a, k) ((a) * (1.0 / (k)))
 #define B3_RSQRT(x) rsqrt(x)
+#define B3_RCPX(x) xg::fast_rcp(x)
+#define B3_SQRTX(x, r) xg::fast_sqrt(x, r)
 #else
-#define B3_RCOL(name, k) (void)0
-#define B3_RCP(name, x) (void)0
-#define B3_DIV(a, b, rb) ((a) / (b))
+#define B3_RCP(name, x) const double name = 1.0 / (x)
+#define B3_DIV(a, b, rb) xg::quotient(a, b, rb)
+#define B3_DIVP(a, b, rb) ((a) / (b))
 #define B3_Q(a, b) ((a) / (b))
 #define B3_DIVK(a, k) ((a) / (k))
 #define B3_RSQRT(x) (1.0 / sqrt(x))
+#define B3_RCPX(x) (1.0 / (x))
+#define B3_SQRTX(x, r) xg::exact_sqrt(x, r)
 #endif
 
 enum B3Mem {
@@ -75,19 +90,20 @@ struct B3Local {
 
 __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Flags f, LoadIO io) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= t.n || !instance_flags(t, i, f)) return;
+  if (ge(i, t.n) || !instance_flags(t, i, f)) return;
   const int nI = t.n;  // instances ("n" is the subthreshold swing below)
   const double *__restrict__ p = t.p;
 #define PRM(k) __ldg(p + (int64_t)(k) * nI + i)
   const int li_Drain = __ldg(t.lid + i), li_Gate = __ldg(t.lid + nI + i);
   const int li_Source = __ldg(t.lid + 2 * nI + i), li_Bulk = __ldg(t.lid + 3 * nI + i);
   const int li_DrainPrime = __ldg(t.lid + 4 * nI + i), li_SourcePrime = __ldg(t.lid + 5 * nI + i);
-  const int dtype = (int)PRM(XG_B3_DTYPE);
-  const int mobMod = (int)PRM(XG_B3_MOBMOD), capMod = (int)PRM(XG_B3_CAPMOD);
+  // the polarity (+-1) as a sign to flip
+  const int pol = __double2hiint(PRM(XG_B3_DTYPE)) & int(0x80000000);
+  const int mobMod = small_int(PRM(XG_B3_MOBMOD)), capMod = small_int(PRM(XG_B3_CAPMOD));
   const double xpart = PRM(XG_B3_XPART), tox = PRM(XG_B3_TOX), cox = PRM(XG_B3_COX);
   const double factor1 = PRM(XG_B3_FACTOR1);
   const double gmin = o.gmin;
-  const int OFF = ((int)PRM(XG_B3_FLAGS)) & 1;
+  const int OFF = small_int(PRM(XG_B3_FLAGS)) & 1;
   double *sto = io.sto + t.sto0 + (int64_t)i * 5;
   double *sta = io.sta + t.sta0 + (int64_t)i * 12;
   const double *csto = io.sto_curr + t.sto0 + (int64_t)i * 5;
@@ -149,7 +165,6 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
   double Cgg, Cgd, Cgb, Cbg, Cbd, Cbb, Csg, Csd, Csb, CoxWL, qinv;
   double qgdo, qgso, cgdo, cgso, capbs, capbd, qbs, qbd, gbs, gbd, cbs, cbd;
   (void)qinv;
-  int Check = 1;
   int ChargeComputationNeeded = (f.tranop || f.acop || f.transient) ? 1 : 0;
   int mode;
 
@@ -158,7 +173,7 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
   double Vsp = sol[li_SourcePrime], Vdp = sol[li_DrainPrime];
   double Vddp = Vd - Vdp, Vssp = Vs - Vsp, Vbsp = Vb - Vsp, Vgsp = Vg - Vsp;
   double Vdpsp = Vdp - Vsp;
-  double vbs = dtype * Vbsp, vgs = dtype * Vgsp, vds = dtype * Vdpsp;
+  double vbs = flip(Vbsp, pol), vgs = flip(Vgsp, pol), vds = flip(Vdpsp, pol);
   double vbd = vbs - vds, vgd = vgs - vds, vgb;
   int origFlag = 1;
   const double vgs_orig = vgs, vds_orig = vds, vbs_orig = vbs, vbd_orig = vbd, vgd_orig = vgd;
@@ -166,7 +181,7 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
   if (f.init_jct && !OFF && o.voltlim) {
     /* inputOP with an all-zero flag vector takes the same branch */
     vbs = 0.0;
-    vgs = dtype * PRM(XG_B3_VTH0) + 0.1;
+    vgs = flip(PRM(XG_B3_VTH0), pol) + 0.1;
     vds = 0.1;
     origFlag = 0;
     vbd = vbs - vds;
@@ -190,26 +205,21 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
     const double vt0 = KBOLTZ * (27.0 + CTOK) / KQ;
     const double vcrit = PRM(XG_B3_VCRIT);
     if (f.newton_iter >= 0) {
-      if (vds_old >= 0.0) {
-        vgs = fetlim(vgs, vgs_old, von_local);
-        vds = vgs - vgd;
-        vds = limvds(vds, vds_old);
-        vgd = vgs - vds;
-      } else {
-        vgd = fetlim(vgd, vgdo, von_local);
-        vds = vgs - vgd;
-        vds = -limvds(-vds, -vds_old);
-        vgs = vgd + vds;
-      }
-      if (vds >= 0.0) {
-        vbs = pnjlim(vbs, vbs_old, vt0, vcrit, &Check);
-        vbd = vbs - vds;
-      } else {
-        vbd = pnjlim(vbd, vbd_old, vt0, vcrit, &Check);
-        vbs = vbd + vds;
-      }
+      // forward: vgs is limited, then vds, and vgd follows; reverse: vgd, -vds, vgs
+      const bool fwd = ge0(vds_old);
+      const int rev = fwd ? 0 : int(0x80000000);
+      const double vg = fetlim_select(fwd ? vgs : vgd, fwd ? vgs_old : vgdo, von_local);
+      vds = (fwd ? vg : vgs) - (fwd ? vgd : vg);
+      vds = flip(limvds_select(flip(vds, rev), flip(vds_old, rev)), rev);
+      const double other = vg + flip(vds, fwd ? int(0x80000000) : 0);
+      vgs = fwd ? vg : other;
+      vgd = fwd ? other : vg;
+      const bool pos = ge0(vds);
+      const double vb = pnjlim_select(pos ? vbs : vbd, pos ? vbs_old : vbd_old, vt0, 1.0 / vt0, vcrit);
+      vbs = pos ? vb : vb + vds;
+      vbd = pos ? vbs - vds : vb;
     }
-    if (vgs_orig != vgs || vds_orig != vds || vbs_orig != vbs || vbd_orig != vbd || vgd_orig != vgd)
+    if (ne(vgs_orig, vgs) || ne(vds_orig, vds) || ne(vbs_orig, vbs) || ne(vbd_orig, vbd) || ne(vgd_orig, vgd))
       origFlag = 0;
   }
   vbd = vbs - vds;
@@ -222,14 +232,14 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
   const double ijth = PRM(XG_B3_IJTH);
   // area * Js + perimeter * Jsw, or 1e-14 with neither (set-up, :4475-4511)
   SourceSatCurrent = PRM(XG_B3_SSAT);
-  if (SourceSatCurrent <= 0.0) {
+  if (le0(SourceSatCurrent)) {
     gbs = gmin;
     cbs = gbs * vbs;
-  } else if (ijth == 0.0) {
+  } else if (eq0(ijth)) {
     evbs = exp(B3_DIV(vbs, Nvtm, rNvtm));
     gbs = B3_DIV(SourceSatCurrent * evbs, Nvtm, rNvtm) + gmin;
     cbs = SourceSatCurrent * (evbs - 1.0) + gmin * vbs;
-  } else if (vbs < PRM(XG_B3_VJSM)) {
+  } else if (lt(vbs, PRM(XG_B3_VJSM))) {
     evbs = exp(B3_DIV(vbs, Nvtm, rNvtm));
     gbs = B3_DIV(SourceSatCurrent * evbs, Nvtm, rNvtm) + gmin;
     cbs = SourceSatCurrent * (evbs - 1.0) + gmin * vbs;
@@ -239,14 +249,14 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
     cbs = PRM(XG_B3_ISEVJSM) - SourceSatCurrent + T0 * (vbs - PRM(XG_B3_VJSM)) + gmin * vbs;
   }
   DrainSatCurrent = PRM(XG_B3_DSAT);
-  if (DrainSatCurrent <= 0.0) {
+  if (le0(DrainSatCurrent)) {
     gbd = gmin;
     cbd = gbd * vbd;
-  } else if (ijth == 0.0) {
+  } else if (eq0(ijth)) {
     evbd = exp(B3_DIV(vbd, Nvtm, rNvtm));
     gbd = B3_DIV(DrainSatCurrent * evbd, Nvtm, rNvtm) + gmin;
     cbd = DrainSatCurrent * (evbd - 1.0) + gmin * vbd;
-  } else if (vbd < PRM(XG_B3_VJDM)) {
+  } else if (lt(vbd, PRM(XG_B3_VJDM))) {
     evbd = exp(B3_DIV(vbd, Nvtm, rNvtm));
     gbd = B3_DIV(DrainSatCurrent * evbd, Nvtm, rNvtm) + gmin;
     cbd = DrainSatCurrent * (evbd - 1.0) + gmin * vbd;
@@ -256,7 +266,7 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
     cbd = PRM(XG_B3_ISEVJDM) - DrainSatCurrent + T0 * (vbd - PRM(XG_B3_VJDM)) + gmin * vbd;
   }
 
-  if (vds >= 0.0) {
+  if (ge0(vds)) {
     mode = 1; Vds = vds; Vgs = vgs; Vbs = vbs;
   } else {
     mode = -1; Vds = -vds; Vgs = vgd; Vbs = vbd;
@@ -267,32 +277,35 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
   B3_RCOL(rPhis3, XG_B3_R_PHIS3);
   B3_RCOL(rSqrtPhi, XG_B3_R_SQRTPHI);
   T0 = Vbs - vbsc - 0.001;
-  double T1global = sqrt(T0 * T0 - 0.004 * vbsc);
+  double rT1global;
+  const double T1global = B3_SQRTX(T0 * T0 - 0.004 * vbsc, &rT1global);
   Vbseff = vbsc + 0.5 * (T0 + T1global);
-  dVbseff_dVb = 0.5 * (1.0 + B3_Q(T0, T1global));
-  if (Vbseff < Vbs) Vbseff = Vbs;
-  if (Vbseff > 0.0) {
+  dVbseff_dVb = 0.5 * (1.0 + B3_DIV(T0, T1global, rT1global));
+  if (lt(Vbseff, Vbs)) Vbseff = Vbs;
+  double rSqrtPhis;
+  if (gt0(Vbseff)) {
     T0 = B3_Q(phi, (phi + Vbseff));
     Phis = phi * T0;
     dPhis_dVb = -T0 * T0;
     sqrtPhis = B3_Q(phis3, (phi + 0.5 * Vbseff));
+    rSqrtPhis = B3_RCPX(sqrtPhis);
     dsqrtPhis_dVb = B3_DIV(-0.5 * sqrtPhis * sqrtPhis, phis3, rPhis3);
   } else {
     Phis = phi - Vbseff;
     dPhis_dVb = -1.0;
-    sqrtPhis = sqrt(Phis);
-    dsqrtPhis_dVb = B3_Q(-0.5, sqrtPhis);
+    sqrtPhis = B3_SQRTX(Phis, &rSqrtPhis);
+    dsqrtPhis_dVb = -0.5 * rSqrtPhis;
   }
   Xdep = B3_DIV(Xdep0 * sqrtPhis, sqrtPhi, rSqrtPhi);
   dXdep_dVb = PRM(XG_B3_XDEP0_SQRTPHI) * dsqrtPhis_dVb;
   Leff = PRM(XG_B3_LEFF);
   Vtm = vtm;
-  T3 = sqrt(Xdep);
-  B3_RCP(rSqXdep, T3);
+  double rSqXdep;
+  T3 = B3_SQRTX(Xdep, &rSqXdep);
   V0 = PRM(XG_B3_V0);
   const double dvt2 = PRM(XG_B3_DVT2), dvt2w = PRM(XG_B3_DVT2W);
   T0 = dvt2 * Vbseff;
-  if (T0 >= -0.5) {
+  if (ge(T0, -0.5)) {
     T1 = 1.0 + T0;
     T2 = dvt2;
   } else {
@@ -303,7 +316,7 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
   lt1 = factor1 * T3 * T1;
   dlt1_dVb = factor1 * (B3_DIV(0.5, T3, rSqXdep) * T1 * dXdep_dVb + T3 * T2);
   T0 = dvt2w * Vbseff;
-  if (T0 >= -0.5) {
+  if (ge(T0, -0.5)) {
     T1 = 1.0 + T0;
     T2 = dvt2w;
   } else {
@@ -315,7 +328,7 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
   dltw_dVb = factor1 * (B3_DIV(0.5, T3, rSqXdep) * T1 * dXdep_dVb + T3 * T2);
   B3_RCP(rlt1, lt1);
   T0 = B3_DIV(PRM(XG_B3_DVT1_LEFF), lt1, rlt1);
-  if (T0 > -EXP_THRESHOLD) {
+  if (gt(T0, -EXP_THRESHOLD)) {
     T1 = exp(T0);
     Theta0 = T1 * (1.0 + 2.0 * T1);
     dT1_dVb = B3_DIV(-T0, lt1, rlt1) * T1 * dlt1_dVb;
@@ -331,7 +344,7 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
   const double weff = PRM(XG_B3_WEFF);
   B3_RCP(rltw, ltw);
   T0 = B3_DIV(PRM(XG_B3_DVT1W_WL), ltw, rltw);
-  if (T0 > -EXP_THRESHOLD) {
+  if (gt(T0, -EXP_THRESHOLD)) {
     T1 = exp(T0);
     T2 = T1 * (1.0 + 2.0 * T1);
     dT1_dVb = B3_DIV(-T0, ltw, rltw) * T1 * dltw_dVb;
@@ -350,7 +363,7 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
   tmp2 = PRM(XG_B3_TOXPHI_W);
   const double etab = PRM(XG_B3_ETAB), theta0vb0 = PRM(XG_B3_THETA0VB0);
   T3 = PRM(XG_B3_ETA0) + etab * Vbseff;
-  if (T3 < 1.0e-4) {
+  if (lt(T3, 1.0e-4)) {
     T9 = B3_Q(1.0, (3.0 - 2.0e4 * T3));
     T3 = (2.0e-4 - T3) * T9;
     T4 = T9 * T9;
@@ -373,7 +386,7 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
   tmp2 = B3_DIV(PRM(XG_B3_NFACTOR_EPSSI), Xdep, rXdep);
   tmp3 = PRM(XG_B3_CDSC) + cdscb * Vbseff + cdscd * Vds;
   tmp4 = B3_DIV(tmp2 + tmp3 * Theta0 + PRM(XG_B3_CIT), cox, rcox);
-  if (tmp4 >= -0.5) {
+  if (ge(tmp4, -0.5)) {
     n = 1.0 + tmp4;
     dn_dVb = B3_DIV(B3_DIV(-tmp2, Xdep, rXdep) * dXdep_dVb + tmp3 * dTheta0_dVb + cdscb * Theta0, cox, rcox);
     dn_dVd = B3_DIV(cdscd * Theta0, cox, rcox);
@@ -387,7 +400,7 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
 
   T0 = PRM(XG_B3_VFB_PHI);
   const double ngate = PRM(XG_B3_NGATE);
-  if ((ngate > 1.e18) && (ngate < 1.e25) && (Vgs > T0)) {
+  if (gt(ngate, 1.e18) && lt(ngate, 1.e25) && gt(Vgs, T0)) {
     T1 = B3_Q(1.0e6 * KQ * EPSSI * ngate, (cox * cox));
     T4 = sqrt(1.0 + B3_Q(2.0 * (Vgs - T0), T1));
     T2 = T1 * (T4 - 1.0);
@@ -408,12 +421,12 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
   B3_RCP(rT10, T10);
   VgstNVt = B3_DIV(Vgst, T10, rT10);
   ExpArg = B3_DIV(2.0 * voff - Vgst, T10, rT10);
-  if (VgstNVt > EXP_THRESHOLD) {
+  if (gt(VgstNVt, EXP_THRESHOLD)) {
     Vgsteff = Vgst;
     dVgsteff_dVg = dVgs_eff_dVg;
     dVgsteff_dVd = -dVth_dVd;
     dVgsteff_dVb = -dVth_dVb;
-  } else if (ExpArg > EXP_THRESHOLD) {
+  } else if (gt(ExpArg, EXP_THRESHOLD)) {
     T0 = B3_Q((Vgst - voff), (n * Vtm));
     ExpVgst = exp(T0);
     Vgsteff = PRM(XG_B3_VTMCDEP_COX) * ExpVgst;
@@ -445,7 +458,7 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
   Weff = weff - 2.0 * (dwg * Vgsteff + dwb * T9);
   dWeff_dVg = -2.0 * dwg;
   dWeff_dVb = -2.0 * dwb * dsqrtPhis_dVb;
-  if (Weff < 2.0e-8) {
+  if (lt(Weff, 2.0e-8)) {
     T0 = B3_Q(1.0, (6.0e-8 - 2.0 * Weff));
     Weff = 2.0e-8 * (4.0e-8 - Weff) * T0;
     T0 *= T0 * 4.0e-16;
@@ -454,7 +467,7 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
   }
   const double prwg = PRM(XG_B3_PRWG), prwb = PRM(XG_B3_PRWB), rds0 = PRM(XG_B3_RDS0);
   T0 = prwg * Vgsteff + prwb * T9;
-  if (T0 >= -0.9) {
+  if (ge(T0, -0.9)) {
     Rds = rds0 * (1.0 + T0);
     dRds_dVg = rds0 * prwg;
     dRds_dVb = rds0 * prwb * dsqrtPhis_dVb;
@@ -466,7 +479,6 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
     dRds_dVb = rds0 * prwb * dsqrtPhis_dVb * T1;
   }
 
-  B3_RCP(rSqrtPhis, sqrtPhis);
   T1 = B3_DIV(0.5 * k1ox, sqrtPhis, rSqrtPhis);
   dT1_dVb = B3_DIV(-T1, sqrtPhis, rSqrtPhis) * dsqrtPhis_dVb;
   T9 = sqrt(PRM(XG_B3_XJ) * Xdep);
@@ -486,12 +498,12 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
   dAbulk_dVg = -T1 * T8;
   Abulk = Abulk0 + dAbulk_dVg * Vgsteff;
   dAbulk_dVb = dAbulk0_dVb - T8 * Vgsteff * (dT1_dVb + 3.0 * T1 * dT2_dVb);
-  if (Abulk0 < 0.1) {
+  if (lt(Abulk0, 0.1)) {
     T9 = B3_Q(1.0, (3.0 - 20.0 * Abulk0));
     Abulk0 = (0.2 - Abulk0) * T9;
     dAbulk0_dVb *= T9 * T9;
   }
-  if (Abulk < 0.1) {
+  if (lt(Abulk, 0.1)) {
     T9 = B3_Q(1.0, (3.0 - 20.0 * Abulk));
     Abulk = (0.2 - Abulk) * T9;
     T10 = T9 * T9;
@@ -500,7 +512,7 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
   }
   const double keta = PRM(XG_B3_KETA);
   T2 = keta * Vbseff;
-  if (T2 >= -0.9) {
+  if (ge(T2, -0.9)) {
     T0 = B3_Q(1.0, (1.0 + T2));
     dT0_dVb = -keta * T0 * T0;
   } else {
@@ -539,7 +551,7 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
     dDenomi_dVd = dDenomi_dVg * 2.0 * dVth_dVd;
     dDenomi_dVb = dDenomi_dVg * 2.0 * dVth_dVb + uc * T4;
   }
-  if (T5 >= -0.8) {
+  if (ge(T5, -0.8)) {
     Denomi = 1.0 + T5;
   } else {
     T9 = B3_Q(1.0, (7.0 + 10.0 * T5));
@@ -570,10 +582,10 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
 
   a1 = PRM(XG_B3_A1);
   const double a2 = PRM(XG_B3_A2);
-  if (a1 == 0.0) {
+  if (eq0(a1)) {
     Lambda = a2;
     dLambda_dVg = 0.0;
-  } else if (a1 > 0.0) {
+  } else if (gt0(a1)) {
     T0 = 1.0 - a2;
     T1 = T0 - a1 * Vgsteff - 0.0001;
     T2 = sqrt(T1 * T1 + 0.0004 * T0);
@@ -588,7 +600,7 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
   Vgst2Vtm = Vgsteff + PRM(XG_B3_VTM2);
   B3_RCP(rVgst2Vtm, Vgst2Vtm);
   B3_RCP(rWeff, Weff);
-  if (Rds > 0) {
+  if (gt0(Rds)) {
     B3_RCP(rRds, Rds);
     tmp2 = B3_DIV(dRds_dVg, Rds, rRds) + B3_DIV(dWeff_dVg, Weff, rWeff);
     tmp3 = B3_DIV(dRds_dVb, Rds, rRds) + B3_DIV(dWeff_dVb, Weff, rWeff);
@@ -596,7 +608,7 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
     tmp2 = B3_DIV(dWeff_dVg, Weff, rWeff);
     tmp3 = B3_DIV(dWeff_dVb, Weff, rWeff);
   }
-  if ((Rds == 0.0) && (Lambda == 1.0)) {
+  if (eq0(Rds) && eq(Lambda, 1.0)) {
     T0 = B3_Q(1.0, (Abulk * EsatL + Vgst2Vtm));
     tmp1 = 0.0;
     T1 = T0 * T0;
@@ -628,14 +640,10 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
     dT2_dVg = EsatL + Vgst2Vtm * dEsatL_dVg + T6 * (4.0 + 2.0 * Vgst2Vtm * tmp2);
     dT2_dVb = Vgst2Vtm * (dEsatL_dVb + 2.0 * T6 * tmp3);
     dT2_dVd = Vgst2Vtm * dEsatL_dVd;
-    T3 = sqrt(T1 * T1 - 2.0 * T0 * T2);
+    double rT3v;
+    T3 = B3_SQRTX(T1 * T1 - 2.0 * T0 * T2, &rT3v);
     B3_RCP(rT0v, T0);
-    B3_RCP(rT3v, T3);
     Vdsat = B3_DIV(T1 - T3, T0, rT0v);
-    dT3_dVg = B3_Q((T1 * dT1_dVg - 2.0 * (T0 * dT2_dVg + T2 * dT0_dVg)), T3);
-    dT3_dVd = B3_Q((T1 * dT1_dVd - 2.0 * (T0 * dT2_dVd + T2 * dT0_dVd)), T3);
-    dT3_dVb = B3_Q((T1 * dT1_dVb - 2.0 * (T0 * dT2_dVb + T2 * dT0_dVb)), T3);
-    (void)dT3_dVg; (void)dT3_dVd; (void)dT3_dVb;
     dVdsat_dVg = B3_DIV(dT1_dVg - B3_DIV(T1 * dT1_dVg - dT0_dVg * T2 - T0 * dT2_dVg, T3, rT3v) - Vdsat * dT0_dVg, T0, rT0v);
     dVdsat_dVb = B3_DIV(dT1_dVb - B3_DIV(T1 * dT1_dVb - dT0_dVb * T2 - T0 * dT2_dVb, T3, rT3v) - Vdsat * dT0_dVb, T0, rT0v);
     dVdsat_dVd = B3_DIV(dT1_dVd - B3_DIV(T1 * dT1_dVd - T0 * dT2_dVd, T3, rT3v), T0, rT0v);
@@ -646,8 +654,8 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
   dT1_dVg = dVdsat_dVg;
   dT1_dVd = dVdsat_dVd - 1.0;
   dT1_dVb = dVdsat_dVb;
-  T2 = sqrt(T1 * T1 + 4.0 * delta * Vdsat);
-  B3_RCP(rT2d, T2);
+  double rT2d;
+  T2 = B3_SQRTX(T1 * T1 + 4.0 * delta * Vdsat, &rT2d);
   T0 = B3_DIV(T1, T2, rT2d);
   T3 = B3_DIV(2.0 * delta, T2, rT2d);
   dT2_dVg = T0 * dT1_dVg + T3 * dVdsat_dVg;
@@ -657,7 +665,7 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
   dVdseff_dVg = dVdsat_dVg - 0.5 * (dT1_dVg + dT2_dVg);
   dVdseff_dVd = dVdsat_dVd - 0.5 * (dT1_dVd + dT2_dVd);
   dVdseff_dVb = dVdsat_dVb - 0.5 * (dT1_dVb + dT2_dVb);
-  if (Vds == 0.0) {
+  if (eq0(Vds)) {
     Vdseff = 0.0;
     dVdseff_dVg = 0.0;
     dVdseff_dVb = 0.0;
@@ -681,11 +689,11 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
   dVasat_dVg = B3_DIV(dT0_dVg - Vasat * dT1_dVg, T1, rT1a);
   dVasat_dVb = B3_DIV(dT0_dVb - Vasat * dT1_dVb, T1, rT1a);
   dVasat_dVd = B3_DIV(dT0_dVd, T1, rT1a);
-  if (Vdseff > Vds) Vdseff = Vds;
+  if (gt(Vdseff, Vds)) Vdseff = Vds;
   diffVds = Vds - Vdseff;
 
   const double pclm = PRM(XG_B3_PCLM), litl = PRM(XG_B3_LITL);
-  if ((pclm > 0.0) && (diffVds > 1.0e-10)) {
+  if (gt0(pclm) && gt(diffVds, 1.0e-10)) {
     T0 = B3_Q(1.0, (pclm * Abulk * litl));
     B3_RCP(rAbulk, Abulk);
     dT0_dVb = B3_DIV(-T0, Abulk, rAbulk) * dAbulk_dVb;
@@ -705,7 +713,7 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
     dVACLM_dVd = dVACLM_dVg = dVACLM_dVb = 0.0;
   }
   const double thetaRout = PRM(XG_B3_THETAROUT), pdiblb = PRM(XG_B3_PDIBLB);
-  if (thetaRout > 0.0) {
+  if (gt0(thetaRout)) {
     T8 = Abulk * Vdsat;
     T0 = Vgst2Vtm * T8;
     dT0_dVg = Vgst2Vtm * Abulk * dVdsat_dVg + T8 + Vgst2Vtm * Vdsat * dAbulk_dVg;
@@ -725,7 +733,7 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
     dVADIBL_dVb = B3_DIV(B3_DIV(-dT0_dVb, T1, rT1r) + B3_DIV(T0 * dT1_dVb, T9, rT9r), T2, rthetaRout);
     dVADIBL_dVd = B3_DIV(B3_DIV(-dT0_dVd, T1, rT1r) + B3_DIV(T0 * dT1_dVd, T9, rT9r), T2, rthetaRout);
     T7 = pdiblb * Vbseff;
-    if (T7 >= -0.9) {
+    if (ge(T7, -0.9)) {
       T3 = B3_Q(1.0, (1.0 + T7));
       VADIBL *= T3;
       dVADIBL_dVg *= T3;
@@ -745,7 +753,7 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
   }
   T8 = B3_DIV(PRM(XG_B3_PVAG), EsatL, rEsatL);
   T9 = T8 * Vgsteff;
-  if (T9 > -0.9) {
+  if (gt(T9, -0.9)) {
     T0 = 1.0 + T9;
     dT0_dVg = T8 * (1.0 - B3_DIV(Vgsteff * dEsatL_dVg, EsatL, rEsatL));
     dT0_dVb = B3_DIV(-T9 * dEsatL_dVb, EsatL, rEsatL);
@@ -774,8 +782,8 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
   dVa_dVb = dVasat_dVb + T1 * dT0_dVb + T0 * dT1_dVb;
 
   const double pscbe1 = PRM(XG_B3_PSCBE1), pscbe2 = PRM(XG_B3_PSCBE2);
-  if (pscbe2 > 0.0) {
-    if (diffVds > PRM(XG_B3_PSCBE1_LITL_ET)) {
+  if (gt0(pscbe2)) {
+    if (gt(diffVds, PRM(XG_B3_PSCBE1_LITL_ET))) {
       B3_RCP(rdiff, diffVds);
       T0 = B3_DIV(PRM(XG_B3_PSCBE1_LITL), diffVds, rdiff);
       VASCBE = B3_DIV(Leff * exp(T0), pscbe2, PRM(XG_B3_R_PSCBE2));
@@ -844,11 +852,11 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
 
   const double beta0 = PRM(XG_B3_BETA0);
   tmp = PRM(XG_B3_ISUB_A);  // alpha0 + alpha1 * Leff
-  if ((tmp <= 0.0) || (beta0 <= 0.0)) {
+  if (le0(tmp) || le0(beta0)) {
     Isub = Gbd = Gbb = Gbg = 0.0;
   } else {
     T2 = PRM(XG_B3_ISUB_T2);
-    if (diffVds > PRM(XG_B3_BETA0_ET)) {
+    if (gt(diffVds, PRM(XG_B3_BETA0_ET))) {
       B3_RCP(rdiffI, diffVds);
       T0 = B3_DIV(-beta0, diffVds, rdiffI);
       T1 = T2 * diffVds * exp(T0);
@@ -884,14 +892,14 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
   const double abulkCVfactor = PRM(XG_B3_ABULKCVFACTOR);
   qgate = qdrn = qsrc = qbulk = 0.0;
   cggb = cgsb = cgdb = cdgb = cdsb = cddb = cbgb = cbsb = cbdb = 0.0;
-  if ((xpart < 0) || (!ChargeComputationNeeded)) {
+  if (lt0(xpart) || (!ChargeComputationNeeded)) {
     qgate = qdrn = qsrc = qbulk = 0.0;
     cggb = cgsb = cgdb = 0.0;
     cdgb = cdsb = cddb = 0.0;
     cbgb = cbsb = cbdb = 0.0;
     goto finished;
   } else if (capMod == 0) {
-    if (Vbseff < 0.0) {
+    if (lt0(Vbseff)) {
       Vbseff = Vbs;
       dVbseff_dVb = 1.0;
     } else {
@@ -907,7 +915,7 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
     (void)dVgst_dVb; (void)dVgst_dVg;
     CoxWL = PRM(XG_B3_COXWL);
     Arg1 = Vgs_eff - Vbseff - Vfb;
-    if (Arg1 <= 0.0) {
+    if (le0(Arg1)) {
       qgate = CoxWL * Arg1;
       qbulk = -qgate;
       qdrn = 0.0;
@@ -919,7 +927,7 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
       cbdb = 0.0;
       cbsb = -cgsb;
       qinv = 0.0;
-    } else if (Vgst <= 0.0) {
+    } else if (le0(Vgst)) {
       T1 = 0.5 * k1ox;
       T2 = sqrt(T1 * T1 + Arg1);
       qgate = CoxWL * k1ox * (T2 - T1);
@@ -942,8 +950,8 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
       Vdsat = B3_Q(Vgst, AbulkCV);
       dVdsat_dVg = B3_Q(dVgs_eff_dVg, AbulkCV);
       dVdsat_dVb = B3_Q(-(Vdsat * dAbulkCV_dVb + dVth_dVb), AbulkCV);
-      if (xpart > 0.5) {
-        if (Vdsat <= Vds) {
+      if (gt(xpart, 0.5)) {
+        if (le(Vdsat, Vds)) {
           T1 = B3_DIVK(Vdsat, 3.0);
           qgate = CoxWL * (Vgs_eff - Vfb - phi - T1);
           T2 = -Two_Third_CoxWL * Vgst;
@@ -997,8 +1005,8 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
           cbsb = -(cgsb + cdsb + T0);
           qinv = -(qgate + qbulk);
         }
-      } else if (xpart < 0.5) {
-        if (Vds >= Vdsat) {
+      } else if (lt(xpart, 0.5)) {
+        if (ge(Vds, Vdsat)) {
           T1 = B3_DIVK(Vdsat, 3.0);
           qgate = CoxWL * (Vgs_eff - Vfb - phi - T1);
           T2 = -Two_Third_CoxWL * Vgst;
@@ -1059,7 +1067,7 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
           qinv = -(qgate + qbulk);
         }
       } else {
-        if (Vds >= Vdsat) {
+        if (ge(Vds, Vdsat)) {
           T1 = B3_DIVK(Vdsat, 3.0);
           qgate = CoxWL * (Vgs_eff - Vfb - phi - T1);
           T2 = -Two_Third_CoxWL * Vgst;
@@ -1111,7 +1119,7 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
       }
     }
   } else {
-    if (Vbseff < 0.0) {
+    if (lt0(Vbseff)) {
       VbseffCV = Vbseff;
       dVbseffCV_dVb = 1.0;
     } else {
@@ -1125,12 +1133,12 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
     T0 = Vtm * noff;
     voffcv = PRM(XG_B3_VOFFCV);
     VgstNVt = B3_Q((Vgst - voffcv), T0);
-    if (VgstNVt > EXP_THRESHOLD) {
+    if (gt(VgstNVt, EXP_THRESHOLD)) {
       Vgsteff = Vgst - voffcv;
       dVgsteff_dVg = dVgs_eff_dVg;
       dVgsteff_dVd = -dVth_dVd;
       dVgsteff_dVb = -dVth_dVb;
-    } else if (VgstNVt < -EXP_THRESHOLD) {
+    } else if (lt(VgstNVt, -EXP_THRESHOLD)) {
       Vgsteff = T0 * log(1.0 + MIN_EXP);
       dVgsteff_dVg = 0.0;
       dVgsteff_dVd = B3_Q(Vgsteff, noff);
@@ -1150,7 +1158,7 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
     if (capMod == 1) {
       Vfb = PRM(XG_B3_VFBZB);
       Arg1 = Vgs_eff - VbseffCV - Vfb - Vgsteff;
-      if (Arg1 <= 0.0) {
+      if (le0(Arg1)) {
         qgate = CoxWL * Arg1;
         Cgg = CoxWL * (dVgs_eff_dVg - dVgsteff_dVg);
         Cgd = -CoxWL * dVgsteff_dVd;
@@ -1173,7 +1181,7 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
       AbulkCV = Abulk0 * abulkCVfactor;
       dAbulkCV_dVb = abulkCVfactor * dAbulk0_dVb;
       VdsatCV = B3_Q(Vgsteff, AbulkCV);
-      if (VdsatCV < Vds) {
+      if (lt(VdsatCV, Vds)) {
         dVdsatCV_dVg = B3_Q(1.0, AbulkCV);
         dVdsatCV_dVb = B3_Q(-VdsatCV * dAbulkCV_dVb, AbulkCV);
         T0 = Vgsteff - B3_DIVK(VdsatCV, 3.0);
@@ -1198,8 +1206,8 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
         Cbg += Cbg1;
         Cbb += Cbb1;
         Cbd += Cbd1;
-        if (xpart > 0.5) T0 = -Two_Third_CoxWL;
-        else if (xpart < 0.5) T0 = -0.4 * CoxWL;
+        if (gt(xpart, 0.5)) T0 = -Two_Third_CoxWL;
+        else if (lt(xpart, 0.5)) T0 = -0.4 * CoxWL;
         else T0 = -One_Third_CoxWL;
         qsrc = T0 * Vgsteff;
         Csg = T0 * dVgsteff_dVg;
@@ -1232,7 +1240,7 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
         Cbg += Cbg1;
         Cbb += Cbb1;
         Cbd += Cbd1;
-        if (xpart > 0.5) {
+        if (gt(xpart, 0.5)) {
           T1 = T1 + T1;
           qsrc = -CoxWL * (0.5 * Vgsteff + 0.25 * T0 - B3_Q(T0 * T0, T1));
           Csg = -CoxWL * (0.5 + B3_Q(B3_Q(24.0 * T0 * Vds, T1), T1) * AbulkCV);
@@ -1241,7 +1249,7 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
           Csd = -CoxWL * (0.25 * AbulkCV - B3_Q(B3_Q(12.0 * AbulkCV * T0, T1), T1) * (4.0 * Vgsteff - T0)) +
                 Csg * dVgsteff_dVd;
           Csg *= dVgsteff_dVg;
-        } else if (xpart < 0.5) {
+        } else if (lt(xpart, 0.5)) {
           T1 = B3_DIVK(T1, 12.0);
           T2 = B3_Q(0.5 * CoxWL, (T1 * T1));
           T3 = Vgsteff * (B3_DIVK(2.0 * T0 * T0, 3.0) + Vgsteff * (Vgsteff - B3_DIVK(4.0 * T0, 3.0))) - B3_DIVK(2.0 * T0 * T0 * T0, 15.0);
@@ -1275,7 +1283,7 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
     } else if (capMod == 2) {
       Vfb = PRM(XG_B3_VFBZB);
       V3 = Vfb - Vgs_eff + VbseffCV - DELTA_3;
-      if (Vfb <= 0.0) {
+      if (le0(Vfb)) {
         T0 = sqrt(V3 * V3 - PRM(XG_B3_D3_VFBZB));  // 4 DELTA_3 Vfb, Vfb = vfbzb
         T2 = B3_Q(-DELTA_3, T0);
       } else {
@@ -1291,10 +1299,10 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
       dQac0_dVb = CoxWL * dVfbeff_dVb;
       T0 = 0.5 * k1ox;
       T3 = Vgs_eff - Vfbeff - VbseffCV - Vgsteff;
-      if (k1ox == 0.0) {
+      if (eq0(k1ox)) {
         T1 = 0.0;
         T2 = 0.0;
-      } else if (T3 < 0.0) {
+      } else if (lt0(T3)) {
         T1 = T0 + B3_Q(T3, k1ox);
         T2 = CoxWL;
       } else {
@@ -1317,7 +1325,7 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
       dVdseffCV_dVg = T3;
       dVdseffCV_dVd = T1;
       dVdseffCV_dVb = -T3 * VdsatCV * dAbulkCV_dVb;
-      if (Vds == 0.0) {
+      if (eq0(Vds)) {
         VdseffCV = 0.0;
         dVdseffCV_dVg = 0.0;
         dVdseffCV_dVb = 0.0;
@@ -1344,7 +1352,7 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
       Cbd1 = CoxWL * T5 * dVdseffCV_dVd + Cbg1 * dVgsteff_dVd;
       Cbb1 = CoxWL * (T5 * dVdseffCV_dVb + T6 * dAbulkCV_dVb) + Cbg1 * dVgsteff_dVb;
       Cbg1 *= dVgsteff_dVg;
-      if (xpart > 0.5) {
+      if (gt(xpart, 0.5)) {
         T1 = T1 + T1;
         qsrc = -CoxWL * (0.5 * Vgsteff + 0.25 * T0 - B3_Q(T0 * T0, T1));
         T7 = B3_Q((4.0 * Vgsteff - T0), (T1 * T1));
@@ -1355,7 +1363,7 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
         Csd = CoxWL * T5 * dVdseffCV_dVd + Csg * dVgsteff_dVd;
         Csb = CoxWL * (T5 * dVdseffCV_dVb + T6 * dAbulkCV_dVb) + Csg * dVgsteff_dVb;
         Csg *= dVgsteff_dVg;
-      } else if (xpart < 0.5) {
+      } else if (lt(xpart, 0.5)) {
         T1 = B3_DIVK(T1, 12.0);
         T2 = B3_Q(0.5 * CoxWL, (T1 * T1));
         T3 = Vgsteff * (B3_DIVK(2.0 * T0 * T0, 3.0) + Vgsteff * (Vgsteff - B3_DIVK(4.0 * T0, 3.0))) - B3_DIVK(2.0 * T0 * T0 * T0, 15.0);
@@ -1399,13 +1407,9 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
     } else if (capMod == 3) {
       const double vfbzb = PRM(XG_B3_VFBZB), acde = PRM(XG_B3_ACDE), ldeb = PRM(XG_B3_LDEB);
       V3 = vfbzb - Vgs_eff + VbseffCV - DELTA_3;
-      if (vfbzb <= 0.0) {
-        T0 = sqrt(V3 * V3 - PRM(XG_B3_D3_VFBZB));
-      } else {
-        T0 = sqrt(V3 * V3 + PRM(XG_B3_D3_VFBZB));
-      }
-      B3_RCP(rT0f, T0);
-      T2 = B3_DIV(vfbzb <= 0.0 ? -DELTA_3 : DELTA_3, T0, rT0f);
+      double rT0f;
+      T0 = B3_SQRTX(V3 * V3 + (le0(vfbzb) ? -PRM(XG_B3_D3_VFBZB) : PRM(XG_B3_D3_VFBZB)), &rT0f);
+      T2 = B3_DIV(le0(vfbzb) ? -DELTA_3 : DELTA_3, T0, rT0f);
       T1 = 0.5 * (1.0 + B3_DIV(V3, T0, rT0f));
       Vfbeff = vfbzb - 0.5 * (V3 + T0);
       dVfbeff_dVg = T1 * dVgs_eff_dVg;
@@ -1417,12 +1421,12 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
       dT0_dVg = B3_DIV(dVgs_eff_dVg, Tox, rTox);
       dT0_dVb = B3_DIV(-dVbseffCV_dVb, Tox, rTox);
       tmp = T0 * acde;
-      if ((-EXP_THRESHOLD < tmp) && (tmp < EXP_THRESHOLD)) {
+      if (lt(-EXP_THRESHOLD, tmp) && lt(tmp, EXP_THRESHOLD)) {
         Tcen = ldeb * exp(tmp);
         dTcen_dVg = acde * Tcen;
         dTcen_dVb = dTcen_dVg * dT0_dVb;
         dTcen_dVg *= dT0_dVg;
-      } else if (tmp <= -EXP_THRESHOLD) {
+      } else if (le(tmp, -EXP_THRESHOLD)) {
         Tcen = ldeb * MIN_EXP;
         dTcen_dVg = dTcen_dVb = 0.0;
       } else {
@@ -1431,9 +1435,10 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
       }
       LINK = PRM(XG_B3_LINK);
       V3 = ldeb - Tcen - LINK;
-      V4 = sqrt(V3 * V3 + PRM(XG_B3_LINK4_LDEB));
+      double rV4;
+      V4 = B3_SQRTX(V3 * V3 + PRM(XG_B3_LINK4_LDEB), &rV4);
       Tcen = ldeb - 0.5 * (V3 + V4);
-      T1 = 0.5 * (1.0 + B3_Q(V3, V4));
+      T1 = 0.5 * (1.0 + B3_DIV(V3, V4, rV4));
       dTcen_dVg *= T1;
       dTcen_dVb *= T1;
       B3_RCP(rTcen, Tcen);
@@ -1452,15 +1457,16 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
       dQac0_dVb = CoxWLcen * dVfbeff_dVb + QovCox * dCoxeff_dVb;
       T0 = 0.5 * k1ox;
       T3 = Vgs_eff - Vfbeff - VbseffCV - Vgsteff;
-      if (k1ox == 0.0) {
+      if (eq0(k1ox)) {
         T1 = 0.0;
         T2 = 0.0;
-      } else if (T3 < 0.0) {
+      } else if (lt0(T3)) {
         T1 = T0 + B3_Q(T3, k1ox);
         T2 = CoxWLcen;
       } else {
-        T1 = sqrt(T0 * T0 + T3);
-        T2 = B3_Q(CoxWLcen * T0, T1);
+        double rT1s;
+        T1 = B3_SQRTX(T0 * T0 + T3, &rT1s);
+        T2 = B3_DIV(CoxWLcen * T0, T1, rT1s);
       }
       Qsub0 = CoxWLcen * k1ox * (T1 - T0);
       QovCox = B3_DIV(Qsub0, Coxeff, rCoxeff);
@@ -1478,7 +1484,7 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
       T3 = 4.0 * (Vth - vfbzb - phi);
       Tox += Tox;
       // the doubled Tox's reciprocal is 0.5 / Tox exactly
-      if (T3 >= 0.0) {
+      if (ge0(T3)) {
         T0 = B3_DIV(Vgsteff + T3, Tox, 0.5 * rTox);
         dT0_dVd = B3_DIV(dVgsteff_dVd + 4.0 * dVth_dVd, Tox, 0.5 * rTox);
         dT0_dVb = B3_DIV(dVgsteff_dVb + 4.0 * dVth_dVb, Tox, 0.5 * rTox);
@@ -1513,9 +1519,9 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
       B3_RCP(rCoxeff2, Coxeff);
       VdsatCV = B3_DIV(Vgsteff - DeltaPhi, AbulkCV, rAbulkCV);
       V4 = VdsatCV - Vds - DELTA_4;
-      T0 = sqrt(V4 * V4 + 4.0 * DELTA_4 * VdsatCV);
+      double rT0g;
+      T0 = B3_SQRTX(V4 * V4 + 4.0 * DELTA_4 * VdsatCV, &rT0g);
       VdseffCV = VdsatCV - 0.5 * (V4 + T0);
-      B3_RCP(rT0g, T0);
       T1 = 0.5 * (1.0 + B3_DIV(V4, T0, rT0g));
       T2 = B3_DIV(DELTA_4, T0, rT0g);
       T3 = B3_DIV(1.0 - T1 - T2, AbulkCV, rAbulkCV);
@@ -1523,7 +1529,7 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
       dVdseffCV_dVg = T4;
       dVdseffCV_dVd = T1;
       dVdseffCV_dVb = -T3 * VdsatCV * dAbulkCV_dVb;
-      if (Vds == 0.0) {
+      if (eq0(Vds)) {
         VdseffCV = 0.0;
         dVdseffCV_dVg = 0.0;
         dVdseffCV_dVb = 0.0;
@@ -1534,7 +1540,7 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
       B3_RCP(rT2h, T2);
       T3 = B3_DIV(T0, T2, rT2h);
       T4 = 1.0 - 12.0 * T3 * T3;
-      T5 = AbulkCV * (B3_DIV(6.0 * T0 * (4.0 * T1 - T0), T2 * T2, rT2h * rT2h) - 0.5);
+      T5 = AbulkCV * (B3_DIVP(6.0 * T0 * (4.0 * T1 - T0), T2 * T2, rT2h * rT2h) - 0.5);
       T6 = B3_DIV(T5 * VdseffCV, AbulkCV, rAbulkCV);
       qgate = qinoi = CoxWLcen * (T1 - T0 * (0.5 - T3));
       QovCox = B3_DIV(qgate, Coxeff, rCoxeff2);
@@ -1544,7 +1550,7 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
       Cgg1 = Cgg1 * dVgsteff_dVg + QovCox * dCoxeff_dVg;
       T7 = 1.0 - AbulkCV;
       T8 = T2 * T2;
-      T9 = B3_DIV(12.0 * T7 * T0 * T0, T8 * AbulkCV, rT2h * rT2h * rAbulkCV);
+      T9 = B3_DIVP(12.0 * T7 * T0 * T0, T8 * AbulkCV, rT2h * rT2h * rAbulkCV);
       T10 = T9 * (1.0 - dDeltaPhi_dVg);
       T11 = B3_DIV(-T7 * T5, AbulkCV, rAbulkCV);
       T12 = -(B3_DIV(T9 * T1, AbulkCV, rAbulkCV) + VdseffCV * (0.5 - B3_DIV(T0, T2, rT2h)));
@@ -1554,7 +1560,7 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
       Cbd1 = CoxWLcen * T11 * dVdseffCV_dVd + Cbg1 * dVgsteff_dVd + QovCox * dCoxeff_dVd;
       Cbb1 = CoxWLcen * (T11 * dVdseffCV_dVb + T12 * dAbulkCV_dVb) + Cbg1 * dVgsteff_dVb + QovCox * dCoxeff_dVb;
       Cbg1 = Cbg1 * dVgsteff_dVg + QovCox * dCoxeff_dVg;
-      if (xpart > 0.5) {
+      if (gt(xpart, 0.5)) {
         qsrc = -CoxWLcen * (B3_DIVK(T1, 2.0) + B3_DIVK(T0, 4.0) - B3_DIV(0.5 * T0 * T0, T2, rT2h));
         QovCox = B3_DIV(qsrc, Coxeff, rCoxeff2);
         T2 += T2;
@@ -1567,10 +1573,10 @@ __global__ void __launch_bounds__(128) bsim3_kernel(DevType t, DevOptions o, Fla
         Csd = CoxWLcen * T5 * dVdseffCV_dVd + Csg * dVgsteff_dVd + QovCox * dCoxeff_dVd;
         Csb = CoxWLcen * (T5 * dVdseffCV_dVb + T6 * dAbulkCV_dVb) + Csg * dVgsteff_dVb + QovCox * dCoxeff_dVb;
         Csg = Csg * dVgsteff_dVg + QovCox * dCoxeff_dVg;
-      } else if (xpart < 0.5) {
+      } else if (lt(xpart, 0.5)) {
         T2 = B3_DIVK(T2, 12.0);
         B3_RCP(rT2x, T2);
-        T3 = B3_DIV(0.5 * CoxWLcen, T2 * T2, rT2x * rT2x);
+        T3 = B3_DIVP(0.5 * CoxWLcen, T2 * T2, rT2x * rT2x);
         T4 = T1 * (B3_DIVK(2.0 * T0 * T0, 3.0) + T1 * (T1 - B3_DIVK(4.0 * T0, 3.0))) -
              B3_DIVK(2.0 * T0 * T0 * T0, 15.0);
         qsrc = -T3 * T4;
@@ -1631,13 +1637,13 @@ finished:
     MJSWG = PRM(XG_B3_MJSWG);
     const double PhiBTemp = PRM(XG_B3_PHIB), PhiBSWTemp = PRM(XG_B3_PHIBSW);
     const double PhiBSWGTemp = PRM(XG_B3_PHIBSWG);
-    if (vbs == 0.0) {
+    if (eq0(vbs)) {
       qbs = 0.0;
       capbs = czbs + czbssw + czbsswg;
-    } else if (vbs < 0.0) {
-      if (czbs > 0.0) {
+    } else if (lt0(vbs)) {
+      if (gt0(czbs)) {
         arg = 1.0 - B3_DIV(vbs, PhiBTemp, PRM(XG_B3_R_PHIB));
-        if (MJ == 0.5) sarg = B3_RSQRT(arg);
+        if (eq(MJ, 0.5)) sarg = B3_RSQRT(arg);
         else sarg = exp(-MJ * log(arg));
         qbs = B3_DIV(PRM(XG_B3_QBS0) * (1.0 - arg * sarg), PRM(XG_B3_OMMJ), PRM(XG_B3_R_OMMJ));
         capbs = czbs * sarg;
@@ -1645,16 +1651,16 @@ finished:
         qbs = 0.0;
         capbs = 0.0;
       }
-      if (czbssw > 0.0) {
+      if (gt0(czbssw)) {
         arg = 1.0 - B3_DIV(vbs, PhiBSWTemp, PRM(XG_B3_R_PHIBSW));
-        if (MJSW == 0.5) sarg = B3_RSQRT(arg);
+        if (eq(MJSW, 0.5)) sarg = B3_RSQRT(arg);
         else sarg = exp(-MJSW * log(arg));
         qbs += B3_DIV(PRM(XG_B3_QBSSW0) * (1.0 - arg * sarg), PRM(XG_B3_OMMJSW), PRM(XG_B3_R_OMMJSW));
         capbs += czbssw * sarg;
       }
-      if (czbsswg > 0.0) {
+      if (gt0(czbsswg)) {
         arg = 1.0 - B3_DIV(vbs, PhiBSWGTemp, PRM(XG_B3_R_PHIBSWG));
-        if (MJSWG == 0.5) sarg = B3_RSQRT(arg);
+        if (eq(MJSWG, 0.5)) sarg = B3_RSQRT(arg);
         else sarg = exp(-MJSWG * log(arg));
         qbs += B3_DIV(PRM(XG_B3_QBSSWG0) * (1.0 - arg * sarg), PRM(XG_B3_OMMJSWG), PRM(XG_B3_R_OMMJSWG));
         capbs += czbsswg * sarg;
@@ -1665,13 +1671,13 @@ finished:
       qbs = vbs * (T0 + 0.5 * T1);
       capbs = T0 + T1;
     }
-    if (vbd == 0.0) {
+    if (eq0(vbd)) {
       qbd = 0.0;
       capbd = czbd + czbdsw + czbdswg;
-    } else if (vbd < 0.0) {
-      if (czbd > 0.0) {
+    } else if (lt0(vbd)) {
+      if (gt0(czbd)) {
         arg = 1.0 - B3_DIV(vbd, PhiBTemp, PRM(XG_B3_R_PHIB));
-        if (MJ == 0.5) sarg = B3_RSQRT(arg);
+        if (eq(MJ, 0.5)) sarg = B3_RSQRT(arg);
         else sarg = exp(-MJ * log(arg));
         qbd = B3_DIV(PRM(XG_B3_QBD0) * (1.0 - arg * sarg), PRM(XG_B3_OMMJ), PRM(XG_B3_R_OMMJ));
         capbd = czbd * sarg;
@@ -1679,16 +1685,16 @@ finished:
         qbd = 0.0;
         capbd = 0.0;
       }
-      if (czbdsw > 0.0) {
+      if (gt0(czbdsw)) {
         arg = 1.0 - B3_DIV(vbd, PhiBSWTemp, PRM(XG_B3_R_PHIBSW));
-        if (MJSW == 0.5) sarg = B3_RSQRT(arg);
+        if (eq(MJSW, 0.5)) sarg = B3_RSQRT(arg);
         else sarg = exp(-MJSW * log(arg));
         qbd += B3_DIV(PRM(XG_B3_QBDSW0) * (1.0 - arg * sarg), PRM(XG_B3_OMMJSW), PRM(XG_B3_R_OMMJSW));
         capbd += czbdsw * sarg;
       }
-      if (czbdswg > 0.0) {
+      if (gt0(czbdswg)) {
         arg = 1.0 - B3_DIV(vbd, PhiBSWGTemp, PRM(XG_B3_R_PHIBSWG));
-        if (MJSWG == 0.5) sarg = B3_RSQRT(arg);
+        if (eq(MJSWG, 0.5)) sarg = B3_RSQRT(arg);
         else sarg = exp(-MJSWG * log(arg));
         qbd += B3_DIV(PRM(XG_B3_QBDSWG0) * (1.0 - arg * sarg), PRM(XG_B3_OMMJSWG), PRM(XG_B3_R_OMMJSWG));
         capbd += czbdswg * sarg;
@@ -1710,7 +1716,7 @@ finished:
       cgso = PRM(XG_B3_CGSO);
       qgso = PRM(XG_B3_CGSO) * vgs;
     } else if (capMod == 1) {
-      if (vgd < 0.0) {
+      if (lt0(vgd)) {
         T1 = sqrt(1.0 - B3_Q(4.0 * vgd, ckappa));
         cgdo = PRM(XG_B3_CGDO) + B3_Q(weffCV * cgdl, T1);
         qgdo = PRM(XG_B3_CGDO) * vgd - weffCV * 0.5 * cgdl * ckappa * (T1 - 1.0);
@@ -1718,7 +1724,7 @@ finished:
         cgdo = PRM(XG_B3_CGDO) + weffCV * cgdl;
         qgdo = (weffCV * cgdl + PRM(XG_B3_CGDO)) * vgd;
       }
-      if (vgs < 0.0) {
+      if (lt0(vgs)) {
         T1 = sqrt(1.0 - B3_Q(4.0 * vgs, ckappa));
         cgso = PRM(XG_B3_CGSO) + B3_Q(weffCV * cgsl, T1);
         qgso = PRM(XG_B3_CGSO) * vgs - weffCV * 0.5 * cgsl * ckappa * (T1 - 1.0);
@@ -1727,19 +1733,20 @@ finished:
         qgso = (weffCV * cgsl + PRM(XG_B3_CGSO)) * vgs;
       }
     } else {
+      double rT1o, rT4o;
       T0 = vgd + DELTA_1;
-      T1 = sqrt(T0 * T0 + 4.0 * DELTA_1);
+      T1 = B3_SQRTX(T0 * T0 + 4.0 * DELTA_1, &rT1o);
       T2 = 0.5 * (T0 - T1);
       T3 = PRM(XG_B3_CGDL_W);  // weffCV * cgdl
-      T4 = sqrt(1.0 - B3_DIV(4.0 * T2, ckappa, PRM(XG_B3_R_CKAPPA)));
-      cgdo = PRM(XG_B3_CGDO_T) - T3 * (1.0 - B3_Q(1.0, T4)) * (0.5 - B3_Q(0.5 * T0, T1));
+      T4 = B3_SQRTX(1.0 - B3_DIV(4.0 * T2, ckappa, PRM(XG_B3_R_CKAPPA)), &rT4o);
+      cgdo = PRM(XG_B3_CGDO_T) - T3 * (1.0 - rT4o) * (0.5 - B3_DIV(0.5 * T0, T1, rT1o));
       qgdo = PRM(XG_B3_CGDO_T) * vgd - T3 * (T2 + PRM(XG_B3_HALF_CKAPPA) * (T4 - 1.0));
       T0 = vgs + DELTA_1;
-      T1 = sqrt(T0 * T0 + 4.0 * DELTA_1);
+      T1 = B3_SQRTX(T0 * T0 + 4.0 * DELTA_1, &rT1o);
       T2 = 0.5 * (T0 - T1);
       T3 = PRM(XG_B3_CGSL_W);  // weffCV * cgsl
-      T4 = sqrt(1.0 - B3_DIV(4.0 * T2, ckappa, PRM(XG_B3_R_CKAPPA)));
-      cgso = PRM(XG_B3_CGSO_T) - T3 * (1.0 - B3_Q(1.0, T4)) * (0.5 - B3_Q(0.5 * T0, T1));
+      T4 = B3_SQRTX(1.0 - B3_DIV(4.0 * T2, ckappa, PRM(XG_B3_R_CKAPPA)), &rT4o);
+      cgso = PRM(XG_B3_CGSO_T) - T3 * (1.0 - rT4o) * (0.5 - B3_DIV(0.5 * T0, T1, rT1o));
       qgso = PRM(XG_B3_CGSO_T) * vgs - T3 * (T2 + PRM(XG_B3_HALF_CKAPPA) * (T4 - 1.0));
     }
     /* setupCapacitors_oldDAE: charge sums and partition (:7640-7898), nqsMod 0 */
@@ -1833,8 +1840,8 @@ finished:
   double gbbdp, gbbsp, gbdpg, gbdpdp, gbdpb, gbdpsp, gbspg, gbspdp, gbspb, gbspsp;
   if (mode >= 0) {
     Gmx = m.gm; Gmbsx = m.gmbs; FwdSum = Gmx + Gmbsx; RevSum = 0.0;
-    cdreq = dtype * (m.cd);
-    ceqbd = -dtype * (m.csub);
+    cdreq = flip(m.cd, pol);
+    ceqbd = -flip(m.csub, pol);
     ceqbs = 0.0;
     gbbdp = -m.gbds;
     gbbsp = (m.gbds + m.gbgs + m.gbbs);
@@ -1843,8 +1850,8 @@ finished:
     gbspg = 0.0; gbspdp = 0.0; gbspb = 0.0; gbspsp = 0.0;
   } else {
     Gmx = -m.gm; Gmbsx = -m.gmbs; FwdSum = 0.0; RevSum = -(Gmx + Gmbsx);
-    cdreq = -dtype * (m.cd);
-    ceqbs = -dtype * (m.csub);
+    cdreq = -flip(m.cd, pol);
+    ceqbs = -flip(m.csub, pol);
     ceqbd = 0.0;
     gbbsp = -m.gbds;
     gbbdp = (m.gbds + m.gbgs + m.gbbs);
@@ -1852,52 +1859,35 @@ finished:
     gbspg = m.gbgs; gbspsp = m.gbds; gbspb = m.gbbs;
     gbspdp = -(gbspg + gbspsp + gbspb);
   }
-  if (dtype > 0) {
-    ceqbs += (cbs);
-    ceqbd += (cbd);
-  } else {
-    ceqbs -= (cbs);
-    ceqbd -= (cbd);
-  }
+  ceqbs += flip(cbs, pol);
+  ceqbd += flip(cbd, pol);
   Terms T{io.terms + t.term0, nI};
-  T.put(0, i, drainConductance != 0.0 ? Idrain * numberParallel : 0.0);
-  T.put(1, i, sourceConductance != 0.0 ? Isource * numberParallel : 0.0);
-  T.put(2, i, (ceqbs + ceqbd) * numberParallel);
-  T.put(3, i, (-(ceqbd - cdreq) - Idrain) * numberParallel);
-  T.put(4, i, (-(cdreq + ceqbs) - Isource) * numberParallel);
+  auto put = [&](int q, double v) { T.put(q, i, v); };
+  put(0, ne0(drainConductance) ? Idrain : 0.0);
+  put(1, ne0(sourceConductance) ? Isource : 0.0);
+  put(2, (ceqbs + ceqbd));
+  put(3, (-(ceqbd - cdreq) - Idrain));
+  put(4, (-(cdreq + ceqbs) - Isource));
   const bool lim = o.voltlim && !origFlag;
   if (lim) {
     double tmpj;
     if (mode >= 0) {
-      tmpj = dtype * (-m.gds * (vds - vds_orig) - Gmx * (vgs - vgs_orig) - Gmbsx * (vbs - vbs_orig));
+      tmpj = flip(-m.gds * (vds - vds_orig) - Gmx * (vgs - vgs_orig) - Gmbsx * (vbs - vbs_orig), pol);
       cdreq_Jdxp += tmpj;
-      cdreq += tmpj;
-      tmpj = -dtype * (-m.gbds * (vds - vds_orig) - m.gbgs * (vgs - vgs_orig) - m.gbbs * (vbs - vbs_orig));
+      tmpj = -flip(-m.gbds * (vds - vds_orig) - m.gbgs * (vgs - vgs_orig) - m.gbbs * (vbs - vbs_orig), pol);
       ceqbd_Jdxp += tmpj;
-      ceqbd += tmpj;
     } else {
-      tmpj = -dtype * (m.gds * (vds - vds_orig) + Gmx * (vgd - vgd_orig) + Gmbsx * (vbd - vbd_orig));
+      tmpj = -flip(m.gds * (vds - vds_orig) + Gmx * (vgd - vgd_orig) + Gmbsx * (vbd - vbd_orig), pol);
       cdreq_Jdxp += tmpj;
-      cdreq += tmpj;
-      tmpj = -dtype * (m.gbds * (vds - vds_orig) - m.gbgs * (vgd - vgd_orig) - m.gbbs * (vbd - vbd_orig));
+      tmpj = -flip(m.gbds * (vds - vds_orig) - m.gbgs * (vgd - vgd_orig) - m.gbbs * (vbd - vbd_orig), pol);
       ceqbd_Jdxp += tmpj;
-      ceqbd += tmpj;
     }
-    if (dtype > 0) {
-      ceqbs_Jdxp += (-gbs * (vbs - vbs_orig));
-      ceqbs += (-gbs * (vbs - vbs_orig));
-      ceqbd_Jdxp += (-gbd * (vbd - vbd_orig));
-      ceqbd += (-gbd * (vbd - vbd_orig));
-    } else {
-      ceqbs_Jdxp -= (-gbs * (vbs - vbs_orig));
-      ceqbs -= (-gbs * (vbs - vbs_orig));
-      ceqbd_Jdxp -= (-gbd * (vbd - vbd_orig));
-      ceqbd -= (-gbd * (vbd - vbd_orig));
-    }
+    ceqbs_Jdxp += flip(-gbs, pol) * (vbs - vbs_orig);
+    ceqbd_Jdxp += flip(-gbd, pol) * (vbd - vbd_orig);
   }
-  T.put(5, i, lim ? -(ceqbs_Jdxp + ceqbd_Jdxp) * numberParallel : 0.0);
-  T.put(6, i, lim ? (ceqbd_Jdxp - cdreq_Jdxp) * numberParallel : 0.0);
-  T.put(7, i, lim ? (cdreq_Jdxp + ceqbs_Jdxp) * numberParallel : 0.0);
+  put(5, lim ? -(ceqbs_Jdxp + ceqbd_Jdxp) : 0.0);
+  put(6, lim ? (ceqbd_Jdxp - cdreq_Jdxp) : 0.0);
+  put(7, lim ? (cdreq_Jdxp + ceqbs_Jdxp) : 0.0);
 
   // auxChargeCalculations (:7477-7573)
   if (ChargeComputationNeeded) {
@@ -1917,67 +1907,67 @@ finished:
     m.sxpart = (1.0 - (m.dxpart = (mode > 0) ? 0.4 : 0.6));
   }
   double Qeqqg, Qeqqb, Qeqqd;
-  if (dtype > 0) {
-    Qeqqg = mem.qg; Qeqqb = mem.qb; Qeqqd = mem.qd;
-  } else {
-    Qeqqg = -mem.qg; Qeqqb = -mem.qb; Qeqqd = -mem.qd;
-  }
-  T.put(8, i, Qeqqg * numberParallel);
-  T.put(9, i, (Qeqqb) * numberParallel);
-  T.put(10, i, (-(-Qeqqd)) * numberParallel);
-  T.put(11, i, (-(+Qeqqg + Qeqqb + Qeqqd)) * numberParallel);
-  if (o.voltlim && dtype <= 0) {
+  Qeqqg = flip(mem.qg, pol); Qeqqb = flip(mem.qb, pol); Qeqqd = flip(mem.qd, pol);
+  put(8, Qeqqg);
+  put(9, (Qeqqb));
+  put(10, (-(-Qeqqd)));
+  put(11, (-(+Qeqqg + Qeqqb + Qeqqd)));
+  if (o.voltlim && pol) {
     mem.Qeqqg_Jdxp = -mem.Qeqqg_Jdxp;
     mem.Qeqqb_Jdxp = -mem.Qeqqb_Jdxp;
     mem.Qeqqd_Jdxp = -mem.Qeqqd_Jdxp;
   }
-  T.put(12, i, lim ? -mem.Qeqqg_Jdxp * numberParallel : 0.0);
-  T.put(13, i, lim ? -(+mem.Qeqqb_Jdxp) * numberParallel : 0.0);
-  T.put(14, i, lim ? (-mem.Qeqqd_Jdxp) * numberParallel : 0.0);
-  T.put(15, i, lim ? (+mem.Qeqqg_Jdxp + mem.Qeqqb_Jdxp + mem.Qeqqd_Jdxp) * numberParallel : 0.0);
+  put(12, lim ? -mem.Qeqqg_Jdxp : 0.0);
+  put(13, lim ? -(+mem.Qeqqb_Jdxp) : 0.0);
+  put(14, lim ? (-mem.Qeqqd_Jdxp) : 0.0);
+  put(15, lim ? (+mem.Qeqqg_Jdxp + mem.Qeqqb_Jdxp + mem.Qeqqd_Jdxp) : 0.0);
 
   // Master::loadDAEMatrices (:9654-9939)
-  const double M = numberParallel;
   const double GD = drainConductance, GS = sourceConductance;
-  T.put(16, i, GD * M);
-  T.put(17, i, -(GD * M));
-  T.put(18, i, GS * M);
-  T.put(19, i, -(GS * M));
-  T.put(20, i, (-m.gbgs) * M);
-  T.put(21, i, (gbd + gbs - m.gbbs) * M);
-  T.put(22, i, (-gbd + gbbdp) * M);
-  T.put(23, i, (-gbs + gbbsp) * M);
-  T.put(24, i, -(GD * M));
-  T.put(25, i, -((gbd - Gmbsx - gbdpb) * M));
-  T.put(26, i, (Gmx + gbdpg) * M);
-  T.put(27, i, (GD + m.gds + gbd + RevSum + gbdpdp) * M);
-  T.put(28, i, -((m.gds + FwdSum - gbdpsp) * M));
-  T.put(29, i, (-Gmx + gbspg) * M);
-  T.put(30, i, -((gbs + Gmbsx - gbspb) * M));
-  T.put(31, i, -(GS * M));
-  T.put(32, i, -((m.gds + RevSum - gbspdp) * M));
-  T.put(33, i, (GS + m.gds + gbs + FwdSum + gbspsp) * M);
+  put(16, GD);
+  put(17, -GD);
+  put(18, GS);
+  put(19, -GS);
+  put(20, (-m.gbgs));
+  put(21, (gbd + gbs - m.gbbs));
+  put(22, (-gbd + gbbdp));
+  put(23, (-gbs + gbbsp));
+  put(24, -GD);
+  put(25, -(gbd - Gmbsx - gbdpb));
+  put(26, (Gmx + gbdpg));
+  put(27, (GD + m.gds + gbd + RevSum + gbdpdp));
+  put(28, -(m.gds + FwdSum - gbdpsp));
+  put(29, (-Gmx + gbspg));
+  put(30, -(gbs + Gmbsx - gbspb));
+  put(31, -GS);
+  put(32, -(m.gds + RevSum - gbspdp));
+  put(33, (GS + m.gds + gbs + FwdSum + gbspsp));
   if (init_tran_step) {
 #pragma unroll
     for (int q = 34; q < 50; ++q) T.put(q, i, 0.0);
   } else {
-    T.put(34, i, (mem.CAPcggb) * M);
-    T.put(35, i, -((mem.CAPcggb + mem.CAPcgdb + mem.CAPcgsb) * M));
-    T.put(36, i, (mem.CAPcgdb) * M);
-    T.put(37, i, (mem.CAPcgsb) * M);
-    T.put(38, i, (mem.CAPcbgb) * M);
-    T.put(39, i, (-mem.CAPcbgb - mem.CAPcbdb - mem.CAPcbsb) * M);
-    T.put(40, i, (mem.CAPcbdb) * M);
-    T.put(41, i, (mem.CAPcbsb) * M);
-    T.put(42, i, -((+mem.CAPcdgb + mem.CAPcddb + mem.CAPcdsb) * M));
-    T.put(43, i, (mem.CAPcdgb) * M);
-    T.put(44, i, (+mem.CAPcddb) * M);
-    T.put(45, i, -((-mem.CAPcdsb) * M));
-    T.put(46, i, (mem.CAPcsgb) * M);
-    T.put(47, i, -((+mem.CAPcsgb + mem.CAPcsdb + mem.CAPcssb) * M));
-    T.put(48, i, -((-mem.CAPcsdb) * M));
-    T.put(49, i, (+mem.CAPcssb) * M);
+    put(34, (mem.CAPcggb));
+    put(35, -(mem.CAPcggb + mem.CAPcgdb + mem.CAPcgsb));
+    put(36, (mem.CAPcgdb));
+    put(37, (mem.CAPcgsb));
+    put(38, (mem.CAPcbgb));
+    put(39, (-mem.CAPcbgb - mem.CAPcbdb - mem.CAPcbsb));
+    put(40, (mem.CAPcbdb));
+    put(41, (mem.CAPcbsb));
+    put(42, -(+mem.CAPcdgb + mem.CAPcddb + mem.CAPcdsb));
+    put(43, (mem.CAPcdgb));
+    put(44, (+mem.CAPcddb));
+    put(45, -(-mem.CAPcdsb));
+    put(46, (mem.CAPcsgb));
+    put(47, -(+mem.CAPcsgb + mem.CAPcsdb + mem.CAPcssb));
+    put(48, -(-mem.CAPcsdb));
+    put(49, (+mem.CAPcssb));
   }
+
+  // each value is times M: instances that are not single scale their stamps
+  // afterwards (a product per stamp for everyone was 50 FP64 instructions)
+  if (ne(numberParallel, 1.0))
+    for (int q = 0; q < 50; ++q) T.put(q, i, T.base[(int64_t)q * nI + i] * numberParallel);
 
   memp[(int64_t)B3M_CAPCGGB * nI] = mem.CAPcggb;
   memp[(int64_t)B3M_CAPCGDB * nI] = mem.CAPcgdb;
