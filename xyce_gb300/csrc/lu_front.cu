@@ -23,6 +23,7 @@
 #include <memory>
 #include <vector>
 
+#include "lu_entries.cuh"
 #include "lu_front.h"
 #include "xg_internal.h"
 #include "xg_smem.cuh"
@@ -126,15 +127,6 @@ size_t factor_smem(int m, int C, size_t tsz) {
   return ((C > 1 ? kNb : 0) + size_t(local_columns(m, 0, C))) * ld * tsz + (kNb * kNb + kNb) * tsz;
 }
 
-__device__ __forceinline__ bool bad_value(double u) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(u);
-  return (b << 1) == 0 || ((b >> 52) & 0x7ff) == 0x7ff;
-}
-__device__ __forceinline__ bool bad_value(float u) {
-  const unsigned b = __float_as_uint(u);
-  return (b << 1) == 0 || ((b >> 23) & 0xff) == 0xff;
-}
-
 __device__ __forceinline__ void report_pivot(unsigned *status, int row) {
   atomicOr(status, 1u);
   atomicMin(status + 1, unsigned(row));
@@ -194,22 +186,6 @@ __device__ void assemble(const FrontDev &d, const Front &f, const double *__rest
     __syncthreads();
   }
 }
-
-// 1 / u: a Halley step (the cubic member of Householder's family: with
-// e = 1 - u x, x (1 + e + e^2) leaves a relative error of e^3) from the
-// hardware's 20-bit approximation, three dependent multiply-adds where the
-// IEEE division has a longer chain; the pivots of a front follow one another
-// at its latency.  The division itself near the ends of the exponent range.
-__device__ __forceinline__ double pivot_reciprocal(double u) {
-  double x;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(u));
-  const double e = fma(-u, x, 1.0);
-  x = fma(x, fma(e, e, e), x);
-  const int ex = (__double2hiint(u) >> 20) & 0x7ff;
-  if (unsigned(ex - 64) > 1918u) x = 1.0 / u;
-  return x;
-}
-__device__ __forceinline__ float pivot_reciprocal(float u) { return 1.0f / u; }
 
 // Eliminates the pivot columns [k0, k0 + nb) that start at base, a row per
 // thread with its entries in registers, after applying the kNb pivots before

@@ -49,6 +49,7 @@
 #include "xg.h"
 #include "xg_internal.h"
 #include "lu_chain.h"
+#include "lu_entries.cuh"
 #include "lu_front.h"
 #include "xg_lu.h"
 #include "xg_smem.cuh"
@@ -1277,316 +1278,98 @@ __global__ void __launch_bounds__(kCtaThreads) lu_solve_cta(LuDev d, const T *__
   }
 }
 
-// ---- small matrices, level by level: one thread per row -------------------------
-// GB300 issues FP64 at two lanes per clock per SM, so an FP64 instruction
-// costs about the same whether one lane of the warp uses it or all 32.  The
-// warp-per-row kernels above leave most lanes idle on the short rows of
-// circuit matrices.  Here the rows of one dependency level (independent of
-// each other) go to different threads, the levels follow one another with a
-// block barrier, and everything the kernel reads sits in shared memory: the
-// values, the pattern, the update schedule and the level lists.  With a
-// nested-dissection order a chain of 1,000 inverters has ~22 levels.  The
-// trailing rows with long L parts (the tail, see LuSymbolic) are done after
-// the levels, one row at a time with all threads.  A Newton step refactors
-// and then solves: lu_factor_solve_lvl does both from one staging of the
-// shared-memory working set.
+// ---- small matrices, level by level in one CTA ----------------------------------
+// The factor and the schedule of lu_entries.cuh sit in shared memory.  The
+// schedule's image comes by one bulk copy while the threads gather A; a Newton
+// step refactors and solves from one staging (lu_factor_solve_lvl).  What
+// bounds it is the chain of levels, each a few shared-memory loads, an FP64
+// multiply-add or a reciprocal, and a barrier.  Measured on the 1,000-stage
+// inverter chain (6,958 entries, nested dissection): a Newton step in 41.0 us;
+// with a thread per row of a dependency level, its index lists loaded one by
+// one, it took 102.4 us.
 
 struct LvlDev {
-  const int *lrow, *lptr, *urow, *uptr;  // rows by L level / by U level
-  const int *lheavy;                     // per L level: where its heavy rows start
-  const int *urp32;                      // update-schedule row starts (int)
-  const int *tail_rowg, *tail_gptr, *tail_glong, *tail_pos, *tail_pp, *tail_pm, *tail_q;
-  int levels, ulevels, nup;
-  int tail0, ntail, ngroups, npos, npairs;
+  const uint32_t *image;
+  LuEntriesHead h;
 };
-
-enum LvlOff { O_VAL, O_RD, O_Y, O_RED, O_CI, O_RP, O_DIAG, O_URP, O_UPOS, O_LROW, O_LPTR, O_UROW,
-              O_UPTR, O_TROWG, O_TGPTR, O_TGLONG, O_TPOS, O_TPP, O_TPM, O_TQ, O_LHEAVY, O_END };
 enum LvlMode { LVL_FACTOR = 1, LVL_SOLVE = 2, LVL_BOTH = 3 };
 
-// Shared-memory layout of the level kernels (the same function on host and
-// device).  The factor uses val, rd, the schedule and the tail; the solve
-// uses val, rd, y, the reduction scratch (one T per thread) and both level
-// lists.  The T arrays come first, each padded to 16 bytes.
-__host__ __device__ inline size_t lvl_layout(int n, int64_t nnz, const LvlDev &v, int threads,
-                                             size_t tsz, int mode, size_t *off) {
-  auto a16 = [](size_t x) { return (x + 15) & ~size_t(15); };
-  const size_t I = sizeof(int);
-  const bool f = mode & LVL_FACTOR, sv = mode & LVL_SOLVE;
-  size_t o = 0;
-  off[O_VAL] = o; o += a16(tsz * size_t(nnz));
-  off[O_RD] = o; o += a16(tsz * size_t(n));
-  off[O_Y] = o; o += sv ? a16(tsz * size_t(n)) : 0;
-  off[O_RED] = o; o += sv ? a16(tsz * size_t(threads)) : 0;
-  off[O_CI] = o; o += I * size_t(nnz);
-  off[O_RP] = o; o += I * size_t(n + 1);
-  off[O_DIAG] = o; o += I * size_t(n);
-  off[O_URP] = o; o += f ? I * size_t(n + 1) : 0;
-  off[O_UPOS] = o; o += f ? I * size_t(v.nup) : 0;
-  off[O_LROW] = o; o += I * size_t(v.tail0);
-  off[O_LPTR] = o; o += I * size_t(v.levels + 1);
-  off[O_UROW] = o; o += sv ? I * size_t(n) : 0;
-  off[O_UPTR] = o; o += sv ? I * size_t(v.ulevels + 1) : 0;
-  off[O_TROWG] = o; o += f ? I * size_t(v.ntail + 1) : 0;
-  off[O_TGPTR] = o; o += f ? I * size_t(v.ngroups + 1) : 0;
-  off[O_TGLONG] = o; o += f ? I * size_t(v.ngroups) : 0;
-  off[O_TPOS] = o; o += f ? I * size_t(v.npos) : 0;
-  off[O_TPP] = o; o += f ? I * size_t(v.npos + 1) : 0;
-  off[O_TPM] = o; o += f ? I * size_t(v.npairs) : 0;
-  off[O_TQ] = o; o += f ? I * size_t(v.npairs) : 0;
-  off[O_LHEAVY] = o; o += f ? I * size_t(v.levels) : 0;
-  off[O_END] = o;
-  return o;
+__host__ __device__ inline size_t pad16(size_t x) { return (x + 15) & ~size_t(15); }
+__host__ __device__ inline int lvl_first_word(const LuEntriesHead &h, int mode) {
+  return mode == LVL_SOLVE ? h.solve0 : 0;
 }
-
-// A zero, infinite or NaN pivot, from the bits (no FP64 instruction).
-__device__ __forceinline__ bool bad_pivot(double u) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(u);
-  return (b << 1) == 0 || ((b >> 52) & 0x7ff) == 0x7ff;
+__host__ __device__ inline int lvl_words(const LuEntriesHead &h, int mode) {
+  return mode == LVL_FACTOR ? h.factor : mode == LVL_SOLVE ? h.words - h.solve0 : h.both;
 }
-__device__ __forceinline__ bool bad_pivot(float u) {
-  const unsigned b = __float_as_uint(u);
-  return (b << 1) == 0 || ((b >> 23) & 0xff) == 0xff;
-}
-
-// Copies count ints into shared memory, four loads in flight per thread.
-__device__ __forceinline__ void stage_ints(int *dst, const int *__restrict__ src, int count) {
-  const int T = blockDim.x;
-  int i = threadIdx.x;
-  for (; i + 3 * T < count; i += 4 * T) {
-    const int a0 = __ldg(src + i), a1 = __ldg(src + i + T), a2 = __ldg(src + i + 2 * T),
-              a3 = __ldg(src + i + 3 * T);
-    dst[i] = a0;
-    dst[i + T] = a1;
-    dst[i + 2 * T] = a2;
-    dst[i + 3 * T] = a3;
-  }
-  for (; i < count; i += T) dst[i] = __ldg(src + i);
+// The copy's barrier, values, reciprocal pivots, solve vector, image.
+inline size_t lvl_smem_bytes(int n, int64_t nnz, const LuEntriesHead &h, size_t tsz, int mode) {
+  return 16 + pad16(tsz * size_t(nnz)) + 2 * pad16(tsz * size_t(n)) + 4 * size_t(lvl_words(h, mode));
 }
 
 template <class T>
-struct LvlSmem {
-  T *val, *rd, *y, *red;
-  int *ci, *rp, *diag, *urp, *upos, *lrow, *lptr, *urow, *uptr;
-  int *trowg, *tgptr, *tglong, *tpos, *tpp, *tpm, *tq, *lheavy;
-};
-
-template <class T>
-__device__ LvlSmem<T> lvl_smem(char *smem, int n, int64_t nnz, const LvlDev &v, int mode) {
-  size_t off[O_END + 1];
-  lvl_layout(n, nnz, v, blockDim.x, sizeof(T), mode, off);
-  LvlSmem<T> m;
-  m.val = (T *)(smem + off[O_VAL]);
-  m.rd = (T *)(smem + off[O_RD]);
-  m.y = (T *)(smem + off[O_Y]);
-  m.red = (T *)(smem + off[O_RED]);
-  m.ci = (int *)(smem + off[O_CI]);
-  m.rp = (int *)(smem + off[O_RP]);
-  m.diag = (int *)(smem + off[O_DIAG]);
-  m.urp = (int *)(smem + off[O_URP]);
-  m.upos = (int *)(smem + off[O_UPOS]);
-  m.lrow = (int *)(smem + off[O_LROW]);
-  m.lptr = (int *)(smem + off[O_LPTR]);
-  m.urow = (int *)(smem + off[O_UROW]);
-  m.uptr = (int *)(smem + off[O_UPTR]);
-  m.trowg = (int *)(smem + off[O_TROWG]);
-  m.tgptr = (int *)(smem + off[O_TGPTR]);
-  m.tglong = (int *)(smem + off[O_TGLONG]);
-  m.tpos = (int *)(smem + off[O_TPOS]);
-  m.tpp = (int *)(smem + off[O_TPP]);
-  m.tpm = (int *)(smem + off[O_TPM]);
-  m.tq = (int *)(smem + off[O_TQ]);
-  m.lheavy = (int *)(smem + off[O_LHEAVY]);
+__device__ EntryView<T> lvl_view(char *smem, int n, int64_t nnz, const LvlDev &v, int mode) {
+  EntryView<T> m;
+  m.val = (T *)(smem + 16);
+  m.rd = (T *)(smem + 16 + pad16(sizeof(T) * size_t(nnz)));
+  m.y = (T *)((char *)m.rd + pad16(sizeof(T) * size_t(n)));
+  m.img = (const uint32_t *)((char *)m.y + pad16(sizeof(T) * size_t(n))) - lvl_first_word(v.h, mode);
+  m.h = v.h;
   return m;
 }
 
-// Stage what `mode` needs.  The factor scatters A into the L\U positions and
-// keeps the FP64 copy of A the refinement uses; the solve takes the factor's
-// values, or (LVL_BOTH) keeps them in place.
+// Stages what `mode` needs; false (in every thread) when the image's copy did
+// not complete in time, which is reported.  The factor scatters A into the
+// L\U positions and keeps the FP64 copy of A the refinement uses; the solve
+// takes the factor's values.
 template <class T>
-__device__ void lvl_stage(const LuDev &d, const LvlDev &v, const LvlSmem<T> &m, int mode,
+__device__ bool lvl_stage(const LuDev &d, const LvlDev &v, const EntryView<T> &m, char *smem, int mode,
                           const double *__restrict__ a, double *__restrict__ a_copy, int64_t nnz_a,
-                          const T *__restrict__ val_in, int64_t nnz, const double *__restrict__ b) {
-  const int n = d.n;
+                          const T *__restrict__ val_in, int nnz, const double *__restrict__ b) {
+  const int n = d.n, tid = threadIdx.x, bd = blockDim.x;
+  const unsigned mb = smem_addr(smem);
+  if (tid == 0) {
+    const int w0 = lvl_first_word(v.h, mode);
+    const unsigned bytes = 4u * unsigned(lvl_words(v.h, mode));
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mb) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    expect_bytes(mb, bytes);
+    bulk_copy((void *)(m.img + w0), v.image + w0, bytes, mb);
+  }
+  constexpr int kU4 = 8;  // gathers in flight per thread
   if (mode & LVL_FACTOR) {
-    for (int64_t p = threadIdx.x; p < nnz; p += blockDim.x) {
-      const int s = __ldg(d.lu2a + p);
-      m.val[p] = s >= 0 ? T(a[s]) : T(0);
+    for (int p = tid; p < nnz; p += kU4 * bd) {
+      int s[kU4];
+      double t[kU4];
+#pragma unroll
+      for (int q = 0; q < kU4; ++q) s[q] = p + q * bd < nnz ? __ldg(d.lu2a + p + q * bd) : -1;
+#pragma unroll
+      for (int q = 0; q < kU4; ++q) t[q] = s[q] >= 0 ? a[s[q]] : 0.0;
+#pragma unroll
+      for (int q = 0; q < kU4; ++q)
+        if (p + q * bd < nnz) m.val[p + q * bd] = T(t[q]);
     }
     if (a_copy != a)
-      for (int64_t p = threadIdx.x; p < nnz_a; p += blockDim.x) a_copy[p] = a[p];
-    stage_ints(m.urp, v.urp32, n + 1);
-    stage_ints(m.upos, d.upos, v.nup);
-    stage_ints(m.trowg, v.tail_rowg, v.ntail + 1);
-    stage_ints(m.tgptr, v.tail_gptr, v.ngroups + 1);
-    stage_ints(m.tglong, v.tail_glong, v.ngroups);
-    stage_ints(m.tpos, v.tail_pos, v.npos);
-    stage_ints(m.tpp, v.tail_pp, v.npos + 1);
-    stage_ints(m.tpm, v.tail_pm, v.npairs);
-    stage_ints(m.tq, v.tail_q, v.npairs);
-    stage_ints(m.lheavy, v.lheavy, v.levels);
+      for (int64_t p = tid; p < nnz_a; p += bd) a_copy[p] = a[p];
   } else {
-    for (int64_t p = threadIdx.x; p < nnz; p += blockDim.x) m.val[p] = val_in[p];
-    for (int i = threadIdx.x; i < n; i += blockDim.x) m.rd[i] = ((const T *)d.rdiag)[i];
+#pragma unroll 4
+    for (int p = tid; p < nnz; p += bd) m.val[p] = val_in[p];
+    for (int i = tid; i < n; i += bd) m.rd[i] = ((const T *)d.rdiag)[i];
   }
-  stage_ints(m.ci, d.ci, int(nnz));
-  stage_ints(m.rp, d.rp, n + 1);
-  stage_ints(m.diag, d.diag, n);
-  stage_ints(m.lrow, v.lrow, v.tail0);
-  stage_ints(m.lptr, v.lptr, v.levels + 1);
-  if (mode & LVL_SOLVE) {
-    stage_ints(m.urow, v.urow, n);
-    stage_ints(m.uptr, v.uptr, v.ulevels + 1);
-    for (int i = threadIdx.x; i < n; i += blockDim.x) m.y[i] = T(b[__ldg(d.P + i)]);
+  if (mode & LVL_SOLVE)
+    for (int i = tid; i < n; i += bd) m.y[i] = T(b[__ldg(d.P + i)]);
+  __syncthreads();  // the barrier's initialisation, and the staged values
+  const int limit = int(__ldg(&d.ctrl[C_SPIN]));
+  if (!__syncthreads_or(!mbar_wait(mb, 0u, limit))) return true;
+  // report it, and let the copy land before the shared memory is released
+  if (tid == 0) {
+    atomicOr(&d.ctrl[C_STATUS], ST_TIMEOUT);
+    mbar_wait(mb, 0u, 1 << 22);
   }
+  __syncthreads();
+  return false;
 }
 
-// The factorisation in shared memory; ends with a barrier.
-template <class T>
-__device__ void lvl_factor(const LuDev &d, const LvlDev &v, const LvlSmem<T> &m) {
-  T *val = m.val, *rd = m.rd;
-  const int *ci = m.ci, *rp = m.rp, *diag = m.diag, *urp = m.urp, *upos = m.upos;
-  unsigned bad = 0xffffffffu;
-  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  for (int lv = 0; lv < v.levels; ++lv) {
-    // heavy rows: a warp each, the updates of one L entry spread over the
-    // lanes, the L entries in order (the same sequence per entry as below)
-    for (int t = m.lheavy[lv] + (threadIdx.x >> 5); t < m.lptr[lv + 1]; t += nw) {
-      const int i = m.lrow[t];
-      const int dp = diag[i];
-      int u = urp[i];
-      for (int p = rp[i]; p < dp; ++p) {
-        const int k = ci[p];
-        const T l = val[p] * rd[k];
-        const int q0 = diag[k] + 1, len = rp[k + 1] - q0;
-        for (int j = lane; j < len; j += 32) val[upos[u + j]] -= l * val[q0 + j];
-        u += len;
-        __syncwarp();
-        if (lane == 0) val[p] = l;
-      }
-      __syncwarp();
-      if (lane == 0) {
-        const T piv = val[dp];
-        if (bad_pivot(piv)) bad = min(bad, unsigned(i));
-        rd[i] = recip(piv);
-      }
-    }
-    for (int t = m.lptr[lv] + threadIdx.x; t < m.lheavy[lv]; t += blockDim.x) {
-      const int i = m.lrow[t];
-      const int dp = diag[i];
-      int u = urp[i];
-      for (int p = rp[i]; p < dp; ++p) {
-        const int k = ci[p];
-        const T l = val[p] * rd[k];
-        val[p] = l;
-        const int q0 = diag[k] + 1, len = rp[k + 1] - q0;
-        // four updates at a time, all loads before the stores: the targets are
-        // distinct positions of row i, the sources lie in row k
-        int j = 0;
-        for (; j + 4 <= len; j += 4) {
-          const int t0 = upos[u + j], t1 = upos[u + j + 1], t2 = upos[u + j + 2],
-                    t3 = upos[u + j + 3];
-          const T s0 = val[q0 + j], s1 = val[q0 + j + 1], s2 = val[q0 + j + 2],
-                  s3 = val[q0 + j + 3];
-          const T v0 = val[t0], v1 = val[t1], v2 = val[t2], v3 = val[t3];
-          val[t0] = v0 - l * s0;
-          val[t1] = v1 - l * s1;
-          val[t2] = v2 - l * s2;
-          val[t3] = v3 - l * s3;
-        }
-        for (; j < len; ++j) val[upos[u + j]] -= l * val[q0 + j];
-        u += len;
-      }
-      const T piv = val[dp];
-      if (bad_pivot(piv)) bad = min(bad, unsigned(i));
-      rd[i] = recip(piv);
-    }
-    __syncthreads();
-  }
-  // the tail: each position pulls its updates, group after group
-  for (int r = 0; r < v.ntail; ++r) {
-    const int i = v.tail0 + r, dp = diag[i];
-    for (int g = m.trowg[r]; g < m.trowg[r + 1]; ++g) {
-      for (int t = m.tgptr[g] + threadIdx.x; t < m.tglong[g]; t += blockDim.x) {
-        const int p = m.tpos[t];
-        T acc = val[p];
-        for (int j = m.tpp[t]; j < m.tpp[t + 1]; ++j) acc -= val[m.tpm[j]] * val[m.tq[j]];
-        val[p] = p < dp ? acc * rd[ci[p]] : acc;
-      }
-      // long pulls: a warp each, lane-strided partial sums added in a fixed
-      // butterfly
-      for (int t = m.tglong[g] + (threadIdx.x >> 5); t < m.tgptr[g + 1]; t += nw) {
-        const int p = m.tpos[t];
-        T part = T(0);
-        for (int j = m.tpp[t] + lane; j < m.tpp[t + 1]; j += 32) part += val[m.tpm[j]] * val[m.tq[j]];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-        if (lane == 0) {
-          const T acc = val[p] - part;
-          val[p] = p < dp ? acc * rd[ci[p]] : acc;
-        }
-      }
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-      const T piv = val[dp];
-      if (bad_pivot(piv)) bad = min(bad, unsigned(i));
-      rd[i] = recip(piv);
-    }
-    __syncthreads();
-  }
-  if (bad != 0xffffffffu) {
-    atomicOr(&d.ctrl[C_STATUS], ST_PIVOT);
-    atomicMin(&d.ctrl[C_BAD_ROW], bad);
-  }
-}
-
-// x(Q) = U \ (L \ b(P)) in shared memory (y staged from b).
-template <class T>
-__device__ void lvl_solve(const LuDev &d, const LvlDev &v, const LvlSmem<T> &m,
-                          double *__restrict__ x) {
-  const int n = d.n;
-  const T *val = m.val, *rd = m.rd;
-  T *y = m.y, *red = m.red;
-  const int *ci = m.ci, *rp = m.rp, *diag = m.diag;
-  // y = L \ b(P): the levels, then the tail rows as block-wide dot products
-  for (int lv = 0; lv < v.levels; ++lv) {
-    for (int t = m.lptr[lv] + threadIdx.x; t < m.lptr[lv + 1]; t += blockDim.x) {
-      const int i = m.lrow[t];
-      T acc = y[i];
-      for (int p = rp[i]; p < diag[i]; ++p) acc -= val[p] * y[ci[p]];
-      y[i] = acc;
-    }
-    __syncthreads();
-  }
-  for (int i = v.tail0; i < n; ++i) {
-    T part = T(0);
-    for (int p = rp[i] + threadIdx.x; p < diag[i]; p += blockDim.x) part += val[p] * y[ci[p]];
-    red[threadIdx.x] = part;
-    __syncthreads();
-    // fixed pairing: the same sum on every run (blockDim is a power of two)
-    for (int h = blockDim.x >> 1; h > 0; h >>= 1) {
-      if (threadIdx.x < h) red[threadIdx.x] += red[threadIdx.x + h];
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) y[i] -= red[0];
-    __syncthreads();
-  }
-  // z = U \ y in place: a row reads only rows of lower U levels
-  for (int lv = 0; lv < v.ulevels; ++lv) {
-    for (int t = m.uptr[lv] + threadIdx.x; t < m.uptr[lv + 1]; t += blockDim.x) {
-      const int i = m.urow[t];
-      T acc = y[i];
-      for (int p = diag[i] + 1; p < rp[i + 1]; ++p) acc -= val[p] * y[ci[p]];
-      y[i] = acc * rd[i];
-    }
-    __syncthreads();
-  }
-  for (int i = threadIdx.x; i < n; i += blockDim.x) x[__ldg(d.Q + i)] = double(y[i]);
-}
-
-template <class T>
-__device__ void lvl_open(const LuDev &d) {
+__device__ __forceinline__ void lvl_open(const LuDev &d) {
   if (threadIdx.x == 0) {
     d.ctrl[C_STATUS] = 0;
     d.ctrl[C_BAD_ROW] = 0xffffffffu;
@@ -1594,52 +1377,53 @@ __device__ void lvl_open(const LuDev &d) {
 }
 
 template <class T>
-__device__ void lvl_store_factor(const LuDev &d, const LvlSmem<T> &m, T *__restrict__ val_out,
-                                 int64_t nnz) {
-  for (int64_t p = threadIdx.x; p < nnz; p += blockDim.x) val_out[p] = m.val[p];
+__device__ void lvl_close_factor(const LuDev &d, const EntryView<T> &m, unsigned bad, T *__restrict__ val_out,
+                                 int nnz) {
+  for (int p = threadIdx.x; p < nnz; p += blockDim.x) val_out[p] = m.val[p];
   for (int i = threadIdx.x; i < d.n; i += blockDim.x) ((T *)d.rdiag)[i] = m.rd[i];
+  if (bad != 0xffffffffu) {
+    atomicOr(&d.ctrl[C_STATUS], ST_PIVOT);
+    atomicMin(&d.ctrl[C_BAD_ROW], bad);
+  }
 }
 
 template <class T>
 __global__ void __launch_bounds__(1024) lu_factor_lvl(LuDev d, LvlDev v, const double *__restrict__ a,
                                                       double *__restrict__ a_copy, int64_t nnz_a,
-                                                      T *__restrict__ val_out, int64_t nnz) {
+                                                      T *__restrict__ val_out, int nnz) {
   extern __shared__ __align__(16) char smem[];
-  const LvlSmem<T> m = lvl_smem<T>(smem, d.n, nnz, v, LVL_FACTOR);
-  lvl_open<T>(d);
-  lvl_stage<T>(d, v, m, LVL_FACTOR, a, a_copy, nnz_a, nullptr, nnz, nullptr);
-  __syncthreads();
-  lvl_factor<T>(d, v, m);
-  lvl_store_factor<T>(d, m, val_out, nnz);
+  const EntryView<T> m = lvl_view<T>(smem, d.n, nnz, v, LVL_FACTOR);
+  lvl_open(d);
+  if (!lvl_stage<T>(d, v, m, smem, LVL_FACTOR, a, a_copy, nnz_a, nullptr, nnz, nullptr)) return;
+  const unsigned bad = factor_entries<T, false>(m);
+  lvl_close_factor<T>(d, m, bad, val_out, nnz);
 }
 
 template <class T>
-__global__ void __launch_bounds__(1024) lu_solve_lvl(LuDev d, LvlDev v, const T *__restrict__ val_in,
-                                                     int64_t nnz, const double *__restrict__ b,
-                                                     double *__restrict__ x) {
+__global__ void __launch_bounds__(1024) lu_solve_lvl(LuDev d, LvlDev v, const T *__restrict__ val_in, int nnz,
+                                                     const double *__restrict__ b, double *__restrict__ x) {
   extern __shared__ __align__(16) char smem[];
-  const LvlSmem<T> m = lvl_smem<T>(smem, d.n, nnz, v, LVL_SOLVE);
-  lvl_stage<T>(d, v, m, LVL_SOLVE, nullptr, nullptr, 0, val_in, nnz, b);
-  __syncthreads();
-  lvl_solve<T>(d, v, m, x);
+  const EntryView<T> m = lvl_view<T>(smem, d.n, nnz, v, LVL_SOLVE);
+  if (!lvl_stage<T>(d, v, m, smem, LVL_SOLVE, nullptr, nullptr, 0, val_in, nnz, b)) return;
+  forward_entries<T>(m);
+  backward_entries<T>(m);
+  for (int i = threadIdx.x; i < d.n; i += blockDim.x) x[__ldg(d.Q + i)] = double(m.y[i]);
 }
 
-// Refactor, keep the factor, then solve with it while it is in shared memory.
+// Refactor with the forward solve in step, keep the factor, solve backward.
 template <class T>
-__global__ void __launch_bounds__(1024) lu_factor_solve_lvl(LuDev d, LvlDev v,
-                                                            const double *__restrict__ a,
-                                                            double *__restrict__ a_copy,
-                                                            int64_t nnz_a, T *__restrict__ val_out,
-                                                            int64_t nnz, const double *__restrict__ b,
-                                                            double *__restrict__ x) {
+__global__ void __launch_bounds__(1024) lu_factor_solve_lvl(LuDev d, LvlDev v, const double *__restrict__ a,
+                                                            double *__restrict__ a_copy, int64_t nnz_a,
+                                                            T *__restrict__ val_out, int nnz,
+                                                            const double *__restrict__ b, double *__restrict__ x) {
   extern __shared__ __align__(16) char smem[];
-  const LvlSmem<T> m = lvl_smem<T>(smem, d.n, nnz, v, LVL_BOTH);
-  lvl_open<T>(d);
-  lvl_stage<T>(d, v, m, LVL_BOTH, a, a_copy, nnz_a, nullptr, nnz, b);
-  __syncthreads();
-  lvl_factor<T>(d, v, m);
-  lvl_store_factor<T>(d, m, val_out, nnz);
-  lvl_solve<T>(d, v, m, x);
+  const EntryView<T> m = lvl_view<T>(smem, d.n, nnz, v, LVL_BOTH);
+  lvl_open(d);
+  if (!lvl_stage<T>(d, v, m, smem, LVL_BOTH, a, a_copy, nnz_a, nullptr, nnz, b)) return;
+  const unsigned bad = factor_entries<T, true>(m);
+  lvl_close_factor<T>(d, m, bad, val_out, nnz);
+  backward_entries<T>(m);
+  for (int i = threadIdx.x; i < d.n; i += blockDim.x) x[__ldg(d.Q + i)] = double(m.y[i]);
 }
 
 // Shared memory of lu_solve_chain: the tile and entry rings, the block's
@@ -1750,7 +1534,7 @@ struct xg_lu {
   size_t smem_lvl_factor = 0, smem_lvl_solve = 0;
   size_t smem_lvl_both = 0;                // > 0: the fused refactor + solve fits
   int lvl_threads = 0;
-  int *d_lvl = nullptr;                    // level lists, row starts and tail, one buffer
+  uint32_t *d_lvl = nullptr;               // the schedule's image
   xg::LvlDev lvl_dev{};
   xg::FrontLu *front = nullptr;            // the multifrontal path (lu_front.h); nothing above then
   bool factored = false;
@@ -1801,7 +1585,7 @@ int refactor_t(xg_lu *lu, const double *dev_values) {
   }
   if (lu->lvl) {
     xg::lu_factor_lvl<T><<<1, lu->lvl_threads, lu->smem_lvl_factor, lu->stream>>>(
-        d, lu->lvl_dev, dev_values, lu->d_a, lu->S.nnz_a, (T *)lu->d_val, lu->nnz_lu);
+        d, lu->lvl_dev, dev_values, lu->d_a, lu->S.nnz_a, (T *)lu->d_val, int(lu->nnz_lu));
     xg::count_launches(1);
     XG_CU(cudaGetLastError());
     return XG_OK;
@@ -1842,7 +1626,7 @@ int solve_once(xg_lu *lu, const double *b, double *x) {
   }
   if (lu->lvl) {
     xg::lu_solve_lvl<T><<<1, lu->lvl_threads, lu->smem_lvl_solve, lu->stream>>>(
-        d, lu->lvl_dev, (const T *)lu->d_val, lu->nnz_lu, b, x);
+        d, lu->lvl_dev, (const T *)lu->d_val, int(lu->nnz_lu), b, x);
     xg::count_launches(1);
     XG_CU(cudaGetLastError());
     return XG_OK;
@@ -1917,7 +1701,7 @@ int refactor_solve_t(xg_lu *lu, const double *dev_values, const double *b, doubl
   }
   xg::LuDev d = lu->dev();
   xg::lu_factor_solve_lvl<T><<<1, lu->lvl_threads, lu->smem_lvl_both, lu->stream>>>(
-      d, lu->lvl_dev, dev_values, lu->d_a, lu->S.nnz_a, (T *)lu->d_val, lu->nnz_lu, b, x);
+      d, lu->lvl_dev, dev_values, lu->d_a, lu->S.nnz_a, (T *)lu->d_val, int(lu->nnz_lu), b, x);
   xg::count_launches(1);
   XG_CU(cudaGetLastError());
   for (int it = 0; it < n_refine; ++it) {
@@ -2063,9 +1847,8 @@ extern "C" int xg_lu_analyze(xg_ctx *ctx, int n, const int *host_rowptr, const i
       (rc = upload(&lu->d_P, S.P)) || (rc = upload(&lu->d_Q, S.Q)) ||
       (rc = upload(&lu->d_urp, S.urp)) || (rc = upload(&lu->d_upos, S.upos)))
     return fail(rc);
-  const int64_t nup = S.urp[n];
-  std::vector<int> urp32;  // the row starts as int, for the level path
-  if (nup < (int64_t(1) << 31)) urp32.assign(S.urp.begin(), S.urp.end());
+  xg::LuEntries entries;  // the level path's schedule
+  const bool have_entries = !std::getenv("XG_LU_NO_LVL") && xg::lu_build_entries(S, &entries);
   // the schedule lives on the device only
   std::vector<int64_t>().swap(lu->S.urp);
   std::vector<int>().swap(lu->S.upos);
@@ -2230,80 +2013,36 @@ extern "C" int xg_lu_analyze(xg_ctx *ctx, int n, const int *host_rowptr, const i
   // level-by-level path when its whole working set fits in shared memory and
   // the levels hold several rows each (a chain of single rows is walked faster
   // by the one lane of the narrow path)
-  if (!std::getenv("XG_LU_NO_LVL") && !lu->narrow && !urp32.empty() &&
-      lu->nnz_lu < (int64_t(1) << 31)) {
-    // lrow | lptr | urow | uptr | urp32 | tail_rowg | tail_gptr | tail_pos | tail_pp | tail_pm |
-    // tail_q | tail_glong | lheavy
-    const std::vector<int> *parts[] = {&S.lrow, &S.lptr, &S.urow, &S.uptr, &urp32, &S.tail_rowg,
-                                       &S.tail_gptr, &S.tail_pos, &S.tail_pp, &S.tail_pm, &S.tail_q,
-                                       &S.tail_glong, &S.lheavy};
-    size_t start[13], total = 0;
-    for (int k = 0; k < 13; ++k) { start[k] = total; total += parts[k]->size(); }
-    xg::LvlDev v{};
-    v.levels = int(S.lptr.size()) - 1;
-    v.ulevels = int(S.uptr.size()) - 1;
-    v.nup = int(nup);
-    v.tail0 = S.tail0;
-    v.ntail = int(S.tail_rowg.size()) - 1;
-    v.ngroups = int(S.tail_gptr.size()) - 1;
-    v.npos = int(S.tail_pos.size());
-    v.npairs = int(S.tail_pm.size());
-    // threads: the widest level or tail group, in warps, 1 to 32
-    int maxw = 1;
-    for (int l = 0; l < v.levels; ++l) maxw = std::max(maxw, S.lptr[l + 1] - S.lptr[l]);
-    for (int l = 0; l < v.ulevels; ++l) maxw = std::max(maxw, S.uptr[l + 1] - S.uptr[l]);
-    for (int g = 0; g < v.ngroups; ++g) maxw = std::max(maxw, S.tail_gptr[g + 1] - S.tail_gptr[g]);
-    // a power of two (the tail reduction); 1,024 threads when there are heavy
-    // rows (a warp each) or the widest level needs them, else 256, so the
-    // staging keeps many loads in flight
-    int threads = 256;
-    for (int l = 0; l < v.levels; ++l)
-      if (S.lheavy[l] < S.lptr[l + 1]) maxw = std::max(maxw, 1024);
-    while (threads < maxw && threads < 1024) threads *= 2;
-    size_t off[xg::O_END + 1];
-    const size_t fb = xg::lvl_layout(n, lu->nnz_lu, v, threads, tsz, xg::LVL_FACTOR, off);
-    const size_t sb = xg::lvl_layout(n, lu->nnz_lu, v, threads, tsz, xg::LVL_SOLVE, off);
-    const size_t bb = xg::lvl_layout(n, lu->nnz_lu, v, threads, tsz, xg::LVL_BOTH, off);
+  if (have_entries && !lu->narrow) {
+    const xg::LuEntriesHead &h = entries.head;
+    // as many threads as the widest level has entries, 256 to 512: more cost
+    // a level's barrier more than they save in its widest levels (the
+    // 1,000-stage chain's step: 48.0, 45.1 and 47.5 us with 256, 512 and 1,024
+    // before a kind of entry started a new warp)
+    const int threads = h.max_width <= 256 ? 256 : 512;
+    const size_t fb = xg::lvl_smem_bytes(n, lu->nnz_lu, h, tsz, xg::LVL_FACTOR);
+    const size_t sb = xg::lvl_smem_bytes(n, lu->nnz_lu, h, tsz, xg::LVL_SOLVE);
+    const size_t bb = xg::lvl_smem_bytes(n, lu->nnz_lu, h, tsz, xg::LVL_BOTH);
     int max_optin = 0;
     cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, lu->device);
     const size_t limit = size_t(max_optin) > 8192 ? size_t(max_optin) - 4096 : 0;
     if (fb <= limit && sb <= limit) {
-      cudaError_t e1, e2;
-      if (precision == XG_LU_FP32) {
-        e1 = xg::allow_dynamic_smem((const void *)xg::lu_factor_lvl<float>, fb);
-        e2 = xg::allow_dynamic_smem((const void *)xg::lu_solve_lvl<float>, sb);
-      } else {
-        e1 = xg::allow_dynamic_smem((const void *)xg::lu_factor_lvl<double>, fb);
-        e2 = xg::allow_dynamic_smem((const void *)xg::lu_solve_lvl<double>, sb);
-      }
+      const bool f32 = precision == XG_LU_FP32;
+      const cudaError_t e1 = xg::allow_dynamic_smem(f32 ? (const void *)xg::lu_factor_lvl<float>
+                                                        : (const void *)xg::lu_factor_lvl<double>, fb);
+      const cudaError_t e2 = xg::allow_dynamic_smem(f32 ? (const void *)xg::lu_solve_lvl<float>
+                                                        : (const void *)xg::lu_solve_lvl<double>, sb);
       if (e1 == cudaSuccess && e2 == cudaSuccess) {
-        std::vector<int> buf;
-        buf.reserve(total);
-        for (auto *pv : parts) buf.insert(buf.end(), pv->begin(), pv->end());
-        if ((rc = upload(&lu->d_lvl, buf))) return fail(rc);
-        const int *b0 = lu->d_lvl;
-        v.lrow = b0 + start[0];
-        v.lptr = b0 + start[1];
-        v.urow = b0 + start[2];
-        v.uptr = b0 + start[3];
-        v.urp32 = b0 + start[4];
-        v.tail_rowg = b0 + start[5];
-        v.tail_gptr = b0 + start[6];
-        v.tail_pos = b0 + start[7];
-        v.tail_pp = b0 + start[8];
-        v.tail_pm = b0 + start[9];
-        v.tail_q = b0 + start[10];
-        v.tail_glong = b0 + start[11];
-        v.lheavy = b0 + start[12];
-        lu->lvl_dev = v;
+        if ((rc = upload(&lu->d_lvl, entries.image))) return fail(rc);
+        lu->lvl_dev = xg::LvlDev{lu->d_lvl, h};
         lu->lvl_threads = threads;
         lu->smem_lvl_factor = fb;
         lu->smem_lvl_solve = sb;
         lu->lvl = true;
         // the fused refactor + solve when both working sets fit together
         if (bb <= limit) {
-          const void *fn = precision == XG_LU_FP32 ? (const void *)xg::lu_factor_solve_lvl<float>
-                                                   : (const void *)xg::lu_factor_solve_lvl<double>;
+          const void *fn = f32 ? (const void *)xg::lu_factor_solve_lvl<float>
+                               : (const void *)xg::lu_factor_solve_lvl<double>;
           if (xg::allow_dynamic_smem(fn, bb) == cudaSuccess) lu->smem_lvl_both = bb;
         }
       } else {

@@ -674,6 +674,163 @@ bool lu_build_updates(LuSymbolic &S) {
   return true;
 }
 
+bool lu_build_entries(const LuSymbolic &S, LuEntries *E) {
+  const int n = S.n, nnz = S.rp[n];
+  *E = LuEntries();
+  if (nnz > 65535 || n > 16383 || S.urp[n] > 65535) return false;
+  LuEntriesHead &h = E->head;
+  // when each entry is final (-1: from the start), and its pairs
+  struct Work {
+    int level, pos, pair0, pairs;
+    uint32_t word;
+  };
+  std::vector<Work> work;
+  std::vector<int> lev(nnz, -1), ylev(n, -1), slev(n, -1), ulev(n, 0);
+  std::vector<std::vector<uint32_t>> pulls;
+  std::vector<uint32_t> pair;
+  for (int i = 0; i < n; ++i) {
+    const int s = S.rp[i], e = S.rp[i + 1], dp = S.diag[i];
+    pulls.assign(size_t(e - s), {});
+    int64_t u = S.urp[i];
+    for (int p = s; p < dp; ++p) {
+      const int k = S.ci[p];
+      for (int q = S.diag[k] + 1; q < S.rp[k + 1]; ++q)
+        pulls[size_t(S.upos[size_t(u++)] - s)].push_back(uint32_t(p) | uint32_t(q) << 16);
+    }
+    for (int p = s; p < e; ++p) {
+      const auto &pl = pulls[size_t(p - s)];
+      if (pl.empty() && p > dp) continue;
+      int l = -1;
+      for (uint32_t pq : pl) l = std::max(l, std::max(lev[pq & 0xffffu], lev[pq >> 16]));
+      if (p < dp) l = std::max(l, lev[S.diag[S.ci[p]]]);
+      lev[p] = l + 1;
+      const uint32_t kind = p < dp ? kEntryL : p == dp ? kEntryPivot : kEntryU;
+      const uint32_t aux = p < dp ? uint32_t(S.ci[p]) : uint32_t(i);
+      work.push_back(Work{lev[p], p, int(pair.size()), int(pl.size()), uint32_t(p) | aux << 16 | kind << 30});
+      pair.insert(pair.end(), pl.begin(), pl.end());
+    }
+    for (int p = s; p < dp; ++p) {
+      const int k = S.ci[p];
+      ylev[i] = std::max(ylev[i], std::max(lev[p], ylev[k]) + 1);
+      slev[i] = std::max(slev[i], slev[k] + 1);
+    }
+  }
+  for (int i = n - 1; i >= 0; --i)
+    for (int p = S.diag[i] + 1; p < S.rp[i + 1]; ++p) ulev[i] = std::max(ulev[i], ulev[S.ci[p]] + 1);
+  for (auto &w : work) h.levels = std::max(h.levels, w.level + 1);
+  for (int i = 0; i < n; ++i) {
+    h.levels = std::max(h.levels, ylev[i] + 1);
+    h.slevels = std::max(h.slevels, slev[i] + 1);
+    h.ulevels = std::max(h.ulevels, ulev[i] + 1);
+  }
+  h.n_work = int(work.size());
+  h.n_pair = int(pair.size());
+  // by level; in a level the short ones first, of one kind and length together
+  auto is_long = [](int c) { return c > kEntryLong; };
+  std::stable_sort(work.begin(), work.end(), [&](const Work &a, const Work &b) {
+    if (a.level != b.level) return a.level < b.level;
+    if (is_long(a.pairs) != is_long(b.pairs)) return is_long(b.pairs);
+    if (a.word >> 30 != b.word >> 30) return a.word >> 30 < b.word >> 30;
+    return a.pairs < b.pairs;
+  });
+  // a kind starts a new warp of its level's threads (a warp would take the
+  // kinds in turn): idle places fill the one before
+  {
+    std::vector<Work> padded;
+    for (size_t k = 0, level0 = 0; k < work.size(); ++k) {
+      const bool new_level = k == 0 || work[k].level != work[k - 1].level;
+      if (new_level) level0 = padded.size();
+      const bool lng = is_long(work[k].pairs);
+      if (!new_level && (work[k].word >> 30 != work[k - 1].word >> 30 || lng) && !is_long(work[k - 1].pairs))
+        while ((padded.size() - level0) % 32) padded.push_back(Work{work[k].level, 0, 0, 0, kEntryNone << 30});
+      padded.push_back(work[k]);
+      const bool last = k + 1 == work.size() || work[k + 1].level != work[k].level;
+      if (last && !lng)
+        while ((padded.size() - level0) % 32) padded.push_back(Work{work[k].level, 0, 0, 0, kEntryNone << 30});
+    }
+    work.swap(padded);
+    h.n_work = int(work.size());
+  }
+  std::vector<uint32_t> &img = E->image;
+  auto align = [&]() {
+    while (img.size() % 4) img.push_back(0);
+    return int(img.size());
+  };
+  auto put16 = [&](const std::vector<int> &v) {
+    const int at = align();
+    for (size_t k = 0; k < v.size(); k += 2)
+      img.push_back(uint32_t(v[k]) | (k + 1 < v.size() ? uint32_t(v[k + 1]) << 16 : 0u));
+    return at;
+  };
+  // per level {first short, first long}, then the end
+  auto bounds = [&](const std::vector<int> &level, const std::vector<char> &lng, int levels) {
+    std::vector<int> b(size_t(2 * levels + 1), 0), shorts(size_t(levels), 0), count(size_t(levels), 0);
+    for (size_t k = 0; k < level.size(); ++k) {
+      ++count[size_t(level[k])];
+      shorts[size_t(level[k])] += !lng[k];
+    }
+    int at = 0;
+    for (int l = 0; l < levels; ++l) {
+      b[size_t(2 * l)] = at;
+      b[size_t(2 * l + 1)] = at + shorts[size_t(l)];
+      at += count[size_t(l)];
+    }
+    b[size_t(2 * levels)] = at;
+    const int word = align();
+    for (int x : b) img.push_back(uint32_t(x));
+    return word;
+  };
+  // rows with a level, by level, short before long
+  auto rows = [&](const std::vector<int> &level, int levels, auto length, int *bound) {
+    std::vector<int> r, lv;
+    std::vector<char> lng;
+    for (int i = 0; i < n; ++i)
+      if (level[i] >= 0) r.push_back(i);
+    std::stable_sort(r.begin(), r.end(), [&](int a, int b) {
+      if (level[a] != level[b]) return level[a] < level[b];
+      if (is_long(length(a)) != is_long(length(b))) return is_long(length(b));
+      return length(a) < length(b);
+    });
+    for (int i : r) {
+      lv.push_back(level[i]);
+      lng.push_back(is_long(length(i)));
+    }
+    *bound = bounds(lv, lng, levels);
+    return put16(r);
+  };
+  auto l_length = [&](int i) { return S.diag[i] - S.rp[i]; };
+  auto u_length = [&](int i) { return S.rp[i + 1] - S.diag[i] - 1; };
+  {
+    std::vector<int> lv;
+    std::vector<char> lng;
+    for (auto &w : work) {
+      lv.push_back(w.level);
+      lng.push_back(is_long(w.pairs));
+    }
+    h.ebound = bounds(lv, lng, h.levels);
+    std::vector<int> width(size_t(h.levels), 0);
+    for (int l : lv) h.max_width = std::max(h.max_width, ++width[size_t(l)]);
+  }
+  h.work = align();
+  for (auto &w : work) {
+    img.push_back(w.word);
+    img.push_back(uint32_t(w.pair0) | uint32_t(w.pairs) << 16);
+  }
+  h.pair = align();
+  img.insert(img.end(), pair.begin(), pair.end());
+  h.factor = align();
+  h.frow = rows(ylev, h.levels, l_length, &h.fbound);
+  h.solve0 = align();
+  h.ci = put16(S.ci);
+  h.rp = put16(S.rp);
+  h.diag = put16(S.diag);
+  h.urow = rows(ulev, h.ulevels, u_length, &h.ubound);
+  h.both = align();
+  h.srow = rows(slev, h.slevels, l_length, &h.sbound);
+  h.words = align();
+  return true;
+}
+
 double lu_model_seconds(const LuSymbolic &S) {
   // dependent steps cost a fixed latency each, independent work a rate
   return S.levels * kLuLevelSeconds + S.refactor_flops * kLuFlopSeconds;

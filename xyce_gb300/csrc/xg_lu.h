@@ -84,7 +84,7 @@ constexpr int kTailMaxRows = 16;
 // multiply-add.
 constexpr int kNdMinLevels = 64;
 constexpr double kNdMaxRowsPerLevel = 8.0;  // and minimum degree averages fewer rows per level
-constexpr int kNdLeaf = 16;
+constexpr int kNdLeaf = 4;  // 1,000-stage chain: 12 row levels against 22 with 16, the same fill
 constexpr double kLuLevelSeconds = 2e-6;
 constexpr double kLuFlopSeconds = 2e-10;
 double lu_model_seconds(const LuSymbolic &S);
@@ -109,6 +109,32 @@ int lu_analyze(int n, const int *rp, const int *ci, const double *val, double pi
 // the L\U pattern; false if an update falls outside the pattern (cannot
 // happen for a pattern lu_analyze made).
 bool lu_build_updates(LuSymbolic &S);
+
+// The elimination of a small factor entry by entry (lu_entries.cuh), as one
+// image of 32-bit words.  Its head says where each part starts; a bound list
+// holds, per level, where its short and its long members start.
+constexpr unsigned kEntryU = 0, kEntryL = 1, kEntryPivot = 2, kEntryNone = 3;
+constexpr int kEntryLong = 12;  // pairs or row entries a thread sums; longer ones take a warp
+struct LuEntriesHead {
+  int words = 0, solve0 = 0, both = 0;  // image; solve-only part [solve0, words); factor and solve [0, both)
+  int factor = 0;                       // factor only [0, factor)
+  int levels = 0, ulevels = 0, slevels = 0;
+  int n_work = 0, n_pair = 0, max_width = 0;
+  int ebound = 0, work = 0, pair = 0;   // entries: {position | row or column << 16 | kind << 30,
+                                        // first pair | pairs << 16}; pairs {L position | U position << 16}
+  int fbound = 0, frow = 0;             // forward rows by entry level
+  int ci = 0, rp = 0, diag = 0;         // the pattern in 16 bits
+  int ubound = 0, urow = 0;             // backward rows
+  int sbound = 0, srow = 0;             // forward rows by row level (a solve on its own)
+};
+struct LuEntries {
+  LuEntriesHead head;
+  std::vector<uint32_t> image;
+};
+// Fills the image from the pattern and the update schedule (lu_build_updates);
+// false when it needs more than 16-bit positions (65,535 entries or pairs,
+// 16,383 rows).
+bool lu_build_entries(const LuSymbolic &S, LuEntries *E);
 
 // Device address of an LU's status word (bits as xg_lu_status reports), for
 // callers that read it back together with other results.
