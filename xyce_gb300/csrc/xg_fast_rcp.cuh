@@ -20,9 +20,17 @@
 
 namespace xg {
 
+// b, opaque to the compiler: a division of it in a rarely taken branch stays
+// in the branch.  (Left to itself the compiler computes the division on the
+// common path too and selects: 361 cycles.)
+__device__ __forceinline__ double kept_apart(double b) {
+  asm volatile("mov.f64 %0, %0;" : "+d"(b));
+  return b;
+}
+
 __device__ __forceinline__ double fast_rcp(double b) {
   const unsigned e = (unsigned(__double2hiint(b)) >> 20) & 0x7ffu;
-  if (e - 23u > 2000u) return 1.0 / b;  // biased exponent outside [23, 2023]
+  if (e - 23u > 2000u) return 1.0 / kept_apart(b);  // biased exponent outside [23, 2023]
   double x;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(b));
   const double t = fma(-b, x, 1.0);
@@ -39,7 +47,7 @@ __device__ __forceinline__ double exact_sqrt(double b, double *r) {
 __device__ __forceinline__ double fast_sqrt(double b, double *r) {
   const unsigned e = unsigned(__double2hiint(b)) >> 20;  // sign included
   if (e - 123u > 1800u) {  // not a positive number of biased exponent [123, 1923]
-    const double s = sqrt(b);
+    const double s = sqrt(kept_apart(b));
     *r = 1.0 / s;
     return s;
   }
