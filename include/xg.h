@@ -258,7 +258,7 @@ int xg_load(xg_circuit *c, const xg_load_flags *flags);
  *                   left-looking threshold-partial-pivot factorisation of the
  *                   given values (KLU's tol 0.001, diagonal preferred) that
  *                   fixes the pivot order and the L\U pattern; uploads them.
- *                   Large matrices (8,192 rows and up) with long dependency
+ *                   Matrices too large for one SM with long dependency
  *                   chains are refactored by dense fronts over a nested-
  *                   dissection tree instead, when their multipliers on the
  *                   given values stay within the same tolerance; xg_lu_info

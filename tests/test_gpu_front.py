@@ -1,5 +1,5 @@
 """The multifrontal LU (lu_front.cu) through the C ABI, on matrices of at
-least 8,192 rows: backward error |b - A x| / (|A| |x| + |b|) <= 1e-13 in FP64
+least 8,192 rows and on smaller ones: backward error |b - A x| / (|A| |x| + |b|) <= 1e-13 in FP64
 and after three refinements of FP32 factors, as for the other LU paths; the
 same solution as the grid path to the error both may have; run-to-run bits;
 pivots and singular values reported."""
@@ -99,3 +99,31 @@ def test_pivots_that_grow_keep_the_grid_path(gpu_ctx):
     b = rng.standard_normal(n)
     x, st, _ = _solve(gpu_ctx, A, A, b, abi.LU_FP64, 0)
     assert st == 0 and _backward_error(A, x, b) <= 1e-13
+
+
+SMALLER = {
+    # too large for the level path and without a solve chain
+    "power_grid_20x20": lambda: netlists.power_grid(20, 20, 200, seed=1),
+    "power_grid_30x28": lambda: netlists.power_grid(30, 28, 400, seed=2),
+    "random_logic_2500": lambda: netlists.random_logic(2500, seed=4),
+    "inverter_chain_1700": lambda: netlists.inverter_chain(1700),
+    "inverter_chain_8000": lambda: netlists.inverter_chain(8000),
+}
+
+
+@pytest.mark.parametrize("precision,n_refine", [(abi.LU_FP64, 0), (abi.LU_FP32, 3)])
+@pytest.mark.parametrize("case", sorted(SMALLER))
+def test_smaller_matrices(case, precision, n_refine, gpu_ctx, oracle_lib, monkeypatch):
+    """Matrices below 8,192 rows: whichever path the rule takes meets the
+    same bound as the row-wise one it replaced."""
+    nl = SMALLER[case]()
+    A0, A = (circuit_jacobian(nl, seed=s, pdt=1e12) for s in (4, 5))
+    b = np.random.default_rng(7).standard_normal(A.shape[0])
+    x, st, info = _solve(gpu_ctx, A0, A, b, precision, n_refine)
+    again = _solve(gpu_ctx, A0, A, b, precision, n_refine)[0]
+    assert st == 0 and info.solve_chain == 0 and np.array_equal(x, again)
+    assert _backward_error(A, x, b) <= 1e-13
+    monkeypatch.setenv("XG_LU_NO_FRONT", "1")
+    other, st, _ = _solve(gpu_ctx, A0, A, b, precision, n_refine)
+    assert st == 0 and _backward_error(A, other, b) <= 1e-13
+    assert np.abs(x - other).max() <= 2e-7 * np.abs(other).max()  # as above

@@ -25,9 +25,9 @@
 //    trailing rows of one or two per level go to the chain kernel, 32
 //    columns at a time (lu_solve_chain, planned in lu_chain.h), and a long
 //    row no other row waits for to a block of its own (lu_solve_long).
-//  * large matrices (8,192 rows and up) whose dependency chains would cost
-//    more than a tree of dense fronts go to the multifrontal path
-//    (lu_front.h, lu_front.cu) instead; try_front below chooses.
+//  * matrices beyond the level path whose dependency chains would cost more
+//    than a tree of dense fronts go to the multifrontal path (lu_front.h,
+//    lu_front.cu) instead; try_front below chooses.
 //  * precision: factors in FP64, or in FP32 with FP64 iterative refinement
 //    (r = b - A x with the FP64 matrix, solve, x += d).
 //
@@ -1716,9 +1716,11 @@ int refactor_solve_t(xg_lu *lu, const double *dev_values, const double *b, doubl
   return XG_OK;
 }
 
-// Where the multifrontal path is tried.  Factors below kFrontMinRows rows
-// keep the bounded waits and the reported chain of the grid path, which their
-// callers observe.
+// Factors of this many rows try the multifrontal path before anything else.
+// Below, the level path is faster where a factor fits it (a 428-row grid 194
+// us against 200, a 1,604-row chain in FP32 98 against 565); the others try it
+// unless the grid path has a chain for them (xg_lu_info::solve_chain) and the
+// caller reads that (xg_lu_analyze; a transient does not).
 constexpr int kFrontMinRows = 8192;
 // The largest multiplier the chosen pivots may give in the tree's order: the
 // analysis accepts a pivot at 0.001 of its column (KLU's tolerance), which is
@@ -1726,25 +1728,30 @@ constexpr int kFrontMinRows = 8192;
 // checked on the analysed values.
 constexpr double kFrontMaxMultiplier = 1e3;
 
-// The grid path's refactor and solve, modelled: 2.8 us a level of its
-// longest dependency chain and 25 ps a multiply-add (power grids of 8,634 to
-// 120,002 rows and logic blocks of 17,000 to 200,000 devices took 0.75 to 1.2
-// times that), and 0.6 us an entry of the longest L row, which one warp walks (a
-// 9,000-stage chain's supply row: 5.5 ms).
-double grid_seconds(const xg::LuSymbolic &S) {
+// Refactor and solve on the row-wise paths, modelled: per level of the
+// longest dependency chain 2.8 us on the grid path with a chain, 5.4 us
+// without, 7 us in one CTA (power grids and logic blocks of 668 to 120,002
+// rows took 0.75 to 1.25 times that), 25 ps a multiply-add, and 0.6 us an entry of
+// the longest L row, which one warp walks (a 9,000-stage chain's supply row:
+// 5.5 ms).
+double row_seconds(const xg::LuSymbolic &S, bool one_cta, bool chain) {
   int longest = 0;
   for (int i = 0; i < S.n; ++i) longest = std::max(longest, S.diag[i] - S.rp[i]);
-  return std::max(2.8e-6 * S.levels + 25e-12 * S.refactor_flops, 0.6e-6 * longest);
+  const double level = one_cta ? 7e-6 : chain ? 2.8e-6 : 5.4e-6;
+  return std::max(level * S.levels + 25e-12 * S.refactor_flops, 0.6e-6 * longest);
 }
 
 // Tries the multifrontal path for an analysed matrix: lu->front when it is
-// modelled faster than the grid path and its multipliers stay within the
-// pivoting bound.  Measured, refactor and solve, grid / multifrontal: 200x200
-// power grid 7.2 / 2.0 ms, logic of 200,000 devices 21.4 / 2.5 ms.
-int try_front(xg_lu *lu, const int *rp, const int *ci, const double *values) {
+// modelled faster than `otherwise` and its multipliers stay within the
+// pivoting bound.  Measured, refactor and solve, row-wise / multifrontal:
+// 20x20 power grid (668 rows, one CTA) 490 / 225 us, 34x34 (1,928 rows, grid)
+// 736 / 366 us, 60x60 with its chain 842 / 605 us, 200x200 7.2 / 2.0 ms, logic
+// of 1,000, 6,000 and 200,000 devices 568 / 339 us, 1.77 / 0.76 ms and
+// 21.4 / 2.5 ms, a 4,000-stage chain 2.5 / 0.26 ms.
+int try_front(xg_lu *lu, const int *rp, const int *ci, const double *values, double otherwise) {
   const xg::LuSymbolic &S = lu->S;
   xg::FrontPlan plan;
-  if (!xg::build_front_plan(S, rp, ci, &plan) || plan.seconds > grid_seconds(S)) return XG_OK;
+  if (!xg::build_front_plan(S, rp, ci, &plan) || plan.seconds > otherwise) return XG_OK;
   int rc = XG_OK;
   xg::FrontLu *f = xg::front_create(plan, S, lu->device, lu->precision, &rc);
   if (!f) return XG_OK;  // no room: the grid path
@@ -1773,10 +1780,10 @@ int try_front(xg_lu *lu, const int *rp, const int *ci, const double *values) {
   return XG_OK;
 }
 
-}  // namespace
-
-extern "C" int xg_lu_analyze(xg_ctx *ctx, int n, const int *host_rowptr, const int *host_colidx,
-                             const double *host_values, int precision, xg_lu **out) {
+// xg_lu_analyze; any_path: no caller reads the chain of a factor below
+// kFrontMinRows.
+int analyze(xg_ctx *ctx, int n, const int *host_rowptr, const int *host_colidx, const double *host_values,
+            int precision, bool any_path, xg_lu **out) {
   if (!ctx || !out || n <= 0 || !host_rowptr || !host_colidx || !host_values ||
       (precision != XG_LU_FP64 && precision != XG_LU_FP32)) {
     xg::set_error("xg_lu_analyze: bad argument");
@@ -1830,8 +1837,12 @@ extern "C" int xg_lu_analyze(xg_ctx *ctx, int n, const int *host_rowptr, const i
       return cuda_fail(e, "xg_lu_analyze: cudaMemcpy");
     }
   }
-  if (n >= kFrontMinRows && !std::getenv("XG_LU_NO_FRONT")) {
-    if ((rc = try_front(lu.get(), host_rowptr, host_colidx, host_values))) return fail(rc);
+  const size_t tsz = precision == XG_LU_FP32 ? sizeof(float) : sizeof(double);
+  const bool front = !std::getenv("XG_LU_NO_FRONT");
+  const bool chain = front && xg::chain_start(S, tsz) < n;
+  if (n >= kFrontMinRows && front) {
+    rc = try_front(lu.get(), host_rowptr, host_colidx, host_values, row_seconds(S, false, chain));
+    if (rc) return fail(rc);
     if (lu->front) {
       *out = lu.release();
       return XG_OK;
@@ -1841,17 +1852,38 @@ extern "C" int xg_lu_analyze(xg_ctx *ctx, int n, const int *host_rowptr, const i
     xg::set_error("xg_lu_analyze: internal error, an update falls outside the L\\U pattern");
     return fail(XG_ERR_ARG);
   }
+  int max_optin = 0;
+  cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, lu->device);
+  const size_t smem_limit = size_t(max_optin) > 8192 ? size_t(max_optin) - 4096 : 0;
+  const size_t cta_bytes = xg::smem_bytes(n, lu->nnz_lu, tsz);
+  const bool cta_fits = cta_bytes <= smem_limit && !std::getenv("XG_LU_NO_CTA");
+  // average rows per level: little parallelism -> the one-lane walk
+  const bool narrow = cta_fits && double(n) / std::max(1, S.levels) < 3.0 && !std::getenv("XG_LU_NO_SEQ");
+  // level-by-level path when its whole working set fits in shared memory and
+  // the levels hold several rows each (a chain of single rows is walked faster
+  // by the one lane of the narrow path)
+  xg::LuEntries entries;
+  const bool level = !narrow && !std::getenv("XG_LU_NO_LVL") && xg::lu_build_entries(S, &entries) &&
+                     xg::lvl_smem_bytes(n, lu->nnz_lu, entries.head, tsz, xg::LVL_FACTOR) <= smem_limit &&
+                     xg::lvl_smem_bytes(n, lu->nnz_lu, entries.head, tsz, xg::LVL_SOLVE) <= smem_limit;
+  // (a switch that turns a row-wise path off asks for the next of them)
+  const bool forced = std::getenv("XG_LU_NO_CTA") || std::getenv("XG_LU_NO_LVL") || std::getenv("XG_LU_NO_SEQ");
+  if (n < kFrontMinRows && front && !forced && !level && !narrow && (cta_fits || any_path || !chain)) {
+    rc = try_front(lu.get(), host_rowptr, host_colidx, host_values, row_seconds(S, cta_fits, chain));
+    if (rc) return fail(rc);
+    if (lu->front) {
+      *out = lu.release();
+      return XG_OK;
+    }
+  }
   if ((rc = upload(&lu->d_rp, S.rp)) || (rc = upload(&lu->d_ci, S.ci)) ||
       (rc = upload(&lu->d_diag, S.diag)) || (rc = upload(&lu->d_lu2a, S.lu2a)) ||
       (rc = upload(&lu->d_P, S.P)) || (rc = upload(&lu->d_Q, S.Q)) ||
       (rc = upload(&lu->d_urp, S.urp)) || (rc = upload(&lu->d_upos, S.upos)))
     return fail(rc);
-  xg::LuEntries entries;  // the level path's schedule
-  const bool have_entries = !std::getenv("XG_LU_NO_LVL") && xg::lu_build_entries(S, &entries);
   // the schedule lives on the device only
   std::vector<int64_t>().swap(lu->S.urp);
   std::vector<int>().swap(lu->S.upos);
-  const size_t tsz = precision == XG_LU_FP32 ? sizeof(float) : sizeof(double);
   if ((e = cudaMalloc(&lu->d_val, tsz * size_t(lu->nnz_lu))) ||
       (e = cudaMalloc(&lu->d_y, tsz * size_t(n))) || (e = cudaMalloc(&lu->d_z, tsz * size_t(n))) ||
       (e = cudaMalloc(&lu->d_rdiag, tsz * size_t(n))))
@@ -1977,12 +2009,8 @@ extern "C" int xg_lu_analyze(xg_ctx *ctx, int n, const int *host_rowptr, const i
   }
   // one-CTA path when the factor (and the solve's extra vectors) fit in shared memory
   {
-    const size_t factor_b = xg::smem_bytes(n, lu->nnz_lu, tsz);
-    const size_t solve_b = factor_b;
-    int max_optin = 0;
-    cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, lu->device);
-    const size_t limit = size_t(max_optin) > 8192 ? size_t(max_optin) - 4096 : 0;
-    if (solve_b <= limit && factor_b <= limit && !std::getenv("XG_LU_NO_CTA")) {
+    const size_t factor_b = cta_bytes, solve_b = cta_bytes;
+    if (cta_fits) {
       cudaError_t e1, e2, e3, e4;
       if (precision == XG_LU_FP32) {
         e1 = xg::allow_dynamic_smem((const void *)xg::lu_factor_cta<float>, factor_b);
@@ -2002,17 +2030,13 @@ extern "C" int xg_lu_analyze(xg_ctx *ctx, int n, const int *host_rowptr, const i
         // as many warps as rows can be in flight, 2 to 32
         const int warps = std::max(2, std::min(32, lu->S.max_width));
         lu->cta_threads = 32 * warps;
-        // average rows per level: little parallelism -> the one-lane walk
-        lu->narrow = double(n) / std::max(1, lu->S.levels) < 3.0 && !std::getenv("XG_LU_NO_SEQ");
+        lu->narrow = narrow;
       } else {
         cudaGetLastError();
       }
     }
   }
-  // level-by-level path when its whole working set fits in shared memory and
-  // the levels hold several rows each (a chain of single rows is walked faster
-  // by the one lane of the narrow path)
-  if (have_entries && !lu->narrow) {
+  if (level) {
     const xg::LuEntriesHead &h = entries.head;
     // as many threads as the widest level has entries, 256 to 512: more cost
     // a level's barrier more than they save in its widest levels (the
@@ -2022,10 +2046,7 @@ extern "C" int xg_lu_analyze(xg_ctx *ctx, int n, const int *host_rowptr, const i
     const size_t fb = xg::lvl_smem_bytes(n, lu->nnz_lu, h, tsz, xg::LVL_FACTOR);
     const size_t sb = xg::lvl_smem_bytes(n, lu->nnz_lu, h, tsz, xg::LVL_SOLVE);
     const size_t bb = xg::lvl_smem_bytes(n, lu->nnz_lu, h, tsz, xg::LVL_BOTH);
-    int max_optin = 0;
-    cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, lu->device);
-    const size_t limit = size_t(max_optin) > 8192 ? size_t(max_optin) - 4096 : 0;
-    if (fb <= limit && sb <= limit) {
+    {
       const bool f32 = precision == XG_LU_FP32;
       const cudaError_t e1 = xg::allow_dynamic_smem(f32 ? (const void *)xg::lu_factor_lvl<float>
                                                         : (const void *)xg::lu_factor_lvl<double>, fb);
@@ -2039,7 +2060,7 @@ extern "C" int xg_lu_analyze(xg_ctx *ctx, int n, const int *host_rowptr, const i
         lu->smem_lvl_solve = sb;
         lu->lvl = true;
         // the fused refactor + solve when both working sets fit together
-        if (bb <= limit) {
+        if (bb <= smem_limit) {
           const void *fn = f32 ? (const void *)xg::lu_factor_solve_lvl<float>
                                : (const void *)xg::lu_factor_solve_lvl<double>;
           if (xg::allow_dynamic_smem(fn, bb) == cudaSuccess) lu->smem_lvl_both = bb;
@@ -2051,6 +2072,18 @@ extern "C" int xg_lu_analyze(xg_ctx *ctx, int n, const int *host_rowptr, const i
   }
   *out = lu.release();
   return XG_OK;
+}
+
+}  // namespace
+
+extern "C" int xg_lu_analyze(xg_ctx *ctx, int n, const int *host_rowptr, const int *host_colidx,
+                             const double *host_values, int precision, xg_lu **out) {
+  return analyze(ctx, n, host_rowptr, host_colidx, host_values, precision, false, out);
+}
+
+int xg::lu_analyze_transient(xg_ctx *ctx, int n, const int *host_rowptr, const int *host_colidx,
+                             const double *host_values, int precision, xg_lu **out) {
+  return analyze(ctx, n, host_rowptr, host_colidx, host_values, precision, true, out);
 }
 
 extern "C" int xg_lu_refactor(xg_lu *lu, const double *dev_values) {

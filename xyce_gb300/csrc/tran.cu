@@ -533,8 +533,8 @@ extern "C" int xg_tran_run(xg_circuit *c, const xg_tran_options *o, const double
     } else {
       reanalysed = true;
     }
-    return xg_lu_analyze(R.v.ctx, n, P.rowptr.data(), P.colidx.data(), hj.data(), o->lu_precision,
-                         &R.lu);
+    return lu_analyze_transient(R.v.ctx, n, P.rowptr.data(), P.colidx.data(), hj.data(), o->lu_precision,
+                                &R.lu);
   };
   const double tstep = o->tstep > 0 ? o->tstep : 1e-10;
   if ((rc = analyse(true, tstep))) { cleanup(); return rc; }

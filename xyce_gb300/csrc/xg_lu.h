@@ -78,11 +78,12 @@ constexpr int kTailMaxRows = 16;
 
 // Ordering choice: nested dissection is tried when minimum degree leaves a
 // dependency chain longer than kNdMinLevels rows with fewer than
-// kNdMaxRowsPerLevel rows per level on average; parts of at most kNdLeaf
-// vertices are ordered by minimum degree.  The refactorisation time model
+// kNdMaxRowsPerLevel rows per level on average (a 60-stage chain: 61 levels in
+// minimum-degree order, refactor and solve 85 us, 7 levels and 27 us in the
+// other); parts of at most kNdLeaf vertices are ordered by minimum degree.  The refactorisation time model
 // charges kLuLevelSeconds per dependent level and kLuFlopSeconds per
 // multiply-add.
-constexpr int kNdMinLevels = 64;
+constexpr int kNdMinLevels = 16;
 constexpr double kNdMaxRowsPerLevel = 8.0;  // and minimum degree averages fewer rows per level
 constexpr int kNdLeaf = 4;  // 1,000-stage chain: 12 row levels against 22 with 16, the same fill
 constexpr double kLuLevelSeconds = 2e-6;
@@ -135,6 +136,11 @@ struct LuEntries {
 // false when it needs more than 16-bit positions (65,535 entries or pairs,
 // 16,383 rows).
 bool lu_build_entries(const LuSymbolic &S, LuEntries *E);
+
+// xg_lu_analyze for a transient, which does not read xg_lu_info: small
+// factors with a solve chain may take the multifrontal path too.
+int lu_analyze_transient(xg_ctx *ctx, int n, const int *host_rowptr, const int *host_colidx,
+                         const double *host_values, int precision, xg_lu **out);
 
 // Device address of an LU's status word (bits as xg_lu_status reports), for
 // callers that read it back together with other results.
