@@ -42,39 +42,7 @@ struct LuSymbolic {
   // row i that U(k, ci[q]) updates.  urp[i] is where row i's updates start.
   std::vector<int64_t> urp;
   std::vector<int> upos;
-  // Rows grouped by dependency level for the level-by-level kernels: lrow
-  // lists the rows of L level 0, 1, ... (a row's L level is one more than the
-  // highest of the rows its L part names), lptr[l] where level l starts;
-  // urow/uptr the same for the backward solve, by U level.
-  std::vector<int> lrow, lptr, urow, uptr;
-  // Within level l the rows with more than kHeavyRowUpdates updates come
-  // last, from lheavy[l] on: a warp factors each of those (when the level
-  // has at most kMaxHeavyRows of them).
-  std::vector<int> lheavy;
-  // Trailing rows with long L parts (a supply rail ordered last has one L
-  // entry per device on it), and the rows after them, are left out of lrow:
-  // one thread would walk them serially.  They are factored one at a time after the levels, each with
-  // all threads: every position of the row pulls its updates (tail_pm[j] the
-  // row's own multiplier, tail_q[j] the U entry, in the order the row-wise
-  // elimination applies them), positions grouped so that a group reads only
-  // multipliers of earlier groups.  tail_pos lists the positions by group,
-  // tail_gptr[g] where group g starts, tail_rowg[r] the first group of row
-  // tail0 + r, tail_pp[t] where the pairs of tail_pos[t] start.  Within a
-  // group the positions with more than kTailLongPulls pairs come last, from
-  // tail_glong[g] on: a warp sums each of those (the diagonal of a supply
-  // rail pulls one pair per device on the rail).
-  int tail0 = 0;
-  std::vector<int> tail_rowg, tail_gptr, tail_glong, tail_pos, tail_pp, tail_pm, tail_q;
 };
-
-constexpr int kTailLongPulls = 32;
-constexpr int kHeavyRowUpdates = 32;
-constexpr int kMaxHeavyRows = 8;
-
-// The tail starts at the first of the last kTailMaxRows rows with more than
-// kTailMinL L entries.
-constexpr int kTailMinL = 64;
-constexpr int kTailMaxRows = 16;
 
 // Ordering choice: nested dissection is tried when minimum degree leaves a
 // dependency chain longer than kNdMinLevels rows with fewer than
