@@ -107,15 +107,18 @@ __global__ void tran_weights(int n, const double *xc, const double *x, double re
 
 // x += dx; optionally refresh the weights from the updated x (DC); partial
 // sums of (dx / w)^2.  Also copies the LU status word behind the partials, so
-// one read brings both back.
+// one read brings both back.  With xn0 (a transient's predictor) also the
+// sums of the local error test on the updated x, so that a step whose Newton
+// solve converges is tested without a pass and a round trip of its own: (x -
+// xn0)^2 and the max of |x_curr|.
 __global__ void __launch_bounds__(kThreads) tran_update(int n, const double *dx, double *x,
                                                         const double *xc, int reweight, double rel,
                                                         double abs_tol, double *w, double *partials,
-                                                        const unsigned *lu_status) {
+                                                        const unsigned *lu_status, const double *xn0) {
   __shared__ double sh[kThreads];
   if (blockIdx.x == 0 && threadIdx.x == 0)
     *reinterpret_cast<unsigned *>(partials + P_N * kRedBlocks) = *lu_status;
-  double s2 = 0.0;
+  double s2 = 0.0, e2 = 0.0, mx = 0.0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     double xi = x[i] + dx[i];
     x[i] = xi;
@@ -123,8 +126,17 @@ __global__ void __launch_bounds__(kThreads) tran_update(int n, const double *dx,
     if (reweight) w[i] = wi;
     double t = dx[i] / wi;
     s2 += t * t;
+    if (xn0) {
+      const double e = xi - xn0[i];
+      e2 += e * e;
+      mx = fmax(mx, fabs(xc[i]));
+    }
   }
   block_reduce(sh, s2, false, partials + P_DXW2 * kRedBlocks + blockIdx.x);
+  if (xn0) {
+    block_reduce(sh, e2, false, partials + P_ERR2 * kRedBlocks + blockIdx.x);
+    block_reduce(sh, mx, true, partials + P_XMAX * kRedBlocks + blockIdx.x);
+  }
 }
 
 // Predictor x = xh0 + b1 xh1 (+ b2 xh2), also kept as xn0; qn0 = qh0.
@@ -139,7 +151,8 @@ __global__ void tran_predict(int n, int order, double b1, double b2, const doubl
   }
 }
 
-// Partial sums of (x - xn0)^2 and the max of |x_curr|.
+// Partial sums of (x - xn0)^2 and the max of |x_curr| (a step without Newton
+// iterations).
 __global__ void __launch_bounds__(kThreads) tran_lte(int n, const double *x, const double *xn0,
                                                      const double *xc, double *partials) {
   __shared__ double sh[kThreads];
@@ -206,6 +219,8 @@ struct Run {
   int stall_count = 0;
   double stall_rate = 0.0;
   bool first_solve = true;
+  bool tested = false;  // the last transient Newton solve left the local error test's sums
+  double err2 = 0.0, xmax = 0.0;
   int grid = 1;
   std::string err;
 
@@ -316,6 +331,7 @@ struct Run {
   // library error code through *rc.
   int newton(bool transient, double h, int order, double time, int init_tran, int *rc) {
     *rc = XG_OK;
+    tested = false;
     const int max_step = transient ? 20 : 200;
     const double rhs_tol = transient ? 1e-2 : 1e-6;
     double dx_tol = transient ? 0.33 : 1.0;
@@ -353,7 +369,7 @@ struct Run {
       st->factorizations++;
       if ((*rc = xg_lu_refactor_solve(lu, jac, rhs, dx, o->n_refine))) return 0;
       tran_update<<<kRedBlocks, kThreads, 0, s>>>(n, dx, x, xc, !transient, rel_tol, abs_tol, w,
-                                                  partials, lu_status_device(lu));
+                                                  partials, lu_status_device(lu), transient ? xn0 : nullptr);
       xg::count_launches(1);
       fl.newton_iter = step;
       fl.init_jct = 0;
@@ -361,7 +377,14 @@ struct Run {
       if ((*rc = load(fl))) return 0;
       if ((*rc = combine(transient, order, h, r, false))) return 0;
       unsigned lu_status = 0;
-      if ((*rc = reduce({P_RHS2, P_RHSMAX, P_LIMMAX, P_DXW2}, r, &lu_status))) return 0;
+      if (transient) {
+        if ((*rc = reduce({P_RHS2, P_RHSMAX, P_LIMMAX, P_DXW2, P_ERR2, P_XMAX}, r, &lu_status))) return 0;
+        tested = true;
+        err2 = r[P_ERR2];
+        xmax = r[P_XMAX];
+      } else if ((*rc = reduce({P_RHS2, P_RHSMAX, P_LIMMAX, P_DXW2}, r, &lu_status))) {
+        return 0;
+      }
       any_limit = r[P_LIMMAX] != 0.0;
       if (lu_status) return -5;
       const double upd = std::sqrt(r[P_DXW2] / n);
@@ -713,12 +736,16 @@ extern "C" int xg_tran_run(xg_circuit *c, const xg_tran_options *o, const double
     bool ok = ns >= 0;
     double est = 0.0;
     if (ok && st->steps >= 1 && !beginning) {
-      tran_lte<<<kRedBlocks, kThreads, 0, R.s>>>(n, R.vec(XG_VEC_SOL_NEXT), R.xn0,
-                                                 R.vec(XG_VEC_SOL_CURR), R.partials); xg::count_launches(1);
-      double q[P_N];
-      if ((rc = R.reduce({P_ERR2, P_XMAX}, q))) { cleanup(); return rc; }
-      const double wt = reltol * q[P_XMAX] + abstol;
-      est = ck * std::sqrt(q[P_ERR2] / n) / wt;
+      if (!R.tested) {
+        tran_lte<<<kRedBlocks, kThreads, 0, R.s>>>(n, R.vec(XG_VEC_SOL_NEXT), R.xn0,
+                                                   R.vec(XG_VEC_SOL_CURR), R.partials); xg::count_launches(1);
+        double q[P_N];
+        if ((rc = R.reduce({P_ERR2, P_XMAX}, q))) { cleanup(); return rc; }
+        R.err2 = q[P_ERR2];
+        R.xmax = q[P_XMAX];
+      }
+      const double wt = reltol * R.xmax + abstol;
+      est = ck * std::sqrt(R.err2 / n) / wt;
       ok = est <= 1.0;
     }
     if (ok) {
