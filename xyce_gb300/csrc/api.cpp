@@ -565,15 +565,16 @@ int xg_update_state(xg_circuit *c, const xg_load_flags *flags) {
               flags->init_tran};
   xg::LoadIO io{c->d_sol[0], c->d_sta[1], c->d_sto[1], c->d_sta[0], c->d_sto[0], c->d_terms,
                 c->d_diode_vd, c->d_b3_mem, c->d_sta[1]};
+  xg::EvalType types[XG_NUM_DEV_TYPES];
+  int n_types = 0;
   for (int k = 0; k < P.n_order; ++k) {
-    int t = P.order[k];
+    const int t = P.order[k];
     const xg::TypeData &T = P.T[t];
-    if (!T.n) continue;
-    xg::DevType dt{T.n, T.nterm, T.sta0, T.sto0, T.term0, T.d_params, T.d_lid};
-    rc = c->opt.fma ? xg::fast::launch_eval(t, dt, o, f, io, c->ctx->stream)
-                    : xg::exact::launch_eval(t, dt, o, f, io, c->ctx->stream);
-    if (rc) return fail(rc, rc == XG_ERR_CUDA ? "eval kernel launch failed" : "unsupported device type");
+    if (T.n) types[n_types++] = {t, {T.n, T.nterm, T.sta0, T.sto0, T.term0, T.d_params, T.d_lid}};
   }
+  rc = c->opt.fma ? xg::fast::launch_evals(types, n_types, o, f, io, c->ctx->stream)
+                  : xg::exact::launch_evals(types, n_types, o, f, io, c->ctx->stream);
+  if (rc) return fail(rc, rc == XG_ERR_CUDA ? "eval kernel launch failed" : "unsupported device type");
   c->state_done = true;
   return XG_OK;
 }

@@ -136,8 +136,7 @@ __device__ __forceinline__ bool instance_live(const DevType &t, int i) {
 }
 
 // ---- resistor (N_DEV_Resistor.C:1073-1135) ---------------------------------
-__global__ void __launch_bounds__(256) res_kernel(DevType t, LoadIO io) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void res_one(const DevType &t, const LoadIO &io, int i) {
   if (i >= t.n || !instance_live(t, i)) return;
   const int n = t.n;
   int lp = ld(t.lid + i), ln = ld(t.lid + n + i);
@@ -153,8 +152,7 @@ __global__ void __launch_bounds__(256) res_kernel(DevType t, LoadIO io) {
 }
 
 // ---- capacitor, constant C, no IC (N_DEV_Capacitor.C:1821-2040) -------------
-__global__ void __launch_bounds__(256) cap_kernel(DevType t, LoadIO io) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void cap_one(const DevType &t, const LoadIO &io, int i) {
   if (i >= t.n || !instance_live(t, i)) return;
   const int n = t.n;
   int lp = ld(t.lid + i), ln = ld(t.lid + n + i);
@@ -189,8 +187,7 @@ __device__ double pulse_value(const double *p, int n, int i, double t) {
 }
 
 // ---- independent voltage source (N_DEV_Vsrc.C:941-1045) ---------------------
-__global__ void __launch_bounds__(256) vsrc_kernel(DevType t, Flags f, LoadIO io) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void vsrc_one(const DevType &t, Flags f, const LoadIO &io, int i) {
   if (i >= t.n || !instance_flags(t, i, f)) return;
   const int n = t.n;
   int lp = ld(t.lid + i), ln = ld(t.lid + n + i), lb = ld(t.lid + 2 * n + i);
@@ -214,8 +211,7 @@ __global__ void __launch_bounds__(256) vsrc_kernel(DevType t, Flags f, LoadIO io
 
 // ---- independent current source (N_DEV_ISRC.C:774-800) ----------------------
 // The source value goes into F at both terminals; there are no matrix entries.
-__global__ void __launch_bounds__(256) isrc_kernel(DevType t, Flags f, LoadIO io) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void isrc_one(const DevType &t, Flags f, const LoadIO &io, int i) {
   if (i >= t.n || !instance_flags(t, i, f)) return;
   const int n = t.n;
   double source;
@@ -229,8 +225,7 @@ __global__ void __launch_bounds__(256) isrc_kernel(DevType t, Flags f, LoadIO io
 }
 
 // ---- junction diode, level 1 (N_DEV_Diode.C:873-1331, 2007-2128) ------------
-__global__ void __launch_bounds__(256) diode_kernel(DevType t, DevOptions o, Flags f, LoadIO io) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void diode_one(const DevType &t, const DevOptions &o, Flags f, const LoadIO &io, int i) {
   if (i >= t.n || !instance_flags(t, i, f)) return;
   const int n = t.n;
   const double *p = t.p;
@@ -440,8 +435,7 @@ __device__ __forceinline__ void junction(double v, double sat, double vt, double
   c = fwd ? sat * (ev - 1) + gmin * v : cv;
 }
 
-__global__ void __launch_bounds__(128) mos1_kernel(DevType t, DevOptions o, Flags f, LoadIO io) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void mos1_one(const DevType &t, const DevOptions &o, Flags f, const LoadIO &io, int i) {
   if (i >= t.n || !instance_flags(t, i, f)) return;
   const int n = t.n;
   const double *p = t.p;
@@ -760,6 +754,58 @@ __global__ void __launch_bounds__(128) mos1_kernel(DevType t, DevOptions o, Flag
 
 #include "bsim3_eval.cuh"
 
+// ---- launches ------------------------------------------------------------------
+__global__ void __launch_bounds__(256) res_kernel(DevType t, LoadIO io) {
+  res_one(t, io, blockIdx.x * blockDim.x + threadIdx.x);
+}
+__global__ void __launch_bounds__(256) cap_kernel(DevType t, LoadIO io) {
+  cap_one(t, io, blockIdx.x * blockDim.x + threadIdx.x);
+}
+__global__ void __launch_bounds__(256) vsrc_kernel(DevType t, Flags f, LoadIO io) {
+  vsrc_one(t, f, io, blockIdx.x * blockDim.x + threadIdx.x);
+}
+__global__ void __launch_bounds__(256) isrc_kernel(DevType t, Flags f, LoadIO io) {
+  isrc_one(t, f, io, blockIdx.x * blockDim.x + threadIdx.x);
+}
+__global__ void __launch_bounds__(256) diode_kernel(DevType t, DevOptions o, Flags f, LoadIO io) {
+  diode_one(t, o, f, io, blockIdx.x * blockDim.x + threadIdx.x);
+}
+__global__ void __launch_bounds__(128) mos1_kernel(DevType t, DevOptions o, Flags f, LoadIO io) {
+  mos1_one(t, o, f, io, blockIdx.x * blockDim.x + threadIdx.x);
+}
+
+// All light types of a small circuit in one launch: where every instance is
+// resident at once a launch per type costs its start and its slowest warp in
+// turn.  Blocks of one warp spread the MOSFETs' FP64 instructions, 66 cycles
+// each on a sub-partition, over as many SMs as there are.  The MOSFETs' blocks
+// come first.  A load of a 101-stage chain (sources, MOSFETs, capacitors):
+// 26.6 us with three launches, 18.3 us with one; above one wave of warps the
+// launches' cost no longer shows.
+constexpr int kFewThreads = 32, kFewWarpsPerSm = 16;
+struct FewArgs {
+  int count;
+  int type[XG_NUM_DEV_TYPES], block0[XG_NUM_DEV_TYPES + 1];
+  DevType t[XG_NUM_DEV_TYPES];
+  DevOptions o;
+  Flags f;
+  LoadIO io;
+};
+__global__ void __launch_bounds__(kFewThreads) few_kernel(const __grid_constant__ FewArgs a) {
+  int k = 0;
+  while (k + 1 < a.count && (int)blockIdx.x >= a.block0[k + 1]) ++k;
+  const int i = ((int)blockIdx.x - a.block0[k]) * kFewThreads + (int)threadIdx.x;
+  const DevType t = a.t[k];
+  switch (a.type[k]) {
+    case XG_DEV_RES: res_one(t, a.io, i); break;
+    case XG_DEV_CAP: cap_one(t, a.io, i); break;
+    case XG_DEV_VSRC: vsrc_one(t, a.f, a.io, i); break;
+    case XG_DEV_ISRC: isrc_one(t, a.f, a.io, i); break;
+    case XG_DEV_DIODE: diode_one(t, a.o, a.f, a.io, i); break;
+    default: mos1_one(t, a.o, a.f, a.io, i); break;
+  }
+}
+
+
 // ---- fixed-order reduction ---------------------------------------------------
 // Each output is the sum of its terms in the reference's statement order,
 // s = ((0 + t1) + t2) + ..., so the result is bit-identical to a serial load.
@@ -860,8 +906,8 @@ int grid_for(int64_t n, int block) { return (int)((n + block - 1) / block); }
 
 }  // namespace
 
-int launch_eval(int dev_type, const DevType &t, const DevOptions &o, const Flags &f,
-                const LoadIO &io, void *stream) {
+static int launch_type(int dev_type, const DevType &t, const DevOptions &o, const Flags &f, const LoadIO &io,
+                       void *stream) {
   if (t.n <= 0) return XG_OK;
   cudaStream_t s = (cudaStream_t)stream;
   switch (dev_type) {
@@ -875,6 +921,40 @@ int launch_eval(int dev_type, const DevType &t, const DevOptions &o, const Flags
     default: return XG_ERR_UNSUPPORTED;
   }
   return cudaGetLastError() == cudaSuccess ? XG_OK : XG_ERR_CUDA;
+}
+
+// Evaluates the given types: one launch for the light ones where they leave
+// every SM at most kFewWarpsPerSm warps and there are two or more, else a
+// launch each.
+int launch_evals(const EvalType *types, int n, const DevOptions &o, const Flags &f, const LoadIO &io, void *stream) {
+  FewArgs a;
+  a.count = 0;
+  int64_t blocks = 0;
+  for (int pass = 0; pass < 2; ++pass)
+    for (int k = 0; k < n; ++k) {
+      const EvalType &e = types[k];
+      if (e.t.n <= 0 || e.type == XG_DEV_BSIM3 || (e.type == XG_DEV_MOS1) != (pass == 0)) continue;
+      if (e.type < 0 || e.type >= XG_NUM_DEV_TYPES || a.count >= XG_NUM_DEV_TYPES) return XG_ERR_UNSUPPORTED;
+      a.type[a.count] = e.type;
+      a.block0[a.count] = (int)std::min<int64_t>(blocks, INT32_MAX);
+      a.t[a.count++] = e.t;
+      blocks += (e.t.n + kFewThreads - 1) / kFewThreads;
+    }
+  const bool few = a.count > 1 && blocks <= (int64_t)sm_count() * kFewWarpsPerSm;
+  if (few) {
+    a.o = o;
+    a.f = f;
+    a.io = io;
+    few_kernel<<<(unsigned)blocks, kFewThreads, 0, (cudaStream_t)stream>>>(a);
+    xg::count_launches(1);
+    if (cudaGetLastError() != cudaSuccess) return XG_ERR_CUDA;
+  }
+  for (int k = 0; k < n; ++k) {
+    if (few && types[k].type != XG_DEV_BSIM3) continue;
+    const int rc = launch_type(types[k].type, types[k].t, o, f, io, stream);
+    if (rc) return rc;
+  }
+  return XG_OK;
 }
 
 int launch_reduce(const ReduceArgs &a, void *stream) {

@@ -89,17 +89,18 @@ extern "C" int xg_load_noalloc(xg_circuit *c, const xg_load_flags *flags, double
   xg::Flags f{flags->dcop, flags->tranop, flags->acop, flags->transient, flags->init_jct,
               flags->init_fix, flags->newton_iter, flags->inputop, flags->pdt, flags->time,
               flags->init_tran};
+  xg::EvalType types[XG_NUM_DEV_TYPES];
+  int n_types = 0;
   for (int k = 0; k < P.n_order; ++k) {
     const int t = P.order[k];
     const xg::TypeData &T = P.T[t];
-    if (!T.n) continue;
-    xg::DevType dt{T.n, T.nterm, T.sta0, T.sto0, T.term0, T.d_params, T.d_lid};
-    rc = v.fma ? xg::fast::launch_eval(t, dt, v.opt, f, io, v.stream)
-               : xg::exact::launch_eval(t, dt, v.opt, f, io, v.stream);
-    if (rc) {
-      xg::set_error("xg_load_noalloc: evaluation kernel launch failed");
-      return rc;
-    }
+    if (T.n) types[n_types++] = {t, {T.n, T.nterm, T.sta0, T.sto0, T.term0, T.d_params, T.d_lid}};
+  }
+  rc = v.fma ? xg::fast::launch_evals(types, n_types, v.opt, f, io, v.stream)
+             : xg::exact::launch_evals(types, n_types, v.opt, f, io, v.stream);
+  if (rc) {
+    xg::set_error("xg_load_noalloc: evaluation kernel launch failed");
+    return rc;
   }
   const xg::ReduceArgs ra = xg::reduce_args(P, scratch, v.red, dev_out, 0,
                                             P.n_out);

@@ -1166,19 +1166,21 @@ int enqueue_iteration(xg_batch *b) {
     count_launches(1);
   }
   Flags unused{};
+  EvalType types[XG_NUM_DEV_TYPES];
+  int n_types = 0;
   for (int k = 0; k < P.n_order; ++k) {
     const int t = P.order[k];
     const TypeData &T = P.T[t];
-    if (!T.n) continue;
-    DevType dt{T.n, T.nterm, T.sta0, T.sto0, T.term0, T.d_params, T.d_lid, b->d_cid[t], b->dev.flags};
-    int rc = v.fma ? fast::launch_eval(t, dt, v.opt, unused, v.io, s)
-                   : exact::launch_eval(t, dt, v.opt, unused, v.io, s);
-    if (rc) return rc;
+    if (T.n)
+      types[n_types++] = {t, {T.n, T.nterm, T.sta0, T.sto0, T.term0, T.d_params, T.d_lid, b->d_cid[t], b->dev.flags}};
   }
+  int rc = v.fma ? fast::launch_evals(types, n_types, v.opt, unused, v.io, s)
+                 : exact::launch_evals(types, n_types, v.opt, unused, v.io, s);
+  if (rc) return rc;
   double *out = nullptr;
   xg_vec_device_ptr(b->ckt, XG_VEC_F, &out);
   const ReduceArgs ra = reduce_args(P, v.io.terms, v.red, out, 0, P.n_out);
-  int rc = v.fma ? fast::launch_reduce(ra, s) : exact::launch_reduce(ra, s);
+  rc = v.fma ? fast::launch_reduce(ra, s) : exact::launch_reduce(ra, s);
   if (rc) return rc;
   batch_combine<<<b->nc, kBatchThreads, 0, s>>>(b->dev);
   // one warp per 32 requests: the step control is FP64-heavy (pow, sqrt,
@@ -2129,18 +2131,17 @@ PoolRed pool_red(const SlotPool *p) {
 // The evaluation launches over every type's whole instance array, with the
 // given circuit and flag arrays (the live ones, or the set-up ones).
 int pool_eval(const SlotPool *p, int *const *cid, const Flags *flags, cudaStream_t s) {
-  const LoadIO io = pool_io(p);
+  EvalType types[kTypes];
+  int n_types = 0;
   for (int t = 0; t < kTypes; ++t) {
     if (!p->NT[t]) continue;
     const TypeLayout &L = type_layout(t);
-    DevType dt{p->NT[t], L.nterm, int(p->sta0[t]), int(p->sto0[t]), p->term0[t], p->params[t],
-               p->lid[t], cid[t], flags};
-    Flags unused{};
-    const int rc = p->dopt.fma ? fast::launch_eval(t, dt, p->opt, unused, io, s)
-                               : exact::launch_eval(t, dt, p->opt, unused, io, s);
-    if (rc) return rc;
+    types[n_types++] = {t, {p->NT[t], L.nterm, int(p->sta0[t]), int(p->sto0[t]), p->term0[t], p->params[t],
+                            p->lid[t], cid[t], flags}};
   }
-  return XG_OK;
+  const Flags unused{};
+  return p->dopt.fma ? fast::launch_evals(types, n_types, p->opt, unused, pool_io(p), s)
+                     : exact::launch_evals(types, n_types, p->opt, unused, pool_io(p), s);
 }
 
 // One request, set up on the host and placed in its slot.

@@ -211,15 +211,19 @@ int ctx_options(xg_ctx *ctx, xg_device_options *o);
 std::vector<double> pulse_breakpoints(const Plan &P, double tstop, const int *lo = nullptr,
                                       const int *hi = nullptr);
 
+// One type's instances of an evaluation.
+struct EvalType {
+  int type;
+  DevType t;
+};
+
 // load_kernels.cu (two builds: bit-exact and FMA-contracted)
 namespace exact {
-int launch_eval(int dev_type, const DevType &t, const DevOptions &o, const Flags &f,
-                const LoadIO &io, void *stream);
+int launch_evals(const EvalType *types, int n, const DevOptions &o, const Flags &f, const LoadIO &io, void *stream);
 int launch_reduce(const ReduceArgs &a, void *stream);
 }  // namespace exact
 namespace fast {
-int launch_eval(int dev_type, const DevType &t, const DevOptions &o, const Flags &f,
-                const LoadIO &io, void *stream);
+int launch_evals(const EvalType *types, int n, const DevOptions &o, const Flags &f, const LoadIO &io, void *stream);
 int launch_reduce(const ReduceArgs &a, void *stream);
 }  // namespace fast
 
