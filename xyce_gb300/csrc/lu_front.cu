@@ -17,8 +17,8 @@
 //
 // Measured: the 253-row root of a 200x200 power grid in 259 us (429 with a
 // barrier per pivot and every CTA of the front reading the owner's shared
-// memory), a whole refactor and solve of that grid 2.04 ms (2.66), of 200,000
-// devices of logic 2.47 ms (2.91).
+// memory), a whole refactor and solve of that grid 1.96 ms, of 200,000 devices
+// of logic 2.37 ms.
 //
 // Every sum has a fixed order: results repeat bit for bit.
 
@@ -579,8 +579,11 @@ __global__ void front_check_rows(RowsDev R, int n, const double *__restrict__ a,
 }
 
 // One round of rows outside the tree (and the tree's right-hand sides, which
-// have no pivot here): a block per long row first, then a thread per row.
-// clear: flags the solve that follows starts from (nullptr: none).
+// have no pivot here): a cluster of kLongCtas blocks per long row first (a
+// supply's row has an entry per device on it: 65 us with a block for each of
+// 200,000 devices of logic's two), then a thread per row.  clear: flags the
+// solve that follows starts from (nullptr: none).
+constexpr int kLongCtas = 8;
 __global__ void __launch_bounds__(1024) front_rows(RowsDev R, int i0, int n_long, int n, const double *__restrict__ a,
                                                    const double *__restrict__ b, const int *__restrict__ P,
                                                    const int *__restrict__ Q, double *xk, double *x,
@@ -589,22 +592,31 @@ __global__ void __launch_bounds__(1024) front_rows(RowsDev R, int i0, int n_long
   const int bd = blockDim.x;
   if (clear)
     for (int k = blockIdx.x * bd + threadIdx.x; k < n_clear; k += gridDim.x * bd) clear[k] = 0;
-  const bool is_long = int(blockIdx.x) < n_long;
-  const int i = is_long ? i0 + int(blockIdx.x) : i0 + n_long + (int(blockIdx.x) - n_long) * bd + int(threadIdx.x);
+  const int block = int(blockIdx.x) - n_long * kLongCtas;
+  const bool is_long = block < 0;
+  const int i = is_long ? i0 + int(blockIdx.x) / kLongCtas : i0 + n_long + block * bd + int(threadIdx.x);
   if (i >= i0 + n) return;
   const int64_t e0 = R.ptr[i], e1 = R.ptr[i + 1];
   const int k = R.row[i], dg = R.diag[i];
   double s = 0.0;
   if (is_long) {
+    __shared__ double sums[kLongCtas];
+    const int rank = int(cluster_rank());
 #pragma unroll 8
-    for (int64_t e = e0 + threadIdx.x; e < e1; e += bd) s += a[R.a[e]] * xk[R.col[e]];
+    for (int64_t e = e0 + rank * bd + threadIdx.x; e < e1; e += kLongCtas * bd) s += a[R.a[e]] * xk[R.col[e]];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
     __syncthreads();
-    if (threadIdx.x) return;
-    s = part[0];
-    for (int w = 1; w < bd >> 5; ++w) s += part[w];
+    if (threadIdx.x == 0) {
+      s = part[0];
+      for (int w = 1; w < bd >> 5; ++w) s += part[w];
+      asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(remote(sums + rank, 0u)), "d"(s) : "memory");
+    }
+    cluster_sync();
+    if (rank || threadIdx.x) return;
+    s = sums[0];
+    for (int w = 1; w < kLongCtas; ++w) s += sums[w];
   } else {
     for (int64_t e = e0; e < e1; ++e) s += a[R.a[e]] * xk[R.col[e]];
   }
@@ -616,159 +628,263 @@ __global__ void __launch_bounds__(1024) front_rows(RowsDev R, int i0, int n_long
   xk[k] = v;
 }
 
-// Children whose border sums (forward) a row gathers: loads of four children
-// in flight at once, added in their order.
+// The children's border sums that row i of a front gathers, in their order.
+// Four children's places are found ahead of the wait for them, and their
+// loads are in flight together.
+constexpr int kAhead = 4;
+__device__ __forceinline__ void find_children(const FrontDev &d, const Front &f, int c0, int i, int64_t (&at)[kAhead]) {
+#pragma unroll
+  for (int q = 0; q < kAhead; ++q) {
+    at[q] = -1;
+    if (c0 + q < f.child1) {
+      const ChildDev &g = d.child[c0 + q];
+      const int k = __ldg(d.inv_map + g.inv + i);
+      if (k >= 0) at[q] = g.bv + k;
+    }
+  }
+}
 template <class T>
-__device__ __forceinline__ T gather_children(const FrontDev &d, const Front &f, int i) {
-  const T *bv = (const T *)d.bv;
-  T s = T(0);
-  int c = f.child0;
-  for (; c + 4 <= f.child1; c += 4) {
-    int at[4];
-    T v[4];
+__device__ __forceinline__ T add_children(const FrontDev &d, T s, const int64_t (&at)[kAhead]) {
+  T v[kAhead];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) at[q] = __ldg(d.inv_map + d.child[c + q].inv + i);
+  for (int q = 0; q < kAhead; ++q) v[q] = at[q] >= 0 ? __ldcg((const T *)d.bv + at[q]) : T(0);
 #pragma unroll
-    for (int q = 0; q < 4; ++q) v[q] = at[q] >= 0 ? __ldcg(bv + d.child[c + q].bv + at[q]) : T(0);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) s += v[q];
-  }
-  for (; c < f.child1; ++c) {
-    const int at = __ldg(d.inv_map + d.child[c].inv + i);
-    if (at >= 0) s += __ldcg(bv + d.child[c].bv + at);
-  }
+  for (int q = 0; q < kAhead; ++q) s += v[q];
   return s;
 }
 
-// y = L \ (right-hand side and the children's sums) for the front's pivots;
-// its border sums go to its parent.  Warp 0 resolves 32 pivots lane to lane
-// while the other warps fetch the entries they apply next (a block of one
-// warp does both in turn).
+// The solves of a front go 32 pivots at a time.  Warp 0 resolves a block lane
+// to lane (a pivot costs a shuffle and one FP64 instruction, 95 cycles); all
+// warps then bring the next 32 rows up to date, and the rows beyond them
+// follow while warp 0 resolves the next block.
+//
+// A block of fewer than 32 columns goes by eights, the last of them repeating
+// its last column with a factor of 0: loads under a condition each would go
+// one by one (up to 32 L2 round trips, 11 us a block).
+//
+// A lane's row of a block of pivots: its entries in the block's other columns
+// that are solved before it (below the diagonal forward, above it backward).
+template <class T, bool kUp>
+__device__ __forceinline__ void load_block(const T *L, int m, int kb, int nb, T (&w)[32]) {
+  const int lane = threadIdx.x & 31;
+  const T *col = L + int64_t(kb) * m + kb + min(lane, nb - 1);
+#pragma unroll
+  for (int g = 0; g < 32; g += 8)
+    if (g < nb)
+#pragma unroll
+      for (int t = g; t < g + 8; ++t) w[t] = col[int64_t(min(t, nb - 1)) * m];
+#pragma unroll
+  for (int t = 0; t < 32; ++t) w[t] = t < nb && lane < nb && (kUp ? lane > t : lane < t) ? w[t] : T(0);
+}
+// v less the columns [kb, kb + nb) in the rows [i0, i1): a row per thread (t
+// of n), ...
 template <class T>
-__device__ __forceinline__ void forward(const FrontDev &d, const Front &f, T *v) {
-  const int m = f.m, p = f.p, tid = threadIdx.x, bd = blockDim.x, lane = tid & 31;
-  const T *L = (const T *)d.l + f.lo;
-  for (int i = tid; i < m; i += bd) {
-    T s = gather_children<T>(d, f, i);
-    if (i < p) s += T(__ldcg(d.xk + __ldg(d.idx + f.idx + i)));
+__device__ __forceinline__ void apply_rows(const T *L, int m, T *v, int kb, int nb, int i0, int i1, int t, int n) {
+  for (int i = i0 + t; i < i1; i += n) {
+    T w[32], s = v[i];
+    if (nb == 32) {
+#pragma unroll
+      for (int q = 0; q < 32; ++q) w[q] = L[int64_t(kb + q) * m + i];
+#pragma unroll
+      for (int q = 0; q < 32; ++q) s -= w[q] * v[kb + q];
+    } else {
+      for (int g = 0; g < nb; g += 8) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) w[q] = L[int64_t(kb + min(g + q, nb - 1)) * m + i];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) s -= (g + q < nb ? w[q] : T(0)) * v[kb + min(g + q, nb - 1)];
+      }
+    }
     v[i] = s;
   }
+}
+// ... and in the 32 rows from i0 on: 8 rows to a warp, 8 columns to a lane.
+template <class T>
+__device__ __forceinline__ void apply_next(const T *L, int m, T *v, int kb, int nb, int i0, int i1) {
+  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5, c0 = (lane >> 3) * 8;
+  for (int g = threadIdx.x >> 5; g < 4; g += nw) {
+    const int i = i0 + 8 * g + (lane & 7), row = min(i, i1 - 1);
+    T w[8], s = T(0);
+#pragma unroll
+    for (int q = 0; q < 8; ++q) w[q] = L[int64_t(kb + min(c0 + q, nb - 1)) * m + row];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) s += (c0 + q < nb ? w[q] : T(0)) * v[kb + min(c0 + q, nb - 1)];
+    s += __shfl_xor_sync(0xffffffffu, s, 8);
+    s += __shfl_xor_sync(0xffffffffu, s, 16);
+    if (lane < 8 && i < i1) v[i] -= s;
+  }
+}
+
+// y = L \\ (right-hand side and the children's sums) for the front's pivots;
+// its border sums go to its parent.  What does not depend on other fronts is
+// loaded ahead: warp 0's first block, the other warps' row of it where it is
+// the only one, the places of the children's sums, the right-hand side.
+template <class T>
+struct Up {
+  T w[32], rhs;
+  int64_t at[kAhead];
+};
+template <class T>
+__device__ __forceinline__ void ahead(const FrontDev &d, const Front &f, Up<T> &a) {
+  const int m = f.m, p = f.p, tid = threadIdx.x, nb = min(32, p), i = nb + tid - 32;
+  const T *L = (const T *)d.l + f.lo;
+  if (tid < 32) {
+    load_block<T, true>(L, m, 0, nb, a.w);
+  } else if (p <= 32) {
+#pragma unroll
+    for (int g = 0; g < 32; g += 8)
+      if (g < nb)
+#pragma unroll
+        for (int q = g; q < g + 8; ++q) a.w[q] = L[int64_t(min(q, nb - 1)) * m + min(i, m - 1)];
+  }
+  a.rhs = tid < p ? T(__ldcg(d.xk + __ldg(d.idx + f.idx + tid))) : T(0);
+  if (tid < m) find_children(d, f, f.child0, tid, a.at);
+}
+template <class T>
+__device__ __forceinline__ void forward(const FrontDev &d, const Front &f, T *v, Up<T> &a) {
+  const int m = f.m, p = f.p, tid = threadIdx.x, bd = blockDim.x, lane = tid & 31, wid = tid >> 5, nw = bd >> 5;
+  const T *L = (const T *)d.l + f.lo;
+  for (int i = tid; i < m; i += bd) {
+    T r = a.rhs;
+    if (i != tid) {
+      r = i < p ? T(__ldcg(d.xk + __ldg(d.idx + f.idx + i))) : T(0);
+      find_children(d, f, f.child0, i, a.at);
+    }
+    T s = add_children<T>(d, T(0), a.at);
+    for (int c = f.child0 + kAhead; c < f.child1; c += kAhead) {
+      find_children(d, f, c, i, a.at);
+      s = add_children<T>(d, s, a.at);
+    }
+    v[i] = s + r;
+  }
   __syncthreads();
-  const int first = bd > 32 ? 32 : 0, step = bd - first;  // threads that apply
   for (int kb = 0; kb < p; kb += 32) {
     const int nb = min(32, p - kb);
-    T w[32];
-    const int i0 = kb + nb + tid - first;
-    if (tid < 32) {
+    if (wid == 0) {
       T s = lane < nb ? v[kb + lane] : T(0);
-#pragma unroll
-      for (int t = 0; t < 32; ++t) w[t] = t < nb && lane > t && lane < nb ? L[int64_t(kb + t) * m + kb + lane] : T(0);
 #pragma unroll
       for (int t = 0; t < 32; ++t) {
         if (t < nb) {
-          const T vt = __shfl_sync(0xffffffffu, s, t);
-          if (lane > t) s -= w[t] * vt;
+          const T vt = __shfl_sync(0xffffffffu, s, t), r = s - a.w[t] * vt;
+          s = lane > t ? r : s;
         }
       }
       if (lane < nb) {
         v[kb + lane] = s;
         ((T *)d.y)[f.pv + kb + lane] = s;
       }
-    } else if (i0 < m) {
-#pragma unroll
-      for (int t = 0; t < 32; ++t) w[t] = t < nb ? L[int64_t(kb + t) * m + i0] : T(0);
     }
+    if (kb > 0 && (wid > 0 || nw == 1))
+      apply_rows<T>(L, m, v, kb - 32, 32, kb + 32, m, nw == 1 ? tid : tid - 32, nw == 1 ? bd : bd - 32);
     __syncthreads();
-    if (tid >= first) {
-      for (int i = i0; i < m; i += step) {
-        if (first == 0 || i != i0) {
-#pragma unroll
-          for (int t = 0; t < 32; ++t) w[t] = t < nb ? L[int64_t(kb + t) * m + i] : T(0);
-        }
+    if (kb + 32 < p) {
+      if (wid == 0) load_block<T, true>(L, m, kb + 32, min(32, p - kb - 32), a.w);
+      apply_next<T>(L, m, v, kb, 32, kb + 32, m);
+    } else if (p <= 32 && nw > 1) {
+      const int i = nb + tid - 32;
+      if (wid > 0 && i < m) {
         T s = v[i];
 #pragma unroll
-        for (int t = 0; t < 32; ++t)
-          if (t < nb) s -= w[t] * v[kb + t];
+        for (int q = 0; q < 32; ++q)
+          if (q < nb) s -= a.w[q] * v[q];
         v[i] = s;
       }
+      apply_rows<T>(L, m, v, 0, nb, nb + bd - 32, m, tid, bd);
+    } else {
+      apply_rows<T>(L, m, v, kb, nb, kb + nb, m, tid, bd);
     }
     __syncthreads();
   }
   for (int i = p + tid; i < m; i += bd) ((T *)d.bv)[f.bv + i - p] = v[i];
 }
 
-// x = U \ (y - the border's part) for the front's pivots, border first; v
-// holds p + b values and one per thread.
+// x = U \\ (y - the border's part) for the front's pivots, border first; v
+// holds m values and p per warp.  Ahead: warp 0's last block, the first of a
+// warp's columns of U, the border's unknowns' places.
+constexpr int kAheadU = 8;
 template <class T>
-__device__ __forceinline__ void backward(const FrontDev &d, const Front &f, T *v, double *x) {
-  const int m = f.m, p = f.p, b = m - p, tid = threadIdx.x, bd = blockDim.x, lane = tid & 31;
-  T *xb = v + p;                      // the border's unknowns
-  T *red = xb + b;                    // partial sums, one per thread
-  const T *L = (const T *)d.l + f.lo, *U = (const T *)d.u + f.uo;
-  for (int j = tid; j < b; j += bd) xb[j] = T(__ldcg(d.xk + __ldg(d.idx + f.idx + p + j)));
-  __syncthreads();
-  // v = y - U x: threads in groups of one row each, a group per slice of the
-  // border, the slices added in order
-  const int rows = min(bd, (p + 31) & ~31), parts = bd / rows, part = tid / rows, ri = tid - part * rows;
-  for (int r0 = 0; r0 < p; r0 += rows) {
-    const int i = r0 + ri;
-    T s = T(0);
-    if (part < parts && i < p) {
-#pragma unroll 8
-      for (int j = part; j < b; j += parts) s += U[int64_t(j) * p + i] * xb[j];
-    }
-    red[tid] = s;
-    __syncthreads();
-    if (part == 0 && i < p) {
-      T t = __ldcg((const T *)d.y + f.pv + i);
-      for (int q = 0; q < parts; ++q) t -= red[q * rows + ri];
-      v[i] = t;
-    }
-    __syncthreads();
+struct Down {
+  T w[32], u[kAheadU], rd;
+  int at, own, own_x;
+};
+template <class T>
+__device__ __forceinline__ void ahead(const FrontDev &d, const Front &f, Down<T> &a) {
+  const int m = f.m, p = f.p, b = m - p, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nw = blockDim.x >> 5;
+  const int kb = (p - 1) / 32 * 32;
+  const T *U = (const T *)d.u + f.uo;
+  if (tid < 32) load_block<T, false>((const T *)d.l + f.lo, m, kb, p - kb, a.w);
+  a.rd = tid < p - kb ? ((const T *)d.rd)[f.pv + kb + tid] : T(0);
+#pragma unroll
+  for (int q = 0; q < kAheadU; ++q) {
+    const int j = wid + q * nw;
+    if (b > 0) a.u[q] = U[int64_t(min(j, b - 1)) * p + min(lane, p - 1)];
   }
-  const int first = bd > 32 ? 32 : 0, step = bd - first;
+  a.at = tid < b ? __ldg(d.idx + f.idx + p + tid) : 0;
+  a.own = tid < p ? __ldg(d.idx + f.idx + tid) : 0;
+  a.own_x = tid < p ? __ldg(d.Q + a.own) : 0;
+}
+template <class T>
+__device__ __forceinline__ void backward(const FrontDev &d, const Front &f, T *v, Down<T> &a, double *x) {
+  const int m = f.m, p = f.p, b = m - p, tid = threadIdx.x, bd = blockDim.x, lane = tid & 31;
+  const int wid = tid >> 5, nw = bd >> 5;
+  T *xb = v + p;                      // the border's unknowns
+  T *red = xb + b;                    // the warps' sums
+  const T *L = (const T *)d.l + f.lo, *U = (const T *)d.u + f.uo;
+  for (int j = tid; j < b; j += bd) xb[j] = T(__ldcg(d.xk + (j == tid ? a.at : __ldg(d.idx + f.idx + p + j))));
+  for (int i = tid; i < p; i += bd) v[i] = __ldcg((const T *)d.y + f.pv + i);
+  __syncthreads();
+  // v = y - U x: every warp a share of the border for all rows, the shares
+  // added in order
+  for (int i = lane; i < p; i += 32) {
+    T s = T(0);
+    int j = wid;
+    if (i == lane) {
+#pragma unroll
+      for (int q = 0; q < kAheadU; ++q, j += nw)
+        if (j < b) s += a.u[q] * xb[j];
+    }
+#pragma unroll 16
+    for (; j < b; j += nw) s += U[int64_t(j) * p + i] * xb[j];
+    red[wid * p + i] = s;
+  }
+  __syncthreads();
+  for (int i = tid; i < p; i += bd) {
+    T t = v[i];
+    for (int q = 0; q < nw; ++q) t -= red[q * p + i];
+    v[i] = t;
+  }
+  __syncthreads();
   for (int kb = ((p - 1) / 32) * 32; kb >= 0; kb -= 32) {
     const int nb = min(32, p - kb);
-    T w[32];
-    const int i0 = tid - first;
-    if (tid < 32) {
+    if (wid == 0) {
       T s = lane < nb ? v[kb + lane] : T(0);
-      const T rd = lane < nb ? ((const T *)d.rd)[f.pv + kb + lane] : T(0);
-#pragma unroll
-      for (int t = 0; t < 32; ++t) w[t] = t < nb && lane < t ? L[int64_t(kb + t) * m + kb + lane] : T(0);
 #pragma unroll
       for (int t = 31; t >= 0; --t) {
         if (t < nb) {
-          if (lane == t) s *= rd;
-          const T vt = __shfl_sync(0xffffffffu, s, t);
-          if (lane < t) s -= w[t] * vt;
+          const T vt = __shfl_sync(0xffffffffu, s, t) * __shfl_sync(0xffffffffu, a.rd, t);
+          const T r = s - a.w[t] * vt;
+          s = lane == t ? vt : lane < t ? r : s;
         }
       }
-      if (lane < nb) {
-        v[kb + lane] = s;
-        const int k = __ldg(d.idx + f.idx + kb + lane);
-        d.xk[k] = double(s);
-        x[__ldg(d.Q + k)] = double(s);
-      }
-    } else if (i0 < kb) {
-#pragma unroll
-      for (int t = 0; t < 32; ++t) w[t] = t < nb ? L[int64_t(kb + t) * m + i0] : T(0);
+      if (lane < nb) v[kb + lane] = s;
     }
+    if (kb + 32 < p && (wid > 0 || nw == 1))
+      apply_rows<T>(L, m, v, kb + 32, min(32, p - kb - 32), 0, kb, nw == 1 ? tid : tid - 32,
+                    nw == 1 ? bd : bd - 32);
     __syncthreads();
-    if (tid >= first) {
-      for (int i = i0; i < kb; i += step) {
-        if (first == 0 || i != i0) {
-#pragma unroll
-          for (int t = 0; t < 32; ++t) w[t] = t < nb ? L[int64_t(kb + t) * m + i] : T(0);
-        }
-        T s = v[i];
-#pragma unroll
-        for (int t = 0; t < 32; ++t)
-          if (t < nb) s -= w[t] * v[kb + t];
-        v[i] = s;
+    if (kb > 0) {
+      if (wid == 0) {
+        load_block<T, false>(L, m, kb - 32, 32, a.w);
+        a.rd = ((const T *)d.rd)[f.pv + kb - 32 + lane];
       }
+      apply_next<T>(L, m, v, kb, nb, kb - 32, kb);
+      __syncthreads();
     }
-    __syncthreads();
+  }
+  for (int i = tid; i < p; i += bd) {
+    const int k = i == tid ? a.own : __ldg(d.idx + f.idx + i);
+    d.xk[k] = double(v[i]);
+    x[i == tid ? a.own_x : __ldg(d.Q + k)] = double(v[i]);
   }
 }
 
@@ -776,13 +892,17 @@ template <class T>
 __global__ void __launch_bounds__(256) front_forward(FrontDev d, int f0) {
   extern __shared__ __align__(16) unsigned char raw[];
   const Front f = d.front[f0 + blockIdx.x];
-  forward<T>(d, f, reinterpret_cast<T *>(raw));
+  Up<T> a;
+  ahead<T>(d, f, a);
+  forward<T>(d, f, reinterpret_cast<T *>(raw), a);
 }
 template <class T>
 __global__ void __launch_bounds__(256) front_backward(FrontDev d, int f0, double *x) {
   extern __shared__ __align__(16) unsigned char raw[];
   const Front f = d.front[f0 + blockIdx.x];
-  backward<T>(d, f, reinterpret_cast<T *>(raw), x);
+  Down<T> a;
+  ahead<T>(d, f, a);
+  backward<T>(d, f, reinterpret_cast<T *>(raw), a, x);
 }
 
 // Polls a flag (acquire) until it is set, at most `limit` times.
@@ -801,11 +921,16 @@ __device__ __forceinline__ bool wait_flag(const unsigned *p, int limit) {
 // (bounded) for its children's border sums, backward for its parent, so a
 // step up or down the tree costs a flag and the front's own work instead of
 // a launch that waits for the whole level.  Every front waited for was
-// claimed earlier by a running block, so the claims always advance.  flow:
+// claimed earlier by a running block, so the claims always advance.  What
+// bounds it is the tree's height: per front the wait, the children's sums,
+// the pivots' chain and the flag, with everything static loaded before the
+// wait (a 28-pivot front 3.6 us up, 8.9 with its loads after it).  Measured:
+// 60x60 power grid 113 us (141), 200x200 361 (440), 200,000 devices of logic
+// 448 (512).  flow:
 // the claim counter, then a forward and a backward flag per front, cleared
 // before the launch.
-template <class T>
-__global__ void __launch_bounds__(kFlowThreads) front_flow(FrontDev d, int first, int nf, unsigned *flow,
+template <class T, int kPerSm>
+__global__ void __launch_bounds__(kFlowThreads, kPerSm) front_flow(FrontDev d, int first, int nf, unsigned *flow,
                                                            const unsigned *limit_at, double *x) {
   extern __shared__ __align__(16) unsigned char raw[];
   __shared__ int claim;
@@ -819,19 +944,24 @@ __global__ void __launch_bounds__(kFlowThreads) front_flow(FrontDev d, int first
     const bool up = t < count;
     const int k = up ? first + t : nf - 1 - (t - count);
     const Front f = d.front[k];
-    bool ok = true;
     if (up) {
+      Up<T> a;
+      ahead<T>(d, f, a);
+      bool ok = true;
       for (int c = f.child0 + tid; c < f.child1; c += kFlowThreads) {
         const int g = d.child[c].front;
         if (g >= first) ok = wait_flag(fwd + g, limit) && ok;
       }
-    } else if (tid == 0) {
-      ok = wait_flag(f.parent >= 0 ? bwd + f.parent : fwd + k, limit);
+      if (!ok) atomicOr(d.status, 2u);
+      __syncthreads();
+      forward<T>(d, f, reinterpret_cast<T *>(raw), a);
+    } else {
+      Down<T> a;
+      ahead<T>(d, f, a);
+      if (tid == 0 && !wait_flag(f.parent >= 0 ? bwd + f.parent : fwd + k, limit)) atomicOr(d.status, 2u);
+      __syncthreads();
+      backward<T>(d, f, reinterpret_cast<T *>(raw), a, x);
     }
-    if (!ok) atomicOr(d.status, 2u);
-    __syncthreads();
-    if (up) forward<T>(d, f, reinterpret_cast<T *>(raw));
-    else backward<T>(d, f, reinterpret_cast<T *>(raw), x);
     __syncthreads();
     if (tid == 0) {
       __threadfence();
@@ -884,6 +1014,7 @@ struct FrontLu {
   FrontDev d{};
   RowsDev before{}, core{}, after{};
   std::vector<int> before_round, core_round, after_round;
+  bool flow_many = false;
   int flow_first = 0, flow_grid = 0;  // fronts from here on (levels above 0) are solved in one launch
   size_t n_low = 0;                   // groups of level 0
   size_t flow_smem = 0;
@@ -941,6 +1072,11 @@ cudaError_t launch_factor(const FrontLu *f, const Group &g, const double *a, con
                                     : cudaLaunchKernelEx(&cfg, front_factor<double>, f->d, a, f->slot + g.slot0, limit);
 }
 
+// Fronts per SM from which the solves' walk takes four blocks an SM, with
+// fewer registers, instead of two: it is then bound by how many fronts are in
+// flight, not by one front's time (200,000 devices of logic, 4,946 fronts: 439
+// us against 498; a 200x200 grid, 2,172 fronts: 402 against 394).
+constexpr int kManyFronts = 16;
 constexpr double kWideWork = 6e4;  // multiply-adds one SM is left with
 
 }  // namespace
@@ -1011,7 +1147,9 @@ FrontLu *front_create(const FrontPlan &plan, const LuSymbolic &S, int device, in
       while ((slot.size() - size_t(g.slot0)) % size_t(g.cluster)) slot.push_back(-1);
       g.grid = int(slot.size()) - g.slot0;
       g.smem_fwd = size_t(m) * tsz;
-      g.smem_bwd = size_t(m + g.solve_threads) * tsz;
+      int most_p = 0;
+      for (int k = g.f0; k < g.f0 + g.n; ++k) most_p = std::max(most_p, front[k].p);
+      g.smem_bwd = (size_t(m) + size_t(g.solve_threads / 32) * size_t(most_p)) * tsz;
       most = std::max(most, g.smem);
       f->group.push_back(g);
     }
@@ -1019,10 +1157,15 @@ FrontLu *front_create(const FrontPlan &plan, const LuSymbolic &S, int device, in
   }
   f->flow_first = plan.level.size() > 1 ? plan.level[1] : f->n_front;
   {
-    int mx = 0;
-    for (int k = f->flow_first; k < f->n_front; ++k) mx = std::max(mx, plan.front[k].m);
-    f->flow_smem = size_t(mx + kFlowThreads) * tsz;
-    const void *flow_fn = precision == XG_LU_FP32 ? (const void *)front_flow<float> : (const void *)front_flow<double>;
+    size_t mx = 0;
+    for (int k = f->flow_first; k < f->n_front; ++k)
+      mx = std::max(mx, size_t(plan.front[k].m) + size_t(kFlowThreads / 32) * size_t(plan.front[k].p));
+    f->flow_smem = mx * tsz;
+    f->flow_many = f->n_front - f->flow_first > kManyFronts * sms;
+    const void *flow_fn = precision == XG_LU_FP32
+                              ? f->flow_many ? (const void *)front_flow<float, 4> : (const void *)front_flow<float, 2>
+                          : f->flow_many ? (const void *)front_flow<double, 4>
+                                         : (const void *)front_flow<double, 2>;
     int occ = 0;
     if (allow_dynamic_smem(flow_fn, f->flow_smem) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, flow_fn, kFlowThreads, f->flow_smem) != cudaSuccess)
@@ -1110,7 +1253,8 @@ static void solve_tree(FrontLu *f, double *x, unsigned *status, const unsigned *
   }
   if (f->flow_first < f->n_front) {
     f->d.status = status;
-    front_flow<T><<<f->flow_grid, kFlowThreads, f->flow_smem, s>>>(f->d, f->flow_first, f->n_front, f->flow, limit, x);
+    (f->flow_many ? front_flow<T, 4> : front_flow<T, 2>)<<<f->flow_grid, kFlowThreads, f->flow_smem, s>>>(
+        f->d, f->flow_first, f->n_front, f->flow, limit, x);
     count_launches(1);
   }
   for (size_t k = f->n_low; k-- > 0;) {
@@ -1127,9 +1271,21 @@ int front_solve(FrontLu *f, const double *a_copy, const double *b, double *x, un
     for (size_t k = 0; k + 2 < round.size(); k += 2) {
       const int i0 = round[k], n_long = round[k + 1] - i0, n = round[k + 2] - i0;
       if (!n) continue;
-      const int bd = n_long ? 1024 : 256;
-      front_rows<<<n_long + (n - n_long + bd - 1) / bd, bd, 0, s>>>(R, i0, n_long, n, a_copy, b, f->d.P, f->d.Q,
-                                                                    f->d.xk, x, clear, 2 * f->n_front + 1);
+      const int bd = n_long ? 1024 : 256, short_blocks = (n - n_long + bd - 1) / bd;
+      cudaLaunchConfig_t cfg{};
+      cfg.gridDim = dim3(unsigned(n_long ? n_long * kLongCtas + (short_blocks + kLongCtas - 1) / kLongCtas * kLongCtas
+                                         : short_blocks));
+      cfg.blockDim = dim3(unsigned(bd));
+      cfg.stream = s;
+      cudaLaunchAttribute at[1];
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim.x = unsigned(n_long ? kLongCtas : 1);
+      at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+      cfg.attrs = at;
+      cfg.numAttrs = 1;
+      if (cudaLaunchKernelEx(&cfg, front_rows, R, i0, n_long, n, a_copy, b, (const int *)f->d.P, (const int *)f->d.Q,
+                             f->d.xk, x, clear, 2 * f->n_front + 1) != cudaSuccess)
+        return;  // (the last error tells front_solve)
       count_launches(1);
     }
   };
