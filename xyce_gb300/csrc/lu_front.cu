@@ -17,8 +17,8 @@
 //
 // Measured: the 253-row root of a 200x200 power grid in 259 us (429 with a
 // barrier per pivot and every CTA of the front reading the owner's shared
-// memory), a whole refactor and solve of that grid 1.96 ms, of 200,000 devices
-// of logic 2.37 ms.
+// memory), a whole refactor and solve of that grid 1.84 ms, of 200,000 devices
+// of logic 2.30 ms.
 //
 // Every sum has a fixed order: results repeat bit for bit.
 
@@ -77,6 +77,18 @@ __device__ __forceinline__ unsigned cluster_size() {
 }
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// Every kernel here is launched with programmatic stream serialization: its
+// blocks start as the last blocks of the one ahead of it leave, and open with
+// this wait for that one's memory, so a launch costs its blocks' start but not
+// the gap before them.  Measured, 15 to 30 launches a step: 20x20 power grid
+// 211 to 178 us, 60x60 577 to 537, 200x200 1,910 to 1,843, 200,000 devices of
+// logic 2,375 to 2,296.  (Letting them start as soon as the blocks ahead have
+// started fills SMs unevenly: the last two took 1,940 and 2,564 us.)
+// (What another kernel wrote is therefore never read through __restrict__ or
+// __ldg, whose loads may be taken for constant over the kernel's life.)
+__device__ __forceinline__ void await_previous() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 __device__ __forceinline__ unsigned smem_u32(const void *p) { return unsigned(__cvta_generic_to_shared(p)); }
 // One arrival at an mbarrier of another CTA of the cluster (its address from
@@ -157,7 +169,7 @@ __device__ __forceinline__ int local_column(int j, int r, int C) {
 // 16 CTAs' columns took 104 us of the 410 us of a 253-row root; a warp per
 // column, children in turn, 50 us for a single front of 32 rows.)
 template <class T>
-__device__ void assemble(const FrontDev &d, const Front &f, const double *__restrict__ a, T *F, int ld, int ncl,
+__device__ void assemble(const FrontDev &d, const Front &f, const double *a, T *F, int ld, int ncl,
                          int r, int C) {
   const int tid = threadIdx.x, bd = blockDim.x;
   constexpr int kE = 8;
@@ -397,7 +409,7 @@ __device__ __forceinline__ int next_block(T *F, int ld, int l0, int l1, int k0, 
 
 // One CTA's part of a front.
 template <class T>
-__device__ void factor_front(const FrontDev &d, const Front f, const double *__restrict__ a, unsigned char *raw,
+__device__ void factor_front(const FrontDev &d, const Front f, const double *a, unsigned char *raw,
                              unsigned long long *bar, int limit) {
   const int C = f.ctas, r = C > 1 ? int(cluster_rank()) & (C - 1) : 0, rank0 = int(cluster_rank()) - r;
   const int m = f.m, p = f.p, ld = column_stride(m), tid = threadIdx.x, bd = blockDim.x;
@@ -540,8 +552,8 @@ __device__ void factor_front(const FrontDev &d, const Front f, const double *__r
 // slot: per CTA of the launch the front it works for (-1: none); a front's
 // Front::ctas CTAs are neighbours in one cluster.
 template <class T>
-__global__ void __launch_bounds__(kFrontMax) front_factor(FrontDev d, const double *__restrict__ a,
-                                                          const int *__restrict__ slot, const unsigned *limit_at) {
+__global__ void __launch_bounds__(kFrontMax) front_factor(FrontDev d, const double *a, const int *__restrict__ slot,
+                                                          const unsigned *limit_at) {
   extern __shared__ __align__(16) unsigned char raw[];
   __shared__ __align__(8) unsigned long long bar[kMaxCtas];
   const int number = __ldg(slot + blockIdx.x), tid = threadIdx.x;
@@ -552,14 +564,16 @@ __global__ void __launch_bounds__(kFrontMax) front_factor(FrontDev d, const doub
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (shared_cluster) cluster_sync();  // every barrier of the cluster is ready
+  await_previous();
   if (number >= 0) factor_front<T>(d, d.front[number], a, raw, bar, int(__ldg(limit_at)));
   if (shared_cluster) cluster_sync();  // no CTA leaves while another may read its columns
 }
 
 // Opens a refactor: keeps A for the rows outside the tree and refinement,
 // resets the status.
-__global__ void front_open(const double *__restrict__ a, double *__restrict__ a_copy, int64_t nnz, unsigned *status) {
+__global__ void front_open(const double *a, double *a_copy, int64_t nnz, unsigned *status) {
   const int64_t t0 = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  await_previous();
   if (t0 == 0) {
     status[0] = 0;
     status[1] = 0xffffffffu;
@@ -573,7 +587,8 @@ struct RowsDev {
   const int64_t *ptr;
 };
 
-__global__ void front_check_rows(RowsDev R, int n, const double *__restrict__ a, unsigned *status) {
+__global__ void front_check_rows(RowsDev R, int n, const double *a, unsigned *status) {
+  await_previous();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
     if (bad_value(a[R.diag[i]])) report_pivot(status, R.row[i]);
 }
@@ -584,12 +599,13 @@ __global__ void front_check_rows(RowsDev R, int n, const double *__restrict__ a,
 // 200,000 devices of logic's two), then a thread per row.  clear: flags the
 // solve that follows starts from (nullptr: none).
 constexpr int kLongCtas = 8;
-__global__ void __launch_bounds__(1024) front_rows(RowsDev R, int i0, int n_long, int n, const double *__restrict__ a,
-                                                   const double *__restrict__ b, const int *__restrict__ P,
+__global__ void __launch_bounds__(1024) front_rows(RowsDev R, int i0, int n_long, int n, const double *a,
+                                                   const double *b, const int *__restrict__ P,
                                                    const int *__restrict__ Q, double *xk, double *x,
-                                                   unsigned *__restrict__ clear, int n_clear) {
+                                                   unsigned *clear, int n_clear) {
   __shared__ double part[32];
   const int bd = blockDim.x;
+  await_previous();
   if (clear)
     for (int k = blockIdx.x * bd + threadIdx.x; k < n_clear; k += gridDim.x * bd) clear[k] = 0;
   const int block = int(blockIdx.x) - n_long * kLongCtas;
@@ -892,6 +908,7 @@ template <class T>
 __global__ void __launch_bounds__(256) front_forward(FrontDev d, int f0) {
   extern __shared__ __align__(16) unsigned char raw[];
   const Front f = d.front[f0 + blockIdx.x];
+  await_previous();
   Up<T> a;
   ahead<T>(d, f, a);
   forward<T>(d, f, reinterpret_cast<T *>(raw), a);
@@ -900,6 +917,7 @@ template <class T>
 __global__ void __launch_bounds__(256) front_backward(FrontDev d, int f0, double *x) {
   extern __shared__ __align__(16) unsigned char raw[];
   const Front f = d.front[f0 + blockIdx.x];
+  await_previous();
   Down<T> a;
   ahead<T>(d, f, a);
   backward<T>(d, f, reinterpret_cast<T *>(raw), a, x);
@@ -936,6 +954,7 @@ __global__ void __launch_bounds__(kFlowThreads, kPerSm) front_flow(FrontDev d, i
   __shared__ int claim;
   const int count = nf - first, limit = int(__ldg(limit_at)), tid = threadIdx.x;
   unsigned *fwd = flow + 1, *bwd = fwd + nf;
+  await_previous();
   for (;;) {
     if (tid == 0) claim = int(atomicAdd(flow, 1u));
     __syncthreads();
@@ -1056,20 +1075,24 @@ const void *factor_fn() {
   return (const void *)front_factor<T>;
 }
 
-cudaError_t launch_factor(const FrontLu *f, const Group &g, const double *a, const unsigned *limit, cudaStream_t s) {
+// Launches a kernel of this file (await_previous).
+template <class... P, class... A>
+cudaError_t launch(void (*fn)(P...), int grid, int threads, size_t smem, int cluster, cudaStream_t s, A... args) {
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(unsigned(g.grid));
-  cfg.blockDim = dim3(unsigned(g.threads));
-  cfg.dynamicSmemBytes = g.smem;
+  cfg.gridDim = dim3(unsigned(grid));
+  cfg.blockDim = dim3(unsigned(threads));
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = unsigned(g.cluster);
-  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = unsigned(cluster);
+  at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
-  return f->precision == XG_LU_FP32 ? cudaLaunchKernelEx(&cfg, front_factor<float>, f->d, a, f->slot + g.slot0, limit)
-                                    : cudaLaunchKernelEx(&cfg, front_factor<double>, f->d, a, f->slot + g.slot0, limit);
+  cfg.numAttrs = cluster > 0 ? 2 : 1;
+  count_launches(1);
+  return cudaLaunchKernelEx(&cfg, fn, P(args)...);
 }
 
 // Fronts per SM from which the solves' walk takes four blocks an SM, with
@@ -1227,74 +1250,64 @@ int front_refactor(FrontLu *f, const double *dev_values, double *a_copy, int64_t
                    const unsigned *limit, void *stream) {
   cudaStream_t s = (cudaStream_t)stream;
   f->d.status = status;
-  front_open<<<int(std::min<int64_t>(1024, (nnz_a + 255) / 256)), 256, 0, s>>>(dev_values, a_copy, nnz_a, status);
-  count_launches(1);
+  cudaError_t e = launch(front_open, int(std::min<int64_t>(1024, (nnz_a + 255) / 256)), 256, 0, 0, s, dev_values,
+                         a_copy, nnz_a, status);
   for (const Group &g : f->group) {
-    if (launch_factor(f, g, dev_values, limit, s) != cudaSuccess) return XG_ERR_CUDA;
-    count_launches(1);
+    if (e != cudaSuccess) return XG_ERR_CUDA;
+    e = launch(f->precision == XG_LU_FP32 ? front_factor<float> : front_factor<double>, g.grid, g.threads, g.smem,
+               g.cluster, s, f->d, dev_values, f->slot + g.slot0, limit);
   }
   const RowsDev *rows[] = {&f->before, &f->after};
   const std::vector<int> *round[] = {&f->before_round, &f->after_round};
   for (int k = 0; k < 2; ++k) {
     if (round[k]->empty() || !round[k]->back()) continue;
     const int n = round[k]->back();
-    front_check_rows<<<std::min(1024, (n + 255) / 256), 256, 0, s>>>(*rows[k], n, a_copy, status);
-    count_launches(1);
+    if (e == cudaSuccess)
+      e = launch(front_check_rows, std::min(1024, (n + 255) / 256), 256, 0, 0, s, *rows[k], n, a_copy, status);
   }
-  return cudaGetLastError() == cudaSuccess ? XG_OK : XG_ERR_CUDA;
+  return e == cudaSuccess && cudaGetLastError() == cudaSuccess ? XG_OK : XG_ERR_CUDA;
 }
 
 template <class T>
-static void solve_tree(FrontLu *f, double *x, unsigned *status, const unsigned *limit, cudaStream_t s) {
-  for (size_t k = 0; k < f->n_low; ++k) {
+static cudaError_t solve_tree(FrontLu *f, double *x, unsigned *status, const unsigned *limit, cudaStream_t s) {
+  cudaError_t e = cudaSuccess;
+  for (size_t k = 0; k < f->n_low && e == cudaSuccess; ++k) {
     const Group &g = f->group[k];
-    front_forward<T><<<g.n, g.solve_threads, g.smem_fwd, s>>>(f->d, g.f0);
-    count_launches(1);
+    e = launch(front_forward<T>, g.n, g.solve_threads, g.smem_fwd, 0, s, f->d, g.f0);
   }
-  if (f->flow_first < f->n_front) {
+  if (f->flow_first < f->n_front && e == cudaSuccess) {
     f->d.status = status;
-    (f->flow_many ? front_flow<T, 4> : front_flow<T, 2>)<<<f->flow_grid, kFlowThreads, f->flow_smem, s>>>(
-        f->d, f->flow_first, f->n_front, f->flow, limit, x);
-    count_launches(1);
+    e = launch(f->flow_many ? front_flow<T, 4> : front_flow<T, 2>, f->flow_grid, kFlowThreads, f->flow_smem, 0, s, f->d,
+               f->flow_first, f->n_front, f->flow, limit, x);
   }
-  for (size_t k = f->n_low; k-- > 0;) {
+  for (size_t k = f->n_low; k-- > 0 && e == cudaSuccess;) {
     const Group &g = f->group[k];
-    front_backward<T><<<g.n, g.solve_threads, g.smem_bwd, s>>>(f->d, g.f0, x);
-    count_launches(1);
+    e = launch(front_backward<T>, g.n, g.solve_threads, g.smem_bwd, 0, s, f->d, g.f0, x);
   }
+  return e;
 }
 
 int front_solve(FrontLu *f, const double *a_copy, const double *b, double *x, unsigned *status, const unsigned *limit,
                 void *stream) {
   cudaStream_t s = (cudaStream_t)stream;
+  cudaError_t e = cudaSuccess;
   auto rows = [&](const RowsDev &R, const std::vector<int> &round, unsigned *clear) {
-    for (size_t k = 0; k + 2 < round.size(); k += 2) {
+    for (size_t k = 0; k + 2 < round.size() && e == cudaSuccess; k += 2) {
       const int i0 = round[k], n_long = round[k + 1] - i0, n = round[k + 2] - i0;
       if (!n) continue;
       const int bd = n_long ? 1024 : 256, short_blocks = (n - n_long + bd - 1) / bd;
-      cudaLaunchConfig_t cfg{};
-      cfg.gridDim = dim3(unsigned(n_long ? n_long * kLongCtas + (short_blocks + kLongCtas - 1) / kLongCtas * kLongCtas
-                                         : short_blocks));
-      cfg.blockDim = dim3(unsigned(bd));
-      cfg.stream = s;
-      cudaLaunchAttribute at[1];
-      at[0].id = cudaLaunchAttributeClusterDimension;
-      at[0].val.clusterDim.x = unsigned(n_long ? kLongCtas : 1);
-      at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-      cfg.attrs = at;
-      cfg.numAttrs = 1;
-      if (cudaLaunchKernelEx(&cfg, front_rows, R, i0, n_long, n, a_copy, b, (const int *)f->d.P, (const int *)f->d.Q,
-                             f->d.xk, x, clear, 2 * f->n_front + 1) != cudaSuccess)
-        return;  // (the last error tells front_solve)
-      count_launches(1);
+      const int grid = n_long ? n_long * kLongCtas + (short_blocks + kLongCtas - 1) / kLongCtas * kLongCtas : short_blocks;
+      e = launch(front_rows, grid, bd, 0, n_long ? kLongCtas : 0, s, R, i0, n_long, n, a_copy, b, f->d.P, f->d.Q,
+                 f->d.xk, x, clear, 2 * f->n_front + 1);
     }
   };
   rows(f->before, f->before_round, nullptr);
   rows(f->core, f->core_round, f->flow);
-  if (f->precision == XG_LU_FP32) solve_tree<float>(f, x, status, limit, s);
-  else solve_tree<double>(f, x, status, limit, s);
+  if (e == cudaSuccess)
+    e = f->precision == XG_LU_FP32 ? solve_tree<float>(f, x, status, limit, s)
+                                   : solve_tree<double>(f, x, status, limit, s);
   rows(f->after, f->after_round, nullptr);
-  return cudaGetLastError() == cudaSuccess ? XG_OK : XG_ERR_CUDA;
+  return e == cudaSuccess && cudaGetLastError() == cudaSuccess ? XG_OK : XG_ERR_CUDA;
 }
 
 int front_max_multiplier(FrontLu *f, double *out, void *stream) {

@@ -1744,10 +1744,10 @@ double row_seconds(const xg::LuSymbolic &S, bool one_cta, bool chain) {
 // Tries the multifrontal path for an analysed matrix: lu->front when it is
 // modelled faster than `otherwise` and its multipliers stay within the
 // pivoting bound.  Measured, refactor and solve, row-wise / multifrontal:
-// 20x20 power grid (668 rows, one CTA) 490 / 225 us, 34x34 (1,928 rows, grid)
-// 736 / 366 us, 60x60 with its chain 842 / 605 us, 200x200 7.2 / 2.0 ms, logic
-// of 1,000, 6,000 and 200,000 devices 568 / 339 us, 1.77 / 0.76 ms and
-// 21.4 / 2.5 ms, a 4,000-stage chain 2.5 / 0.26 ms.
+// 20x20 power grid (668 rows, one CTA) 490 / 178 us, 40x40 (2,668 rows, grid)
+// 809 / 381 us, 60x60 with its chain 842 / 537 us, 200x200 7.2 / 1.84 ms, logic
+// of 3,000 and 200,000 devices 844 / 600 us and 21.4 / 2.30 ms, a 7,000-stage
+// chain 4.3 / 0.32 ms.
 int try_front(xg_lu *lu, const int *rp, const int *ci, const double *values, double otherwise) {
   const xg::LuSymbolic &S = lu->S;
   xg::FrontPlan plan;
