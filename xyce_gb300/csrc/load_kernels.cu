@@ -26,6 +26,7 @@
 
 #include "xg_dcmp.cuh"
 #include "xg_fast_rcp.cuh"
+#include "xg_launch.cuh"
 #include "xg_internal.h"
 
 #ifndef XG_NS
@@ -141,7 +142,7 @@ __device__ __forceinline__ void res_one(const DevType &t, const LoadIO &io, int 
   const int n = t.n;
   int lp = ld(t.lid + i), ln = ld(t.lid + n + i);
   double G = ld(t.p + i);
-  double i0 = (ld(io.sol + lp) - ld(io.sol + ln)) * G;
+  double i0 = (io.sol[lp] - io.sol[ln]) * G;
   Terms T{io.terms + t.term0, n};
   T.put(0, i, i0);
   T.put(1, i, -i0);
@@ -157,7 +158,7 @@ __device__ __forceinline__ void cap_one(const DevType &t, const LoadIO &io, int 
   const int n = t.n;
   int lp = ld(t.lid + i), ln = ld(t.lid + n + i);
   double C = ld(t.p + i);
-  double vcap = ld(io.sol + lp) - ld(io.sol + ln);
+  double vcap = io.sol[lp] - io.sol[ln];
   double q0 = C * vcap;
   io.sta[t.sta0 + i] = q0;
   Terms T{io.terms + t.term0, n};
@@ -196,8 +197,8 @@ __device__ __forceinline__ void vsrc_one(const DevType &t, Flags f, const LoadIO
     source = pulse_value(t.p, n, i, f.time);
   else
     source = ld(t.p + XG_V_V1 * n + i);
-  double srcCurrent = ld(io.sol + lb);
-  double srcDrop = (ld(io.sol + lp) - ld(io.sol + ln));
+  double srcCurrent = io.sol[lb];
+  double srcDrop = (io.sol[lp] - io.sol[ln]);
   Terms T{io.terms + t.term0, n};
   T.put(0, i, srcCurrent);
   T.put(1, i, -srcCurrent);
@@ -242,7 +243,7 @@ __device__ __forceinline__ void diode_one(const DevType &t, const DevOptions &o,
   // Master::updateState stores the previous limited Vd before the update.
   const double vd_member = io.diode_vd[i];
   *sto = vd_member;
-  double Vpp = ld(io.sol + li_Pri), Vn = ld(io.sol + li_Neg), Vp = ld(io.sol + li_Pos);
+  double Vpp = io.sol[li_Pri], Vn = io.sol[li_Neg], Vp = io.sol[li_Pos];
   double Vd = Vpp - Vn;
   double Isat = PRM(XG_D_ISAT);
   double Vte = N * PRM(XG_D_VT);
@@ -254,7 +255,7 @@ __device__ __forceinline__ void diode_one(const DevType &t, const DevOptions &o,
       else if (off) Vd = 0.0;
       else Vd = tVcrit;
     }
-    Vd_old = f.dcop ? Vd : ld(io.sto_curr + t.sto0 + i);
+    Vd_old = f.dcop ? Vd : io.sto_curr[t.sto0 + i];
   } else {
     Vd_old = vd_member;
   }
@@ -435,11 +436,14 @@ __device__ __forceinline__ void junction(double v, double sat, double vt, double
   c = fwd ? sat * (ev - 1) + gmin * v : cv;
 }
 
+template <bool kStill>
 __device__ __forceinline__ void mos1_one(const DevType &t, const DevOptions &o, Flags f, const LoadIO &io, int i) {
   if (i >= t.n || !instance_flags(t, i, f)) return;
   const int n = t.n;
   const double *p = t.p;
 #define PRM(k) ld(p + (k) * n + i)
+  // (a launch that starts before the one ahead has ended reads no constants of its)
+  auto sol = [&](int k) { return kStill ? ld(io.sol + k) : io.sol[k]; };
   const int li_d = ld(t.lid + i), li_g = ld(t.lid + n + i), li_s = ld(t.lid + 2 * n + i);
   const int li_b = ld(t.lid + 3 * n + i), li_dp = ld(t.lid + 4 * n + i), li_sp = ld(t.lid + 5 * n + i);
   // the polarity (+-1) as a sign to flip
@@ -456,8 +460,8 @@ __device__ __forceinline__ void mos1_one(const DevType &t, const DevOptions &o, 
   enum { S_QGS, S_QGD, S_QGB, S_CAPGS, S_CAPGD, S_CAPGB, S_QBD, S_QBS };
   enum { O_VBD, O_VBS, O_VGS, O_VDS, O_VON };
 
-  const double Vd = ld(io.sol + li_d), Vg = ld(io.sol + li_g), Vs = ld(io.sol + li_s);
-  const double Vb = ld(io.sol + li_b), Vsp = ld(io.sol + li_sp), Vdp = ld(io.sol + li_dp);
+  const double Vd = sol(li_d), Vg = sol(li_g), Vs = sol(li_s);
+  const double Vb = sol(li_b), Vsp = sol(li_sp), Vdp = sol(li_dp);
   double vbs = flip(Vb - Vsp, pol), vgs = flip(Vg - Vsp, pol), vds = flip(Vdp - Vsp, pol);
   double vbd = vbs - vds, vgd = vgs - vds;
   const double vgs_orig = vgs, vds_orig = vds, vbs_orig = vbs, vbd_orig = vbd, vgd_orig = vgd;
@@ -771,7 +775,7 @@ __global__ void __launch_bounds__(256) diode_kernel(DevType t, DevOptions o, Fla
   diode_one(t, o, f, io, blockIdx.x * blockDim.x + threadIdx.x);
 }
 __global__ void __launch_bounds__(128) mos1_kernel(DevType t, DevOptions o, Flags f, LoadIO io) {
-  mos1_one(t, o, f, io, blockIdx.x * blockDim.x + threadIdx.x);
+  mos1_one<true>(t, o, f, io, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 // All light types of a small circuit in one launch: where every instance is
@@ -779,8 +783,9 @@ __global__ void __launch_bounds__(128) mos1_kernel(DevType t, DevOptions o, Flag
 // turn.  Blocks of one warp spread the MOSFETs' FP64 instructions, 66 cycles
 // each on a sub-partition, over as many SMs as there are.  The MOSFETs' blocks
 // come first.  A load of a 101-stage chain (sources, MOSFETs, capacitors):
-// 26.6 us with three launches, 18.3 us with one; above one wave of warps the
-// launches' cost no longer shows.
+// 26.6 us with three launches, 18.3 us with one, 13.2 us with the reduction
+// close behind it (xg_launch.cuh); above one wave of warps the launches' cost
+// no longer shows.
 constexpr int kFewThreads = 32, kFewWarpsPerSm = 16;
 struct FewArgs {
   int count;
@@ -795,13 +800,14 @@ __global__ void __launch_bounds__(kFewThreads) few_kernel(const __grid_constant_
   while (k + 1 < a.count && (int)blockIdx.x >= a.block0[k + 1]) ++k;
   const int i = ((int)blockIdx.x - a.block0[k]) * kFewThreads + (int)threadIdx.x;
   const DevType t = a.t[k];
+  await_previous();
   switch (a.type[k]) {
     case XG_DEV_RES: res_one(t, a.io, i); break;
     case XG_DEV_CAP: cap_one(t, a.io, i); break;
     case XG_DEV_VSRC: vsrc_one(t, a.f, a.io, i); break;
     case XG_DEV_ISRC: isrc_one(t, a.f, a.io, i); break;
     case XG_DEV_DIODE: diode_one(t, a.o, a.f, a.io, i); break;
-    default: mos1_one(t, a.o, a.f, a.io, i); break;
+    default: mos1_one<false>(t, a.o, a.f, a.io, i); break;
   }
 }
 
@@ -820,6 +826,7 @@ constexpr int kRedChunk = 256;
 
 __global__ void __launch_bounds__(kRedThreads) reduce_kernel(ReduceArgs a, int long_blocks) {
   if ((int)blockIdx.x < long_blocks) {
+    await_previous();
 #if XG_SPLIT_SUMS
     // a block per long output: every thread sums a strided share of its terms,
     // then a fixed butterfly per warp and the warps in order
@@ -831,7 +838,7 @@ __global__ void __launch_bounds__(kRedThreads) reduce_kernel(ReduceArgs a, int l
       double s = 0.0;
 #pragma unroll 4
       for (int64_t j = b + threadIdx.x; j < e; j += blockDim.x)
-        s += __ldg(a.terms + __ldg(a.red_idx + j));
+        s += a.terms[__ldg(a.red_idx + j)];
 #pragma unroll
       for (int m = 16; m > 0; m >>= 1) s += __shfl_xor_sync(0xffffffffu, s, m);
       if (lane == 0) part[wid] = s;
@@ -855,7 +862,7 @@ __global__ void __launch_bounds__(kRedThreads) reduce_kernel(ReduceArgs a, int l
       for (int64_t base = b; base < e; base += kRedChunk) {
         const int cnt = (int)(e - base < kRedChunk ? e - base : kRedChunk);
         for (int j = lane; j < cnt; j += 32)
-          buf[wid][j] = __ldg(a.terms + __ldg(a.red_idx + base + j));
+          buf[wid][j] = a.terms[__ldg(a.red_idx + base + j)];
         __syncwarp();
         if (lane == 0)
           for (int j = 0; j < cnt; ++j) s += buf[wid][j];
@@ -880,15 +887,16 @@ __global__ void __launch_bounds__(kRedThreads) reduce_kernel(ReduceArgs a, int l
   }
   const EllBucket B = a.ell[lo];
   const int64_t k0 = (g - B.block0) * kEllPerBlock + threadIdx.x, k1 = k0 + kEllThreads;
-  if (k0 >= B.m) return;
   const uint32_t *ix = a.ell_idx + B.idx0;
+  await_previous();
+  if (k0 >= B.m) return;
   if (k1 < B.m) {
     double s0 = 0.0, s1 = 0.0;
 #pragma unroll 4
     for (int j = 0; j < B.c; ++j) {
       const int64_t row = (int64_t)j * B.m;
-      const double t0 = __ldg(a.terms + __ldg(ix + row + k0));
-      const double t1 = __ldg(a.terms + __ldg(ix + row + k1));
+      const double t0 = a.terms[__ldg(ix + row + k0)];
+      const double t1 = a.terms[__ldg(ix + row + k1)];
       s0 += t0;
       s1 += t1;
     }
@@ -897,7 +905,7 @@ __global__ void __launch_bounds__(kRedThreads) reduce_kernel(ReduceArgs a, int l
   } else {
     double s = 0.0;
 #pragma unroll 8
-    for (int j = 0; j < B.c; ++j) s += __ldg(a.terms + __ldg(ix + (int64_t)j * B.m + k0));
+    for (int j = 0; j < B.c; ++j) s += a.terms[__ldg(ix + (int64_t)j * B.m + k0)];
     a.out[__ldg(a.ell_out + B.out0 + k0)] = s;
   }
 }
@@ -945,9 +953,8 @@ int launch_evals(const EvalType *types, int n, const DevOptions &o, const Flags 
     a.o = o;
     a.f = f;
     a.io = io;
-    few_kernel<<<(unsigned)blocks, kFewThreads, 0, (cudaStream_t)stream>>>(a);
-    xg::count_launches(1);
-    if (cudaGetLastError() != cudaSuccess) return XG_ERR_CUDA;
+    if (launch_close(few_kernel, blocks, kFewThreads, 0, 0, (cudaStream_t)stream, a) != cudaSuccess)
+      return XG_ERR_CUDA;
   }
   for (int k = 0; k < n; ++k) {
     if (few && types[k].type != XG_DEV_BSIM3) continue;
@@ -968,9 +975,10 @@ int launch_reduce(const ReduceArgs &a, void *stream) {
   const int long_blocks = (int)std::min<int64_t>((a.n_long + kRedWarps - 1) / kRedWarps, sms * 8);
 #endif
   if (grid + long_blocks <= 0) return XG_OK;
-  reduce_kernel<<<(unsigned)(grid + long_blocks), kRedThreads, 0, (cudaStream_t)stream>>>(a, long_blocks);
-  xg::count_launches(1);
-  return cudaGetLastError() == cudaSuccess ? XG_OK : XG_ERR_CUDA;
+  return launch_close(reduce_kernel, grid + long_blocks, kRedThreads, 0, 0, (cudaStream_t)stream, a, long_blocks) ==
+                 cudaSuccess
+             ? XG_OK
+             : XG_ERR_CUDA;
 }
 
 }  // namespace XG_NS

@@ -32,6 +32,7 @@
 #include "lu_entries.cuh"
 #include "lu_front.h"
 #include "xg_internal.h"
+#include "xg_launch.cuh"
 #include "xg_smem.cuh"
 
 namespace xg {
@@ -78,18 +79,11 @@ __device__ __forceinline__ unsigned cluster_size() {
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// Every kernel here is launched with programmatic stream serialization: its
-// blocks start as the last blocks of the one ahead of it leave, and open with
-// this wait for that one's memory, so a launch costs its blocks' start but not
-// the gap before them.  Measured, 15 to 30 launches a step: 20x20 power grid
-// 211 to 178 us, 60x60 577 to 537, 200x200 1,910 to 1,843, 200,000 devices of
-// logic 2,375 to 2,296.  (Letting them start as soon as the blocks ahead have
-// started fills SMs unevenly: the last two took 1,940 and 2,564 us.)
-// (What another kernel wrote is therefore never read through __restrict__ or
-// __ldg, whose loads may be taken for constant over the kernel's life.)
-__device__ __forceinline__ void await_previous() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-}
+// The kernels here follow one another closely (xg_launch.cuh), 15 to 30 a
+// step.  Measured: 20x20 power grid 211 to 178 us, 60x60 577 to 537, 200x200
+// 1,910 to 1,843, 200,000 devices of logic 2,375 to 2,296.  (Letting them start
+// as soon as the blocks ahead have started fills SMs unevenly: the last two
+// took 1,940 and 2,564 us.)
 __device__ __forceinline__ unsigned smem_u32(const void *p) { return unsigned(__cvta_generic_to_shared(p)); }
 // One arrival at an mbarrier of another CTA of the cluster (its address from
 // remote()); what the caller saw or wrote before is visible to whoever sees it.
@@ -1075,26 +1069,6 @@ const void *factor_fn() {
   return (const void *)front_factor<T>;
 }
 
-// Launches a kernel of this file (await_previous).
-template <class... P, class... A>
-cudaError_t launch(void (*fn)(P...), int grid, int threads, size_t smem, int cluster, cudaStream_t s, A... args) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(unsigned(grid));
-  cfg.blockDim = dim3(unsigned(threads));
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute at[2];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  at[1].id = cudaLaunchAttributeClusterDimension;
-  at[1].val.clusterDim.x = unsigned(cluster);
-  at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = cluster > 0 ? 2 : 1;
-  count_launches(1);
-  return cudaLaunchKernelEx(&cfg, fn, P(args)...);
-}
-
 // Fronts per SM from which the solves' walk takes four blocks an SM, with
 // fewer registers, instead of two: it is then bound by how many fronts are in
 // flight, not by one front's time (200,000 devices of logic, 4,946 fronts: 439
@@ -1250,11 +1224,11 @@ int front_refactor(FrontLu *f, const double *dev_values, double *a_copy, int64_t
                    const unsigned *limit, void *stream) {
   cudaStream_t s = (cudaStream_t)stream;
   f->d.status = status;
-  cudaError_t e = launch(front_open, int(std::min<int64_t>(1024, (nnz_a + 255) / 256)), 256, 0, 0, s, dev_values,
+  cudaError_t e = launch_close(front_open, int(std::min<int64_t>(1024, (nnz_a + 255) / 256)), 256, 0, 0, s, dev_values,
                          a_copy, nnz_a, status);
   for (const Group &g : f->group) {
     if (e != cudaSuccess) return XG_ERR_CUDA;
-    e = launch(f->precision == XG_LU_FP32 ? front_factor<float> : front_factor<double>, g.grid, g.threads, g.smem,
+    e = launch_close(f->precision == XG_LU_FP32 ? front_factor<float> : front_factor<double>, g.grid, g.threads, g.smem,
                g.cluster, s, f->d, dev_values, f->slot + g.slot0, limit);
   }
   const RowsDev *rows[] = {&f->before, &f->after};
@@ -1263,7 +1237,7 @@ int front_refactor(FrontLu *f, const double *dev_values, double *a_copy, int64_t
     if (round[k]->empty() || !round[k]->back()) continue;
     const int n = round[k]->back();
     if (e == cudaSuccess)
-      e = launch(front_check_rows, std::min(1024, (n + 255) / 256), 256, 0, 0, s, *rows[k], n, a_copy, status);
+      e = launch_close(front_check_rows, std::min(1024, (n + 255) / 256), 256, 0, 0, s, *rows[k], n, a_copy, status);
   }
   return e == cudaSuccess && cudaGetLastError() == cudaSuccess ? XG_OK : XG_ERR_CUDA;
 }
@@ -1273,16 +1247,16 @@ static cudaError_t solve_tree(FrontLu *f, double *x, unsigned *status, const uns
   cudaError_t e = cudaSuccess;
   for (size_t k = 0; k < f->n_low && e == cudaSuccess; ++k) {
     const Group &g = f->group[k];
-    e = launch(front_forward<T>, g.n, g.solve_threads, g.smem_fwd, 0, s, f->d, g.f0);
+    e = launch_close(front_forward<T>, g.n, g.solve_threads, g.smem_fwd, 0, s, f->d, g.f0);
   }
   if (f->flow_first < f->n_front && e == cudaSuccess) {
     f->d.status = status;
-    e = launch(f->flow_many ? front_flow<T, 4> : front_flow<T, 2>, f->flow_grid, kFlowThreads, f->flow_smem, 0, s, f->d,
+    e = launch_close(f->flow_many ? front_flow<T, 4> : front_flow<T, 2>, f->flow_grid, kFlowThreads, f->flow_smem, 0, s, f->d,
                f->flow_first, f->n_front, f->flow, limit, x);
   }
   for (size_t k = f->n_low; k-- > 0 && e == cudaSuccess;) {
     const Group &g = f->group[k];
-    e = launch(front_backward<T>, g.n, g.solve_threads, g.smem_bwd, 0, s, f->d, g.f0, x);
+    e = launch_close(front_backward<T>, g.n, g.solve_threads, g.smem_bwd, 0, s, f->d, g.f0, x);
   }
   return e;
 }
@@ -1297,7 +1271,7 @@ int front_solve(FrontLu *f, const double *a_copy, const double *b, double *x, un
       if (!n) continue;
       const int bd = n_long ? 1024 : 256, short_blocks = (n - n_long + bd - 1) / bd;
       const int grid = n_long ? n_long * kLongCtas + (short_blocks + kLongCtas - 1) / kLongCtas * kLongCtas : short_blocks;
-      e = launch(front_rows, grid, bd, 0, n_long ? kLongCtas : 0, s, R, i0, n_long, n, a_copy, b, f->d.P, f->d.Q,
+      e = launch_close(front_rows, grid, bd, 0, n_long ? kLongCtas : 0, s, R, i0, n_long, n, a_copy, b, f->d.P, f->d.Q,
                  f->d.xk, x, clear, 2 * f->n_front + 1);
     }
   };

@@ -50,6 +50,7 @@
 #include "xg_internal.h"
 #include "lu_chain.h"
 #include "lu_entries.cuh"
+#include "xg_launch.cuh"
 #include "lu_front.h"
 #include "xg_lu.h"
 #include "xg_smem.cuh"
@@ -1323,8 +1324,8 @@ __device__ EntryView<T> lvl_view(char *smem, int n, int64_t nnz, const LvlDev &v
 // takes the factor's values.
 template <class T>
 __device__ bool lvl_stage(const LuDev &d, const LvlDev &v, const EntryView<T> &m, char *smem, int mode,
-                          const double *__restrict__ a, double *__restrict__ a_copy, int64_t nnz_a,
-                          const T *__restrict__ val_in, int nnz, const double *__restrict__ b) {
+                          const double *a, double *a_copy, int64_t nnz_a,
+                          const T *val_in, int nnz, const double *b) {
   const int n = d.n, tid = threadIdx.x, bd = blockDim.x;
   const unsigned mb = smem_addr(smem);
   if (tid == 0) {
@@ -1334,6 +1335,11 @@ __device__ bool lvl_stage(const LuDev &d, const LvlDev &v, const EntryView<T> &m
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     expect_bytes(mb, bytes);
     bulk_copy((void *)(m.img + w0), v.image + w0, bytes, mb);
+  }
+  await_previous();
+  if (tid == 0 && (mode & LVL_FACTOR)) {
+    d.ctrl[C_STATUS] = 0;
+    d.ctrl[C_BAD_ROW] = 0xffffffffu;
   }
   constexpr int kU4 = 8;  // gathers in flight per thread
   if (mode & LVL_FACTOR) {
@@ -1369,15 +1375,8 @@ __device__ bool lvl_stage(const LuDev &d, const LvlDev &v, const EntryView<T> &m
   return false;
 }
 
-__device__ __forceinline__ void lvl_open(const LuDev &d) {
-  if (threadIdx.x == 0) {
-    d.ctrl[C_STATUS] = 0;
-    d.ctrl[C_BAD_ROW] = 0xffffffffu;
-  }
-}
-
 template <class T>
-__device__ void lvl_close_factor(const LuDev &d, const EntryView<T> &m, unsigned bad, T *__restrict__ val_out,
+__device__ void lvl_close_factor(const LuDev &d, const EntryView<T> &m, unsigned bad, T *val_out,
                                  int nnz) {
   for (int p = threadIdx.x; p < nnz; p += blockDim.x) val_out[p] = m.val[p];
   for (int i = threadIdx.x; i < d.n; i += blockDim.x) ((T *)d.rdiag)[i] = m.rd[i];
@@ -1388,20 +1387,19 @@ __device__ void lvl_close_factor(const LuDev &d, const EntryView<T> &m, unsigned
 }
 
 template <class T>
-__global__ void __launch_bounds__(1024) lu_factor_lvl(LuDev d, LvlDev v, const double *__restrict__ a,
-                                                      double *__restrict__ a_copy, int64_t nnz_a,
-                                                      T *__restrict__ val_out, int nnz) {
+__global__ void __launch_bounds__(1024) lu_factor_lvl(LuDev d, LvlDev v, const double *a,
+                                                      double *a_copy, int64_t nnz_a,
+                                                      T *val_out, int nnz) {
   extern __shared__ __align__(16) char smem[];
   const EntryView<T> m = lvl_view<T>(smem, d.n, nnz, v, LVL_FACTOR);
-  lvl_open(d);
   if (!lvl_stage<T>(d, v, m, smem, LVL_FACTOR, a, a_copy, nnz_a, nullptr, nnz, nullptr)) return;
   const unsigned bad = factor_entries<T, false>(m);
   lvl_close_factor<T>(d, m, bad, val_out, nnz);
 }
 
 template <class T>
-__global__ void __launch_bounds__(1024) lu_solve_lvl(LuDev d, LvlDev v, const T *__restrict__ val_in, int nnz,
-                                                     const double *__restrict__ b, double *__restrict__ x) {
+__global__ void __launch_bounds__(1024) lu_solve_lvl(LuDev d, LvlDev v, const T *val_in, int nnz,
+                                                     const double *b, double *x) {
   extern __shared__ __align__(16) char smem[];
   const EntryView<T> m = lvl_view<T>(smem, d.n, nnz, v, LVL_SOLVE);
   if (!lvl_stage<T>(d, v, m, smem, LVL_SOLVE, nullptr, nullptr, 0, val_in, nnz, b)) return;
@@ -1412,13 +1410,12 @@ __global__ void __launch_bounds__(1024) lu_solve_lvl(LuDev d, LvlDev v, const T 
 
 // Refactor with the forward solve in step, keep the factor, solve backward.
 template <class T>
-__global__ void __launch_bounds__(1024) lu_factor_solve_lvl(LuDev d, LvlDev v, const double *__restrict__ a,
-                                                            double *__restrict__ a_copy, int64_t nnz_a,
-                                                            T *__restrict__ val_out, int nnz,
-                                                            const double *__restrict__ b, double *__restrict__ x) {
+__global__ void __launch_bounds__(1024) lu_factor_solve_lvl(LuDev d, LvlDev v, const double *a,
+                                                            double *a_copy, int64_t nnz_a,
+                                                            T *val_out, int nnz,
+                                                            const double *b, double *x) {
   extern __shared__ __align__(16) char smem[];
   const EntryView<T> m = lvl_view<T>(smem, d.n, nnz, v, LVL_BOTH);
-  lvl_open(d);
   if (!lvl_stage<T>(d, v, m, smem, LVL_BOTH, a, a_copy, nnz_a, nullptr, nnz, b)) return;
   const unsigned bad = factor_entries<T, true>(m);
   lvl_close_factor<T>(d, m, bad, val_out, nnz);
@@ -1584,9 +1581,8 @@ int refactor_t(xg_lu *lu, const double *dev_values) {
     return rc ? cuda_fail(cudaGetLastError(), "multifrontal refactor") : XG_OK;
   }
   if (lu->lvl) {
-    xg::lu_factor_lvl<T><<<1, lu->lvl_threads, lu->smem_lvl_factor, lu->stream>>>(
+    xg::launch_close(xg::lu_factor_lvl<T>, 1, lu->lvl_threads, lu->smem_lvl_factor, 0, lu->stream,
         d, lu->lvl_dev, dev_values, lu->d_a, lu->S.nnz_a, (T *)lu->d_val, int(lu->nnz_lu));
-    xg::count_launches(1);
     XG_CU(cudaGetLastError());
     return XG_OK;
   }
@@ -1625,9 +1621,8 @@ int solve_once(xg_lu *lu, const double *b, double *x) {
     return rc ? cuda_fail(cudaGetLastError(), "multifrontal solve") : XG_OK;
   }
   if (lu->lvl) {
-    xg::lu_solve_lvl<T><<<1, lu->lvl_threads, lu->smem_lvl_solve, lu->stream>>>(
+    xg::launch_close(xg::lu_solve_lvl<T>, 1, lu->lvl_threads, lu->smem_lvl_solve, 0, lu->stream,
         d, lu->lvl_dev, (const T *)lu->d_val, int(lu->nnz_lu), b, x);
-    xg::count_launches(1);
     XG_CU(cudaGetLastError());
     return XG_OK;
   }
@@ -1700,9 +1695,8 @@ int refactor_solve_t(xg_lu *lu, const double *dev_values, const double *b, doubl
     return rc ? rc : solve_t<T>(lu, b, x, n_refine);
   }
   xg::LuDev d = lu->dev();
-  xg::lu_factor_solve_lvl<T><<<1, lu->lvl_threads, lu->smem_lvl_both, lu->stream>>>(
+  xg::launch_close(xg::lu_factor_solve_lvl<T>, 1, lu->lvl_threads, lu->smem_lvl_both, 0, lu->stream,
       d, lu->lvl_dev, dev_values, lu->d_a, lu->S.nnz_a, (T *)lu->d_val, int(lu->nnz_lu), b, x);
-  xg::count_launches(1);
   XG_CU(cudaGetLastError());
   for (int it = 0; it < n_refine; ++it) {
     const int nb = std::min(1024, (lu->S.n + 255) / 256);

@@ -29,6 +29,7 @@
 
 #include "xg.h"
 #include "xg_internal.h"
+#include "xg_launch.cuh"
 #include "xg_lu.h"
 
 namespace xg {
@@ -65,6 +66,7 @@ struct CombineArgs {
 
 // The trapezoid / DC combine, plus partial norms of the residual.
 __global__ void __launch_bounds__(kThreads) tran_combine(CombineArgs a) {
+  await_previous();
   __shared__ double sh[kThreads];
   const int stride = gridDim.x * blockDim.x;
   const int t0 = blockIdx.x * blockDim.x + threadIdx.x;
@@ -94,6 +96,7 @@ __global__ void __launch_bounds__(kThreads) tran_combine(CombineArgs a) {
 
 // gmin shunts on the node rows' diagonals (after the combine wrote J).
 __global__ void tran_shunt(int n_nodes, const int64_t *diag, double g, double *jac) {
+  await_previous();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_nodes; i += gridDim.x * blockDim.x)
     if (diag[i] >= 0) jac[diag[i]] += g;
 }
@@ -101,6 +104,7 @@ __global__ void tran_shunt(int n_nodes, const int64_t *diag, double g, double *j
 // Newton weights rel * max(|x_curr|, |x|) + abs.
 __global__ void tran_weights(int n, const double *xc, const double *x, double rel, double abs_tol,
                              double *w) {
+  await_previous();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
     w[i] = rel * fmax(fabs(xc[i]), fabs(x[i])) + abs_tol;
 }
@@ -115,6 +119,7 @@ __global__ void __launch_bounds__(kThreads) tran_update(int n, const double *dx,
                                                         const double *xc, int reweight, double rel,
                                                         double abs_tol, double *w, double *partials,
                                                         const unsigned *lu_status, const double *xn0) {
+  await_previous();
   __shared__ double sh[kThreads];
   if (blockIdx.x == 0 && threadIdx.x == 0)
     *reinterpret_cast<unsigned *>(partials + P_N * kRedBlocks) = *lu_status;
@@ -142,6 +147,7 @@ __global__ void __launch_bounds__(kThreads) tran_update(int n, const double *dx,
 // Predictor x = xh0 + b1 xh1 (+ b2 xh2), also kept as xn0; qn0 = qh0.
 __global__ void tran_predict(int n, int order, double b1, double b2, const double *xh0,
                              const double *xh1, const double *xh2, double *xn0, double *x) {
+  await_previous();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     double v = xh0[i];
     v = b1 * xh1[i] + v;
@@ -155,6 +161,7 @@ __global__ void tran_predict(int n, int order, double b1, double b2, const doubl
 // iterations).
 __global__ void __launch_bounds__(kThreads) tran_lte(int n, const double *x, const double *xn0,
                                                      const double *xc, double *partials) {
+  await_previous();
   __shared__ double sh[kThreads];
   double s2 = 0.0, mx = 0.0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -169,6 +176,7 @@ __global__ void __launch_bounds__(kThreads) tran_lte(int n, const double *x, con
 // OneStep::initialize history: xh0 = x, xh1 = 0, qh0 = Q, qh1 = -h F.
 __global__ void tran_init_hist(int n, double h, const double *x, const double *q, const double *f,
                                double *xh0, double *xh1, double *qh0, double *qh1) {
+  await_previous();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     xh0[i] = x[i];
     xh1[i] = 0.0;
@@ -181,6 +189,7 @@ __global__ void tran_init_hist(int n, double h, const double *x, const double *q
 __global__ void tran_history(int n, int order, const double *x, const double *q, const double *f,
                              double *xh0, double *xh1, double *xh2, double *qh0, double *qh1,
                              double *qh2) {
+  await_previous();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     if (order == 2) {
       xh2[i] = xh1[i];
@@ -194,6 +203,7 @@ __global__ void tran_history(int n, int order, const double *x, const double *q,
 }
 
 __global__ void tran_record(int n_out, const int *idx, const double *x, double *row) {
+  await_previous();
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n_out; k += gridDim.x * blockDim.x)
     row[k] = x[idx[k]];
 }
@@ -292,10 +302,9 @@ struct Run {
     a.rhs = rhs;
     a.jac = jac;
     a.partials = partials;
-    tran_combine<<<kRedBlocks, kThreads, 0, s>>>(a); xg::count_launches(1);
+    launch_close(tran_combine, kRedBlocks, kThreads, 0, 0, s, a);
     if (!transient && gshunt > 0.0) {
-      tran_shunt<<<grid, kThreads, 0, s>>>(n_nodes, diag, gshunt, jac);
-      xg::count_launches(1);
+      launch_close(tran_shunt, grid, kThreads, 0, 0, s, n_nodes, diag, gshunt, jac);
     }
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fail_cuda(e, "tran_combine");
@@ -360,17 +369,15 @@ struct Run {
     double norm_old = norm_rhs;
     double *x = vec(XG_VEC_SOL_NEXT), *xc = vec(XG_VEC_SOL_CURR);
     if (transient) {
-      tran_weights<<<grid, kThreads, 0, s>>>(n, xc, x, rel_tol, abs_tol, w);
-      xg::count_launches(1);
+      launch_close(tran_weights, grid, kThreads, 0, 0, s, n, xc, x, rel_tol, abs_tol, w);
     }
     int status = 0, step = 0;
     while (status == 0) {
       ++step;
       st->factorizations++;
       if ((*rc = xg_lu_refactor_solve(lu, jac, rhs, dx, o->n_refine))) return 0;
-      tran_update<<<kRedBlocks, kThreads, 0, s>>>(n, dx, x, xc, !transient, rel_tol, abs_tol, w,
+      launch_close(tran_update, kRedBlocks, kThreads, 0, 0, s, n, dx, x, xc, !transient, rel_tol, abs_tol, w,
                                                   partials, lu_status_device(lu), transient ? xn0 : nullptr);
-      xg::count_launches(1);
       fl.newton_iter = step;
       fl.init_jct = 0;
       fl.init_fix = !transient && st->dcop_solves == 0 && any_limit;
@@ -600,7 +607,7 @@ extern "C" int xg_tran_run(xg_circuit *c, const xg_tran_options *o, const double
     if (np >= max_points) return;
     host_t[np] = t;
     if (n_out)
-      tran_record<<<1, 128, 0, R.s>>>(n_out, d_idx, R.vec(XG_VEC_SOL_CURR), d_rec + (size_t)np * n_out); xg::count_launches(1);
+      launch_close(tran_record, 1, 128, 0, 0, R.s, n_out, d_idx, R.vec(XG_VEC_SOL_CURR), d_rec + (size_t)np * n_out);
     ++np;
   };
   auto copy_vec = [&](int dst, int src, int64_t len) -> int {
@@ -703,8 +710,8 @@ extern "C" int xg_tran_run(xg_circuit *c, const xg_tran_options *o, const double
       h_sum = 2.0 * h;
       h_last = h;
       next_time = t + h;
-      tran_init_hist<<<R.grid, kThreads, 0, R.s>>>(n, h, R.vec(XG_VEC_SOL_CURR), R.vec(XG_VEC_Q),
-                                                   R.vec(XG_VEC_F), R.xh0, R.xh1, R.qh0, R.qh1); xg::count_launches(1);
+      launch_close(tran_init_hist, R.grid, kThreads, 0, 0, R.s, n, h, R.vec(XG_VEC_SOL_CURR), R.vec(XG_VEC_Q),
+                                                   R.vec(XG_VEC_F), R.xh0, R.xh1, R.qh0, R.qh1);
       n_steps = 0;
       order = 1;
       psi[0] = h;
@@ -722,8 +729,8 @@ extern "C" int xg_tran_run(xg_circuit *c, const xg_tran_options *o, const double
       beta[1] = h / psi[1];
       ck = h / h_sum;
     }
-    tran_predict<<<R.grid, kThreads, 0, R.s>>>(n, order, beta[1], beta[2], R.xh0, R.xh1, R.xh2,
-                                               R.xn0, R.vec(XG_VEC_SOL_NEXT)); xg::count_launches(1);
+    launch_close(tran_predict, R.grid, kThreads, 0, 0, R.s, n, order, beta[1], beta[2], R.xh0, R.xh1, R.xh2,
+                                               R.xn0, R.vec(XG_VEC_SOL_NEXT));
     if ((rc = copy_vec(XG_VEC_STA_NEXT, XG_VEC_STA_CURR, P.n_state)) ||
         (rc = copy_vec(XG_VEC_STO_NEXT, XG_VEC_STO_CURR, P.n_store))) {
       cleanup();
@@ -737,8 +744,8 @@ extern "C" int xg_tran_run(xg_circuit *c, const xg_tran_options *o, const double
     double est = 0.0;
     if (ok && st->steps >= 1 && !beginning) {
       if (!R.tested) {
-        tran_lte<<<kRedBlocks, kThreads, 0, R.s>>>(n, R.vec(XG_VEC_SOL_NEXT), R.xn0,
-                                                   R.vec(XG_VEC_SOL_CURR), R.partials); xg::count_launches(1);
+        launch_close(tran_lte, kRedBlocks, kThreads, 0, 0, R.s, n, R.vec(XG_VEC_SOL_NEXT), R.xn0,
+                                                   R.vec(XG_VEC_SOL_CURR), R.partials);
         double q[P_N];
         if ((rc = R.reduce({P_ERR2, P_XMAX}, q))) { cleanup(); return rc; }
         R.err2 = q[P_ERR2];
@@ -770,9 +777,9 @@ extern "C" int xg_tran_run(xg_circuit *c, const xg_tran_options *o, const double
         hn = rr * h;
       }
       st->steps++;
-      tran_history<<<R.grid, kThreads, 0, R.s>>>(n, order, R.vec(XG_VEC_SOL_NEXT), R.vec(XG_VEC_Q),
+      launch_close(tran_history, R.grid, kThreads, 0, 0, R.s, n, order, R.vec(XG_VEC_SOL_NEXT), R.vec(XG_VEC_Q),
                                                  R.vec(XG_VEC_F), R.xh0, R.xh1, R.xh2, R.qh0,
-                                                 R.qh1, R.qh2); xg::count_launches(1);
+                                                 R.qh1, R.qh2);
       const double min_step = t * 10.0 * DBL_EPSILON;
       hn = std::max(hn, min_step);
       hn = std::min(hn, max_step);
