@@ -76,8 +76,14 @@ __device__ __forceinline__ unsigned cluster_size() {
   asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
   return r;
 }
+// The two halves of a barrier over the cluster; a block's shared memory may be
+// touched by others only once it is known to have started, so a kernel that
+// does passes one before.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  cluster_arrive();
+  cluster_wait();
 }
 // The kernels here follow one another closely (xg_launch.cuh), 15 to 30 a
 // step.  Measured: 20x20 power grid 211 to 178 us, 60x60 577 to 537, 200x200
@@ -599,11 +605,14 @@ __global__ void __launch_bounds__(1024) front_rows(RowsDev R, int i0, int n_long
                                                    unsigned *clear, int n_clear) {
   __shared__ double part[32];
   const int bd = blockDim.x;
+  // (a long row's blocks are one cluster, all of them; its barrier is waited
+  // for behind the sums)
+  const int block = int(blockIdx.x) - n_long * kLongCtas;
+  const bool is_long = block < 0;
+  if (is_long) cluster_arrive();
   await_previous();
   if (clear)
     for (int k = blockIdx.x * bd + threadIdx.x; k < n_clear; k += gridDim.x * bd) clear[k] = 0;
-  const int block = int(blockIdx.x) - n_long * kLongCtas;
-  const bool is_long = block < 0;
   const int i = is_long ? i0 + int(blockIdx.x) / kLongCtas : i0 + n_long + block * bd + int(threadIdx.x);
   if (i >= i0 + n) return;
   const int64_t e0 = R.ptr[i], e1 = R.ptr[i + 1];
@@ -617,6 +626,7 @@ __global__ void __launch_bounds__(1024) front_rows(RowsDev R, int i0, int n_long
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
+    cluster_wait();  // every block of the row has started
     __syncthreads();
     if (threadIdx.x == 0) {
       s = part[0];
