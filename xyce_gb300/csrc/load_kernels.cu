@@ -47,8 +47,13 @@ constexpr double kE = 2.718281828459045;         // CONSTe = exp(1.0), correctly
 __device__ __forceinline__ double dmin(double a, double b) { return a < b ? a : b; }  // Xycemin
 __device__ __forceinline__ double dmax(double a, double b) { return a > b ? a : b; }  // Xycemax
 
-template <typename T>
-__device__ __forceinline__ T ld(const T *p) { return __ldg(p); }
+// Loads of what stays as it is while the kernel runs.  kStill: no kernel that
+// is still running when this one starts may have written it, and the loads may
+// be taken for constant; without it they are ordered behind await_previous()
+// (few_kernel starts early, and a caller's kernel or a slot's set-up may have
+// written any of it just ahead: vectors, parameters, circuit numbers).
+template <bool kStill, typename T>
+__device__ __forceinline__ T ld(const T *p) { return kStill ? __ldg(p) : *p; }
 
 // ---- SPICE3 limiting, DeviceSupport (N_DEV_DeviceSupport.C:186-430) --------
 __device__ __forceinline__ double limvds(double vnew, double vold) {
@@ -122,26 +127,29 @@ struct Terms {
 
 // Batched loads: take instance i's circuit flags; false when the instance is
 // not evaluated (no circuit: an unused place in a slot; or a finished one).
+template <bool kStill>
 __device__ __forceinline__ bool instance_flags(const DevType &t, int i, Flags &f) {
   if (!t.cid) return true;
-  const int c = __ldg(t.cid + i);
+  const int c = ld<kStill>(t.cid + i);
   if (c < 0) return false;
   if (!t.cflags) return true;
   f = t.cflags[c];
   return !f.skip;
 }
+template <bool kStill>
 __device__ __forceinline__ bool instance_live(const DevType &t, int i) {
   if (!t.cid) return true;
-  const int c = __ldg(t.cid + i);
+  const int c = ld<kStill>(t.cid + i);
   return c >= 0 && !(t.cflags && t.cflags[c].skip);
 }
 
 // ---- resistor (N_DEV_Resistor.C:1073-1135) ---------------------------------
+template <bool kStill>
 __device__ __forceinline__ void res_one(const DevType &t, const LoadIO &io, int i) {
-  if (i >= t.n || !instance_live(t, i)) return;
+  if (i >= t.n || !instance_live<kStill>(t, i)) return;
   const int n = t.n;
-  int lp = ld(t.lid + i), ln = ld(t.lid + n + i);
-  double G = ld(t.p + i);
+  int lp = ld<kStill>(t.lid + i), ln = ld<kStill>(t.lid + n + i);
+  double G = ld<kStill>(t.p + i);
   double i0 = (io.sol[lp] - io.sol[ln]) * G;
   Terms T{io.terms + t.term0, n};
   T.put(0, i, i0);
@@ -153,11 +161,12 @@ __device__ __forceinline__ void res_one(const DevType &t, const LoadIO &io, int 
 }
 
 // ---- capacitor, constant C, no IC (N_DEV_Capacitor.C:1821-2040) -------------
+template <bool kStill>
 __device__ __forceinline__ void cap_one(const DevType &t, const LoadIO &io, int i) {
-  if (i >= t.n || !instance_live(t, i)) return;
+  if (i >= t.n || !instance_live<kStill>(t, i)) return;
   const int n = t.n;
-  int lp = ld(t.lid + i), ln = ld(t.lid + n + i);
-  double C = ld(t.p + i);
+  int lp = ld<kStill>(t.lid + i), ln = ld<kStill>(t.lid + n + i);
+  double C = ld<kStill>(t.p + i);
   double vcap = io.sol[lp] - io.sol[ln];
   double q0 = C * vcap;
   io.sta[t.sta0 + i] = q0;
@@ -171,12 +180,13 @@ __device__ __forceinline__ void cap_one(const DevType &t, const LoadIO &io, int 
 }
 
 // PulseData::updateSource (N_DEV_SourceData.C:928-1031) with bpTol = 0.
+template <bool kStill>
 __device__ double pulse_value(const double *p, int n, int i, double t) {
   const double bpTol = 0.0;
-  double V1 = ld(p + XG_V_V1 * n + i), V2 = ld(p + XG_V_V2 * n + i);
-  double TD = ld(p + XG_V_TD * n + i), TR = ld(p + XG_V_TR * n + i);
-  double TF = ld(p + XG_V_TF * n + i), PW = ld(p + XG_V_PW * n + i);
-  double PER = ld(p + XG_V_PER * n + i);
+  double V1 = ld<kStill>(p + XG_V_V1 * n + i), V2 = ld<kStill>(p + XG_V_V2 * n + i);
+  double TD = ld<kStill>(p + XG_V_TD * n + i), TR = ld<kStill>(p + XG_V_TR * n + i);
+  double TF = ld<kStill>(p + XG_V_TF * n + i), PW = ld<kStill>(p + XG_V_PW * n + i);
+  double PER = ld<kStill>(p + XG_V_PER * n + i);
   double time = t - TD;
   if (time > PER && PER != 0.0) time -= PER * floor(time / PER);
   if (time <= 0 || (time > (TR + PW + TF) && (fabs(time - (TR + PW + TF)) > bpTol))) return V1;
@@ -188,15 +198,16 @@ __device__ double pulse_value(const double *p, int n, int i, double t) {
 }
 
 // ---- independent voltage source (N_DEV_Vsrc.C:941-1045) ---------------------
+template <bool kStill>
 __device__ __forceinline__ void vsrc_one(const DevType &t, Flags f, const LoadIO &io, int i) {
-  if (i >= t.n || !instance_flags(t, i, f)) return;
+  if (i >= t.n || !instance_flags<kStill>(t, i, f)) return;
   const int n = t.n;
-  int lp = ld(t.lid + i), ln = ld(t.lid + n + i), lb = ld(t.lid + 2 * n + i);
+  int lp = ld<kStill>(t.lid + i), ln = ld<kStill>(t.lid + n + i), lb = ld<kStill>(t.lid + 2 * n + i);
   double source;
-  if ((f.tranop || f.transient) && ld(t.p + XG_V_KIND * n + i) == XG_SRC_PULSE)
-    source = pulse_value(t.p, n, i, f.time);
+  if ((f.tranop || f.transient) && ld<kStill>(t.p + XG_V_KIND * n + i) == XG_SRC_PULSE)
+    source = pulse_value<kStill>(t.p, n, i, f.time);
   else
-    source = ld(t.p + XG_V_V1 * n + i);
+    source = ld<kStill>(t.p + XG_V_V1 * n + i);
   double srcCurrent = io.sol[lb];
   double srcDrop = (io.sol[lp] - io.sol[ln]);
   Terms T{io.terms + t.term0, n};
@@ -212,26 +223,28 @@ __device__ __forceinline__ void vsrc_one(const DevType &t, Flags f, const LoadIO
 
 // ---- independent current source (N_DEV_ISRC.C:774-800) ----------------------
 // The source value goes into F at both terminals; there are no matrix entries.
+template <bool kStill>
 __device__ __forceinline__ void isrc_one(const DevType &t, Flags f, const LoadIO &io, int i) {
-  if (i >= t.n || !instance_flags(t, i, f)) return;
+  if (i >= t.n || !instance_flags<kStill>(t, i, f)) return;
   const int n = t.n;
   double source;
-  if ((f.tranop || f.transient) && ld(t.p + XG_V_KIND * n + i) == XG_SRC_PULSE)
-    source = pulse_value(t.p, n, i, f.time);
+  if ((f.tranop || f.transient) && ld<kStill>(t.p + XG_V_KIND * n + i) == XG_SRC_PULSE)
+    source = pulse_value<kStill>(t.p, n, i, f.time);
   else
-    source = ld(t.p + XG_V_V1 * n + i);
+    source = ld<kStill>(t.p + XG_V_V1 * n + i);
   Terms T{io.terms + t.term0, n};
   T.put(0, i, source);
   T.put(1, i, -source);
 }
 
 // ---- junction diode, level 1 (N_DEV_Diode.C:873-1331, 2007-2128) ------------
+template <bool kStill>
 __device__ __forceinline__ void diode_one(const DevType &t, const DevOptions &o, Flags f, const LoadIO &io, int i) {
-  if (i >= t.n || !instance_flags(t, i, f)) return;
+  if (i >= t.n || !instance_flags<kStill>(t, i, f)) return;
   const int n = t.n;
   const double *p = t.p;
-#define PRM(k) ld(p + (k) * n + i)
-  const int li_Pos = ld(t.lid + i), li_Neg = ld(t.lid + n + i), li_Pri = ld(t.lid + 2 * n + i);
+#define PRM(k) ld<kStill>(p + (k) * n + i)
+  const int li_Pos = ld<kStill>(t.lid + i), li_Neg = ld<kStill>(t.lid + n + i), li_Pri = ld<kStill>(t.lid + 2 * n + i);
   const double gmin = o.gmin;
   const double M = PRM(XG_D_M), BV = PRM(XG_D_BV), N = PRM(XG_D_N), TT = PRM(XG_D_TT);
   const double tVcrit = PRM(XG_D_TVCRIT), tBrkdwnV = PRM(XG_D_TBRKDWNV);
@@ -438,14 +451,13 @@ __device__ __forceinline__ void junction(double v, double sat, double vt, double
 
 template <bool kStill>
 __device__ __forceinline__ void mos1_one(const DevType &t, const DevOptions &o, Flags f, const LoadIO &io, int i) {
-  if (i >= t.n || !instance_flags(t, i, f)) return;
+  if (i >= t.n || !instance_flags<kStill>(t, i, f)) return;
   const int n = t.n;
   const double *p = t.p;
-#define PRM(k) ld(p + (k) * n + i)
-  // (a launch that starts before the one ahead has ended reads no constants of its)
-  auto sol = [&](int k) { return kStill ? ld(io.sol + k) : io.sol[k]; };
-  const int li_d = ld(t.lid + i), li_g = ld(t.lid + n + i), li_s = ld(t.lid + 2 * n + i);
-  const int li_b = ld(t.lid + 3 * n + i), li_dp = ld(t.lid + 4 * n + i), li_sp = ld(t.lid + 5 * n + i);
+#define PRM(k) ld<kStill>(p + (k) * n + i)
+  auto sol = [&](int k) { return ld<kStill>(io.sol + k); };
+  const int li_d = ld<kStill>(t.lid + i), li_g = ld<kStill>(t.lid + n + i), li_s = ld<kStill>(t.lid + 2 * n + i);
+  const int li_b = ld<kStill>(t.lid + 3 * n + i), li_dp = ld<kStill>(t.lid + 4 * n + i), li_sp = ld<kStill>(t.lid + 5 * n + i);
   // the polarity (+-1) as a sign to flip
   const int pol = __double2hiint(PRM(XG_M1_DTYPE)) & int(0x80000000);
   const double gamma = PRM(XG_M1_GAMMA);
@@ -488,9 +500,9 @@ __device__ __forceinline__ void mos1_one(const DevType &t, const DevOptions &o, 
   double Von, vbs_old, vbd_old, vgs_old, vds_old;
   if (f.newton_iter == 0) {
     if (!f.dcop) {
-      vbs_old = ld(csto + O_VBS); vbd_old = ld(csto + O_VBD);
-      vgs_old = ld(csto + O_VGS); vds_old = ld(csto + O_VDS);
-      Von = flip(ld(csto + O_VON), pol);
+      vbs_old = ld<kStill>(csto + O_VBS); vbd_old = ld<kStill>(csto + O_VBD);
+      vgs_old = ld<kStill>(csto + O_VGS); vds_old = ld<kStill>(csto + O_VDS);
+      Von = flip(ld<kStill>(csto + O_VON), pol);
     } else {
       vbs_old = vbs; vbd_old = vbd; vgs_old = vgs; vds_old = vds;
       Von = 0.0;
@@ -634,9 +646,9 @@ __device__ __forceinline__ void mos1_one(const DevType &t, const DevOptions &o, 
       Capgd = 2.0 * capgd + cgdo;
       Capgb = 2.0 * capgb + cgbo;
     } else {
-      Capgs = (capgs + ld(csta + S_CAPGS) + cgso);
-      Capgd = (capgd + ld(csta + S_CAPGD) + cgdo);
-      Capgb = (capgb + ld(csta + S_CAPGB) + cgbo);
+      Capgs = (capgs + ld<kStill>(csta + S_CAPGS) + cgso);
+      Capgd = (capgd + ld<kStill>(csta + S_CAPGD) + cgdo);
+      Capgb = (capgb + ld<kStill>(csta + S_CAPGB) + cgbo);
     }
     Capgs = magnitude(Capgs);
     Capgd = magnitude(Capgd);
@@ -657,8 +669,8 @@ __device__ __forceinline__ void mos1_one(const DevType &t, const DevOptions &o, 
   if (f.dcop) {
     qgs = Capgs * vgs; qgd = Capgd * vgd; qgb = Capgb * Vgb;
   } else {
-    qgs = ld(csta + S_QGS); qgd = ld(csta + S_QGD); qgb = ld(csta + S_QGB);
-    double vgs1 = ld(csto + O_VGS), vbs1 = ld(csto + O_VBS), vds1 = ld(csto + O_VDS);
+    qgs = ld<kStill>(csta + S_QGS); qgd = ld<kStill>(csta + S_QGD); qgb = ld<kStill>(csta + S_QGB);
+    double vgs1 = ld<kStill>(csto + O_VGS), vbs1 = ld<kStill>(csto + O_VBS), vds1 = ld<kStill>(csto + O_VDS);
     if (wild || ne0(Capgs) || ne0(Capgd) || ne0(Capgb) || !finite_bits(vgs1) || !finite_bits(vbs1) ||
         !finite_bits(vds1)) {
       double vgb1 = vgs1 - vbs1, vgd1 = vgs1 - vds1;
@@ -760,19 +772,19 @@ __device__ __forceinline__ void mos1_one(const DevType &t, const DevOptions &o, 
 
 // ---- launches ------------------------------------------------------------------
 __global__ void __launch_bounds__(256) res_kernel(DevType t, LoadIO io) {
-  res_one(t, io, blockIdx.x * blockDim.x + threadIdx.x);
+  res_one<true>(t, io, blockIdx.x * blockDim.x + threadIdx.x);
 }
 __global__ void __launch_bounds__(256) cap_kernel(DevType t, LoadIO io) {
-  cap_one(t, io, blockIdx.x * blockDim.x + threadIdx.x);
+  cap_one<true>(t, io, blockIdx.x * blockDim.x + threadIdx.x);
 }
 __global__ void __launch_bounds__(256) vsrc_kernel(DevType t, Flags f, LoadIO io) {
-  vsrc_one(t, f, io, blockIdx.x * blockDim.x + threadIdx.x);
+  vsrc_one<true>(t, f, io, blockIdx.x * blockDim.x + threadIdx.x);
 }
 __global__ void __launch_bounds__(256) isrc_kernel(DevType t, Flags f, LoadIO io) {
-  isrc_one(t, f, io, blockIdx.x * blockDim.x + threadIdx.x);
+  isrc_one<true>(t, f, io, blockIdx.x * blockDim.x + threadIdx.x);
 }
 __global__ void __launch_bounds__(256) diode_kernel(DevType t, DevOptions o, Flags f, LoadIO io) {
-  diode_one(t, o, f, io, blockIdx.x * blockDim.x + threadIdx.x);
+  diode_one<true>(t, o, f, io, blockIdx.x * blockDim.x + threadIdx.x);
 }
 __global__ void __launch_bounds__(128) mos1_kernel(DevType t, DevOptions o, Flags f, LoadIO io) {
   mos1_one<true>(t, o, f, io, blockIdx.x * blockDim.x + threadIdx.x);
@@ -802,11 +814,11 @@ __global__ void __launch_bounds__(kFewThreads) few_kernel(const __grid_constant_
   const DevType t = a.t[k];
   await_previous();
   switch (a.type[k]) {
-    case XG_DEV_RES: res_one(t, a.io, i); break;
-    case XG_DEV_CAP: cap_one(t, a.io, i); break;
-    case XG_DEV_VSRC: vsrc_one(t, a.f, a.io, i); break;
-    case XG_DEV_ISRC: isrc_one(t, a.f, a.io, i); break;
-    case XG_DEV_DIODE: diode_one(t, a.o, a.f, a.io, i); break;
+    case XG_DEV_RES: res_one<false>(t, a.io, i); break;
+    case XG_DEV_CAP: cap_one<false>(t, a.io, i); break;
+    case XG_DEV_VSRC: vsrc_one<false>(t, a.f, a.io, i); break;
+    case XG_DEV_ISRC: isrc_one<false>(t, a.f, a.io, i); break;
+    case XG_DEV_DIODE: diode_one<false>(t, a.o, a.f, a.io, i); break;
     default: mos1_one<false>(t, a.o, a.f, a.io, i); break;
   }
 }
