@@ -319,6 +319,12 @@ int xg_lu_solve_host(xg_lu *lu, const double *host_values, const double *host_b,
  * has no device waits.  Synchronises the stream first. */
 int xg_lu_set_wait_limit(xg_lu *lu, int polls);
 int xg_lu_get_info(const xg_lu *lu, xg_lu_info *info);
+/* The kernels that refactor and solve with this analysis (-1: no analysis),
+ * for tests and reports: rows over the whole GPU, rows in one CTA, rows by one
+ * lane of it, entries level by level in one CTA, or dense fronts. */
+enum xg_lu_path { XG_LU_PATH_GRID = 0, XG_LU_PATH_CTA = 1, XG_LU_PATH_LANE = 2, XG_LU_PATH_LEVEL = 3,
+                  XG_LU_PATH_FRONT = 4 };
+int xg_lu_get_path(const xg_lu *lu);
 /* host copies of the analysis: P, Q (n each), L\U row pointers (n+1), columns (nnz_lu) */
 int xg_lu_get_symbolic(const xg_lu *lu, int *P, int *Q, int *lu_rowptr, int *lu_colidx);
 int xg_lu_destroy(xg_lu *lu);

@@ -76,6 +76,7 @@ class XgCircuitInfo(C.Structure):
 
 
 LU_FP64, LU_FP32 = 0, 1
+LU_PATH_GRID, LU_PATH_CTA, LU_PATH_LANE, LU_PATH_LEVEL, LU_PATH_FRONT = range(5)
 
 
 class XgLuInfo(C.Structure):

@@ -2175,6 +2175,16 @@ extern "C" int xg_lu_status(xg_lu *lu, int *status, int *bad_row) {
   return XG_OK;
 }
 
+// (the order refactor_t and solve_once choose in)
+extern "C" int xg_lu_get_path(const xg_lu *lu) {
+  if (!lu) return -1;
+  return lu->front ? XG_LU_PATH_FRONT
+         : lu->lvl ? XG_LU_PATH_LEVEL
+         : lu->narrow ? XG_LU_PATH_LANE
+         : lu->smem_factor ? XG_LU_PATH_CTA
+                   : XG_LU_PATH_GRID;
+}
+
 extern "C" int xg_lu_set_wait_limit(xg_lu *lu, int polls) {
   if (!lu || polls < 1) {
     xg::set_error("xg_lu_set_wait_limit: bad argument");

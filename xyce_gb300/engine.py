@@ -87,6 +87,7 @@ def lib():
     L.xg_lu_status.argtypes = [vp, C.POINTER(i), C.POINTER(i)]
     L.xg_lu_set_wait_limit.argtypes = [vp, i]
     L.xg_lu_get_info.argtypes = [vp, C.POINTER(abi.XgLuInfo)]
+    L.xg_lu_get_path.argtypes = [vp]
     L.xg_lu_get_symbolic.argtypes = [vp, vp, vp, vp, vp]
     L.xg_lu_destroy.argtypes = [vp]
     L.xg_lu_order.argtypes = [i, vp, vp, vp, C.POINTER(i)]
@@ -307,6 +308,11 @@ class LU:
         st, row = C.c_int(), C.c_int()
         check(lib().xg_lu_status(self.h, C.byref(st), C.byref(row)))
         return st.value, row.value
+
+    @property
+    def path(self):
+        """The kernels that refactor and solve (abi.LU_PATH_*)."""
+        return lib().xg_lu_get_path(self.h)
 
     def set_wait_limit(self, polls):
         """Polls a device wait makes before it gives up (status bit 2)."""
