@@ -598,8 +598,8 @@ __global__ void front_check_rows(RowsDev R, int n, const double *a, unsigned *st
 // supply's row has an entry per device on it: 65 us with a block for each of
 // 200,000 devices of logic's two), then a thread per row.  clear: flags the
 // solve that follows starts from (nullptr: none).
-constexpr int kLongCtas = 8;
-__global__ void __launch_bounds__(1024) front_rows(RowsDev R, int i0, int n_long, int n, const double *a,
+constexpr int kLongCtas = 8, kLongThreads = 1024;
+__global__ void __launch_bounds__(kLongThreads) front_rows(RowsDev R, int i0, int n_long, int n, const double *a,
                                                    const double *b, const int *__restrict__ P,
                                                    const int *__restrict__ Q, double *xk, double *x,
                                                    unsigned *clear, int n_clear) {
@@ -1054,10 +1054,7 @@ namespace {
 template <class V>
 bool take(FrontLu *f, V **p, size_t count) {
   *p = nullptr;
-  if (cudaMalloc((void **)p, sizeof(V) * std::max<size_t>(count, 1)) != cudaSuccess) {
-    cudaGetLastError();
-    return false;
-  }
+  if (cudaMalloc((void **)p, sizeof(V) * std::max<size_t>(count, 1)) != cudaSuccess) return false;
   f->owned.push_back(*p);
   return true;
 }
@@ -1074,6 +1071,24 @@ bool give_rows(FrontLu *f, RowsDev *R, const FrontRows &H) {
          give(f, &R->ptr, H.ptr);
 }
 
+// Whether the device can run clusters of so many such blocks at all (a
+// partition of it may hold fewer SMs a cluster than the whole).
+bool granted(const void *fn, int cluster, int threads, size_t smem) {
+  if (cluster <= 1) return true;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(unsigned(cluster));
+  cfg.blockDim = dim3(unsigned(threads));
+  cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = unsigned(cluster);
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  int clusters = 0;
+  return cudaOccupancyMaxActiveClusters(&clusters, fn, &cfg) == cudaSuccess && clusters > 0;
+}
+
 template <class T>
 const void *factor_fn() {
   return (const void *)front_factor<T>;
@@ -1088,8 +1103,7 @@ constexpr double kWideWork = 6e4;  // multiply-adds one SM is left with
 
 }  // namespace
 
-FrontLu *front_create(const FrontPlan &plan, const LuSymbolic &S, int device, int precision, int *rc) {
-  *rc = XG_OK;
+FrontLu *front_create(const FrontPlan &plan, const LuSymbolic &S, int device, int precision) {
   std::unique_ptr<FrontLu> f(new FrontLu);
   f->n = plan.n;
   f->n_front = int(plan.front.size());
@@ -1179,10 +1193,12 @@ FrontLu *front_create(const FrontPlan &plan, const LuSymbolic &S, int device, in
       return nullptr;
     f->flow_grid = std::max(1, std::min(sms * std::max(occ, 1), f->n_front - f->flow_first));
   }
-  if (allow_dynamic_smem(fn, most) != cudaSuccess) {
-    cudaGetLastError();
-    return nullptr;
-  }
+  if (allow_dynamic_smem(fn, most) != cudaSuccess) return nullptr;
+  for (const Group &g : f->group)
+    if (!granted(fn, g.cluster, g.threads, g.smem)) return nullptr;
+  for (const FrontRows *R : {&plan.before, &plan.core, &plan.after})
+    for (size_t k = 0; k + 2 < R->round.size(); k += 2)
+      if (R->round[k + 1] > R->round[k] && !granted((const void *)front_rows, kLongCtas, kLongThreads, 0)) return nullptr;
   std::vector<ChildDev> child(plan.child.size());
   std::vector<int> own(plan.map.size(), 0), own_at;
   for (const Front &h : front)
@@ -1212,10 +1228,7 @@ FrontLu *front_create(const FrontPlan &plan, const LuSymbolic &S, int device, in
                   take(f.get(), &f->flow, size_t(2 * f->n_front + 1)) && take(f.get(), &d.xk, size_t(plan.n)) &&
                   give_rows(f.get(), &f->before, plan.before) && give_rows(f.get(), &f->core, plan.core) &&
                   give_rows(f.get(), &f->after, plan.after);
-  if (!ok) {
-    *rc = XG_ERR_OOM;
-    return nullptr;
-  }
+  if (!ok) return nullptr;
   d.l = l;
   d.u = u;
   d.c = c;
@@ -1279,7 +1292,7 @@ int front_solve(FrontLu *f, const double *a_copy, const double *b, double *x, un
     for (size_t k = 0; k + 2 < round.size() && e == cudaSuccess; k += 2) {
       const int i0 = round[k], n_long = round[k + 1] - i0, n = round[k + 2] - i0;
       if (!n) continue;
-      const int bd = n_long ? 1024 : 256, short_blocks = (n - n_long + bd - 1) / bd;
+      const int bd = n_long ? kLongThreads : 256, short_blocks = (n - n_long + bd - 1) / bd;
       const int grid = n_long ? n_long * kLongCtas + (short_blocks + kLongCtas - 1) / kLongCtas * kLongCtas : short_blocks;
       e = launch_close(front_rows, grid, bd, 0, n_long ? kLongCtas : 0, s, R, i0, n_long, n, a_copy, b, f->d.P, f->d.Q,
                  f->d.xk, x, clear, 2 * f->n_front + 1);

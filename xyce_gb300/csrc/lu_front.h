@@ -23,7 +23,7 @@ namespace xg {
 
 constexpr int kFrontMax = 512;          // rows of the largest front the kernels take
 constexpr int kFrontMiddle = 64, kFrontLow = 32;  // rows that part a level's fronts into size classes
-constexpr int kFrontMaxChildren = 512;  // children of a front (one warp adds them in turn)
+constexpr int kFrontMaxChildren = 512;  // children of a front (a CTA adds them in turn)
 
 // Rows of B solved outside the tree.  A row with one entry left (a source's
 // branch equation) gives its unknown before the tree, a column with one
@@ -87,8 +87,9 @@ bool build_front_plan(const LuSymbolic &S, const int *rp, const int *ci, FrontPl
 
 // Device side (lu_front.cu).
 struct FrontLu;
-// Uploads the plan; nullptr with *rc set when device memory runs out.
-FrontLu *front_create(const FrontPlan &plan, const LuSymbolic &S, int device, int precision, int *rc);
+// Uploads the plan; nullptr when device memory runs out, a front is too large
+// for shared memory or the device does not grant a launch its clusters.
+FrontLu *front_create(const FrontPlan &plan, const LuSymbolic &S, int device, int precision);
 void front_destroy(FrontLu *f);
 // Refactors from dev_values (an FP64 copy goes to a_copy); status[0] collects
 // status bits (1: zero or non-finite pivot, 2: a wait gave up after *limit

@@ -1737,41 +1737,37 @@ double row_seconds(const xg::LuSymbolic &S, bool one_cta, bool chain) {
 
 // Tries the multifrontal path for an analysed matrix: lu->front when it is
 // modelled faster than `otherwise` and its multipliers stay within the
-// pivoting bound.  Measured, refactor and solve, row-wise / multifrontal:
+// pivoting bound.  Whatever else refuses it (memory, a launch the device does
+// not grant) leaves the row-wise paths, and no error behind.  Measured,
+// refactor and solve, row-wise / multifrontal:
 // 20x20 power grid (668 rows, one CTA) 490 / 178 us, 40x40 (2,668 rows, grid)
 // 809 / 381 us, 60x60 with its chain 842 / 537 us, 200x200 7.2 / 1.84 ms, logic
 // of 3,000 and 200,000 devices 844 / 600 us and 21.4 / 2.30 ms, a 7,000-stage
 // chain 4.3 / 0.32 ms.
-int try_front(xg_lu *lu, const int *rp, const int *ci, const double *values, double otherwise) {
+void try_front(xg_lu *lu, const int *rp, const int *ci, const double *values, double otherwise) {
   const xg::LuSymbolic &S = lu->S;
   xg::FrontPlan plan;
-  if (!xg::build_front_plan(S, rp, ci, &plan) || plan.seconds > otherwise) return XG_OK;
-  int rc = XG_OK;
-  xg::FrontLu *f = xg::front_create(plan, S, lu->device, lu->precision, &rc);
-  if (!f) return XG_OK;  // no room: the grid path
+  if (!xg::build_front_plan(S, rp, ci, &plan) || plan.seconds > otherwise) return;
+  xg::FrontLu *f = xg::front_create(plan, S, lu->device, lu->precision);
   double *dev_values = nullptr, most = 0.0;
   unsigned status[2] = {1u, 0u};
-  cudaError_t e = cudaMalloc((void **)&dev_values, sizeof(double) * size_t(S.nnz_a));
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(dev_values, values, sizeof(double) * size_t(S.nnz_a), cudaMemcpyHostToDevice, lu->stream);
-  if (e == cudaSuccess) {
-    rc = xg::front_refactor(f, dev_values, dev_values, S.nnz_a, lu->d_ctrl + xg::C_STATUS, lu->d_ctrl + xg::C_SPIN,
-                            lu->stream);
-    if (!rc) rc = xg::front_max_multiplier(f, &most, lu->stream);
-    e = cudaMemcpyAsync(status, lu->d_ctrl + xg::C_STATUS, sizeof(status), cudaMemcpyDeviceToHost, lu->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(lu->stream);
-  }
+  const size_t bytes = sizeof(double) * size_t(S.nnz_a);
+  const bool tried =
+      f && cudaMalloc((void **)&dev_values, bytes) == cudaSuccess &&
+      cudaMemcpyAsync(dev_values, values, bytes, cudaMemcpyHostToDevice, lu->stream) == cudaSuccess &&
+      xg::front_refactor(f, dev_values, dev_values, S.nnz_a, lu->d_ctrl + xg::C_STATUS, lu->d_ctrl + xg::C_SPIN,
+                         lu->stream) == XG_OK &&
+      xg::front_max_multiplier(f, &most, lu->stream) == XG_OK &&
+      cudaMemcpyAsync(status, lu->d_ctrl + xg::C_STATUS, sizeof(status), cudaMemcpyDeviceToHost, lu->stream) ==
+          cudaSuccess &&
+      cudaStreamSynchronize(lu->stream) == cudaSuccess;
   if (dev_values) cudaFree(dev_values);
-  if (rc || e != cudaSuccess || status[0] || !(most <= kFrontMaxMultiplier)) {
-    xg::front_destroy(f);
-    if (e == cudaErrorMemoryAllocation) {
-      cudaGetLastError();
-      return XG_OK;
-    }
-    return rc ? rc : e != cudaSuccess ? cuda_fail(e, "xg_lu_analyze") : XG_OK;
+  if (tried && !status[0] && most <= kFrontMaxMultiplier) {
+    lu->front = f;
+    return;
   }
-  lu->front = f;
-  return XG_OK;
+  if (f) xg::front_destroy(f);
+  cudaGetLastError();
 }
 
 // xg_lu_analyze; any_path: no caller reads the chain of a factor below
@@ -1835,8 +1831,7 @@ int analyze(xg_ctx *ctx, int n, const int *host_rowptr, const int *host_colidx, 
   const bool front = !std::getenv("XG_LU_NO_FRONT");
   const bool chain = front && xg::chain_start(S, tsz) < n;
   if (n >= kFrontMinRows && front) {
-    rc = try_front(lu.get(), host_rowptr, host_colidx, host_values, row_seconds(S, false, chain));
-    if (rc) return fail(rc);
+    try_front(lu.get(), host_rowptr, host_colidx, host_values, row_seconds(S, false, chain));
     if (lu->front) {
       *out = lu.release();
       return XG_OK;
@@ -1863,8 +1858,7 @@ int analyze(xg_ctx *ctx, int n, const int *host_rowptr, const int *host_colidx, 
   // (a switch that turns a row-wise path off asks for the next of them)
   const bool forced = std::getenv("XG_LU_NO_CTA") || std::getenv("XG_LU_NO_LVL") || std::getenv("XG_LU_NO_SEQ");
   if (n < kFrontMinRows && front && !forced && !level && !narrow && (cta_fits || any_path || !chain)) {
-    rc = try_front(lu.get(), host_rowptr, host_colidx, host_values, row_seconds(S, cta_fits, chain));
-    if (rc) return fail(rc);
+    try_front(lu.get(), host_rowptr, host_colidx, host_values, row_seconds(S, cta_fits, chain));
     if (lu->front) {
       *out = lu.release();
       return XG_OK;
