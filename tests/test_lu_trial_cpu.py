@@ -51,7 +51,8 @@ def test_granted_everything_the_tree_is_taken(run):
     assert run()[:4] == (0, "front", 0, 0)
 
 
-@pytest.mark.parametrize("refusal", [("cluster", 8), ("cluster", 4), ("launch", 8), ("copies", 1), ("copies", 2)])
+@pytest.mark.parametrize("refusal", [("cluster", 8), ("cluster", 4), ("launch", 8), ("copies", 1), ("copies", 2),
+                                     ("pivot",)])
 def test_refused_the_rows_are(run, refusal):
     assert run(*refusal)[:4] == (0, "rows", 0, 0)
 

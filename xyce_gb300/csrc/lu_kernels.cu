@@ -1767,6 +1767,7 @@ void try_front(xg_lu *lu, const int *rp, const int *ci, const double *values, do
     return;
   }
   if (f) xg::front_destroy(f);
+  cudaMemset(lu->d_ctrl + xg::C_STATUS, 0, sizeof(status));  // the trial's findings are not the caller's
   cudaGetLastError();
 }
 
