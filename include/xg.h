@@ -197,6 +197,12 @@ int xg_probe_fp64_rate(int cuda_device, double *flops_per_second);
  * approximation) of n values on the current device, for testing it against
  * 1.0 / b.  No counterpart in the reference. */
 int xg_probe_reciprocal(int n, const double *host_b, double *host_out);
+/* The kernels' other FP64 arithmetic, value by value, for testing it against
+ * IEEE's: a / b from b's rounded reciprocal (the loads' quotients), sqrt(b) of
+ * the FMA load build, the reciprocal that comes with it, and the LU's
+ * reciprocal of a pivot b.  host_a may be NULL but for the quotient. */
+enum xg_probe_op { XG_PROBE_QUOTIENT = 0, XG_PROBE_SQRT = 1, XG_PROBE_RSQRT = 2, XG_PROBE_PIVOT = 3 };
+int xg_probe_arithmetic(int op, int n, const double *host_a, const double *host_b, double *host_out);
 
 /* ---- context: one GPU, one stream (replaces the DeviceMgr singleton) -------- */
 int xg_ctx_create(int cuda_device, xg_ctx **out);

@@ -2,11 +2,14 @@
 // the roofline denominator for the device-evaluation kernels, which are
 // bound by the FP64 pipe (GB300 issues two FP64 thread operations per cycle
 // per SM).  Eight independent DFMA chains per thread, one block per SM slot,
-// timed with CUDA events.
+// timed with CUDA events.  Beside it probes of the kernels' own FP64
+// arithmetic, for tests.
 
 #include <cuda_runtime.h>
 
+#include "lu_entries.cuh"
 #include "xg.h"
+#include "xg_dcmp.cuh"
 #include "xg_fast_rcp.cuh"
 #include "xg_internal.h"
 
@@ -28,6 +31,16 @@ __global__ void reciprocals(const double *b, double *out, int n) {
   if (i < n) out[i] = xg::fast_rcp(b[i]);
 }
 
+__global__ void arithmetic(int op, const double *a, const double *b, double *out, int n) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  double r = 0.0;
+  if (op == XG_PROBE_QUOTIENT) out[i] = xg::quotient(a[i], b[i], 1.0 / b[i]);
+  else if (op == XG_PROBE_SQRT) out[i] = xg::fast_sqrt(b[i], &r);
+  else if (op == XG_PROBE_RSQRT) xg::fast_sqrt(b[i], &r), out[i] = r;
+  else out[i] = xg::pivot_reciprocal(b[i]);
+}
+
 }  // namespace
 
 extern "C" int xg_probe_reciprocal(int n, const double *host_b, double *host_out) {
@@ -42,6 +55,26 @@ extern "C" int xg_probe_reciprocal(int n, const double *host_b, double *host_out
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) e = cudaMemcpy(host_out, d + n, sizeof(double) * n, cudaMemcpyDeviceToHost);
+  cudaFree(d);
+  return e == cudaSuccess ? XG_OK : XG_ERR_CUDA;
+}
+
+extern "C" int xg_probe_arithmetic(int op, int n, const double *host_a, const double *host_b, double *host_out) {
+  if (op < XG_PROBE_QUOTIENT || op > XG_PROBE_PIVOT || n < 0 || (n && (!host_b || !host_out)) ||
+      (n && op == XG_PROBE_QUOTIENT && !host_a))
+    return XG_ERR_ARG;
+  if (!n) return XG_OK;
+  const size_t bytes = sizeof(double) * size_t(n);
+  double *d = nullptr;
+  if (cudaMalloc(&d, 3 * bytes) != cudaSuccess) return XG_ERR_OOM;
+  cudaError_t e = cudaMemcpy(d, host_b, bytes, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess && host_a) e = cudaMemcpy(d + n, host_a, bytes, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) {
+    arithmetic<<<(n + 255) / 256, 256>>>(op, d + n, d, d + 2 * size_t(n), n);
+    xg::count_launches(1);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaMemcpy(host_out, d + 2 * size_t(n), bytes, cudaMemcpyDeviceToHost);
   cudaFree(d);
   return e == cudaSuccess ? XG_OK : XG_ERR_CUDA;
 }

@@ -80,6 +80,7 @@ def lib():
     L.xg_load_noalloc.argtypes = [vp, C.POINTER(abi.XgLoadFlags), vp, C.c_int64]
     L.xg_probe_fp64_rate.argtypes = [i, C.POINTER(C.c_double)]
     L.xg_probe_reciprocal.argtypes = [i, vp, vp]
+    L.xg_probe_arithmetic.argtypes = [i, i, vp, vp, vp]
     L.xg_lu_analyze.argtypes = [vp, i, vp, vp, vp, i, C.POINTER(vp)]
     L.xg_lu_refactor.argtypes = [vp, vp]
     L.xg_lu_solve.argtypes = [vp, vp, vp, i]
