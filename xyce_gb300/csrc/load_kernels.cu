@@ -45,7 +45,6 @@ constexpr double kMaxExpArg = 100.0;             // CONSTMAX_EXP_ARG
 constexpr double kE = 2.718281828459045;         // CONSTe = exp(1.0), correctly rounded
 
 __device__ __forceinline__ double dmin(double a, double b) { return a < b ? a : b; }  // Xycemin
-__device__ __forceinline__ double dmax(double a, double b) { return a > b ? a : b; }  // Xycemax
 
 // Loads of what stays as it is while the kernel runs.  kStill: no kernel that
 // is still running when this one starts may have written it, and the loads may
@@ -55,18 +54,8 @@ __device__ __forceinline__ double dmax(double a, double b) { return a > b ? a : 
 template <bool kStill, typename T>
 __device__ __forceinline__ T ld(const T *p) { return kStill ? __ldg(p) : *p; }
 
-// ---- SPICE3 limiting, DeviceSupport (N_DEV_DeviceSupport.C:186-430) --------
-__device__ __forceinline__ double limvds(double vnew, double vold) {
-  if (vold >= 3.5) {
-    if (vnew > vold) vnew = dmin(vnew, (3.0 * vold) + 2.0);
-    else if (vnew < 3.5) vnew = dmax(vnew, 2.0);
-  } else {
-    if (vnew > vold) vnew = dmin(vnew, 4.0);
-    else vnew = dmax(vnew, -0.5);
-  }
-  return vnew;
-}
-
+// ---- SPICE3 junction limiting, DeviceSupport (N_DEV_DeviceSupport.C:186-430);
+// the MOSFETs' limiters in a form without divergence stand with level 1 ------
 __device__ __forceinline__ double pnjlim(double vnew, double vold, double vt, double vcrit,
                                          int *icheck) {
   if ((vnew > vcrit) && (fabs(vnew - vold) > (vt + vt))) {
@@ -79,40 +68,6 @@ __device__ __forceinline__ double pnjlim(double vnew, double vold, double vt, do
     *icheck = 1;
   } else {
     *icheck = 0;
-  }
-  return vnew;
-}
-
-__device__ __forceinline__ double fetlim(double vnew, double vold, double vto) {
-  double vtsthi = fabs(2 * (vold - vto)) + 2;
-  double vtstlo = vtsthi / 2 + 2;
-  double vtox = vto + 3.5;
-  double delv = vnew - vold;
-  if (vold >= vto) {
-    if (vold >= vtox) {
-      if (delv <= 0) {
-        if (vnew >= vtox) {
-          if (-delv > vtstlo) vnew = vold - vtstlo;
-        } else {
-          vnew = dmax(vnew, vto + 2.0);
-        }
-      } else if (delv >= vtsthi) {
-        vnew = vold + vtsthi;
-      }
-    } else {
-      vnew = delv <= 0 ? dmax(vnew, vto - 0.5) : dmin(vnew, vto + 4.0);
-    }
-  } else {
-    if (delv <= 0) {
-      if (-delv > vtsthi) vnew = vold - vtsthi;
-    } else {
-      double vtemp = vto + 0.5;
-      if (vnew <= vtemp) {
-        if (delv > vtstlo) vnew = vold + vtstlo;
-      } else {
-        vnew = vtemp;
-      }
-    }
   }
   return vnew;
 }
