@@ -74,8 +74,9 @@ std::vector<int> amd_order(int n, const int *rp, const int *ci, int *n_dense);
 int lu_analyze(int n, const int *rp, const int *ci, const double *val, double pivot_tol,
                LuSymbolic *out, std::string *err, int ordering = -1);
 
-// Fills the update schedule (urp, upos) from the L\U pattern; false if an update falls outside the pattern (cannot
-// happen for a pattern lu_analyze made).
+// Fills the update schedule (urp, upos) from the L\U pattern; false if an
+// update falls outside the pattern (cannot happen for a pattern lu_analyze
+// made).
 bool lu_build_updates(LuSymbolic &S);
 
 // The elimination of a small factor entry by entry (lu_entries.cuh), as one
