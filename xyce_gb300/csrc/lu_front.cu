@@ -143,7 +143,18 @@ __host__ __device__ inline int local_columns(int m, int r, int C) {
 // An odd column stride: lanes on consecutive columns touch different banks.
 __host__ __device__ inline int column_stride(int m) { return m | 1; }
 
+// Fronts of at most kFrontDouble rows are eliminated in FP64 whatever the
+// factors are kept in: that is where FP32 arithmetic loses most, and the tree
+// would be less accurate than the minimum-degree order.  Forward error after
+// two refinements of FP32 factors, row by row / tree in FP32 / tree so: 50x30
+// power grid 3.8e-14 / 6.0e-13 / 2.6e-15, 72x72 1.2e-14 / 2.4e-12 / 5.5e-15,
+// 150x150 9.8e-13 / 1.0e-12 / 4.2e-14.  (At 32 rows it would still be five
+// times the row-wise one, at 40 three times after one refinement.)  The
+// refactors take 240 -> 288 us (72x72), 510 -> 567 us (20,000 devices of logic)
+// and 915 -> 1,016 us (150,000); another refinement step would cost 105, 177
+// and 308 us.
 size_t factor_smem(int m, int C, size_t tsz) {
+  if (m <= kFrontDouble) tsz = sizeof(double);
   const size_t ld = size_t(column_stride(m));
   return ((C > 1 ? kNb : 0) + size_t(local_columns(m, 0, C))) * ld * tsz + (kNb * kNb + kNb) * tsz;
 }
@@ -168,8 +179,8 @@ __device__ __forceinline__ int local_column(int j, int r, int C) {
 // a child's L2 round trip.  (Looking at every entry of a child for the few of
 // 16 CTAs' columns took 104 us of the 410 us of a 253-row root; a warp per
 // column, children in turn, 50 us for a single front of 32 rows.)
-template <class T>
-__device__ void assemble(const FrontDev &d, const Front &f, const double *a, T *F, int ld, int ncl,
+template <class W, class T>
+__device__ void assemble(const FrontDev &d, const Front &f, const double *a, W *F, int ld, int ncl,
                          int r, int C) {
   const int tid = threadIdx.x, bd = blockDim.x;
   constexpr int kE = 8;
@@ -201,12 +212,12 @@ __device__ void assemble(const FrontDev &d, const Front &f, const double *a, T *
     }
   };
   load(at, v);
-  for (int e = tid; e < ncl * ld; e += bd) F[e] = T(0);
+  for (int e = tid; e < ncl * ld; e += bd) F[e] = W(0);
   __syncthreads();
   const int64_t e0 = f.acol, e1 = f.acol + f.na;
   for (int64_t e = e0 + tid; e < e1; e += bd) {
     const int to = __ldg(d.apos + e), lc = local_column(to / kFrontMax, r, C);
-    if (lc >= 0) F[size_t(lc) * ld + to % kFrontMax] = T(a[__ldg(d.aidx + e)]);
+    if (lc >= 0) F[size_t(lc) * ld + to % kFrontMax] = W(a[__ldg(d.aidx + e)]);
   }
   __syncthreads();
   if (f.child0 == f.child1) return;
@@ -215,7 +226,7 @@ __device__ void assemble(const FrontDev &d, const Front &f, const double *a, T *
     load(at_next, v_next);
 #pragma unroll
     for (int q = 0; q < kE; ++q) {
-      if (at[q] >= 0) F[at[q]] += v[q];
+      if (at[q] >= 0) F[at[q]] += W(v[q]);
       at[q] = at_next[q];
       v[q] = v_next[q];
     }
@@ -407,37 +418,37 @@ __device__ __forceinline__ int next_block(T *F, int ld, int l0, int l1, int k0, 
   return done;
 }
 
-// One CTA's part of a front.
-template <class T>
+// One CTA's part of a front, in W arithmetic; T is what is kept.
+template <class W, class T>
 __device__ void factor_front(const FrontDev &d, const Front f, const double *a, unsigned char *raw,
                              unsigned long long *bar, int limit) {
   const int C = f.ctas, r = C > 1 ? int(cluster_rank()) & (C - 1) : 0, rank0 = int(cluster_rank()) - r;
   const int m = f.m, p = f.p, ld = column_stride(m), tid = threadIdx.x, bd = blockDim.x;
   const int ncl = local_columns(m, r, C);
-  T *su = reinterpret_cast<T *>(raw);       // pivot rows of the block being eliminated
-  T *sr = su + kNb * kNb;                   // and their reciprocal pivots
-  T *pb = sr + kNb;                         // another CTA's pivot columns
-  T *F = pb + (C > 1 ? size_t(kNb) * ld : 0);
-  assemble<T>(d, f, a, F, ld, ncl, r, C);
+  W *su = reinterpret_cast<W *>(raw);       // pivot rows of the block being eliminated
+  W *sr = su + kNb * kNb;                   // and their reciprocal pivots
+  W *pb = sr + kNb;                         // another CTA's pivot columns
+  W *F = pb + (C > 1 ? size_t(kNb) * ld : 0);
+  assemble<W, T>(d, f, a, F, ld, ncl, r, C);
   __syncthreads();
   const int blocks = (p + kNb - 1) / kNb;
   if (C == 1) {
-    if (tid < 32) pivot_rows<T>(F, ld, 0, min(kNb, p), m, su, sr);
+    if (tid < 32) pivot_rows<W>(F, ld, 0, min(kNb, p), m, su, sr);
     __syncthreads();
-    lower_rows<T>(F, ld, 0, min(kNb, p), m, su, sr);
+    lower_rows<W>(F, ld, 0, min(kNb, p), m, su, sr);
     __syncthreads();
     for (int jb = 0; jb < blocks; ++jb) {
       const int k0 = jb * kNb, nb = min(kNb, p - k0), nbn = min(kNb, p - k0 - kNb);
-      const T *pan = F + size_t(k0) * ld;
+      const W *pan = F + size_t(k0) * ld;
       int l0 = k0 + nb, done = 0;
       if (jb + 1 < blocks) {
-        done = next_block<T, true>(F, ld, l0, m, k0, nbn, m, pan, su, sr);
+        done = next_block<W, true>(F, ld, l0, m, k0, nbn, m, pan, su, sr);
         l0 += nbn;
       } else {
-        update_u<T>(F, ld, l0, m, pan, k0, nb, tid, bd);
+        update_u<W>(F, ld, l0, m, pan, k0, nb, tid, bd);
         __syncthreads();
       }
-      update_rest<T>(F, ld, l0, pan, k0, nb, m, done, (m - k0 - nb) * (m - l0), tid, bd);
+      update_rest<W>(F, ld, l0, pan, k0, nb, m, done, (m - k0 - nb) * (m - l0), tid, bd);
       __syncthreads();
     }
   } else {
@@ -457,23 +468,23 @@ __device__ void factor_front(const FrontDev &d, const Front f, const double *a, 
         return;
       }
       if (tid == 0 && next >= 0) signal(remote(bar + jb % C, unsigned(rank0 + next)));
-      const T *src = F + size_t((jb / C) * kNb) * ld;
+      const W *src = F + size_t((jb / C) * kNb) * ld;
       T *dst = (T *)d.l + f.lo + int64_t(k0) * m;
       for (int i = k0 + tid; i < m; i += bd)
-        for (int q = 0; q < nb; ++q) dst[int64_t(q) * m + i] = src[q * ld + i];
+        for (int q = 0; q < nb; ++q) dst[int64_t(q) * m + i] = T(src[q * ld + i]);
       __syncthreads();
       if (tid < C && tid != next) signal(remote(bar + jb % C, unsigned(rank0 + tid)));
     };
     if (r == 0) {
-      if (tid < 32) pivot_rows<T>(F, ld, 0, min(kNb, p), m, su, sr);
+      if (tid < 32) pivot_rows<W>(F, ld, 0, min(kNb, p), m, su, sr);
       __syncthreads();
-      lower_rows<T>(F, ld, 0, min(kNb, p), m, su, sr);
+      lower_rows<W>(F, ld, 0, min(kNb, p), m, su, sr);
       hand_over(0);
     }
     for (int jb = 0; jb < blocks; ++jb) {
       const int k0 = jb * kNb, nb = min(kNb, p - k0), own = jb % C, lc0 = (jb / C) * kNb;
       if (!await(smem_u32(bar + own), unsigned(jb / C) & 1u, limit)) atomicOr(d.status, 2u);
-      const T *pan = F + size_t(lc0) * ld;
+      const W *pan = F + size_t(lc0) * ld;
       // this CTA's first column after the block
       const int passed = jb >= r ? (jb - r) / C + 1 : 0;
       const bool next = jb + 1 < blocks && r == (jb + 1) % C;
@@ -481,8 +492,8 @@ __device__ void factor_front(const FrontDev &d, const Front f, const double *a, 
       if (r != own && l0 < ncl) {
         const int rows = m - k0, cnt = nb * rows;
         for (int e = tid; e < cnt; e += 4 * bd) {
-          T *dst[4];
-          T v[4];
+          W *dst[4];
+          W v[4];
           if (next || !wide) {
             unsigned src[4];
 #pragma unroll
@@ -498,7 +509,7 @@ __device__ void factor_front(const FrontDev &d, const Front f, const double *a, 
             for (int z = 0; z < 4; ++z) {
               const int ez = min(e + z * bd, cnt - 1), q = ez / rows, i = k0 + ez - q * rows;
               dst[z] = pb + q * ld + i;
-              v[z] = __ldcg(src + int64_t(q) * m + i);
+              v[z] = W(__ldcg(src + int64_t(q) * m + i));
             }
           }
 #pragma unroll
@@ -509,14 +520,14 @@ __device__ void factor_front(const FrontDev &d, const Front f, const double *a, 
       __syncthreads();
       if (next) {
         const int nbn = min(kNb, p - k0 - kNb);
-        next_block<T, false>(F, ld, l0, ncl, k0, nbn, m, pan, su, sr);
+        next_block<W, false>(F, ld, l0, ncl, k0, nbn, m, pan, su, sr);
         hand_over(jb + 1);
         l0 += nbn;
       }
       if (l0 < ncl) {
-        update_u<T>(F, ld, l0, ncl, pan, k0, nb, tid, bd);
+        update_u<W>(F, ld, l0, ncl, pan, k0, nb, tid, bd);
         __syncthreads();
-        update_rest<T>(F, ld, l0, pan, k0, nb, m, 0, (m - k0 - nb) * (ncl - l0), tid, bd);
+        update_rest<W>(F, ld, l0, pan, k0, nb, m, 0, (m - k0 - nb) * (ncl - l0), tid, bd);
       }
       __syncthreads();
     }
@@ -526,25 +537,25 @@ __device__ void factor_front(const FrontDev &d, const Front f, const double *a, 
   for (int lc = tid; lc < ncl; lc += bd) {
     const int j = ((lc / kNb) * C + r) * kNb + lc % kNb;
     if (j < p) {
-      const T pivot = F[size_t(lc) * ld + j];
-      ((T *)d.rd)[f.pv + j] = pivot_reciprocal(pivot);
-      if (bad_value(pivot)) report_pivot(d.status, __ldg(d.idx + f.idx + j));
+      const W pivot = F[size_t(lc) * ld + j];
+      ((T *)d.rd)[f.pv + j] = T(pivot_reciprocal(pivot));
+      if (bad_value(T(pivot))) report_pivot(d.status, __ldg(d.idx + f.idx + j));
     }
   }
   const int lane = tid & 31, b = m - p;
   for (int lc = tid >> 5; lc < ncl; lc += bd >> 5) {
     const int j = ((lc / kNb) * C + r) * kNb + lc % kNb;
-    const T *col = F + size_t(lc) * ld;
+    const W *col = F + size_t(lc) * ld;
     if (j < p) {
       // (a wide front's hand-over wrote the rows of the block and below)
       T *dst = (T *)d.l + f.lo + int64_t(j) * m;
       const int e = C > 4 ? j / kNb * kNb : m;
-      for (int i = lane; i < e; i += 32) dst[i] = col[i];
+      for (int i = lane; i < e; i += 32) dst[i] = T(col[i]);
     } else {
       T *dst = (T *)d.u + f.uo + int64_t(j - p) * p;
-      for (int i = lane; i < p; i += 32) dst[i] = col[i];
+      for (int i = lane; i < p; i += 32) dst[i] = T(col[i]);
       dst = (T *)d.c + f.co + int64_t(j - p) * b;
-      for (int i = lane; i < b; i += 32) dst[i] = col[p + i];
+      for (int i = lane; i < b; i += 32) dst[i] = T(col[p + i]);
     }
   }
 }
@@ -565,7 +576,12 @@ __global__ void __launch_bounds__(kFrontMax) front_factor(FrontDev d, const doub
   }
   if (shared_cluster) cluster_sync();  // every barrier of the cluster is ready
   await_previous();
-  if (number >= 0) factor_front<T>(d, d.front[number], a, raw, bar, int(__ldg(limit_at)));
+  if (number >= 0) {
+    const Front f = d.front[number];
+    const int limit = int(__ldg(limit_at));
+    if (sizeof(T) == sizeof(double) || f.m <= kFrontDouble) factor_front<double, T>(d, f, a, raw, bar, limit);
+    else factor_front<T, T>(d, f, a, raw, bar, limit);
+  }
   if (shared_cluster) cluster_sync();  // no CTA leaves while another may read its columns
 }
 

@@ -23,6 +23,7 @@ namespace xg {
 
 constexpr int kFrontMax = 512;          // rows of the largest front the kernels take
 constexpr int kFrontMiddle = 64, kFrontLow = 32;  // rows that part a level's fronts into size classes
+constexpr int kFrontDouble = 48;         // rows up to which FP32 factors' fronts are eliminated in FP64
 constexpr int kFrontMaxChildren = 512;  // children of a front (a CTA adds them in turn)
 
 // Rows of B solved outside the tree.  A row with one entry left (a source's
