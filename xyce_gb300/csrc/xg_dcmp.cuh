@@ -61,18 +61,14 @@ __device__ __forceinline__ int small_int(double x) {
   return e < 0 ? 0 : (1 << e) | ((hi & 0xfffff) >> (20 - e));
 }
 
-// b, opaque to the compiler: a division of it in a rarely taken branch stays
-// in the branch.  (Left to itself the compiler computes the division on the
-// common path too and selects: 361 cycles.)
-__device__ __forceinline__ double kept_apart(double b) {
-  asm volatile("mov.f64 %0, %0;" : "+d"(b));
-  return b;
-}
-
 // How far x's exponent lies above 2^-480, in units of 2^21; at most kMiddling
 // for 2^-480 <= |x| < 2^480 (an integer instruction each).
 constexpr unsigned kMiddling = (960u << 21) - 1u;
 __device__ __forceinline__ unsigned above_low(double x) { return 2u * unsigned(__double2hiint(x)) - (543u << 21); }
+
+// The division where the three instructions of quotient() do not do, out of
+// line: inline it stood between the quotients, and a warp ran them one by one.
+static __device__ __noinline__ double plain_quotient(double a, double b) { return a / b; }
 
 // a / b from y, the correctly rounded reciprocal of b: the quotient a y and
 // one correction by its remainder, which gives IEEE's rounding (P. Markstein,
@@ -81,15 +77,14 @@ __device__ __forceinline__ unsigned above_low(double x) { return 2u * unsigned(_
 // the normal numbers: three FP64 instructions where the division takes 8.6 of
 // their time.  With a and b between 2^-480 and 2^480 all of it is well inside
 // (the remainder's last bit is at least 2^-105 of a); a zero over such a b is
-// the product, and the rest is left to the division.  The two tests cost the
-// exact BSIM3 evaluation 2% (30,001 devices, a whole load: 222.4 us against
-// 218.2 without; with the zero among the first test's operands 232.7).
+// the product, and the rest is left to the division.  The tests cost exact
+// BSIM3 loads 1.5% (300,000 devices: 1.635 ms against 1.611; 1.789 with the
+// division inline, 1.745 with the zeros out of line too).
 __device__ __forceinline__ double quotient(double a, double b, double y) {
   const double q = a * y, r = fma(-b, q, a), z = fma(r, y, q);
   const unsigned ha = above_low(a), hb = above_low(b);
-  if ((ha > hb ? ha : hb) <= kMiddling) return z;
-  if (eq0(a) && hb <= kMiddling) return q;
-  return a / kept_apart(b);
+  if ((ha > hb ? ha : hb) > kMiddling) return eq0(a) && hb <= kMiddling ? q : plain_quotient(a, b);
+  return z;
 }
 
 }  // namespace xg

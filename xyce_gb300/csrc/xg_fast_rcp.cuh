@@ -18,9 +18,15 @@
 // negative operands) IEEE's own operations are used, chosen by an integer test.
 #pragma once
 
-#include "xg_dcmp.cuh"
-
 namespace xg {
+
+// b, opaque to the compiler: a division of it in a rarely taken branch stays
+// in the branch.  (Left to itself the compiler computes the division on the
+// common path too and selects: 361 cycles.)
+__device__ __forceinline__ double kept_apart(double b) {
+  asm volatile("mov.f64 %0, %0;" : "+d"(b));
+  return b;
+}
 
 __device__ __forceinline__ double fast_rcp(double b) {
   const unsigned e = (unsigned(__double2hiint(b)) >> 20) & 0x7ffu;
