@@ -458,7 +458,7 @@ def run_serve(args, world, rank, local, dist, emit=True):
         "newton_iters_per_s": float(np.mean([r[0]["newton_iters_per_s"] for r in runs])),
         "roofline": {"kernel": "batch iteration", "bound": "hbm", "achieved": None, "peak": measured_peaks()[0],
                      "unit": "GB/s", "frac": None, "traffic": None,
-                     "note": "latency-bound: each request's factor runs level by level in one 128-thread block"},
+                     "note": "latency-bound: each request's factor runs by its entry schedule in one 256-thread block"},
         "e2e": {"value": value, "unit": "solves/s",
                 "h2d_bytes_per_step": int(sum(8 * len(r.x0) for r in runs[0][1])),
                 "d2h_bytes_per_step": int(sum(r.result[1].nbytes + r.result[0].nbytes for r in runs[0][1]))},

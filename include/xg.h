@@ -276,8 +276,10 @@ int xg_load(xg_circuit *c, const xg_load_flags *flags);
  *                   analyses again).
  * xg_lu_solve     : GPU forward/backward solves, x = A^-1 b (device buffers,
  *                   length n, distinct).  With XG_LU_FP32 the factors and
- *                   solves are FP32 and n_refine steps of FP64 iterative
- *                   refinement follow (r = b - A x with the FP64 matrix).
+ *                   solves are FP32 (small dense fronts are eliminated in
+ *                   FP64 and kept in FP32) and n_refine steps of FP64
+ *                   iterative refinement follow (r = b - A x with the FP64
+ *                   matrix).
  * xg_lu_status    : synchronises; status bits 1 = zero/non-finite pivot (bad_row
  *                   = first such row of B), 2 = a wait gave up, 4 = pattern error.
  */

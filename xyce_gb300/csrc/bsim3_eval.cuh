@@ -14,13 +14,13 @@
 // charge-partition derivatives, all zero for nqsMod = 0) are left out: adding
 // +-0 never changes a sum's value.
 //
-// Bound by FP64 issue (81-85% of the pipe's cycles): comparisons are made on
+// Bound by FP64 issue (80-84% of the pipe's cycles): comparisons are made on
 // the bits, polarity is a sign flip and the limiting evaluates one alternative
 // (xg_dcmp.cuh and the level-1 kernel's helpers), quotients share reciprocals
-// and square roots come with theirs.  On 300,000 devices a warp issues 1,724
-// FP64 instructions in the FMA build (2,002 with the model's branches and
-// comparisons as they stand) and 2,523 in the exact build (3,339): 1.185 ->
-// 1.043 ms and 1.92 -> 1.47 ms.
+// and square roots come with theirs.  On 300,000 devices a warp issues 1,720
+// FP64 instructions in the FMA build and 2,543 in the exact build: 1.196 ->
+// 1.050 ms and 1.931 -> 1.495 ms against the model's branches and comparisons
+// as they stand (ncu; profiles/bsim3_kernel_single_load_bsim3_300k.md).
 //
 // Members the reference refreshes only when charges are computed (CAP*
 // capacitances, Qeqq*_Jdxp limiter charges, qg/qb/qd/qbs/qbd) live in a

@@ -314,17 +314,17 @@ __device__ __forceinline__ void diode_one(const DevType &t, const DevOptions &o,
 
 // ---- MOSFET level 1 (N_DEV_MOSFET1.C:2618-3427, 4103-4722), newMeyer off ----
 // Bound by FP64 issue, and a warp pays for every instruction any of its lanes
-// takes: with the model's branches as branches, a warp of the random netlist
-// issued 806 FP64 instructions where one thread needs 287.  So each
-// alternative is a choice of operands for one evaluation (the direction of
+// takes: with the model's branches as branches, most of what a warp of the
+// random netlist issued was for other lanes' alternatives.  So each alternative is a choice of operands for one evaluation (the direction of
 // the channel, the junction that is limited, saturation or not) with the
 // arithmetic of the branch it stands for; comparisons are made on the bits
 // and polarity and mode are sign flips (xg_dcmp.cuh); quotients by vt share
 // one reciprocal; and a warp whose instances all have M = 1 skips the
 // products by M.  Nothing is formed that a card without body effect
-// (GAMMA = 0) or oxide capacitance would multiply by that zero.  On 300,000
-// devices: 806 -> 213 FP64 instructions a warp, 0.47 -> 0.133 ms (FMA build),
-// 0.49 -> 0.138 ms (exact build), FP64 pipe 82% busy.
+// (GAMMA = 0) or oxide capacitance would multiply by that zero.  On a million
+// devices a warp issues 244 FP64 instructions (FMA build; exact 259), 84% of
+// the FP64 pipe's cycles: 1.532 -> 0.470 ms (exact 0.502; ncu,
+// profiles/mos1_reduce_single_load_mos1_1M.md).
 
 // fetlim: the limit is a bound on the step (s) or on the value (t).
 __device__ __forceinline__ double fetlim_select(double vnew, double vold, double vto) {
@@ -750,7 +750,7 @@ __global__ void __launch_bounds__(128) mos1_kernel(DevType t, DevOptions o, Flag
 // turn.  Blocks of one warp spread the MOSFETs' FP64 instructions, 66 cycles
 // each on a sub-partition, over as many SMs as there are.  The MOSFETs' blocks
 // come first.  A load of a 101-stage chain (sources, MOSFETs, capacitors):
-// 26.6 us with three launches, 18.3 us with one, 13.2 us with the reduction
+// 26.6 us with three launches, 18.3 us with one, 13.6 us with the reduction
 // close behind it (xg_launch.cuh); above one wave of warps the launches' cost
 // no longer shows.
 constexpr int kFewThreads = 32, kFewWarpsPerSm = 16;

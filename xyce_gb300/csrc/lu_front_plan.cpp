@@ -460,6 +460,7 @@ struct Draft {
   bool gone = false;
 };
 
+constexpr double kModelSms = 152.0;  // SMs of the GB300 whose times the model below follows
 constexpr int kSmallPivots = 16, kSmallRows = 48;
 constexpr double kSmallGrowth = 4.0, kGrowth = 0.2;
 
@@ -733,7 +734,7 @@ bool build_front_plan(const LuSymbolic &S, const int *rp, const int *ci, FrontPl
       longest = std::max(longest, front_work(P.front[k].p, P.front[k].m));
       pivots = std::max(pivots, double(P.front[k].p));
     }
-    const double sms = std::min(16.0, std::max(1.0, 152.0 / (P.level[l + 1] - P.level[l])));
+    const double sms = std::min(16.0, std::max(1.0, kModelSms / (P.level[l + 1] - P.level[l])));
     P.seconds += 20e-6 + pivots * 1.1e-6 + std::max(longest / (sms * 4e9), total / 600e9);
   }
   return true;
